@@ -1,7 +1,7 @@
 """Benchmark: SuBSENSE Mpix/s on the 64-stream mixed-resolution workload, batched vs plain.
 
 A step is one frame tick of all 64 streams (16x320x240, 24x640x480, 16x1280x720, 8x1920x1080;
-48 BGR + 16 grayscale; 39,936,000 pixels) processed by one batched frame step (15 kernel launches,
+48 BGR + 16 grayscale; 39,936,000 pixels) processed by one batched frame step (9 kernel launches,
 each over all streams). ``value`` is measured with the frames already resident in HBM; ``e2e`` goes through the
 C-ABI (lvbgs_batch_apply) with pinned host frames and host masks, so the host->device frame copies
 and device->host mask copies are inside the timed region. The plain form (one stream per launch,
@@ -97,8 +97,7 @@ class ClockSampler:
                 "samples": len(srt)}
 
 
-KERNELS = ["eval", "longscan", "resolve", "repair", "commit", "runs", "vunion", "holes", "combine",
-           "hcount", "median", "epilogue", "dilate", "reset", "close"]
+KERNELS = ["eval", "longscan", "resolve", "repair", "commit", "unite", "fill", "final", "close"]
 
 
 def algorithmic_bytes(px_by_c):

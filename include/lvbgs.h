@@ -100,7 +100,7 @@ lvbgs_status lvbgs_apply(lvbgs_handle h, const uint8_t* image, size_t stride, ui
 
 /* Batched frame step: one frame of each of the n streams (handles on the same device, all
  * initialized). The SuBSENSE streams run in one sequence of phase kernels over a per-stream
- * descriptor table (15 launches per group; large batches run as up to four concurrent groups, see
+ * descriptor table (9 launches per group; large batches run as up to four concurrent groups, see
  * lvbgs_set_batch_groups), enqueued on cuda_stream. The PAWCS streams' frame steps run on their
  * handles' own CUDA streams, forked from cuda_stream and joined back into it, all in flight together;
  * a PAWCS step waits on the host for its fixed-point rounds, so the call returns once every PAWCS
@@ -251,10 +251,9 @@ lvbgs_status lvbgs_get_scalars(lvbgs_handle h, lvbgs_scalars* out);
 /* Per-kernel timing of frame steps (inspection): lvbgs_debug_set_timing(h, batched, n) records CUDA
  * events around each kernel of the next n steps launched by h (batched != 0: the batched steps it
  * leads; 0 disables); lvbgs_debug_tick_profile() waits for them and returns the average duration in
- * ms of each kernel, in launch order: evaluation, long sample scans, ghost resolution, repair, commit/closing, row runs,
- * vertical unions, holes, erosion/combination, median row-window counts, median, frame-level epilogue,
- * dilation/blinks,
- * automatic model reset, frame close. Returns the number of values written. */
+ * ms of each kernel, in launch order: evaluation, long sample scans, ghost resolution, repair, commit/closing,
+ * row-run unions with the frame-level epilogue, holes/erosion/combination, median/averages/dilation/blinks,
+ * automatic model reset and frame close. Returns the number of values written. */
 lvbgs_status lvbgs_debug_set_timing(lvbgs_handle h, int batched, int n_ticks);
 int lvbgs_debug_tick_profile(lvbgs_handle h, int batched, double* out_ms, int max_n);
 /* Phase durations (microseconds) of the repair kernel of the last step launched by h (batched != 0:

@@ -127,7 +127,7 @@ struct StreamDev {
     int W, H, C, npx;
     int tilesX, tilesY, tileBase, nTiles;
     int rowBase, rowWords;  // first row of this stream in the batch's row index space; bit-plane words per row
-    int segBase, nSegs;     // first median column segment of this stream in the batch, and its count
+    int segBase, nSegs;     // first final-mask tile of this stream in the batch, and its count
     int dsW, dsH;  // size of the frame-level down-sampled frame (W/8, H/8)
     int N, nreq, minColor, descOff, stabColorOff, nmv;
     float relThr;
@@ -150,8 +150,7 @@ struct StreamDev {
     uint8_t* roi;
     uint8_t *blinks, *lastRawFG, *lastFG, *dilInv, *lastRawBlink;
     uint32_t* bits;   // mask bit planes (BP_*): rowWords words per row, bit b of word w = pixel 32w + b
-    uint8_t* hcount;  // set pixels of the combined mask in each pixel's median row window
-    int* label;
+    int* label;       // union-find nodes of the hole filling, one per 0-run of a closed-mask row
     uint32_t* intent;
     uint32_t *stampD, *stampR;
     uint4* goodRec;  // long scans of the frame: frame tag, stop position, good samples (index, distances)
@@ -185,7 +184,7 @@ struct TickParams {
     unsigned long long* dlist[2];  // (stream << 40) | pixel
     unsigned long long* rlist[2];
     unsigned int listCap;
-    int totalSegs, colBlocks;  // median: column segments of all streams; 256-pixel column blocks of the widest
+    int totalSegs;  // final-mask tiles of all streams
     unsigned long long barrierNs;  // limit of one grid-barrier wait of the repair, then ERR_BARRIER_TIMEOUT
     int maxRepairIters;            // repair rounds before ERR_REPAIR_LIMIT
     int dbgFault;                  // injected fault (lvbgs_debug_inject_fault), 0: none
@@ -195,8 +194,14 @@ constexpr unsigned long long kDebugBarrierNs = 2000000ull;  // 2 ms, for the inj
 constexpr int kRepairIterLimit = 4096;
 
 // mask bit planes of a stream (scratch of one frame step; bits beyond the frame width are 0)
-enum { BP_CLOSED = 0, BP_RAW, BP_HOLES, BP_COMB, BP_FG, BP_COUNT };
-constexpr int kMedSegRows = 32;  // rows of one median column segment
+enum { BP_CLOSED = 0, BP_RAW, BP_COMB, BP_COUNT };
+// a block of the final-mask kernel: 8 rows of 4 words, a quad of pixels per thread. Small, so that also a
+// 320x240 frame gives 90 blocks
+constexpr int kFinWords = 4, kFinH = 8;
+static_assert(kFinWords * 32 * kFinH == 4 * kThreads, "one quad of pixels per thread");
+inline int final_tiles(int W, int H) {
+    return ((W + 32 * kFinWords - 1) / (32 * kFinWords)) * ((H + kFinH - 1) / kFinH);
+}
 constexpr int kResolveTiles = 4;  // tiles per block of the ghost-resolution kernel
 constexpr int kScanCap = 8;      // samples the evaluation scans per pixel before deferring to a long scan
 __host__ __device__ __forceinline__ uint32_t* bit_plane(const StreamDev& S, int i) {

@@ -1123,6 +1123,8 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_blink_close(PwParams P) {
         bit_plane(D, BP_RAW)[o] = rawW;
         bit_plane(D, BP_CLOSED)[o] = closedW;
     }
+    // the nodes of the hole filling: the run starts of the row's 0-pixels (a word's first pixel counts)
+    if (x < W && y < H && ((~closedW & ~(~closedW << 1)) >> lx) & 1u) D.label[y * W + x] = y * W + x;
 }
 
 // down-sampled frame (INTER_AREA, integral scale), its rolling averages (accumulateWeighted) and the

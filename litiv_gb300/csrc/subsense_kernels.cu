@@ -1245,6 +1245,9 @@ __device__ void phaseF_tile(const TickParams& P, const StreamDev& S, int lt, uin
         bit_plane(S, BP_RAW)[o] = rawW;
         bit_plane(S, BP_CLOSED)[o] = closedW;
     }
+    // hole filling: every run start of the row's 0-pixels is its own node. A word's first pixel counts as
+    // a start here (the word to its left belongs to another block); nodes that no run uses are not read.
+    if (x < W && y < H && ((~closedW & ~(~closedW << 1)) >> lx) & 1u) S.label[y * W + x] = y * W + x;
     block_add_stats(&S.ctl->st_writes, (unsigned long long)nw, &S.ctl->st_samples, (unsigned long long)ne);
 }
 
@@ -1253,7 +1256,7 @@ __device__ void phaseF_tile(const TickParams& P, const StreamDev& S, int lt, uin
 // over the runs of 0-pixels of each row. The closed mask is 0 on the 2-pixel frame border (no ROI
 // pixel lies there, and a 3x3 closing cannot reach it), so the flood-filled region is the
 // 4-connected component of 0-pixels that contains that border ring. Every row's first and last
-// run touch the ring and link straight to root 0; interior runs are united with the runs they
+// run touch the ring and are root 0 itself; interior runs are united with the runs they
 // overlap in the row above. Holes are the 0-pixels whose run's root is not 0.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ int uf_find(int* L, int a, TickWork* w) {
@@ -1285,26 +1288,6 @@ __device__ void uf_union(int* L, int a, int b, TickWork* w) {
     atomicOr(&w->err, ERR_UF_LIMIT);
 }
 
-// run start (x of the first pixel of the run of set bits) for each lane of a 32-pixel chunk
-struct RunTracker {
-    uint32_t carry;   // bit 31 of the previous chunk
-    int prevStart;    // start of the run that reached the end of the previous chunk
-    __device__ __forceinline__ void reset() {
-        carry = 0;
-        prevStart = -1;
-    }
-    // returns the run start of this lane (undefined when its bit is 0) and advances
-    __device__ __forceinline__ int step(uint32_t ball, int x0, int lane) {
-        const uint32_t starts = ball & ~((ball << 1) | carry);
-        const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
-        const int rs = upto ? x0 + 31 - __clz(upto) : prevStart;
-        const int rs31 = __shfl_sync(0xffffffffu, rs, 31);
-        if (ball >> 31) prevStart = rs31;
-        carry = ball >> 31;
-        return rs;
-    }
-};
-
 __device__ __forceinline__ int find_stream_by_row(const TickParams& P, int r) {
     int lo = 0, hi = P.nStreams - 1;
     while (lo < hi) {
@@ -1321,293 +1304,420 @@ __device__ __forceinline__ uint32_t valid_bits(int w, int W) {
     return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);
 }
 
-// runs pass: initializes the label of each run start (0 for runs touching the border ring)
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_runs(TickParams P) {
+// The 0-runs of a row, 32 words at a time with one word per lane. A lane holds its word's 0-pixels and
+// run starts; the start of a run that enters the word from the left comes from the nearest lower lane
+// that has a start (or from the previous chunk), by one ballot and one shuffle. So a 1920-pixel row takes
+// two steps of a warp, where a walk with one lane per pixel took sixty.
+struct RowRuns {
+    const uint32_t* row;
+    int RW, W;
+    uint32_t z, starts;  // this lane's word: 0-pixels, run starts
+    int entry;           // start of the run that continues from the previous word (if bit 0 of z is set and no start)
+    uint32_t carryZ;
+    int carryStart;
+    __device__ __forceinline__ void reset(const uint32_t* r, int rw, int w) {
+        row = r;
+        RW = rw;
+        W = w;
+        carryZ = 0u;
+        carryStart = -1;
+    }
+    // loads words c .. c+31 (every lane of the warp calls it)
+    __device__ __forceinline__ void load(int c, int lane) {
+        const int w = c + lane;
+        z = w < RW ? ~__ldcg(&row[w]) & valid_bits(w, W) : 0u;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, z >> 31, 1);
+        if (lane == 0) prev = carryZ;
+        starts = z & ~((z << 1) | prev);
+        const unsigned m = __ballot_sync(0xffffffffu, starts != 0u);
+        const int v = 32 * w + 31 - __clz(starts);
+        const unsigned lower = m & ((1u << lane) - 1u);
+        const int fromLane = __shfl_sync(0xffffffffu, v, lower ? 31 - __clz(lower) : 0);
+        entry = lower ? fromLane : carryStart;
+        const int last = __shfl_sync(0xffffffffu, v, m ? 31 - __clz(m) : 0);
+        if (m) carryStart = last;
+        carryZ = __shfl_sync(0xffffffffu, z >> 31, 31);
+    }
+    // start of the run that holds bit b of word w (this lane's word)
+    __device__ __forceinline__ int run_start(int w, int b) const {
+        const uint32_t upto = starts & (0xffffffffu >> (31 - b));
+        return upto ? 32 * w + 31 - __clz(upto) : entry;
+    }
+    // the last run start of the row: the run that reaches x = W-1 (every lane calls it)
+    __device__ __forceinline__ int last_start(int lane) const {
+        for (int c = (RW - 1) & ~31; c >= 0; c -= 32) {
+            const int w = c + lane;
+            int v = -1;
+            if (w < RW) {
+                const uint32_t zz = ~__ldcg(&row[w]) & valid_bits(w, W);
+                const uint32_t prev = w > 0 ? ~__ldcg(&row[w - 1]) >> 31 : 0u;
+                const uint32_t st = zz & ~((zz << 1) | prev);
+                if (st) v = 32 * w + 31 - __clz(st);
+            }
+            v = __reduce_max_sync(0xffffffffu, v);
+            if (v >= 0) return v;
+        }
+        return -1;
+    }
+};
+
+__device__ void stream_epilogue(const TickParams& P, const StreamDev& S);
+
+// Unites each run with the runs it overlaps in the row above: a warp per row, a word per lane. A run's
+// node is the index of its first pixel, labelled with itself by the kernel that wrote the closed mask;
+// a run that touches the ring (it holds x = 0 or x = W-1, or lies in the first or last row) stands for
+// node 0 without any memory access, so on a mostly empty mask few unions remain. The blocks past the rows
+// run the frame-level epilogue of one stream each (it touches nothing that these rows read).
+// Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before.
+extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
+    const int rowBlocks = (P.totalRows + 7) / 8;
+    if ((int)blockIdx.x >= rowBlocks) {
+        stream_epilogue(P, P.streams[blockIdx.x - rowBlocks]);
+        return;
+    }
     const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (gr >= P.totalRows) return;
     const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
-    const int y = gr - S.rowBase, W = S.W, H = S.H;
-    const uint32_t* row = bit_plane(S, BP_CLOSED) + (size_t)y * S.rowWords;
-    RunTracker rt;
-    rt.reset();
-    int last = -1;
+    const int y = gr - S.rowBase, W = S.W, H = S.H, RW = S.rowWords;
+    const uint32_t* row = bit_plane(S, BP_CLOSED) + (size_t)y * RW;
+    const bool edgeRow = y < 2 || y >= H - 2;
+    RowRuns rc, ru;
+    rc.reset(row, RW, W);
+    ru.reset(row - (y > 0 ? RW : 0), RW, W);
+    const int lastC = y > 0 ? rc.last_start(lane) : -1, lastU = y > 0 ? ru.last_start(lane) : -1;
+    uint32_t carryOv = 0u;
     bool ringOk = true;
-    for (int x0 = 0; x0 < W; x0 += 32) {
-        const int x = x0 + lane;
-        const uint32_t ball = ~__ldcg(&row[x0 >> 5]) & valid_bits(x0 >> 5, W);  // 0-pixels of the chunk
-        const bool z = (ball >> lane) & 1u;
-        if (x < W && (x < 2 || x >= W - 2 || y < 2 || y >= H - 2) && !z) ringOk = false;
-        const uint32_t starts = ball & ~((ball << 1) | rt.carry);
-        const int rs = rt.step(ball, x0, lane);
-        if ((starts >> lane) & 1u) {
-            const int idx = y * W + x;
-            S.label[idx] = (x == 0 || y == 0 || y == H - 1) ? 0 : idx;
+    for (int c = 0; c < RW; c += 32) {
+        const int w = c + lane;
+        rc.load(c, lane);
+        ru.load(c, lane);
+        const uint32_t vb = valid_bits(w, W);
+        uint32_t ring = edgeRow ? vb : 0u;  // pixels of the 2-pixel border ring in this word
+        if (w == 0) ring |= 3u & vb;
+        if (w == (W - 1) >> 5) ring |= 1u << ((W - 1) & 31);
+        if (W > 1 && w == (W - 2) >> 5) ring |= 1u << ((W - 2) & 31);
+        if (ring & ~rc.z) ringOk = false;
+        const uint32_t ov = rc.z & ru.z;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, ov >> 31, 1);
+        if (lane == 0) prev = carryOv;
+        carryOv = __shfl_sync(0xffffffffu, ov >> 31, 31);
+        uint32_t seg = y > 0 ? ov & ~((ov << 1) | prev) : 0u;
+        while (seg) {
+            const int b = __ffs(seg) - 1;
+            seg &= seg - 1u;
+            const int sc = rc.run_start(w, b), su = ru.run_start(w, b);
+            const int ic = (sc == 0 || sc == lastC || y == H - 1) ? 0 : y * W + sc;
+            const int iu = (su == 0 || su == lastU || y == 1) ? 0 : (y - 1) * W + su;
+            if (ic != iu) uf_union(S.label, ic, iu, P.work);
         }
-        if (z) last = rs;
     }
-    // the last run of the row reaches x = W-1, on the ring (held by the lane that read x = W-1)
-    const int lastRun = __shfl_sync(0xffffffffu, last, (W - 1) & 31);
-    if (lane == 0 && lastRun >= 0) S.label[y * W + lastRun] = 0;
     if (__any_sync(0xffffffffu, !ringOk) && lane == 0) atomicOr(&P.work->err, ERR_RING);
 }
 
-// vertical pass: unites each run with the runs it overlaps in the row above
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_vunion(TickParams P) {
-    const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
-    if (gr >= P.totalRows) return;
-    const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
-    const int y = gr - S.rowBase, W = S.W;
-    if (y == 0) return;
-    const uint32_t* row = bit_plane(S, BP_CLOSED) + (size_t)y * S.rowWords;
-    const uint32_t* up = row - S.rowWords;
-    RunTracker rc, ru;
-    rc.reset();
-    ru.reset();
-    uint32_t ovCarry = 0;
-    for (int x0 = 0; x0 < W; x0 += 32) {
-        const uint32_t vb = valid_bits(x0 >> 5, W);
-        const uint32_t bc = ~__ldcg(&row[x0 >> 5]) & vb, bu = ~__ldcg(&up[x0 >> 5]) & vb;
-        const int rsc = rc.step(bc, x0, lane), rsu = ru.step(bu, x0, lane);
-        const uint32_t ov = bc & bu;
-        const uint32_t segStarts = ov & ~((ov << 1) | ovCarry);
-        ovCarry = ov >> 31;
-        if ((segStarts >> lane) & 1u) uf_union(S.label, y * W + rsc, (y - 1) * W + rsu, P.work);
-    }
-}
-
-// holes pass: the 0-pixels whose run is not connected to the ring
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_holes(TickParams P) {
-    const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
-    if (gr >= P.totalRows) return;
-    const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
-    const int y = gr - S.rowBase, W = S.W;
-    const uint32_t* row = bit_plane(S, BP_CLOSED) + (size_t)y * S.rowWords;
-    uint32_t* holes = bit_plane(S, BP_HOLES) + (size_t)y * S.rowWords;
-    // one root lookup per run: at the lane where the run starts; a run that continues from the
-    // previous chunk keeps that chunk's answer
-    uint32_t carry = 0;
-    bool carryHole = false;
-    for (int x0 = 0; x0 < W; x0 += 32) {
-        const uint32_t ball = ~__ldcg(&row[x0 >> 5]) & valid_bits(x0 >> 5, W);
-        const uint32_t starts = ball & ~((ball << 1) | carry);
-        const bool isStart = (starts >> lane) & 1u;
-        const bool h = isStart && uf_find(S.label, y * W + x0 + lane, P.work) != 0;
-        const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
-        const int src = upto ? 31 - __clz(upto) : 0;
-        const bool hs = __shfl_sync(0xffffffffu, h, src);
-        const bool hole = ((ball >> lane) & 1u) && (upto ? hs : carryHole);
-        const uint32_t hw = __ballot_sync(0xffffffffu, hole);
-        if (lane == 0) holes[x0 >> 5] = hw;
-        carryHole = (hw >> 31) & 1u;
-        carry = ball >> 31;
-    }
-}
-
-// word w of a bit-plane row with the pixels outside [0, W) set to fill (0 or ~0)
-__device__ __forceinline__ uint32_t row_word(const uint32_t* row, int w, int RW, int W, uint32_t fill) {
-    if (w < 0 || w >= RW) return fill;
-    const uint32_t vb = valid_bits(w, W);
-    return (__ldcg(&row[w]) & vb) | (fill & ~vb);
-}
-
-// 7-pixel horizontal AND (erode) or OR (dilate) of word w of a row; pixels outside the frame take
-// the value that never wins
-template <bool AND>
-__device__ __forceinline__ uint32_t row_box7(const uint32_t* row, int w, int RW, int W) {
-    const uint32_t fill = AND ? 0xffffffffu : 0u;
-    const uint32_t L = row_word(row, w - 1, RW, W, fill), C = row_word(row, w, RW, W, fill),
-                   R = row_word(row, w + 1, RW, W, fill);
-    uint32_t v = C;
-#pragma unroll
-    for (int d = 1; d <= 3; ++d) {
-        const uint32_t a = __funnelshift_r(C, R, d), b = __funnelshift_l(L, C, d);  // pixels x+d, x-d
-        v = AND ? (v & a & b) : (v | a | b);
-    }
-    return v;
-}
-
-// 3-fold 3x3 erosion of the closed mask (a clipped 7x7 minimum) and mask |= holes | eroded (:544-546);
-// one warp per row, one thread per 32-pixel word
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_combine(TickParams P) {
+// Combined mask |= holes | 3-fold 3x3 erosion of the closed mask (a clipped 7x7 minimum) (:541-546): a
+// warp per row, a word per lane. Holes are the 0-runs whose root is not 0 (one lookup per run and word;
+// runs on the ring need none). The erosion is separable: seven row words are ANDed, then the neighbour
+// words come from the neighbour lanes (the two edge lanes of a chunk load theirs). One kernel where the
+// hole words took a pass of their own through memory: 20 + 6 us on a 1920x1080 frame before.
+extern "C" __global__ void __launch_bounds__(256) lvbgs_k_fill(TickParams P) {
     const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (gr >= P.totalRows) return;
     const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
     const int y = gr - S.rowBase, W = S.W, H = S.H, RW = S.rowWords;
     const uint32_t* closed = bit_plane(S, BP_CLOSED);
-    for (int w = lane; w < RW; w += 32) {
-        uint32_t er = 0xffffffffu;
-        for (int yy = max(0, y - 3); yy <= min(H - 1, y + 3); ++yy) er &= row_box7<true>(closed + (size_t)yy * RW, w, RW, W);
-        const size_t o = (size_t)y * RW + w;
-        bit_plane(S, BP_COMB)[o] = (__ldcg(&bit_plane(S, BP_RAW)[o]) | __ldcg(&bit_plane(S, BP_HOLES)[o]) | er) & valid_bits(w, W);
-    }
-}
-
-// median, part 1: for each pixel, the number of set pixels of the combined mask in its row window
-// [x - r, x + r] (replicate border: pixels left of 0 / right of W-1 repeat those two pixels); one
-// block per row, four 32-pixel words per warp step
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_hcount(TickParams P) {
-    const int gr = blockIdx.x, lane = threadIdx.x & 31;
-    if (gr >= P.totalRows) return;
-    const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
-    const int y = gr - S.rowBase, W = S.W, RW = S.rowWords;
-    const int r = S.ctl->median_k / 2;  // <= 15
-    const uint32_t* row = bit_plane(S, BP_COMB) + (size_t)y * RW;
-    const uint32_t lastFill = ((__ldcg(&row[(W - 1) >> 5]) >> ((W - 1) & 31)) & 1u) ? 0xffffffffu : 0u;
-    const uint32_t firstFill = (__ldcg(&row[0]) & 1u) ? 0xffffffffu : 0u;
-    const unsigned long long win = (2ull << (2 * r)) - 1ull;
-    const int nw = blockDim.x >> 5;
-    for (int w0 = (threadIdx.x >> 5) * 4; w0 < RW; w0 += 4 * nw) {
-        // words w0-1 .. w0+4 first, then the four words' counts
-        uint32_t v[6];
+    RowRuns rr;
+    rr.reset(closed + (size_t)y * RW, RW, W);
+    const int last = rr.last_start(lane);
+    const int ya = max(0, y - 3), yb = min(H - 1, y + 3);
+    // word w of the rows' minimum; pixels outside the frame never win
+    auto column_and = [&](int w) {
+        uint32_t v = 0xffffffffu;
+        if (w < 0 || w >= RW) return v;
+        for (int yy = ya; yy <= yb; ++yy) v &= __ldcg(&closed[(size_t)yy * RW + w]);
+        return v | ~valid_bits(w, W);
+    };
+    for (int c = 0; c < RW; c += 32) {
+        const int w = c + lane;
+        const uint32_t er0 = column_and(w);
+        uint32_t erL = __shfl_up_sync(0xffffffffu, er0, 1), erR = __shfl_down_sync(0xffffffffu, er0, 1);
+        if (lane == 0) erL = column_and(w - 1);
+        if (lane == 31) erR = column_and(w + 1);
+        uint32_t er = er0;
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            const int w = w0 - 1 + j;
-            v[j] = w < 0 ? firstFill : row_word(row, w, RW, W, lastFill);
+        for (int d = 1; d <= 3; ++d) er &= __funnelshift_r(er0, erR, d) & __funnelshift_l(erL, er0, d);
+        rr.load(c, lane);
+        uint32_t holes = 0u, rem = rr.z;
+        while (rem) {
+            const int b = __ffs(rem) - 1;
+            const uint32_t inv = ~(rem >> b);
+            const int len = inv ? __ffs(inv) - 1 : 32;  // pixels of the run in this word
+            const uint32_t m = (len >= 32 ? 0xffffffffu : (1u << len) - 1u) << b;
+            rem &= ~m;
+            const int s = rr.run_start(w, b);
+            if (s != 0 && s != last && y > 0 && y < H - 1 && uf_find(S.label, y * W + s, P.work) != 0) holes |= m;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            // bits 16..79 of the 96-bit row segment L | C | R: pixel x - r is bit 16 + lane - r
-            const unsigned long long M =
-                ((unsigned long long)v[j + 2] << 48) | ((unsigned long long)v[j + 1] << 16) | (v[j] >> 16);
-            const int x = 32 * (w0 + j) + lane;
-            if (x < W) S.hcount[(size_t)y * W + x] = (uint8_t)__popcll((M >> (16 + lane - r)) & win);
+        if (w < RW) {
+            const size_t o = (size_t)y * RW + w;
+            bit_plane(S, BP_COMB)[o] = (__ldcg(&bit_plane(S, BP_RAW)[o]) | holes | er) & valid_bits(w, W);
         }
     }
 }
 
-// median, part 2 (:547, :552-554): binary median blur (majority of the k x k window, replicate border)
-// of the combined mask -> final mask, its row words, and the final-segmentation EMAs (addWeighted).
-// One thread per pixel column of a 64-row segment, sliding the window sum down the rows.
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_median(TickParams P) {
-    const int gs = blockIdx.y;
-    if (gs >= P.totalSegs) return;
+// bit-sliced arithmetic on 32 pixels at once: carry of a full adder
+__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (a & c) | (b & c); }
+
+// number of set pixels of each pixel's row window [x - r, x + r], r < 2^(HB-1): bit planes h[0..HB-1] of
+// word C with its neighbour words L and R
+template <int HB>
+__device__ __forceinline__ void row_window_planes(uint32_t L, uint32_t C, uint32_t R, int r, uint32_t (&h)[HB]) {
+    h[0] = C;
+#pragma unroll
+    for (int i = 1; i < HB; ++i) h[i] = 0u;
+    int d = 1;
+    for (; d + 1 <= r; d += 2) {
+        const uint32_t a = __funnelshift_r(C, R, d), b = __funnelshift_l(L, C, d);
+        const uint32_t e = __funnelshift_r(C, R, d + 1), f = __funnelshift_l(L, C, d + 1);
+        const uint32_t s = h[0] ^ a ^ b, c1 = maj3(h[0], a, b);
+        h[0] = s ^ e ^ f;
+        const uint32_t c2 = maj3(s, e, f);
+        uint32_t c = maj3(h[1], c1, c2);
+        h[1] ^= c1 ^ c2;
+#pragma unroll
+        for (int i = 2; i < HB; ++i) {
+            const uint32_t t = h[i] & c;
+            h[i] ^= c;
+            c = t;
+        }
+    }
+    if (d <= r) {
+        const uint32_t a = __funnelshift_r(C, R, d), b = __funnelshift_l(L, C, d);
+        uint32_t c = maj3(h[0], a, b);
+        h[0] ^= a ^ b;
+#pragma unroll
+        for (int i = 1; i < HB; ++i) {
+            const uint32_t t = h[i] & c;
+            h[i] ^= c;
+            c = t;
+        }
+    }
+}
+
+// shared memory of one tile of the final-mask kernel: the combined mask's words with their halo, the row
+// window counts as bit planes, the final mask with the dilation's halo, the dilated words
+constexpr int kFinMaxR = 15;                            // median radius (kernel size at most 31)
+constexpr int kFinRows = kFinH + 6 + 2 * kFinMaxR;      // combined-mask rows
+constexpr int kFinFG = kFinH + 6;                       // final-mask rows
+struct FinSmem {
+    uint32_t comb[kFinRows][kFinWords + 4];
+    uint32_t h[5][kFinRows][kFinWords + 2];
+    uint32_t fg[kFinFG][kFinWords + 2];
+    uint32_t dil[kFinH][kFinWords];
+};
+
+// row window counts, then the window sums of the final mask's words and their comparison with half the
+// window (threads take one word each)
+template <int HB>
+__device__ __forceinline__ void median_words(FinSmem& sm, int r, int half, int y0, int w0, int W, int H, int RW) {
+    const int nRows = kFinFG + 2 * r;
+    for (int i = threadIdx.x; i < nRows * (kFinWords + 2); i += blockDim.x) {
+        const int rr = i / (kFinWords + 2), ww = i % (kFinWords + 2);
+        uint32_t h[HB];
+        row_window_planes<HB>(sm.comb[rr][ww], sm.comb[rr][ww + 1], sm.comb[rr][ww + 2], r, h);
+#pragma unroll
+        for (int b = 0; b < HB; ++b) sm.h[b][rr][ww] = h[b];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kFinFG * (kFinWords + 2); i += blockDim.x) {
+        const int fr = i / (kFinWords + 2), fw = i % (kFinWords + 2);
+        const int y = y0 - 3 + fr, w = w0 - 1 + fw;
+        uint32_t fg = 0u;
+        if (y >= 0 && y < H && w >= 0 && w < RW) {
+            uint32_t a[2 * HB];
+#pragma unroll
+            for (int b = 0; b < 2 * HB; ++b) a[b] = b < HB ? sm.h[b < HB ? b : 0][fr][fw] : 0u;
+            for (int j = 1; j <= 2 * r; ++j) {
+                uint32_t c = 0u;
+#pragma unroll
+                for (int b = 0; b < HB; ++b) {
+                    const uint32_t v = sm.h[b][fr + j][fw];
+                    const uint32_t s = a[b] ^ v ^ c;
+                    c = maj3(a[b], v, c);
+                    a[b] = s;
+                }
+#pragma unroll
+                for (int b = HB; b < 2 * HB; ++b) {
+                    const uint32_t t = a[b] & c;
+                    a[b] ^= c;
+                    c = t;
+                }
+            }
+            // sum > half, from the lowest bit up
+#pragma unroll
+            for (int b = 0; b < 2 * HB; ++b) fg = ((half >> b) & 1) ? (a[b] & fg) : (a[b] | fg);
+            fg &= valid_bits(w, W);
+        }
+        sm.fg[fr][fw] = fg;
+    }
+}
+
+// The final mask and everything that follows from it (:547-554): binary median blur of the combined mask
+// (majority of the k x k window, replicated border), the final-segmentation averages (addWeighted), the
+// mask bytes, its 3-fold 3x3 dilation (a clipped 7x7 maximum) and the blink masking with the previous and
+// the new inverted dilated masks. A block takes 8 rows of 4 words (128 pixels) and counts on bit planes:
+// 32 pixels per word operation, full adders over the row window, then over the rows, with the halo of the
+// dilation recomputed (84 words for 32), so that no per-pixel count goes through memory and the three
+// passes of before (7.8 + 15.9 + 10.2 us on a 1920x1080 frame) are one. The pixels' maps are requested
+// first and used last; a thread holds four neighbouring pixels, so the mask leaves in 128-byte rows also
+// when it is in host memory. Bound by the 22 B/px of maps and by the latency of the short word phases.
+extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams P) {
+    __shared__ FinSmem sm;
+    const int gt = blockIdx.x;
+    if (gt >= P.totalSegs) return;
     int lo = 0, hi = P.nStreams - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (P.streams[mid].segBase <= gs) lo = mid;
+        if (P.streams[mid].segBase <= gt) lo = mid;
         else hi = mid - 1;
     }
     const StreamDev& S = P.streams[lo];
-    const int W = S.W, H = S.H, npx = S.npx;
-    const int x0 = blockIdx.x * 256;
-    if (x0 >= W) return;
-    const int x = x0 + threadIdx.x, lane = threadIdx.x & 31;
-    const bool in = x < W;
-    const int y0 = (gs - S.segBase) * kMedSegRows, y1 = min(H, y0 + kMedSegRows);
+    const int W = S.W, H = S.H, npx = S.npx, RW = S.rowWords;
+    const int tilesX = (RW + kFinWords - 1) / kFinWords;
+    const int lt = gt - S.segBase, y0 = (lt / tilesX) * kFinH, w0 = (lt % tilesX) * kFinWords;
     const int k = S.ctl->median_k, r = k / 2;
     const FrameK F = frame_consts(S);
-    const float* fcur = S.fm + (size_t)F.cur * kNumFloatMaps * npx;
-    float* fn = S.fm + (size_t)F.nxt * kNumFloatMaps * npx;
+    // the four pixels of this thread
+    const int row = threadIdx.x >> 5, quad = threadIdx.x & 31;
+    const int y = y0 + row, x = w0 * 32 + quad * 4, q = y * W + x;
+    const int n = y < H ? min(4, W - x) : 0;  // pixels of the quad inside the frame
+    const float* cLT = S.fm + ((size_t)F.cur * kNumFloatMaps + FM_FIN_LT) * npx;
+    const float* cST = S.fm + ((size_t)F.cur * kNumFloatMaps + FM_FIN_ST) * npx;
+    float* nLT = S.fm + ((size_t)F.nxt * kNumFloatMaps + FM_FIN_LT) * npx;
+    float* nST = S.fm + ((size_t)F.nxt * kNumFloatMaps + FM_FIN_ST) * npx;
+    const bool vec = (W & 3) == 0;  // then a quad is whole, and aligned in every plane
+    float fl[4] = {0, 0, 0, 0}, fs[4] = {0, 0, 0, 0};
+    uint32_t bl = 0u, di = 0u;
+    if (vec && n > 0) {
+        const float4 a = *(const float4*)(cLT + q), b = *(const float4*)(cST + q);
+        fl[0] = a.x, fl[1] = a.y, fl[2] = a.z, fl[3] = a.w;
+        fs[0] = b.x, fs[1] = b.y, fs[2] = b.z, fs[3] = b.w;
+        bl = *(const uint32_t*)(S.blinks + q);
+        di = *(const uint32_t*)(S.dilInv + q);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < n) {
+                fl[i] = cLT[q + i];
+                fs[i] = cST[q + i];
+                bl |= (uint32_t)S.blinks[q + i] << (8 * i);
+                di |= (uint32_t)S.dilInv[q + i] << (8 * i);
+            }
+    }
+    const uint32_t* comb = bit_plane(S, BP_COMB);
+    const int nRows = kFinFG + 2 * r;
+    for (int i = threadIdx.x; i < nRows * (kFinWords + 4); i += blockDim.x) {
+        const int rr = i / (kFinWords + 4), ww = i % (kFinWords + 4);
+        const uint32_t* src = comb + (size_t)min(max(y0 - 3 - r + rr, 0), H - 1) * RW;
+        const int w = w0 - 2 + ww;
+        uint32_t v;
+        if (w < 0) {
+            v = (__ldcg(&src[0]) & 1u) ? 0xffffffffu : 0u;
+        } else if (w < RW - 1) {
+            v = __ldcg(&src[w]);
+        } else {
+            const uint32_t lw = __ldcg(&src[RW - 1]);
+            const uint32_t fill = ((lw >> ((W - 1) & 31)) & 1u) ? 0xffffffffu : 0u;
+            const uint32_t vb = valid_bits(w, W);
+            v = (lw & vb) | (fill & ~vb);
+        }
+        sm.comb[rr][ww] = v;
+    }
+    __syncthreads();
+    // 2 * sum > k * k
+    if (r < 8) median_words<4>(sm, r, k * k / 2, y0, w0, W, H, RW);
+    else median_words<5>(sm, r, k * k / 2, y0, w0, W, H, RW);
+    __syncthreads();
+    if (threadIdx.x < kFinH * kFinWords) {
+        const int dr = threadIdx.x / kFinWords, dw = threadIdx.x % kFinWords;
+        uint32_t a = 0u, b = 0u, c = 0u;
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            a |= sm.fg[dr + j][dw];
+            b |= sm.fg[dr + j][dw + 1];
+            c |= sm.fg[dr + j][dw + 2];
+        }
+        uint32_t v = b;
+#pragma unroll
+        for (int d = 1; d <= 3; ++d) v |= __funnelshift_r(b, c, d) | __funnelshift_l(a, b, d);
+        sm.dil[dr][dw] = v;
+    }
+    __syncthreads();
+    if (n <= 0) return;
+    const uint32_t fg4 = (sm.fg[row + 3][1 + (quad >> 3)] >> ((quad & 7) * 4)) & 15u;
+    const uint32_t dl4 = (sm.dil[row][quad >> 3] >> ((quad & 7) * 4)) & 15u;
+    // bit i -> byte i, as 0 or 255
+    const uint32_t fgb = ((fg4 * 0x00204081u) & 0x01010101u) * 255u;
+    const uint32_t inv = ~(((dl4 * 0x00204081u) & 0x01010101u) * 255u);
     const float aL = 1.0f - F.fLT, bL = S.ctl->bLT;
     const float aS = 1.0f - F.fST, bS = S.ctl->bST;
-    const uint8_t* hc = S.hcount + (in ? x : 0);
-    int sum = 0;
-    if (in)
-        for (int yy = y0 - r; yy <= y0 + r; ++yy) sum += __ldcg(&hc[(size_t)min(max(yy, 0), H - 1) * W]);
-    uint32_t* fgRow = bit_plane(S, BP_FG) + (x0 >> 5) + (threadIdx.x >> 5);
-    // four rows per step: every load of the step is issued before its stores
-    for (int yb = y0; yb < y1; yb += 4) {
-        int add[4], sub[4];
-        float fl[4], fs[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int y = yb + j;
-            add[j] = sub[j] = 0;
-            fl[j] = fs[j] = 0.0f;
-            if (in && y < y1) {
-                const int q = y * W + x;
-                add[j] = __ldcg(&hc[(size_t)min(y + r + 1, H - 1) * W]);
-                sub[j] = __ldcg(&hc[(size_t)max(y - r, 0) * W]);
-                fl[j] = fcur[FM_FIN_LT * npx + q];
-                fs[j] = fcur[FM_FIN_ST * npx + q];
-            }
-        }
+    for (int i = 0; i < 4; ++i) {
+        const float m = (float)((fgb >> (8 * i)) & 255u);
+        fl[i] = (fl[i] * aL + m * bL) + 0.0f;
+        fs[i] = (fs[i] * aS + m * bS) + 0.0f;
+    }
+    const uint32_t nb = bl & di & inv;
+    if (vec) {
+        *(float4*)(nLT + q) = make_float4(fl[0], fl[1], fl[2], fl[3]);
+        *(float4*)(nST + q) = make_float4(fs[0], fs[1], fs[2], fs[3]);
+        *(uint32_t*)(S.lastFG + q) = fgb;
+        *(uint32_t*)(S.blinks + q) = nb;
+        *(uint32_t*)(S.dilInv + q) = inv;
+    } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int y = yb + j;
-            if (y >= y1) break;
-            const bool fg = in && 2 * sum > k * k;
-            const unsigned ball = __ballot_sync(0xffffffffu, fg);
-            if (in) {
-                const int q = y * W + x;
-                const uint8_t fgv = fg ? 255 : 0;
-                __stcg(&S.lastFG[q], fgv);
-                if (S.maskOut) S.maskOut[q] = fgv;
-                const float m = (float)fgv;
-                fn[FM_FIN_LT * npx + q] = (fl[j] * aL + m * bL) + 0.0f;
-                fn[FM_FIN_ST * npx + q] = (fs[j] * aS + m * bS) + 0.0f;
-                sum += add[j] - sub[j];
+        for (int i = 0; i < 4; ++i)
+            if (i < n) {
+                nLT[q + i] = fl[i];
+                nST[q + i] = fs[i];
+                S.lastFG[q + i] = (uint8_t)(fgb >> (8 * i));
+                S.blinks[q + i] = (uint8_t)(nb >> (8 * i));
+                S.dilInv[q + i] = (uint8_t)(inv >> (8 * i));
             }
-            if (lane == 0 && x < W) fgRow[(size_t)y * S.rowWords] = ball;
+    }
+    if (S.maskOut) {
+        if (vec && ((uintptr_t)S.maskOut & 3) == 0) {
+            *(uint32_t*)(S.maskOut + q) = fgb;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < n) S.maskOut[q + i] = (uint8_t)(fgb >> (8 * i));
         }
     }
 }
 
-// 3-fold 3x3 dilation of the final mask (a clipped 7x7 maximum) and blink masking with the previous
-// and the new inverted dilated masks (:548-551); one block per row, four 32-pixel words per warp step,
-// one lane per pixel of each
-extern "C" __global__ void __launch_bounds__(256) lvbgs_k_dilate(TickParams P) {
-    const int gr = blockIdx.x, lane = threadIdx.x & 31;
-    if (gr >= P.totalRows) return;
-    const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
-    const int y = gr - S.rowBase, W = S.W, H = S.H, RW = S.rowWords;
-    const uint32_t* fgp = bit_plane(S, BP_FG);
-    const int nw = blockDim.x >> 5;
-    for (int w0 = (threadIdx.x >> 5) * 4; w0 < RW; w0 += 4 * nw) {
-        // lane l < 28 dilates row y - 3 + l/4 of word w0 + l%4; an OR over the lanes of equal l%4
-        const int j = lane & 3, yy = y - 3 + (lane >> 2);
-        uint32_t d = 0;
-        if (lane < 28 && yy >= 0 && yy < H && w0 + j < RW) d = row_box7<false>(fgp + (size_t)yy * RW, w0 + j, RW, W);
-        d |= __shfl_xor_sync(0xffffffffu, d, 4);
-        d |= __shfl_xor_sync(0xffffffffu, d, 8);
-        d |= __shfl_xor_sync(0xffffffffu, d, 16);
-        uint32_t dw[4];
-        uint8_t bl[4], di[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            dw[i] = __shfl_sync(0xffffffffu, d, i);
-            const int x = 32 * (w0 + i) + lane;
-            bl[i] = di[i] = 0;
-            if (x < W) {
-                bl[i] = S.blinks[y * W + x];
-                di[i] = S.dilInv[y * W + x];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int x = 32 * (w0 + i) + lane;
-            if (x < W) {
-                const uint8_t inv = ((dw[i] >> lane) & 1u) ? 0 : 255;
-                S.blinks[y * W + x] = (uint8_t)(bl[i] & di[i] & inv);
-                S.dilInv[y * W + x] = inv;
-            }
-        }
-    }
-}
-
-// frame-level epilogue of one stream (:555-611): LBSP threshold LUT adaptation, camera-motion
-// analysis, automatic model reset decision and learning-rate caps
+// frame-level epilogue of one stream (:555-611), one block of 256 threads: LBSP threshold LUT adaptation
+// (one entry per thread), then, on thread 0, camera-motion analysis, automatic model reset decision and
+// learning-rate caps
 __device__ void stream_epilogue(const TickParams& P, const StreamDev& S) {
     StreamCtl* ctl = S.ctl;
     const float relThr = S.relThr;
     const unsigned int lbspOff = S.lbspOff;
     const unsigned long long nz = ctl->nz_acc;
-    ctl->last_nz = nz;
-    ctl->nz_acc = 0;
     const float ratio = __ull2float_rn(nz) / __ull2float_rn(ctl->n_rel);
     const float last = ctl->last_nz_ratio;
+    const int t = threadIdx.x;
     if (ratio < 0.100f && last < 0.100f) {
-        for (int t = 0; t <= 255; ++t) {
-            const float v = ceilf((float)t * relThr / 4) + (float)lbspOff;
-            const int lim = v > 255.0f ? 255 : (int)v;
-            if ((int)ctl->lut[t] > lim) --ctl->lut[t];
-        }
+        const float v = ceilf((float)t * relThr / 4) + (float)lbspOff;
+        const int lim = v > 255.0f ? 255 : (int)v;
+        if ((int)ctl->lut[t] > lim) --ctl->lut[t];
     } else if (ratio > 0.500f && last > 0.500f) {
         int lim = __float2int_rn((float)lbspOff + 255 * relThr);
         lim = lim < 0 ? 0 : lim > 255 ? 255 : lim;
-        for (int t = 0; t <= 255; ++t)
-            if ((int)ctl->lut[t] < lim) ++ctl->lut[t];
+        if ((int)ctl->lut[t] < lim) ++ctl->lut[t];
     }
+    __syncthreads();  // every thread has read the ratios
+    if (t != 0) return;
+    ctl->last_nz = nz;
+    ctl->nz_acc = 0;
     ctl->last_nz_ratio = ratio;
     ctl->refresh_pending = 0;
     ctl->ksent = 0;
@@ -1642,6 +1752,15 @@ __device__ void stream_epilogue(const TickParams& P, const StreamDev& S) {
             ctl->t_hi = 256.0f;
         }
         if (ctl->cooldown > 0ull) --ctl->cooldown;
+    }
+    if (ctl->refresh_pending) {
+        // nRefreshSampleStartPos = rand() % N, drawn with the frame-level (sentinel) counter (:86)
+        DrawState ds;
+        ds.blk = 0xffffffffu;
+        const uint32_t f = (uint32_t)(ctl->frame_idx + 1ull);
+        ctl->refresh_start = draw_k(S.seed, f, kSentinelPx, 0u, ds) % (uint32_t)S.N;
+        ctl->ksent = 1;
+        atomicExch(&P.work->anyReset, 1u);
     }
 }
 
@@ -1881,29 +2000,27 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_commit(TickParams
 }
 
 
-
-// frame-level epilogue of every stream (one thread per stream)
-extern "C" __global__ void lvbgs_k_epilogue(TickParams P) {
-    for (int si = blockIdx.x * blockDim.x + threadIdx.x; si < P.nStreams; si += gridDim.x * blockDim.x) {
-        const StreamDev& S = P.streams[si];
-        stream_epilogue(P, S);
-        if (S.ctl->refresh_pending) {
-            // nRefreshSampleStartPos = rand() % N, drawn with the frame-level (sentinel) counter (:86)
-            DrawState ds;
-            ds.blk = 0xffffffffu;
-            const uint32_t f = (uint32_t)(S.ctl->frame_idx + 1ull);
-            S.ctl->refresh_start = draw_k(S.seed, f, kSentinelPx, 0u, ds) % (uint32_t)S.N;
-            S.ctl->ksent = 1;
-            atomicExch(&P.work->anyReset, 1u);
-        }
+// closes the frame of every stream: frame index (and so the buffer parity), repair statistics
+__device__ __forceinline__ void close_streams(const TickParams& P) {
+    const unsigned int its = P.work->iters;
+    for (int si = threadIdx.x; si < P.nStreams; si += blockDim.x) {
+        StreamCtl* ctl = P.streams[si].ctl;
+        ctl->frame_idx += 1ull;
+        ctl->st_rounds += its;
+        ctl->stamp_base += its + 4u;
+        frame_factors(ctl->frame_idx + 1ull, P.streams[si].nmv, &ctl->fLT, &ctl->fST, &ctl->bLT, &ctl->bST);
     }
 }
 
-
-// automatic model reset: refreshModel(0.1) and T(x) := 1 everywhere (:588-593); a small grid
-// strides over the tiles of the streams that reset this frame
-extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_reset(TickParams P) {
-    if (ld_volatile(&P.work->anyReset) == 0u) return;
+// The end of the frame. Nearly always block 0 closes the streams and the others leave at once. When a
+// stream resets its model -- refreshModel(0.1) and T(x) := 1 everywhere (:588-593) -- the grid strides over
+// the tiles of those streams, and the block that finishes last closes the streams (the others still read
+// the frame index until then).
+extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_close(TickParams P) {
+    if (ld_volatile(&P.work->anyReset) == 0u) {
+        if (blockIdx.x == 0) close_streams(P);
+        return;
+    }
     for (int t = blockIdx.x; t < P.totalTiles; t += gridDim.x) {
         const int si = find_stream_by_tile(P, t);
         const StreamDev& S = P.streams[si];
@@ -1921,18 +2038,12 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_reset(TickParams 
         S.fm[(size_t)0 * kNumFloatMaps * S.npx + FM_T * S.npx + p] = 1.0f;
         S.fm[(size_t)1 * kNumFloatMaps * S.npx + FM_T * S.npx + p] = 1.0f;
     }
-}
-
-// closes the frame of every stream: frame index (and so the buffer parity), repair statistics
-extern "C" __global__ void lvbgs_k_close(TickParams P) {
-    const unsigned int its = P.work->iters;
-    for (int si = blockIdx.x * blockDim.x + threadIdx.x; si < P.nStreams; si += gridDim.x * blockDim.x) {
-        StreamCtl* ctl = P.streams[si].ctl;
-        ctl->frame_idx += 1ull;
-        ctl->st_rounds += its;
-        ctl->stamp_base += its + 4u;
-        frame_factors(ctl->frame_idx + 1ull, P.streams[si].nmv, &ctl->fLT, &ctl->fST, &ctl->bLT, &ctl->bST);
-    }
+    __shared__ int sLast;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sLast = atomicAdd(&P.work->done_ctas, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (sLast) close_streams(P);
 }
 
 // ------------------------------------------------------------------------------------------

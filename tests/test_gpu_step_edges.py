@@ -1,0 +1,38 @@
+"""SuBSENSE's frame step at the edges of its kernels' tiles, words and chunks, against the oracle (bit-exact)."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_parity import run_pair
+
+pytestmark = pytest.mark.gpu
+
+
+def hollow_frames(W, H, channels, n, seed):
+    """A textured background with hollow rectangles (holes to fill), specks and a bar across the frame."""
+    rng = np.random.default_rng(seed)
+    base = rng.integers(40, 90, (H, W, 3)).astype(np.int16)
+    frames = []
+    for t in range(n):
+        img = base + rng.integers(-3, 4, base.shape)
+        for _ in range(6 if t else 0):
+            w, h = int(rng.integers(6, max(7, W // 2))), int(rng.integers(6, max(7, H - 2)))
+            x, y = int(rng.integers(0, max(1, W - 4))), int(rng.integers(0, max(1, H - 4)))
+            keep = img[y + 2:y + h - 2, x + 2:x + w - 2].copy()
+            img[y:y + h, x:x + w] = rng.integers(150, 255, 3)
+            img[y + 2:y + 2 + keep.shape[0], x + 2:x + 2 + keep.shape[1]] = keep
+        speck = rng.random((H, W)) < 0.01
+        img[speck & (t > 0)] = 250
+        if t % 3 == 2:
+            img[H // 2:H // 2 + 2] = 200
+        img = np.clip(img, 0, 255).astype(np.uint8)
+        frames.append(img if channels == 3 else np.ascontiguousarray(img[:, :, 0]))
+    return frames
+
+
+@pytest.mark.parametrize("W,H,k,channels", [(31, 9, 1, 1), (32, 8, 3, 3), (33, 17, 15, 3), (127, 23, 17, 1),
+                                            (128, 24, 31, 3), (130, 25, 9, 1), (1024, 16, 13, 1), (1061, 19, 9, 3),
+                                            (2053, 11, 5, 1)])
+def test_post_processing_at_word_tile_and_chunk_edges(W, H, k, channels):
+    """Hole filling over rows of one word up to three 32-word chunks, every median width class (window counts
+    of four and of five bit planes), frames that end inside a word, a tile and a quad of pixels."""
+    run_pair(hollow_frames(W, H, channels, 7, W * 31 + H), seed=W, nDefaultMedianBlurKernelSize=k)
