@@ -163,7 +163,7 @@ struct StreamDev {
 struct TickWork {
     unsigned int bar_count, bar_gen, err, err_info;
     unsigned int phase_ctr[16];  // repair: re-matched items of rounds 0..15 (phase profile)
-    unsigned int dcount[2], rcount[2];
+    unsigned int dcount[4], rcount[2];  // repair lists' lengths (dcount: by dcount_slot, rcount: by round parity)
     unsigned int done_ctas, iters;
     unsigned long long rematched;
     unsigned long long ts[40];  // %globaltimer after each grid barrier (CTA 0), for the phase profile

@@ -50,9 +50,9 @@ __device__ __forceinline__ unsigned long long gtimer() {
 }
 __device__ __forceinline__ unsigned int ld_volatile(const unsigned int* p) { return *(const volatile unsigned int*)p; }
 
-// Grid-wide barrier for a cooperative launch (all CTAs co-resident). The wait is bounded: after
+// Barrier over the first nCtas CTAs of a cooperative launch (all co-resident). The wait is bounded: after
 // timeoutNs the CTA records ERR_BARRIER_TIMEOUT and every CTA leaves at its next check.
-__device__ bool grid_sync(TickWork* w, unsigned long long timeoutNs) {
+__device__ bool grid_sync(TickWork* w, unsigned int nCtas, unsigned long long timeoutNs) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -60,7 +60,7 @@ __device__ bool grid_sync(TickWork* w, unsigned long long timeoutNs) {
         __threadfence();
         const unsigned int arrived = atomicAdd(&w->bar_count, 1u) + 1u;
         int ok = 1;
-        if (arrived == gridDim.x) {
+        if (arrived == nCtas) {
             atomicExch(&w->bar_count, 0u);
             __threadfence();
             atomicAdd(&w->bar_gen, 1u);
@@ -312,21 +312,6 @@ __device__ __forceinline__ bool sample_match(const uint8_t* __restrict__ lut, co
     }
 }
 
-// the ordered sample scan, continued from state st until nreq good samples or sample sEnd; dA/cA and
-// dB/cB hold samples st.s and st.s+1 (they arrive with the feedback maps), and the loop requests
-// sample s+2 while it evaluates sample s. OVR: the samples that earlier pixels overwrite this frame
-// (repair)
-// L2 prefetch of sample k of pixel p (both planes): a hint without registers, so that a long scan keeps
-// several samples in flight
-template <int C>
-__device__ __forceinline__ void prefetch_sample(const StreamDev& S, int k, int p) {
-    const void* a = C == 3 ? (const void*)((const uint64_t*)S.sD + (size_t)k * S.npx + p)
-                           : (const void*)((const uint16_t*)S.sD + (size_t)k * S.npx + p);
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(S.sC + (size_t)k * S.npx + p));
-}
-constexpr int kScanPrefetch = 8;  // samples prefetched ahead of the loads of a long scan
-
 template <int C>
 __device__ __forceinline__ void scan_init(ScanSt& st) {
     st.s = 0;
@@ -336,59 +321,33 @@ __device__ __forceinline__ void scan_init(ScanSt& st) {
     st.minDesc = C == 1 ? 16u : 48u;
     st.minSum = C == 1 ? 255u : 765u;
 }
-template <int C, bool OVR, bool REC = true>
+// the evaluation's ordered sample scan: until nreq good samples or kScanCap samples; dA/cA and dB/cB hold
+// samples 0 and 1 (they arrive with the feedback maps), and the loop requests sample s+2 while it evaluates
+// sample s. The first good sample's index is tracked (a deferred scan's record keeps it), not the distances.
+template <int C>
 __device__ __forceinline__ void scan_samples(const StreamDev& S, const uint8_t* __restrict__ lut, int p,
                                              const uint32_t (&vals)[C][4], const uint32_t (&curr)[C],
-                                             const uint32_t (&intra)[C], const EvalThr& th, const Ovr* ov, int nov,
-                                             uint64_t ovmask, int sEnd, uint64_t dA, uint32_t cA, uint64_t dB,
-                                             uint32_t cB, ScanSt& st) {
-    const int npx = S.npx, N = S.N, nreq = S.nreq;
-    const int sMax = sEnd < N ? sEnd : N;
-    int nGood = st.nGood, s = st.s;
+                                             const uint32_t (&intra)[C], const EvalThr& th, uint64_t dA, uint32_t cA,
+                                             uint64_t dB, uint32_t cB, ScanSt& st) {
+    const int npx = S.npx, nreq = S.nreq;
+    const int sMax = kScanCap < S.N ? kScanCap : S.N;
+    int nGood = 0, s = 0, g0 = -1;
     uint32_t minDesc = st.minDesc, minSum = st.minSum;
-    int g0 = st.g0, g1 = st.g1;
-    uint32_t g0d = st.g0d, g0s = st.g0s, g1d = st.g1d, g1s = st.g1s;
-    // scans that may run past the evaluation's cap (long scans, repair) prefetch ahead into L2
-    const bool deep = sMax > kScanCap;
-    if (deep && nGood < nreq)
-        for (int k = s + 2; k < min(N, s + 2 + kScanPrefetch); ++k) prefetch_sample<C>(S, k, p);
     while (nGood < nreq && s < sMax) {
-        uint64_t d = dA;
-        uint32_t c2 = cA;
+        const uint64_t d = dA;
+        const uint32_t c2 = cA;
         dA = dB;
         cA = cB;
         if (s + 2 < sMax) {
             dB = C == 3 ? ((const uint64_t*)S.sD)[(size_t)(s + 2) * npx + p]
                         : (uint64_t)((const uint16_t*)S.sD)[(size_t)(s + 2) * npx + p];
             cB = S.sC[(size_t)(s + 2) * npx + p];
-            if (deep && s + 2 + kScanPrefetch < N) prefetch_sample<C>(S, s + 2 + kScanPrefetch, p);
-        }
-        if (OVR && ((ovmask >> s) & 1ull)) {
-            int k = nov - 1;
-            while (ov[k].s != s) --k;
-            if (C == 3) {
-                d = ov[k].desc | ((uint64_t)(ov[k].col & 0xffffu) << 48);
-                c2 = (ov[k].col >> 16) & 0xffu;
-            } else {
-                d = ov[k].desc & 0xffffu;
-                c2 = ov[k].col & 0xffu;
-            }
         }
         uint32_t dd, sd;
         if (sample_match<C>(lut, vals, curr, intra, th, d, c2, dd, sd)) {
             if (minDesc > dd) minDesc = dd;
             if (minSum > sd) minSum = sd;
-            if (g0 < 0) {
-                g0 = s;
-                if (REC) {
-                    g0d = dd;
-                    g0s = sd;
-                }
-            } else if (REC && g1 < 0) {
-                g1 = s;
-                g1d = dd;
-                g1s = sd;
-            }
+            if (g0 < 0) g0 = s;
             ++nGood;
         }
         ++s;
@@ -398,11 +357,6 @@ __device__ __forceinline__ void scan_samples(const StreamDev& S, const uint8_t* 
     st.minDesc = minDesc;
     st.minSum = minSum;
     st.g0 = g0;
-    st.g0d = g0d;
-    st.g0s = g0s;
-    st.g1 = g1;
-    st.g1d = g1d;
-    st.g1s = g1s;
 }
 
 // With nreq <= 2 a scan's outcome is fixed by its stop position and its (at most two) good samples:
@@ -420,6 +374,215 @@ __device__ __forceinline__ void record_scan(const StreamDev& S, const FrameK& F,
     r.z = (st.g0d & 0xffffu) | (st.g1d << 16);
     r.w = (st.g0s & 0xffffu) | (st.g1s << 16);
     S.goodRec[p] = r;
+}
+
+// L2 prefetch of sample k of pixel p (both planes): a hint without registers
+template <int C>
+__device__ __forceinline__ void prefetch_sample(const StreamDev& S, int k, int p) {
+    const void* a = C == 3 ? (const void*)((const uint64_t*)S.sD + (size_t)k * S.npx + p)
+                           : (const void*)((const uint16_t*)S.sD + (size_t)k * S.npx + p);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(S.sC + (size_t)k * S.npx + p));
+}
+
+constexpr int kScanPrefetch = 8;  // samples prefetched ahead of the loads of a lane's own scan
+
+// The ordered scan of one pixel's samples by one lane, continued from st (see coop_scan for the masks)
+template <int C, bool REC>
+__device__ __forceinline__ void lane_scan(const StreamDev& S, int p, const uint32_t (&vals)[C][4],
+                                          const uint32_t (&curr)[C], const uint32_t (&intra)[C], const EvalThr& th,
+                                          uint64_t ovMask, uint64_t ovGood, ScanSt& st) {
+    const int N = S.N, nreq = S.nreq;
+    const size_t npx = (size_t)S.npx;
+    const uint8_t* lut = S.ctl->lut;
+    const uint64_t* d3 = (const uint64_t*)S.sD + p;
+    const uint16_t* d1 = (const uint16_t*)S.sD + p;
+    const uint8_t* sc = S.sC + p;
+    auto desc = [&](int k) { return C == 3 ? d3[(size_t)k * npx] : (uint64_t)d1[(size_t)k * npx]; };
+    int s = st.s;
+    uint64_t dA = 0, dB = 0;
+    uint32_t cA = 0, cB = 0;
+    if (s < N) {
+        dA = desc(s);
+        cA = sc[(size_t)s * npx];
+    }
+    if (s + 1 < N) {
+        dB = desc(s + 1);
+        cB = sc[(size_t)(s + 1) * npx];
+    }
+    for (int k = s + 2; k < min(N, s + 2 + kScanPrefetch); ++k) prefetch_sample<C>(S, k, p);
+    while (st.nGood < nreq && s < N) {
+        const uint64_t d = dA;
+        const uint32_t c2 = cA;
+        dA = dB;
+        cA = cB;
+        if (s + 2 < N) {
+            dB = desc(s + 2);
+            cB = sc[(size_t)(s + 2) * npx];
+            if (s + 2 + kScanPrefetch < N) prefetch_sample<C>(S, s + 2 + kScanPrefetch, p);
+        }
+        if (!REC && ((ovMask >> s) & 1ull)) {
+            st.nGood += (int)((ovGood >> s) & 1ull);
+        } else {
+            uint32_t dd, sd;
+            if (sample_match<C>(lut, vals, curr, intra, th, d, c2, dd, sd)) {
+                st.minDesc = min(st.minDesc, dd);
+                st.minSum = min(st.minSum, sd);
+                if (REC) {
+                    if (st.g0 < 0) {
+                        st.g0 = s;
+                        st.g0d = dd;
+                        st.g0s = sd;
+                    } else if (st.g1 < 0) {
+                        st.g1 = s;
+                        st.g1d = dd;
+                        st.g1s = sd;
+                    }
+                }
+                ++st.nGood;
+            }
+        }
+        ++s;
+    }
+    st.s = s;
+}
+
+// The ordered scan of one pixel's samples by eight lanes. One lane that walks 50 samples waits ~0.4 us for
+// each (a chain of a sample's loads, LUT look-ups and ~130 instructions), 20 us in all, whatever the
+// machine holds beside it; eight lanes take eight samples a step, and the ballot of their verdicts gives the
+// ordered result: the scan stops at the nreq-th good sample, and samples past it count for nothing.
+// A warp has four groups of eight lanes; lane j < m of a group owns an item (want: it has a scan to
+// continue, from st), and the group scans its owners' items in turn. Every lane of the warp calls it. With
+// eight owners a group (m == 8: a list that fills the machine) every lane scans its own item instead: the
+// latency is then hidden by the other warps, and the groups' shuffles and the samples past the stop would
+// cost issue slots (64-stream tick 6.39 ms with groups only, 6.35 ms before).
+// ovMask: samples that earlier pixels overwrite this frame (repair), ovGood: those of them that match now
+// (their distances stay with the owner). REC: also reports the first two good samples.
+template <int C, bool REC>
+__device__ __forceinline__ void coop_scan(const TickParams& P, bool want, int m, int si, int p,
+                                          const uint32_t (&vals)[C][4], const uint32_t (&curr)[C],
+                                          const uint32_t (&intra)[C], const EvalThr& th, uint64_t ovMask,
+                                          uint64_t ovGood, ScanSt& st) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    if (m == 8) {
+        if (want) lane_scan<C, REC>(P.streams[si], p, vals, curr, intra, th, ovMask, ovGood, st);
+        return;
+    }
+    for (int j = 0; j < m; ++j) {
+        const int src = (lane & 24) + j;
+        const bool go = __shfl_sync(kAll, (int)want, src) != 0;
+        if (!__any_sync(kAll, go)) continue;
+        const int bsi = __shfl_sync(kAll, si, src), bp = __shfl_sync(kAll, p, src);
+        uint32_t bv[C][4], bc[C], bi[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bv[c][i] = __shfl_sync(kAll, vals[c][i], src);
+            bc[c] = __shfl_sync(kAll, curr[c], src);
+            bi[c] = __shfl_sync(kAll, intra[c], src);
+        }
+        EvalThr bt;
+        bt.colThr = __shfl_sync(kAll, th.colThr, src);
+        bt.descThr = __shfl_sync(kAll, th.descThr, src);
+        bt.uNew = 0u;
+        int s = __shfl_sync(kAll, st.s, src), ng = __shfl_sync(kAll, st.nGood, src);
+        const uint64_t bm = REC ? 0ull : __shfl_sync(kAll, ovMask, src);
+        const uint64_t bg = REC ? 0ull : __shfl_sync(kAll, ovGood, src);
+        const StreamDev& S = P.streams[go ? bsi : 0];
+        const int N = go ? S.N : 0, nreq = S.nreq;
+        const size_t npx = (size_t)S.npx;
+        const uint8_t* lut = S.ctl->lut;
+        const uint64_t* d3 = (const uint64_t*)S.sD + bp;
+        const uint16_t* d1 = (const uint16_t*)S.sD + bp;
+        const uint8_t* sc = S.sC + bp;
+        int k = s + sub;
+        uint64_t d = 0;
+        uint32_t c2 = 0;
+        if (k < N) {
+            d = C == 3 ? d3[(size_t)k * npx] : (uint64_t)d1[(size_t)k * npx];
+            c2 = sc[(size_t)k * npx];
+        }
+        uint32_t mins = 0xffffffffu;  // descriptor minimum | summed minimum, 16 bits each
+        uint32_t first = 0xffffffffu, second = 0xffffffffu;  // this lane's good samples: index, distances
+        while (__any_sync(kAll, ng < nreq && s < N)) {
+            const bool act = ng < nreq && s < N;
+            uint64_t dn = 0;
+            uint32_t cn = 0;
+            if (act && k + 8 < N) {
+                dn = C == 3 ? d3[(size_t)(k + 8) * npx] : (uint64_t)d1[(size_t)(k + 8) * npx];
+                cn = sc[(size_t)(k + 8) * npx];
+            }
+            uint32_t dd = 0, sd = 0;
+            const bool good = act && k < N && (REC || !((bm >> k) & 1ull)) &&
+                              sample_match<C>(lut, bv, bc, bi, bt, d, c2, dd, sd);
+            uint32_t b = (__ballot_sync(kAll, good) >> (lane & 24)) & 0xffu;
+            if (act) {
+                if (!REC) b |= (uint32_t)(bg >> s) & 0xffu;
+                const int need = nreq - ng, cnt = __popc(b);
+                int stop = min(8, N - s);
+                if (cnt >= need) {
+                    uint32_t t = b;
+                    for (int i = 1; i < need; ++i) t &= t - 1u;
+                    stop = __ffs(t);
+                    ng = nreq;
+                } else {
+                    ng += cnt;
+                }
+                if (good && sub < stop) {
+                    mins = __vminu2(mins, (dd << 16) | sd);
+                    if (REC) {
+                        const uint32_t key = ((uint32_t)k << 24) | (dd << 16) | sd;
+                        if (first == 0xffffffffu) first = key;
+                        else if (second == 0xffffffffu) second = key;
+                    }
+                }
+                s += stop;
+            }
+            d = dn;
+            c2 = cn;
+            k += 8;
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) mins = __vminu2(mins, __shfl_xor_sync(kAll, mins, o));
+        uint32_t k0 = 0xffffffffu, k1 = 0xffffffffu;
+        if (REC) {
+            k0 = first;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) k0 = min(k0, __shfl_xor_sync(kAll, k0, o));
+            k1 = first == k0 ? second : first;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) k1 = min(k1, __shfl_xor_sync(kAll, k1, o));
+        }
+        if (go && sub == j) {
+            st.s = s;
+            st.nGood = ng;
+            st.minDesc = min(st.minDesc, mins >> 16);
+            st.minSum = min(st.minSum, mins & 0xffffu);
+            if (REC) {
+                if (st.g0 < 0 && k0 != 0xffffffffu) {
+                    st.g0 = (int)(k0 >> 24);
+                    st.g0d = (k0 >> 16) & 0xffu;
+                    st.g0s = k0 & 0xffffu;
+                    k0 = k1;
+                }
+                if (st.g0 >= 0 && st.g1 < 0 && k0 != 0xffffffffu) {
+                    st.g1 = (int)(k0 >> 24);
+                    st.g1d = (k0 >> 16) & 0xffu;
+                    st.g1s = k0 & 0xffffu;
+                }
+            }
+        }
+    }
+}
+// Items of a list that one group of eight lanes owns at a time: one while the machine has a group for
+// every item, up to four, then eight (every lane owns one and scans it alone). Re-match round 0 with all
+// groups / lanes alone from 5 / from 3 on: 24,000 items (three a group) 46 / 46 / 52 us, 42,000 (five)
+// 75 / 70 / 70 us, 122,000 on a quarter of the machine 321 / 231 / 231 us.
+__device__ __forceinline__ int coop_share(unsigned int n, unsigned int ctas) {
+    const unsigned int groups = ctas * (blockDim.x >> 5) * 4u;
+    const unsigned int m = (n + groups - 1u) / groups;
+    return m > 4u ? 8 : (int)max(1u, m);
 }
 
 // the rest of one evaluation after the sample scan (:254-330 / :396-481): D_last, D_min, the raw
@@ -549,19 +712,6 @@ __device__ uint32_t eval_tail(const StreamDev& S, const FrameK& F, int x, int y,
         __stcg(&ldn[c], (uint16_t)intra[c]);
     }
     return intent;
-}
-
-// a full evaluation: thresholds, the whole ordered scan, the tail (the repair's re-match)
-template <int C, bool OVR>
-__device__ uint32_t eval_pixel(const StreamDev& S, const FrameK& F, const uint8_t* __restrict__ lut, int x, int y,
-                               int p, const PixIn<C>& in, const uint32_t (&vals)[C][4], const uint32_t (&curr)[C],
-                               const uint32_t (&intra)[C], const Ovr* ov, int nov, uint64_t ovmask, int& e_out) {
-    const EvalThr th = eval_thresholds(S, in.R, in.RwLT, in.RwST, in.FnLT, in.FnST, in.uOld);
-    ScanSt st;
-    scan_init<C>(st);
-    scan_samples<C, OVR>(S, lut, p, vals, curr, intra, th, ov, nov, ovmask, S.N, in.d0, in.c0, in.d1, in.c1, st);
-    e_out = st.s;
-    return eval_tail<C>(S, F, x, y, p, in, curr, intra, th.uNew, st);
 }
 
 // non-zero LBSP descriptor test of the frame-level statistics (:264-265 / :405-407)
@@ -743,10 +893,7 @@ __device__ void phaseA_tile(const TickParams& P, int si, const StreamDev& S, int
             const EvalThr th = eval_thresholds(S, tR, tRwLT, tRwST, tFnLT, tFnST, tU);
             ScanSt st;
             scan_init<C>(st);
-            // the first good sample's index is tracked (the long-scan record keeps it), not the distances
-            // of the first two good samples (only a scan that ends unsettled records them)
-            scan_samples<C, false, false>(S, lut, p, vals, curr, intra, th, nullptr, 0, 0ull, kScanCap, d0, c0, d1,
-                                          c1, st);
+            scan_samples<C>(S, lut, p, vals, curr, intra, th, d0, c0, d1, c1, st);
             if (st.nGood < S.nreq) {
                 // a long scan, or a scan that ended unsettled within the cap (N <= kScanCap): continued,
                 // recorded and finished by lvbgs_k_longscan over the compacted list, so that its warps
@@ -928,28 +1075,74 @@ __device__ void ds_item(const StreamDev& S, int i) {
     if (dmax) atomicAdd(&S.ctl->colordiff_acc, (unsigned long long)dmax);
 }
 
+// Place of the length of round i's list: the lists themselves alternate, but a round without re-resolutions
+// ends in one barrier, so the length that a round resets (that of round i + 2) must not be one that a CTA
+// may still read: three places rotate after round 0's.
+__device__ __forceinline__ int dcount_slot(int i) { return i == 0 ? 0 : 1 + (i - 1) % 3; }
+
 // ------------------------------------------------------------------------------------------
 // repair loop bodies
 // ------------------------------------------------------------------------------------------
+// Re-matches the items of a warp's owner lanes (own: this lane holds pixel q of stream si; every lane of
+// the warp calls it): the scan of q's samples with those that earlier pixels overwrite this frame, the tail
+// of its evaluation, and the list entries that follow from a changed decision.
 template <int C>
-__device__ bool rematch_item(const TickParams& P, int si, const StreamDev& S, int q, uint32_t stampNext,
-                             int iterParity) {
+__device__ bool rematch_items(const TickParams& P, bool own, int m, int si, int q, uint32_t stampNext, int iter) {
+    const StreamDev& S = P.streams[si];
     const int W = S.W, x = q % W, y = q / W;
     const FrameK F = frame_consts(S);
-    const uint32_t wOld = __ldcg(&S.intent[q]);
-    if (!(wOld & kInValid)) return false;
-    // overrides: earlier pixels of the 5x5 window whose neighbour update targets q, raster order
+    const uint32_t wOld = own ? __ldcg(&S.intent[q]) : 0u;
+    own = own && (wOld & kInValid);
+    // overrides: earlier pixels of the 5x5 window whose neighbour update targets q, raster order. All
+    // twelve intents are requested before any is looked at.
     Ovr ov[12];
     int nov = 0;
-    uint64_t mask = 0;
-    for (int dy = -2; dy <= 0; ++dy)
-        for (int dx = -2; dx <= 2; ++dx) {
-            if (dy == 0 && dx >= 0) break;
+    uint64_t mask = 0, good = 0;
+    uint32_t vals[C][4], curr[C], intra[C];
+    PixIn<C> in;
+    EvalThr th;
+    ScanSt st;
+    scan_init<C>(st);
+    th.colThr = th.descThr = th.uNew = 0u;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        curr[c] = intra[c] = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) vals[c][j] = 0u;
+    }
+    bool scan = own;
+    if (own) {
+        uint32_t wn[12];
+#pragma unroll
+        for (int j = 0; j < 12; ++j) {
+            const int dy = j / 5 - 2, dx = j % 5 - 2;
             const int px = x + dx, py = y + dy;
-            if (px < 0 || px >= W || py < 0) continue;
-            const int p = py * W + px;
-            const uint32_t w = __ldcg(&S.intent[p]);
-            if (!in_nb_writes(w) || (int)in_code(w) != (-dy + 2) * 5 + (-dx + 2)) continue;
+            wn[j] = (px >= 0 && px < W && py >= 0) ? __ldcg(&S.intent[py * W + px]) : 0u;
+        }
+        const uint4 gr = S.nreq <= 2 ? __ldcg(&S.goodRec[q]) : make_uint4(0u, 0u, 0u, 0u);
+        const uint8_t* base = S.frame + (size_t)q * C;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t wv = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int n = j * 4 + i;
+                    wv |= (uint32_t)__ldg(base + (c_lbsp_dy[n] * W + c_lbsp_dx[n]) * C + c) << (8 * i);
+                }
+                vals[c][j] = wv;
+            }
+            curr[c] = __ldg(base + c);
+        }
+        load_pix<C>(S, F, q, in);
+        th = eval_thresholds(S, in.R, in.RwLT, in.RwST, in.FnLT, in.FnST, in.uOld);
+#pragma unroll
+        for (int c = 0; c < C; ++c) intra[c] = lbsp_thr(vals[c], curr[c], S.ctl->lut[curr[c]]);
+        for (int j = 0; j < 12; ++j) {
+            const uint32_t w = wn[j];
+            if (!in_nb_writes(w) || (int)in_code(w) != 24 - j) continue;
+            const int p = (y + j / 5 - 2) * W + x + j % 5 - 2;
             const int sn = (int)in_snb(w);
             uint32_t col = 0;
             uint64_t desc = 0;
@@ -966,58 +1159,10 @@ __device__ bool rematch_item(const TickParams& P, int si, const StreamDev& S, in
             ov[k].desc = desc;
             mask |= 1ull << sn;
         }
-    // order matters only within one sample index (last writer wins); entries with distinct s are
-    // independent, and an overwritten entry keeps its slot but takes the latest writer's values
-    uint32_t vals[C][4], curr[C], intra[C];
-    const uint8_t* base = S.frame + (size_t)q * C;
-    for (int c = 0; c < C; ++c) {
-        for (int j = 0; j < 4; ++j) {
-            uint32_t wv = 0;
-            for (int i = 0; i < 4; ++i) {
-                const int n = j * 4 + i;
-                wv |= (uint32_t)__ldg(base + (c_lbsp_dy[n] * W + c_lbsp_dx[n]) * C + c) << (8 * i);
-            }
-            vals[c][j] = wv;
-        }
-        curr[c] = __ldg(base + c);
-        intra[c] = lbsp_thr(vals[c], curr[c], S.ctl->lut[curr[c]]);
-    }
-    int e = 0;
-    PixIn<C> in;
-    load_pix<C>(S, F, q, in);
-    uint32_t wNew;
-    const uint4 gr = S.nreq <= 2 ? __ldcg(&S.goodRec[q]) : make_uint4(0u, 0u, 0u, 0u);
-    if (S.nreq <= 2 && gr.x == F.frame) {
-        // q's frame-start scan is recorded: up to its stop eA, its good samples are the recorded ones
-        // not overwritten and the overwritten ones that match now. The ordered scan over them stops
-        // at the nreq-th good index, with minima over the good samples up to there; with fewer, it
-        // goes on from eA (with the overwrites) as a scan from the start would.
-        const EvalThr th = eval_thresholds(S, in.R, in.RwLT, in.RwST, in.FnLT, in.FnST, in.uOld);
-        const int eA = (int)(gr.y & 255u), nA = (int)((gr.y >> 8) & 255u);
-        int gi[2] = {S.N, S.N};  // the two smallest good indices
-        uint32_t gd[2] = {0u, 0u}, gs[2] = {0u, 0u};
-        int cnt = 0;
-        auto add = [&](int idx, uint32_t dd, uint32_t sd) {
-            ++cnt;
-            if (idx < gi[0]) {
-                gi[1] = gi[0];
-                gd[1] = gd[0];
-                gs[1] = gs[0];
-                gi[0] = idx;
-                gd[0] = dd;
-                gs[0] = sd;
-            } else if (idx < gi[1]) {
-                gi[1] = idx;
-                gd[1] = dd;
-                gs[1] = sd;
-            }
-        };
-        for (int j = 0; j < nA; ++j) {
-            const int g = (int)((gr.y >> (16 + 8 * j)) & 255u);
-            if (!((mask >> g) & 1ull)) add(g, (j ? gr.z >> 16 : gr.z) & 0xffffu, (j ? gr.w >> 16 : gr.w) & 0xffffu);
-        }
+        // order matters only within one sample index (last writer wins); entries with distinct s are
+        // independent, and an overwritten entry keeps its slot but takes the latest writer's values.
+        // The overwritten samples that match now: their entries keep the distances (col, desc)
         for (int k = 0; k < nov; ++k) {
-            if (ov[k].s >= eA) continue;
             uint64_t d;
             uint32_t c2;
             if (C == 3) {
@@ -1028,39 +1173,64 @@ __device__ bool rematch_item(const TickParams& P, int si, const StreamDev& S, in
                 c2 = ov[k].col & 0xffu;
             }
             uint32_t dd, sd;
-            if (sample_match<C>(S.ctl->lut, vals, curr, intra, th, d, c2, dd, sd)) add(ov[k].s, dd, sd);
-        }
-        ScanSt st;
-        scan_init<C>(st);
-        const int take = cnt < S.nreq ? cnt : S.nreq;
-        for (int j = 0; j < take; ++j) {
-            if (st.minDesc > gd[j]) st.minDesc = gd[j];
-            if (st.minSum > gs[j]) st.minSum = gs[j];
-        }
-        st.nGood = take;
-        if (cnt >= S.nreq) {
-            st.s = gi[S.nreq - 1] + 1;
-        } else {
-            st.s = eA;
-            if (eA < S.N) {
-                const int npx = S.npx;
-                uint64_t dA = 0, dB = 0;
-                uint32_t cA = 0, cB = 0;
-                dA = C == 3 ? ((const uint64_t*)S.sD)[(size_t)eA * npx + q] : (uint64_t)((const uint16_t*)S.sD)[(size_t)eA * npx + q];
-                cA = S.sC[(size_t)eA * npx + q];
-                if (eA + 1 < S.N) {
-                    dB = C == 3 ? ((const uint64_t*)S.sD)[(size_t)(eA + 1) * npx + q]
-                                : (uint64_t)((const uint16_t*)S.sD)[(size_t)(eA + 1) * npx + q];
-                    cB = S.sC[(size_t)(eA + 1) * npx + q];
-                }
-                scan_samples<C, true>(S, S.ctl->lut, q, vals, curr, intra, th, ov, nov, mask, S.N, dA, cA, dB, cB, st);
+            if (sample_match<C>(S.ctl->lut, vals, curr, intra, th, d, c2, dd, sd)) {
+                good |= 1ull << ov[k].s;
+                ov[k].col = dd;
+                ov[k].desc = sd;
             }
         }
-        e = st.s;
-        wNew = eval_tail<C>(S, F, x, y, q, in, curr, intra, th.uNew, st);
-    } else {
-        wNew = eval_pixel<C, true>(S, F, S.ctl->lut, x, y, q, in, vals, curr, intra, ov, nov, mask, e);
+        if (S.nreq <= 2 && gr.x == F.frame) {
+            // q's frame-start scan is recorded: up to its stop eA, its good samples are the recorded ones
+            // not overwritten and the overwritten ones that match now. The ordered scan over them stops
+            // at the nreq-th good index, with minima over the good samples up to there; with fewer, it
+            // goes on from eA (with the overwrites) as a scan from the start would.
+            const int eA = (int)(gr.y & 255u), nA = (int)((gr.y >> 8) & 255u);
+            int gi[2] = {S.N, S.N};  // the two smallest good indices
+            uint32_t gd[2] = {0u, 0u}, gs[2] = {0u, 0u};
+            int cnt = 0;
+            auto add = [&](int idx, uint32_t dd, uint32_t sd) {
+                ++cnt;
+                if (idx < gi[0]) {
+                    gi[1] = gi[0];
+                    gd[1] = gd[0];
+                    gs[1] = gs[0];
+                    gi[0] = idx;
+                    gd[0] = dd;
+                    gs[0] = sd;
+                } else if (idx < gi[1]) {
+                    gi[1] = idx;
+                    gd[1] = dd;
+                    gs[1] = sd;
+                }
+            };
+            for (int j = 0; j < nA; ++j) {
+                const int g = (int)((gr.y >> (16 + 8 * j)) & 255u);
+                if (!((mask >> g) & 1ull)) add(g, (j ? gr.z >> 16 : gr.z) & 0xffffu, (j ? gr.w >> 16 : gr.w) & 0xffffu);
+            }
+            for (int k = 0; k < nov; ++k)
+                if (ov[k].s < eA && ((good >> ov[k].s) & 1ull)) add(ov[k].s, ov[k].col, (uint32_t)ov[k].desc);
+            const int take = cnt < S.nreq ? cnt : S.nreq;
+            for (int j = 0; j < take; ++j) {
+                if (st.minDesc > gd[j]) st.minDesc = gd[j];
+                if (st.minSum > gs[j]) st.minSum = gs[j];
+            }
+            st.nGood = take;
+            st.s = cnt >= S.nreq ? gi[S.nreq > 0 ? S.nreq - 1 : 0] + 1 : eA;
+            scan = cnt < S.nreq && eA < S.N;
+        }
     }
+    const int s0 = st.s;
+    coop_scan<C, false>(P, scan, m, si, q, vals, curr, intra, th, mask, good, st);
+    if (!own) return false;
+    // the overwritten samples that the scan counted
+    if (scan)
+        for (int k = 0; k < nov; ++k)
+            if (ov[k].s >= s0 && ov[k].s < st.s && ((good >> ov[k].s) & 1ull)) {
+                st.minDesc = min(st.minDesc, ov[k].col);
+                st.minSum = min(st.minSum, (uint32_t)ov[k].desc);
+            }
+    const int e = st.s;
+    uint32_t wNew = eval_tail<C>(S, F, x, y, q, in, curr, intra, th.uNew, st);
     const bool decChanged = ((wNew ^ wOld) & kInFG) != 0u;
     if (!decChanged) {
         // same decision: same draws, same updates; keep the resolved neighbour state
@@ -1069,8 +1239,8 @@ __device__ bool rematch_item(const TickParams& P, int si, const StreamDev& S, in
         return true;
     }
     __stcg(&S.intent[q], wNew);
-    unsigned int* dcnt = &P.work->dcount[iterParity ^ 1];
-    unsigned long long* dl = P.dlist[iterParity ^ 1];
+    unsigned int* dcnt = &P.work->dcount[dcount_slot(iter + 1)];
+    unsigned long long* dl = P.dlist[(iter & 1) ^ 1];
     // the write that disappeared or appeared changes what its (later) target reads
     if (in_nb_writes(wOld)) {
         const int t = code_target((int)in_code(wOld), x, y, W);
@@ -1082,25 +1252,24 @@ __device__ bool rematch_item(const TickParams& P, int si, const StreamDev& S, in
     }
     // the raw-segmentation value of q changed: re-resolve ghost tests that read it (q itself and
     // later pixels of its 5x5 window), and q's own new pending test
-    unsigned long long* rl = P.rlist[iterParity];
-    unsigned int* rcnt = &P.work->rcount[iterParity];
+    unsigned long long* rl = P.rlist[iter & 1];
+    unsigned int* rcnt = &P.work->rcount[iter & 1];
     const uint32_t rstamp = stampNext;  // separate stamp array: one generation per iteration
-    for (int dy = 0; dy <= 2; ++dy)
-        for (int dx = -2; dx <= 2; ++dx) {
-            if (dy == 0 && dx < 0) continue;
-            const int px = x + dx, py = y + dy;
-            if (px < 0 || px >= W || py >= S.H) continue;
-            const int p = py * W + px;
-            const uint32_t w = (p == q) ? wNew : __ldcg(&S.intent[p]);
-            if (in_ghost(w) && code_target((int)in_code(w), px, py, W) == q)
-                push_item(rl, rcnt, P.listCap, S.stampR, rstamp, si, p, P.work);
-        }
+    uint32_t wl[13];  // q and the later pixels of its window, requested together
+#pragma unroll
+    for (int j = 0; j < 13; ++j) {
+        const int px = x + (j + 12) % 5 - 2, py = y + (j + 12) / 5 - 2;
+        wl[j] = j == 0 ? wNew : (px >= 0 && px < W && py < S.H) ? __ldcg(&S.intent[py * W + px]) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 13; ++j)  // window slot 12 + j targets q with code 24 - (12 + j)
+        if (in_ghost(wl[j]) && (int)in_code(wl[j]) == 12 - j)
+            push_item(rl, rcnt, P.listCap, S.stampR, rstamp, si, (y + (j + 12) / 5 - 2) * W + x + (j + 12) % 5 - 2, P.work);
     if (in_nst(wNew) == NB_PENDING) push_item(rl, rcnt, P.listCap, S.stampR, rstamp, si, q, P.work);
     return true;
 }
 
-__device__ void reresolve_item(const TickParams& P, int si, const StreamDev& S, int p, uint32_t stampNext,
-                               int iterParity) {
+__device__ void reresolve_item(const TickParams& P, int si, const StreamDev& S, int p, uint32_t stampNext, int iter) {
     const int W = S.W, x = p % W, y = p / W;
     const uint32_t w = __ldcg(&S.intent[p]);
     if (!in_ghost(w)) return;
@@ -1113,8 +1282,7 @@ __device__ void reresolve_item(const TickParams& P, int si, const StreamDev& S, 
     // readers during the last re-match pass saw PENDING as "no write"
     const bool wroteBefore = old == NB_GHOST_WRITE, writesNow = st == NB_GHOST_WRITE;
     if (wroteBefore != writesNow && q > p)
-        push_item(P.dlist[iterParity ^ 1], &P.work->dcount[iterParity ^ 1], P.listCap, S.stampD, stampNext, si, q,
-                  P.work);
+        push_item(P.dlist[(iter & 1) ^ 1], &P.work->dcount[dcount_slot(iter + 1)], P.listCap, S.stampD, stampNext, si, q, P.work);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1833,13 +2001,11 @@ extern "C" __global__ void __launch_bounds__(kThreads, 5) lvbgs_k_eval(TickParam
 // keep whole warps of the evaluation waiting on a few lanes.
 // ------------------------------------------------------------------------------------------
 template <int C>
-__device__ void longscan_item(const TickParams& P, unsigned int i) {
-    const unsigned long long key = __ldcg(&P.rlist[0][i]);
-    const unsigned long long sw = __ldcg(&P.rlist[1][i]);
-    const int si = (int)(key >> 40), p = (int)(key & 0xffffffffffull);
+__device__ void longscan_items(const TickParams& P, bool own, int m, unsigned long long key, unsigned long long sw) {
+    const int si = own ? (int)(key >> 40) : 0, p = own ? (int)(key & 0xffffffffffull) : 0;
     const StreamDev& S = P.streams[si];
     const FrameK F = frame_consts(S);
-    const int W = S.W, x = p % W, y = p / W, npx = S.npx, N = S.N;
+    const int W = S.W, x = p % W, y = p / W, npx = S.npx;
     ScanSt st;
     st.s = (int)(sw & 0xffu);
     st.nGood = (int)((sw >> 8) & 0xffu);
@@ -1852,37 +2018,34 @@ __device__ void longscan_item(const TickParams& P, unsigned int i) {
     st.g0s = st.minSum;
     st.g1 = -1;
     st.g1d = st.g1s = 0;
-    // samples s and s+1 with the feedback maps
-    uint64_t dA = 0, dB = 0;
-    uint32_t cA = 0, cB = 0;
-    if (st.s < N) {
-        dA = C == 3 ? ((const uint64_t*)S.sD)[(size_t)st.s * npx + p] : (uint64_t)((const uint16_t*)S.sD)[(size_t)st.s * npx + p];
-        cA = S.sC[(size_t)st.s * npx + p];
-    }
-    if (st.s + 1 < N) {
-        dB = C == 3 ? ((const uint64_t*)S.sD)[(size_t)(st.s + 1) * npx + p]
-                    : (uint64_t)((const uint16_t*)S.sD)[(size_t)(st.s + 1) * npx + p];
-        cB = S.sC[(size_t)(st.s + 1) * npx + p];
-    }
-    // the scan needs the thresholds only; the feedback maps of the tail are loaded after it, which
-    // keeps the register peak (and so the occupancy) of this latency-bound kernel down
-    const float* fc = S.fm + (size_t)F.cur * kNumFloatMaps * npx;
-    const EvalThr th = eval_thresholds(S, fc[FM_R * npx + p], fc[FM_RAW_LT * npx + p], fc[FM_RAW_ST * npx + p],
-                                       fc[FM_FIN_LT * npx + p], fc[FM_FIN_ST * npx + p],
-                                       S.unst[(size_t)F.cur * npx + p]);
+    EvalThr th;
+    th.colThr = th.descThr = th.uNew = 0u;
     uint32_t curr[C], intra[C];
     {
         uint32_t vals[C][4];
-        const uint8_t* base = S.frame + (size_t)p * C;
-        const uint8_t* lut = S.ctl->lut;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            gather_taps<C>(base, W * C, c, vals[c]);
-            curr[c] = __ldg(base + c);
-            intra[c] = lbsp_thr(vals[c], curr[c], lut[curr[c]]);
+            curr[c] = intra[c] = 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) vals[c][j] = 0u;
         }
-        scan_samples<C, false>(S, lut, p, vals, curr, intra, th, nullptr, 0, 0ull, N, dA, cA, dB, cB, st);
+        if (own) {
+            // the scan needs the thresholds only; the feedback maps of the tail are loaded after it
+            const float* fc = S.fm + (size_t)F.cur * kNumFloatMaps * npx;
+            th = eval_thresholds(S, fc[FM_R * npx + p], fc[FM_RAW_LT * npx + p], fc[FM_RAW_ST * npx + p],
+                                 fc[FM_FIN_LT * npx + p], fc[FM_FIN_ST * npx + p], S.unst[(size_t)F.cur * npx + p]);
+            const uint8_t* base = S.frame + (size_t)p * C;
+            const uint8_t* lut = S.ctl->lut;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                gather_taps<C>(base, W * C, c, vals[c]);
+                curr[c] = __ldg(base + c);
+                intra[c] = lbsp_thr(vals[c], curr[c], lut[curr[c]]);
+            }
+        }
+        coop_scan<C, true>(P, own, m, si, p, vals, curr, intra, th, 0ull, 0ull, st);
     }
+    if (!own) return;
     record_scan(S, F, p, st);
     PixIn<C> in;
     load_pix<C>(S, F, p, in);
@@ -1891,10 +2054,16 @@ __device__ void longscan_item(const TickParams& P, unsigned int i) {
 
 extern "C" __global__ void __launch_bounds__(256, 3) lvbgs_k_longscan(TickParams P) {
     const unsigned int n = min(ld_volatile(&P.work->lcount), P.listCap);
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int si = (int)(__ldcg(&P.rlist[0][i]) >> 40);
-        if (P.streams[si].C == 3) longscan_item<3>(P, i);
-        else longscan_item<1>(P, i);
+    const int m = coop_share(n, gridDim.x), lane = threadIdx.x & 31, sub = lane & 7;
+    const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const unsigned int step = gridDim.x * (blockDim.x >> 5) * 4u * m;
+    for (unsigned int base = warp * 4u * m; base < n; base += step) {
+        const unsigned int i = base + (unsigned)(lane >> 3) * m + sub;
+        const bool own = sub < m && i < n;
+        const unsigned long long key = own ? __ldcg(&P.rlist[0][i]) : 0ull, sw = own ? __ldcg(&P.rlist[1][i]) : 0ull;
+        const bool c3 = own && P.streams[(int)(key >> 40)].C == 3;
+        if (__any_sync(0xffffffffu, c3)) longscan_items<3>(P, c3, m, key, sw);
+        if (__any_sync(0xffffffffu, own && !c3)) longscan_items<1>(P, own && !c3, m, key, sw);
     }
 }
 
@@ -1916,20 +2085,29 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParam
     ds_item(P.streams[lo], (int)(i - dsBase[lo]));
 }
 
-// repair to the raster-order fixed point (cooperative launch: all CTAs resident)
-extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_repair(TickParams P) {
+// Repair to the raster-order fixed point (cooperative launch: all CTAs resident). Every round re-matches
+// the listed pixels (M), then re-resolves the ghost tests that read a changed one (R). Most rounds change
+// no decision, so R has nothing to do and its barrier is left out. Only as many CTAs take part as the first
+// list has work for (later lists are shorter): a barrier over 28 CTAs costs a third of one over 304.
+extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickParams P) {
     TickWork* w = P.work;
     if (blockIdx.x == 0 && threadIdx.x == 0 && w->nts < 40u) w->ts[w->nts++] = gtimer();  // phase profile
     if (P.dbgFault == LVBGS_FAULT_BARRIER_TIMEOUT) {
         // injected fault: every CTA but CTA 0 waits at a barrier CTA 0 never reaches; each wait gives
         // up after P.barrierNs and records ERR_BARRIER_TIMEOUT, and every CTA returns
-        if (blockIdx.x != 0) grid_sync(w, P.barrierNs);
+        if (blockIdx.x != 0) grid_sync(w, gridDim.x, P.barrierNs);
         return;
     }
+    const int lane = threadIdx.x & 31;
+    // the CTAs of this repair: a group of eight lanes for every item of the first list (whose length stays
+    // as it is while the kernel runs, so that a CTA that starts late decides alike)
+    const unsigned int n0 = ld_volatile(&w->dcount[0]);
+    const unsigned int ctas = min(gridDim.x, max(1u, (n0 + 31u) / 32u));
+    if (blockIdx.x >= ctas) return;
     int iter = 0;
     for (;;) {
         const int par = iter & 1;
-        const unsigned int n = ld_volatile(&w->dcount[par]);
+        const unsigned int n = ld_volatile(&w->dcount[dcount_slot(iter)]);
         if (n == 0u) break;
         if (iter >= P.maxRepairIters) {
             if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&w->err, ERR_REPAIR_LIMIT);
@@ -1938,55 +2116,54 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_repair(TickParams
         const unsigned int nItems = n < P.listCap ? n : P.listCap;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             w->rcount[par ^ 1] = 0u;
+            w->dcount[dcount_slot(iter + 2)] = 0u;
+            w->fetchD[par ^ 1] = 0u;
+            w->fetchR[par ^ 1] = 0u;
             w->rematched += nItems;
             if (iter < 16) w->phase_ctr[iter] = nItems;
         }
-        // items are fetched 32 at a time by each warp from a counter (not strided): per-item costs
-        // vary widely, and every round waits for its slowest thread at the grid barrier
-        const int lane = threadIdx.x & 31;
+        // items are fetched by each warp from a counter (not strided): per-item costs vary widely, and
+        // every round waits for its slowest warp at the barrier. A fetch is 4 items (one for each
+        // group of eight lanes) while there is a group for every item, up to 32.
+        const int m = coop_share(nItems, ctas);
         for (;;) {
             unsigned int base = 0;
-            if (lane == 0) base = atomicAdd(&w->fetchD[par], 32u);
+            if (lane == 0) base = atomicAdd(&w->fetchD[par], 4u * m);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (base >= nItems) break;
-            const unsigned int i = base + lane;
-            if (i < nItems) {
-                const unsigned long long item = __ldcg(&P.dlist[par][i]);
-                const int si = (int)(item >> 40), q = (int)(item & 0xffffffffffull);
-                const StreamDev& S = P.streams[si];
-                const uint32_t stampNext = S.ctl->stamp_base + (uint32_t)iter + 2u;
-                const bool counted = S.C == 3 ? rematch_item<3>(P, si, S, q, stampNext, par)
-                                              : rematch_item<1>(P, si, S, q, stampNext, par);
-                // re-match statistics: one atomic per stream among the lanes here
-                const unsigned am = __activemask();
-                const unsigned grp = __match_any_sync(am, counted ? si : -1 - (int)(threadIdx.x & 31));
-                if (counted && (int)(threadIdx.x & 31) == __ffs(grp) - 1)
-                    atomicAdd(&S.ctl->st_rematched, (unsigned long long)__popc(grp));
-            }
+            const unsigned int i = base + (unsigned)(lane >> 3) * m + (lane & 7);
+            const bool own = (lane & 7) < m && i < nItems;
+            const unsigned long long item = own ? __ldcg(&P.dlist[par][i]) : 0ull;
+            const int si = (int)(item >> 40), q = (int)(item & 0xffffffffffull);
+            const StreamDev& S = P.streams[si];
+            const bool c3 = own && S.C == 3;
+            const uint32_t stampNext = S.ctl->stamp_base + (uint32_t)iter + 2u;
+            bool counted = false;
+            if (__any_sync(0xffffffffu, c3)) counted = rematch_items<3>(P, c3, m, si, q, stampNext, iter);
+            if (__any_sync(0xffffffffu, own && !c3)) counted |= rematch_items<1>(P, own && !c3, m, si, q, stampNext, iter);
+            // re-match statistics: one atomic per stream among the lanes here
+            const unsigned grp = __match_any_sync(0xffffffffu, counted ? si : -1 - lane);
+            if (counted && lane == __ffs(grp) - 1) atomicAdd(&S.ctl->st_rematched, (unsigned long long)__popc(grp));
         }
-        if (!grid_sync(w, P.barrierNs)) return;
+        if (!grid_sync(w, ctas, P.barrierNs)) return;
         const unsigned int nr0 = ld_volatile(&w->rcount[par]);
         const unsigned int nr = nr0 < P.listCap ? nr0 : P.listCap;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            w->dcount[par] = 0u;
-            // the next round's counters (last used a round ago; visible after the next barrier)
-            w->fetchD[par ^ 1] = 0u;
-            w->fetchR[par ^ 1] = 0u;
-        }
-        for (;;) {
-            unsigned int base = 0;
-            if (lane == 0) base = atomicAdd(&w->fetchR[par], 32u);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= nr) break;
-            const unsigned int i = base + lane;
-            if (i < nr) {
-                const unsigned long long item = __ldcg(&P.rlist[par][i]);
-                const int si = (int)(item >> 40), p = (int)(item & 0xffffffffffull);
-                const StreamDev& S = P.streams[si];
-                reresolve_item(P, si, S, p, S.ctl->stamp_base + (uint32_t)iter + 2u, par);
+        if (nr != 0u) {  // the same value in every CTA: rcount[par] is reset only in the next round, from 0
+            for (;;) {
+                unsigned int base = 0;
+                if (lane == 0) base = atomicAdd(&w->fetchR[par], 32u);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (base >= nr) break;
+                const unsigned int i = base + lane;
+                if (i < nr) {
+                    const unsigned long long item = __ldcg(&P.rlist[par][i]);
+                    const int si = (int)(item >> 40), p = (int)(item & 0xffffffffffull);
+                    const StreamDev& S = P.streams[si];
+                    reresolve_item(P, si, S, p, S.ctl->stamp_base + (uint32_t)iter + 2u, iter);
+                }
             }
+            if (!grid_sync(w, ctas, P.barrierNs)) return;
         }
-        if (!grid_sync(w, P.barrierNs)) return;
         ++iter;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) w->iters = (unsigned)iter;

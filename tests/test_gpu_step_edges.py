@@ -36,3 +36,16 @@ def test_post_processing_at_word_tile_and_chunk_edges(W, H, k, channels):
     """Hole filling over rows of one word up to three 32-word chunks, every median width class (window counts
     of four and of five bit planes), frames that end inside a word, a tile and a quad of pixels."""
     run_pair(hollow_frames(W, H, channels, 7, W * 31 + H), seed=W, nDefaultMedianBlurKernelSize=k)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("N,nreq", [(1, 1), (5, 2), (8, 3), (9, 2), (17, 1), (50, 4), (64, 2), (50, 0)])
+def test_ordered_scans_by_groups_and_by_lanes(N, nreq, channels):
+    """Sample counts around the evaluation's cap and the groups' steps of eight, and one to four required
+    matches: the scans' stops and minima, with dense overwrites (learning rate 1) and foreground shares from
+    a few pixels (one item a group) to most of the frame (every lane its own)."""
+    frames = hollow_frames(96, 64, channels, 9, 100 * N + nreq)
+    rng = np.random.default_rng(N)
+    frames[5] = rng.integers(0, 256, frames[5].shape, dtype=np.uint8)
+    lrs = [1.0 if t in (2, 3, 4, 6, 7) else 0.0 for t in range(len(frames))]
+    run_pair(frames, seed=nreq + 3, lrs=lrs, nBGSamples=N, nRequiredBGSamples=nreq)
