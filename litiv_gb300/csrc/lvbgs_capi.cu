@@ -22,7 +22,7 @@
 namespace lvbgs {
 extern "C" __global__ void lvbgs_k_eval(TickParams P);
 extern "C" __global__ void lvbgs_k_longscan(TickParams P);
-extern "C" __global__ void lvbgs_k_resolve(TickParams P, unsigned long long dsTotal, const unsigned long long* dsBase);
+extern "C" __global__ void lvbgs_k_resolve(TickParams P, unsigned long long dsTotal);
 extern "C" __global__ void lvbgs_k_repair(TickParams P);
 extern "C" __global__ void lvbgs_k_commit(TickParams P);
 extern "C" __global__ void lvbgs_k_unite(TickParams P);
@@ -102,13 +102,12 @@ size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 struct Workspace {
     TickWork* work = nullptr;
     StreamDev* d_streams = nullptr;
-    unsigned long long* d_dsBase = nullptr;
+    unsigned int* h_err = nullptr;        // page-locked: error flags of the last completed tick
     unsigned long long* lists = nullptr;  // 4 lists of `cap` entries
     size_t cap = 0;
     int nStreamsCap = 0;
     int repairDiv = 1;  // the repair kernel's cooperative grid: 1/repairDiv of the co-resident blocks
     std::vector<StreamDev> h_streams;
-    std::vector<unsigned long long> h_dsBase;
     // optional per-kernel timing: a ring of kTimedKernels+1 events per tick
     std::vector<cudaEvent_t> tev;
     int tevTicks = 0, tevNext = 0, tevRecorded = 0;
@@ -121,21 +120,22 @@ struct Workspace {
         free_events();
         cudaFree(work);
         cudaFree(d_streams);
-        cudaFree(d_dsBase);
+        cudaFreeHost(h_err);
         cudaFree(lists);
         *this = Workspace();
     }
     cudaError_t ensure(size_t px, int nStreams) {
         cudaError_t e = cudaSuccess;
+        if (!h_err) {
+            if ((e = cudaHostAlloc((void**)&h_err, sizeof(unsigned int), cudaHostAllocMapped)) != cudaSuccess) return e;
+            *h_err = 0u;
+        }
         if (!work && (e = cudaMalloc(&work, sizeof(TickWork))) != cudaSuccess) return e;
         if (nStreams > nStreamsCap) {
             cudaFree(d_streams);
-            cudaFree(d_dsBase);
             d_streams = nullptr;
-            d_dsBase = nullptr;
             const int n = std::max(nStreams, 8);
             if ((e = cudaMalloc(&d_streams, sizeof(StreamDev) * n)) != cudaSuccess) return e;
-            if ((e = cudaMalloc(&d_dsBase, sizeof(unsigned long long) * (n + 1))) != cudaSuccess) return e;
             nStreamsCap = n;
         }
         if (px > cap) {
@@ -362,10 +362,33 @@ cudaError_t coop_grid(int* maxBlocks) {
     return cudaSuccess;
 }
 
-// enqueue one tick over the n streams described in hS (tileBase etc. filled here); hDs holds n+1
-// entries. Both are host arrays the descriptor uploads read from (pinned for ticks in flight).
-lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t st, StreamDev* hS,
-                         unsigned long long* hDs) {
+// Opens a tick: the stream descriptors travel as kernel arguments (copied at the launch, so the host array
+// is free at once and nothing is staged) and the work area is cleared, one launch where two pageable uploads
+// and a memset were enqueued.
+template <int NB>
+struct TableArg {
+    StreamDev s[NB];
+};
+template <int NB>
+__global__ void __launch_bounds__(256) lvbgs_k_begin(const __grid_constant__ TableArg<NB> T, StreamDev* dst, int n,
+                                                     TickWork* work) {
+    static_assert(sizeof(StreamDev) % 4 == 0 && sizeof(TickWork) % 4 == 0, "copied as words");
+    const uint32_t* src = (const uint32_t*)&T;
+    for (int i = threadIdx.x; i < n * (int)(sizeof(StreamDev) / 4); i += blockDim.x) ((uint32_t*)dst)[i] = src[i];
+    if (work)
+        for (int i = threadIdx.x; i < (int)(sizeof(TickWork) / 4); i += blockDim.x) ((uint32_t*)work)[i] = 0u;
+}
+constexpr int kTableChunk = 64;
+static_assert(sizeof(TableArg<kTableChunk>) < 32000, "kernel arguments are limited to 32,764 bytes");
+template <int NB>
+void launch_begin(const StreamDev* hS, int n, StreamDev* dst, TickWork* work, cudaStream_t st) {
+    TableArg<NB> T;
+    std::memcpy(T.s, hS, sizeof(StreamDev) * n);
+    lvbgs_k_begin<NB><<<1, 256, 0, st>>>(T, dst, n, work);
+}
+
+// enqueue one tick over the n streams described in hS (tileBase etc. filled here)
+lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t st, StreamDev* hS) {
     int totalTiles = 0, totalRows = 0, totalSegs = 0;
     size_t totalPx = 0;
     unsigned long long ds = 0;
@@ -378,18 +401,19 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
         totalRows += S.H;
         totalSegs += S.nSegs;
         totalPx += (size_t)S.npx;
-        hDs[i] = ds;
+        S.dsBase = ds;
         // only streams with the frame-level analysis enabled down-sample
         if (S.lrScaling) ds += (unsigned long long)S.dsW * S.dsH;
     }
-    hDs[n] = ds;
     LV_CUDA(errh, ws.ensure(totalPx, n), "workspace allocation");
-    LV_CUDA(errh, cudaMemcpyAsync(ws.d_streams, hS, sizeof(StreamDev) * n, cudaMemcpyHostToDevice, st),
-            "descriptor upload");
-    LV_CUDA(errh, cudaMemcpyAsync(ws.d_dsBase, hDs, sizeof(unsigned long long) * (n + 1),
-                                  cudaMemcpyHostToDevice, st),
-            "descriptor upload");
-    LV_CUDA(errh, cudaMemsetAsync(ws.work, 0, sizeof(TickWork), st), "work reset");
+    if (n == 1) {
+        launch_begin<1>(hS, 1, ws.d_streams, ws.work, st);
+    } else if (n <= 16) {
+        launch_begin<16>(hS, n, ws.d_streams, ws.work, st);
+    } else {
+        for (int i = 0; i < n; i += kTableChunk)
+            launch_begin<kTableChunk>(hS + i, std::min(kTableChunk, n - i), ws.d_streams + i, i == 0 ? ws.work : nullptr, st);
+    }
     int maxBlocks = 0;
     LV_CUDA(errh, coop_grid(&maxBlocks), "occupancy query");
     if (maxBlocks <= 0) return fail(errh, LVBGS_DEVICE_ERROR, "repair kernel cannot be resident on this device");
@@ -411,7 +435,7 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
     P.rlist[1] = ws.lists + 3 * ws.cap;
     P.listCap = (unsigned)std::min<size_t>(ws.cap, 0xffffffffu);
     P.totalSegs = totalSegs;
-    const unsigned long long* dsb = ws.d_dsBase;
+    P.hostErr = ws.h_err;
     const dim3 blk(kThreads);
     const int rowBlocks = (totalRows + 7) / 8;
     const int dsBlocks = (int)((ds + kThreads - 1) / kThreads);
@@ -424,15 +448,15 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
 #define LV_TMARK(i) \
     if (tev) cudaEventRecord(tev[i], st)
     LV_TMARK(0);
-    lvbgs_k_eval<<<totalTiles, blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_eval, dim3(totalTiles), blk, st, P);
     LV_TMARK(1);
     {
         // long scans: a grid sized to the device, striding over the list the evaluation built
         const int longBlocks = std::max(1, std::min(g_sm_count * 8, (int)((totalPx + kThreads - 1) / kThreads)));
-        lvbgs_k_longscan<<<longBlocks, blk, 0, st>>>(P);
+        launch_chained(lvbgs_k_longscan, dim3(longBlocks), blk, st, P);
         LV_TMARK(2);
     }
-    lvbgs_k_resolve<<<(totalTiles + kResolveTiles - 1) / kResolveTiles + dsBlocks, blk, 0, st>>>(P, ds, dsb);
+    launch_chained(lvbgs_k_resolve, dim3((totalTiles + kResolveTiles - 1) / kResolveTiles + dsBlocks), blk, st, P, ds);
     LV_TMARK(3);
     {
         const int grid = std::max(1, std::min(maxBlocks / std::max(1, ws.repairDiv), std::max(1, totalTiles)));
@@ -441,37 +465,36 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
                 "repair kernel launch");
     }
     LV_TMARK(4);
-    lvbgs_k_commit<<<totalTiles, blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_commit, dim3(totalTiles), blk, st, P);
     LV_TMARK(5);
-    lvbgs_k_unite<<<rowBlocks + n, blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_unite, dim3(rowBlocks + n), blk, st, P);
     LV_TMARK(6);
-    lvbgs_k_fill<<<rowBlocks, blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_fill, dim3(rowBlocks), blk, st, P);
     LV_TMARK(7);
-    lvbgs_k_final<<<std::max(1, totalSegs), blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_final, dim3(std::max(1, totalSegs)), blk, st, P);
     LV_TMARK(8);
-    lvbgs_k_close<<<std::max(1, std::min(totalTiles, g_sm_count * 8)), blk, 0, st>>>(P);
+    launch_chained(lvbgs_k_close, dim3(std::max(1, std::min(totalTiles, g_sm_count * 8))), blk, st, P);
     LV_TMARK(9);
 #undef LV_TMARK
     LV_CUDA(errh, cudaGetLastError(), "frame step launch");
     return LVBGS_OK;
 }
 lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t st) {
-    ws.h_dsBase.resize(n + 1);
-    return launch_tick(errh, ws, n, st, ws.h_streams.data(), ws.h_dsBase.data());
+    return launch_tick(errh, ws, n, st, ws.h_streams.data());
 }
 
 // the device-side error flags of a tick as a status
-lvbgs_status status_from_work(lvbgs_handle errh, const TickWork& w) {
-    if (w.err & ERR_BARRIER_TIMEOUT) return fail(errh, LVBGS_DEVICE_TIMEOUT, "grid barrier wait timed out");
-    if (w.err & ERR_REPAIR_LIMIT) return fail(errh, LVBGS_DEVICE_ERROR, "raster-order repair did not converge");
-    if (w.err & ERR_UF_LIMIT) return fail(errh, LVBGS_DEVICE_ERROR, "hole-filling union-find exceeded its bound");
-    if (w.err & ERR_RING) return fail(errh, LVBGS_DEVICE_ERROR, "closed mask is not zero at pixel (0,0)");
+lvbgs_status status_from_flags(lvbgs_handle errh, unsigned int err) {
+    if (err & ERR_BARRIER_TIMEOUT) return fail(errh, LVBGS_DEVICE_TIMEOUT, "grid barrier wait timed out");
+    if (err & ERR_REPAIR_LIMIT) return fail(errh, LVBGS_DEVICE_ERROR, "raster-order repair did not converge");
+    if (err & ERR_UF_LIMIT) return fail(errh, LVBGS_DEVICE_ERROR, "hole-filling union-find exceeded its bound");
+    if (err & ERR_RING) return fail(errh, LVBGS_DEVICE_ERROR, "closed mask is not zero at pixel (0,0)");
     return LVBGS_OK;
 }
+// (after a wait for the tick: its last kernel wrote the flags)
 lvbgs_status read_work_status(lvbgs_handle errh, Workspace& ws) {
-    TickWork w;
-    LV_CUDA(errh, cudaMemcpy(&w, ws.work, sizeof(TickWork), cudaMemcpyDeviceToHost), "status read-back");
-    return status_from_work(errh, w);
+    if (!ws.work) return cuda_fail(errh, cudaErrorInvalidValue, "status read-back");
+    return status_from_flags(errh, *(volatile unsigned int*)ws.h_err);
 }
 
 // stages a frame for the kernel: returns the device pointer the kernel reads
@@ -1122,7 +1145,7 @@ lvbgs_status pw_advance(lvbgs_ctx* h, bool& done) {
     e = cudaMemcpy(&tw, h->d_work, sizeof(TickWork), cudaMemcpyDeviceToHost);
     h->pw_host_ms[4] += pw_ms_since(t0);
     if (e != cudaSuccess) return finish(cuda_fail(h, e, "status read-back"));
-    return finish(status_from_work(h, tw));
+    return finish(status_from_flags(h, tw.err));
 }
 
 lvbgs_status pw_apply(lvbgs_ctx* h, const uint8_t* img, size_t stride, uint8_t* mask, double lr, cudaStream_t st) {
@@ -1705,10 +1728,8 @@ struct lvbgs_batch_ctx {
     Workspace ws;
     cudaStream_t stream = nullptr;  // the stream of the ticks in flight
     struct Slot {
-        StreamDev* hS = nullptr;             // pinned descriptor table of the tick
-        unsigned long long* hDs = nullptr;   // pinned down-sampling offsets
+        std::vector<StreamDev> hS;           // descriptor table of the tick being enqueued
         TickWork* hWork = nullptr;           // pinned copy of the tick's status
-        int cap = 0;
         cudaEvent_t done = nullptr;
         uint64_t ticket = 0;
         bool busy = false;
@@ -1716,25 +1737,6 @@ struct lvbgs_batch_ctx {
     uint64_t next = 1;
     int inflight = 0;
 };
-
-namespace {
-void free_slot(lvbgs_batch_ctx::Slot& sl) {
-    cudaFreeHost(sl.hS);
-    cudaFreeHost(sl.hDs);
-    sl.hS = nullptr;
-    sl.hDs = nullptr;
-    sl.cap = 0;
-}
-cudaError_t grow_slot(lvbgs_batch_ctx::Slot& sl, int n) {
-    if (n <= sl.cap) return cudaSuccess;
-    free_slot(sl);
-    const int cap = std::max(n + n / 2, 16);
-    cudaError_t e = cudaHostAlloc((void**)&sl.hS, sizeof(StreamDev) * cap, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&sl.hDs, sizeof(unsigned long long) * (cap + 1), cudaHostAllocDefault);
-    if (e == cudaSuccess) sl.cap = cap;
-    return e;
-}
-}  // namespace
 
 lvbgs_status lvbgs_batch_create(int device_id, size_t reserve_px, int reserve_streams, lvbgs_batch* out) {
     if (!out) return fail(nullptr, LVBGS_BAD_ARG, "null output");
@@ -1747,7 +1749,6 @@ lvbgs_status lvbgs_batch_create(int device_id, size_t reserve_px, int reserve_st
     for (auto& sl : b->slots) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaHostAlloc((void**)&sl.hWork, sizeof(TickWork), cudaHostAllocDefault);
-        if (e == cudaSuccess) e = grow_slot(sl, std::max(reserve_streams, 1));
     }
     if (e != cudaSuccess) {
         lvbgs_batch_destroy(b);
@@ -1763,7 +1764,6 @@ lvbgs_status lvbgs_batch_destroy(lvbgs_batch b) {
     for (auto& sl : b->slots)
         if (sl.busy && sl.done) cudaEventSynchronize(sl.done);
     for (auto& sl : b->slots) {
-        free_slot(sl);
         cudaFreeHost(sl.hWork);
         if (sl.done) cudaEventDestroy(sl.done);
     }
@@ -1805,9 +1805,9 @@ lvbgs_status lvbgs_batch_submit(lvbgs_batch b, const lvbgs_handle* hs, const lvb
     for (int i = 0; i < n; ++i) px += hs[i]->npx;
     if (b->inflight > 0 && (px > b->ws.cap || n > b->ws.nStreamsCap))
         return fail(lead, LVBGS_BAD_ARG, "batch exceeds the context's reservation while ticks are in flight");
-    LV_CUDA(lead, grow_slot(sl, n), "descriptor table allocation");
-    if ((s = prepare_batch(hs, frames, n, st, sl.hS)) != LVBGS_OK) return s;
-    if ((s = launch_tick(lead, b->ws, n, st, sl.hS, sl.hDs)) != LVBGS_OK) return s;
+    sl.hS.resize(n);
+    if ((s = prepare_batch(hs, frames, n, st, sl.hS.data())) != LVBGS_OK) return s;
+    if ((s = launch_tick(lead, b->ws, n, st, sl.hS.data())) != LVBGS_OK) return s;
     if ((s = download_masks(hs, frames, n, st)) != LVBGS_OK) return s;
     LV_CUDA(lead, cudaMemcpyAsync(sl.hWork, b->ws.work, sizeof(TickWork), cudaMemcpyDeviceToHost, st), "status copy");
     LV_CUDA(lead, cudaEventRecord(sl.done, st), "completion event");
@@ -1839,7 +1839,7 @@ lvbgs_status lvbgs_batch_complete(lvbgs_batch b, uint64_t ticket) {
     sl.busy = false;
     --b->inflight;
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "batched frame step");
-    return status_from_work(nullptr, *sl.hWork);
+    return status_from_flags(nullptr, sl.hWork->err);
 }
 
 lvbgs_status lvbgs_get_background(lvbgs_handle h, uint8_t* out) {

@@ -139,6 +139,7 @@ struct StreamDev {
     uint8_t* maskOut;      // device output mask (may be null)
     int lrMode;            // 0: per-pixel ceil(T(x)); 1: fixed value lrFixed
     int lrScaling;         // frame-level analysis enabled (host copy of StreamCtl::lr_scaling)
+    unsigned long long dsBase;  // first down-sampled pixel of this stream in the batch's index space
     unsigned long long lrFixed;
     // state
     float* fm;
@@ -188,6 +189,7 @@ struct TickParams {
     unsigned long long barrierNs;  // limit of one grid-barrier wait of the repair, then ERR_BARRIER_TIMEOUT
     int maxRepairIters;            // repair rounds before ERR_REPAIR_LIMIT
     int dbgFault;                  // injected fault (lvbgs_debug_inject_fault), 0: none
+    unsigned int* hostErr;         // page-locked host copy of the tick's error flags, written by its last kernel
 };
 constexpr unsigned long long kBarrierNs = 2000000000ull;  // 2 s
 constexpr unsigned long long kDebugBarrierNs = 2000000ull;  // 2 ms, for the injected barrier timeout
@@ -257,5 +259,31 @@ LV_HD uint8_t area_resample(int W, int H, int dW, int dH, int x, int y, Get get)
     }
     return area_round_ties_even(num, (unsigned long long)W * (unsigned long long)H);
 }
+
+#if defined(__CUDACC__)
+// Programmatic dependent launch. A kernel of a chain calls pdl_entry() first: the next kernel of the stream,
+// if launched with launch_chained, may then be set up while this one runs, and this one waits until the one
+// before it is complete and its writes are visible. A chain's kernels all call it, so the wait reaches back
+// over the whole chain; a kernel launched normally waits as ever.
+__device__ __forceinline__ void pdl_entry() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+template <typename... KArgs, typename... Args>
+inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);  // errors are read by the caller's cudaGetLastError()
+}
+#endif
 
 }  // namespace lvbgs

@@ -1538,6 +1538,7 @@ __device__ void stream_epilogue(const TickParams& P, const StreamDev& S);
 // run the frame-level epilogue of one stream each (it touches nothing that these rows read).
 // Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
+    pdl_entry();
     const int rowBlocks = (P.totalRows + 7) / 8;
     if ((int)blockIdx.x >= rowBlocks) {
         stream_epilogue(P, P.streams[blockIdx.x - rowBlocks]);
@@ -1588,6 +1589,7 @@ extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
 // words come from the neighbour lanes (the two edge lanes of a chunk load theirs). One kernel where the
 // hole words took a pass of their own through memory: 20 + 6 us on a 1920x1080 frame before.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_fill(TickParams P) {
+    pdl_entry();
     const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (gr >= P.totalRows) return;
     const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
@@ -1738,6 +1740,7 @@ __device__ __forceinline__ void median_words(FinSmem& sm, int r, int half, int y
 // first and used last; a thread holds four neighbouring pixels, so the mask leaves in 128-byte rows also
 // when it is in host memory. Bound by the 22 B/px of maps and by the latency of the short word phases.
 extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams P) {
+    pdl_entry();
     __shared__ FinSmem sm;
     const int gt = blockIdx.x;
     if (gt >= P.totalSegs) return;
@@ -1988,6 +1991,7 @@ __device__ void refresh_pixel(const StreamDev& S, int p, uint32_t frame, int sta
     const int lt = t - S.tileBase;
 
 extern "C" __global__ void __launch_bounds__(kThreads, 5) lvbgs_k_eval(TickParams P) {
+    pdl_entry();
     __shared__ __align__(16) uint8_t smem[kTileRW<3> * (kTileH + 2 * kBorder) + 256];
     LV_TILE_KERNEL_PROLOGUE
     if (S.C == 3) phaseA_tile<3>(P, si, S, lt, smem);
@@ -2053,6 +2057,7 @@ __device__ void longscan_items(const TickParams& P, bool own, int m, unsigned lo
 }
 
 extern "C" __global__ void __launch_bounds__(256, 3) lvbgs_k_longscan(TickParams P) {
+    pdl_entry();
     const unsigned int n = min(ld_volatile(&P.work->lcount), P.listCap);
     const int m = coop_share(n, gridDim.x), lane = threadIdx.x & 31, sub = lane & 7;
     const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -2067,8 +2072,8 @@ extern "C" __global__ void __launch_bounds__(256, 3) lvbgs_k_longscan(TickParams
     }
 }
 
-extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParams P, unsigned long long dsTotal,
-                                                                       const unsigned long long* dsBase) {
+extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParams P, unsigned long long dsTotal) {
+    pdl_entry();
     const int tileBlocks = (P.totalTiles + kResolveTiles - 1) / kResolveTiles;
     if ((int)blockIdx.x < tileBlocks) {
         phaseB_tiles(P, blockIdx.x * kResolveTiles);
@@ -2079,10 +2084,10 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParam
     int lo = 0, hi = P.nStreams - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (dsBase[mid] <= i) lo = mid;
+        if (P.streams[mid].dsBase <= i) lo = mid;
         else hi = mid - 1;
     }
-    ds_item(P.streams[lo], (int)(i - dsBase[lo]));
+    ds_item(P.streams[lo], (int)(i - P.streams[lo].dsBase));
 }
 
 // Repair to the raster-order fixed point (cooperative launch: all CTAs resident). Every round re-matches
@@ -2170,6 +2175,7 @@ extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickPar
 }
 
 extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_commit(TickParams P) {
+    pdl_entry();
     __shared__ __align__(16) uint8_t smem[(kTileW + 4) * (kTileH + 4) * 4 + (kTileW + 2) * (kTileH + 2)];
     LV_TILE_KERNEL_PROLOGUE
     if (S.C == 3) phaseF_tile<3>(P, S, lt, smem);
@@ -2180,6 +2186,8 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_commit(TickParams
 // closes the frame of every stream: frame index (and so the buffer parity), repair statistics
 __device__ __forceinline__ void close_streams(const TickParams& P) {
     const unsigned int its = P.work->iters;
+    // the tick's error flags go to the host with the kernel's end: no copy to enqueue and wait for
+    if (threadIdx.x == 0 && P.hostErr) *(volatile unsigned int*)P.hostErr = ld_volatile(&P.work->err);
     for (int si = threadIdx.x; si < P.nStreams; si += blockDim.x) {
         StreamCtl* ctl = P.streams[si].ctl;
         ctl->frame_idx += 1ull;
@@ -2194,6 +2202,7 @@ __device__ __forceinline__ void close_streams(const TickParams& P) {
 // the tiles of those streams, and the block that finishes last closes the streams (the others still read
 // the frame index until then).
 extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_close(TickParams P) {
+    pdl_entry();
     if (ld_volatile(&P.work->anyReset) == 0u) {
         if (blockIdx.x == 0) close_streams(P);
         return;
