@@ -37,9 +37,9 @@ def _stale(target, deps):
 
 def build(verbose=False, force=False, ptxas_verbose=False):
     os.makedirs(OUT, exist_ok=True)
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers += [os.path.join(HERE, "..", "include", f) for f in os.listdir(os.path.join(HERE, "..", "include"))
-                if f.endswith(".h")]
+                if f.endswith((".h", ".cuh"))]
     procs, objs = [], []
     for src in SOURCES:
         s = os.path.join(CSRC, src)

@@ -2,7 +2,32 @@
 #pragma once
 #include <stdint.h>
 
+#include "lvbgs_internal.h"
+
 namespace lvbgs {
+
+// LBSP 16-bit double-cross pattern (LBSP.hpp:297-298): column and row offset of tap n, four bits each.
+// Constant expressions, so that the taps of an unrolled gather become address immediates: from a table in
+// constant memory (which the host could rewrite) every tap cost a load and the address arithmetic.
+LV_HD constexpr int lbsp_dx(int n) { return (int)((0x1331321204402240ull >> (4 * n)) & 15u) - 2; }
+LV_HD constexpr int lbsp_dy(int n) { return (int)((0x3131212304044022ull >> (4 * n)) & 15u) - 2; }
+static_assert(lbsp_dx(0) == -2 && lbsp_dy(0) == 0 && lbsp_dx(5) == 2 && lbsp_dy(5) == -2 && lbsp_dx(15) == -1 &&
+                  lbsp_dy(15) == 1,
+              "tap order");
+
+// Neighbour tables (opencv.hpp:945-964) in closed form: both list the window row by row from dy = +r down to
+// -r, left to right, without the centre. By arithmetic, because the lanes of a warp draw different entries,
+// which constant memory serves one after the other.
+__device__ __forceinline__ void nb3_offset(int r, int& dx, int& dy) {
+    const int k = r + (r >= 4);
+    dx = k % 3 - 1;
+    dy = 1 - k / 3;
+}
+__device__ __forceinline__ void nb5_offset(int r, int& dx, int& dy) {
+    const int k = r + (r >= 12);
+    dx = k % 5 - 2;
+    dy = 2 - k / 5;
+}
 
 // bit 7 of each byte = (a > b) for the unsigned bytes of a and b, given nb = ~b and nbL = nb & 0x7f7f7f7f:
 // a > b exactly when a + ~b carries out of the byte. The low seven bits of each byte are added without

@@ -438,7 +438,7 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
     P.hostErr = ws.h_err;
     const dim3 blk(kThreads);
     const int rowBlocks = (totalRows + 7) / 8;
-    const int dsBlocks = (int)((ds + kThreads - 1) / kThreads);
+    const int dsBlocks = (int)((ds + kThreads / 8 - 1) / (kThreads / 8));  // eight lanes per down-sampled pixel
     cudaEvent_t* tev = nullptr;
     if (ws.tevTicks > 0) {
         tev = &ws.tev[(size_t)ws.tevNext * (kTimedKernels + 1)];
@@ -1049,8 +1049,8 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool& motion) {
     lvbgs_k_final<<<TP.totalSegs, blk, 0, st>>>(TP);
     const int nds = (h->W / 8) * (h->H / 8);
     if (nds > 0) {
-        if (c3) pw3_k_ds<<<(nds + 255) / 256, 256, 0, st>>>(P);
-        else pw_k_ds<<<(nds + 255) / 256, 256, 0, st>>>(P);
+        if (c3) pw3_k_ds<<<(nds + 31) / 32, 256, 0, st>>>(P);
+        else pw_k_ds<<<(nds + 31) / 32, 256, 0, st>>>(P);
     }
     pw_k_epilogue<<<1, 256, 0, st>>>(P);
     const uint32_t t = (uint32_t)(h->pw_frames + 1);

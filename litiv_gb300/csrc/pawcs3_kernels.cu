@@ -20,6 +20,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "area_device.cuh"
 #include "pawcs_device.cuh"
 
 namespace lvbgs {
@@ -930,18 +931,17 @@ extern "C" __global__ void pw3_k_ds(PwParams P) {
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per output
     if (i >= nds) return;
+    uint32_t v[3];
+    area_resample_group<3>(D.frame, D.W, D.H, D.dsW, D.dsH, i % D.dsW, i / D.dsW, v);
+    if (threadIdx.x & 7) return;
     const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
     float fLT, fST;
     pw_factors(t, (int)S.nmv, &fLT, &fST);
-    const int bx = i % D.dsW, by = i / D.dsW;
     float e = 0.0f;
     for (int c = 0; c < 3; ++c) {
-        const uint8_t* fr = D.frame;
-        const int W = D.W;
-        const uint8_t vb = area_resample(D.W, D.H, D.dsW, D.dsH, bx, by,
-                                         [&](int sx, int sy) { return (int)fr[((size_t)sy * W + sx) * 3 + c]; });
+        const uint8_t vb = (uint8_t)v[c];
         const size_t k = (size_t)i * 3 + c;
         const float lt = (float)vb * fLT + D.dsLT[k] * (1.0f - fLT);
         const float st = (float)vb * fST + D.dsST[k] * (1.0f - fST);

@@ -5,19 +5,14 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "lbsp_device.cuh"
 #include "pawcs_internal.h"
 
 namespace lvbgs {
 
-// LBSP double-cross taps (LBSP.hpp:297-298), sampling tables (opencv.hpp:915-964)
-static __constant__ int pw_dx[16] = {-2, 2, 0, 0, -2, 2, 2, -2, 0, -1, 0, 1, -1, 1, 1, -1};
-static __constant__ int pw_dy[16] = {0, 0, -2, 2, 2, -2, 2, -2, 1, 0, -1, 0, -1, 1, -1, 1};
+// sampling weights (opencv.hpp:915-923)
 static __constant__ int pw_pat7[49] = {2, 4, 6, 7, 6, 4, 2, 4, 8, 12, 14, 12, 8, 4, 6, 12, 21, 25, 21, 12, 6, 7, 14, 25, 28,
                                 25, 14, 7, 6, 12, 21, 25, 21, 12, 6, 4, 8, 12, 14, 12, 8, 4, 2, 4, 6, 7, 6, 4, 2};
-static __constant__ int pw_nb3[8][2] = {{-1, 1}, {0, 1}, {1, 1}, {-1, 0}, {1, 0}, {-1, -1}, {0, -1}, {1, -1}};
-static __constant__ int pw_nb5[24][2] = {{-2, 2}, {-1, 2}, {0, 2},   {1, 2},   {2, 2},   {-2, 1},  {-1, 1}, {0, 1},
-                                  {1, 1},  {2, 1},  {-2, 0},  {-1, 0},  {1, 0},   {2, 0},   {-2, -1}, {-1, -1},
-                                  {0, -1}, {1, -1}, {2, -1},  {-2, -2}, {-1, -2}, {0, -2},  {1, -2},  {2, -2}};
 
 constexpr float kTLower = 1.0f, kTUpper = 256.0f, kTIncr = 0.5f, kTDecr = 0.25f;
 constexpr float kVIncr = 1.0f, kVDecr = 0.1f, kRVar = 0.01f, kUnstRatio = 0.1f, kUnstR = 3.0f;
@@ -98,7 +93,7 @@ __device__ __forceinline__ uint32_t pw_absdiff(uint32_t a, uint32_t b) { return 
 // current frame: LBSP lookups of pixel (x, y) and its descriptor
 __device__ __forceinline__ void pw_taps(const uint8_t* img, int W, int x, int y, uint8_t taps[16]) {
 #pragma unroll
-    for (int n = 0; n < 16; ++n) taps[n] = __ldg(img + (size_t)(y + pw_dy[n]) * W + (x + pw_dx[n]));
+    for (int n = 0; n < 16; ++n) taps[n] = __ldg(img + (size_t)(y + lbsp_dy(n)) * W + (x + lbsp_dx(n)));
 }
 __device__ __forceinline__ uint32_t pw_lbsp(const uint8_t taps[16], uint32_t ref, uint32_t thr) {
     uint32_t d = 0;
@@ -164,7 +159,7 @@ __device__ __forceinline__ uint32_t pw3_hd(uint32_t a01, uint32_t a2, uint32_t b
 __device__ __forceinline__ void pw3_taps(const uint8_t* img, int W, int x, int y, uint8_t taps[3][16]) {
 #pragma unroll
     for (int n = 0; n < 16; ++n) {
-        const uint8_t* q = img + ((size_t)(y + pw_dy[n]) * W + (x + pw_dx[n])) * 3;
+        const uint8_t* q = img + ((size_t)(y + lbsp_dy(n)) * W + (x + lbsp_dx(n))) * 3;
         taps[0][n] = q[0];
         taps[1][n] = q[1];
         taps[2][n] = q[2];

@@ -8,6 +8,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "area_device.cuh"
 #include "pawcs_device.cuh"
 
 namespace lvbgs {
@@ -580,15 +581,10 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_nbr(PwParams P) {
     if (upd) {
         const uint32_t r = pw_draw(D.seed, t, (uint32_t)p, k++);
         int nx, ny;
-        if (flat || border || moving) {
-            const int i = (int)(r % 24u);
-            nx = x + pw_nb5[i][0];
-            ny = y + pw_nb5[i][1];
-        } else {
-            const int i = (int)(r % 8u);
-            nx = x + pw_nb3[i][0];
-            ny = y + pw_nb3[i][1];
-        }
+        if (flat || border || moving) nb5_offset((int)(r % 24u), nx, ny);
+        else nb3_offset((int)(r % 8u), nx, ny);
+        nx += x;
+        ny += y;
         nx = nx < 2 ? 2 : nx >= D.W - 2 ? D.W - 3 : nx;
         ny = ny < 2 ? 2 : ny >= D.H - 2 ? D.H - 3 : ny;
         const int q = ny * D.W + nx;
@@ -1133,16 +1129,15 @@ extern "C" __global__ void pw_k_ds(PwParams P) {
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per output
     if (i >= nds) return;
+    uint32_t v[1];
+    area_resample_group<1>(D.frame, D.W, D.H, D.dsW, D.dsH, i % D.dsW, i / D.dsW, v);
+    if (threadIdx.x & 7) return;
     const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
     float fLT, fST;
     pw_factors(t, (int)S.nmv, &fLT, &fST);
-    const int bx = i % D.dsW, by = i / D.dsW;
-    const uint8_t* fr = D.frame;
-    const int W = D.W;
-    const uint8_t vb = area_resample(D.W, D.H, D.dsW, D.dsH, bx, by,
-                                     [&](int sx, int sy) { return (int)fr[(size_t)sy * W + sx]; });
+    const uint8_t vb = (uint8_t)v[0];
     const float lt = (float)vb * fLT + D.dsLT[i] * (1.0f - fLT);
     const float st = (float)vb * fST + D.dsST[i] * (1.0f - fST);
     D.dsLT[i] = lt;

@@ -22,21 +22,15 @@
 // the same tick.
 #include <cuda_runtime.h>
 
+#include "area_device.cuh"
 #include "lbsp_device.cuh"
 #include "lvbgs_internal.h"
 
 namespace lvbgs {
 
-// LBSP 16-bit double-cross pattern (LBSP.hpp:297-298)
-__constant__ int c_lbsp_dx[16] = {-2, 2, 0, 0, -2, 2, 2, -2, 0, -1, 0, 1, -1, 1, 1, -1};
-__constant__ int c_lbsp_dy[16] = {0, 0, -2, 2, 2, -2, 2, -2, 1, 0, -1, 0, -1, 1, -1, 1};
-// 7x7 Gaussian sampling weights (opencv.hpp:915-923) and 3x3 / 5x5 neighbour tables (opencv.hpp:945-964)
+// 7x7 Gaussian sampling weights (opencv.hpp:915-923)
 __constant__ int c_pat7[49] = {2, 4, 6, 7, 6, 4, 2,     4, 8, 12, 14, 12, 8, 4, 6, 12, 21, 25, 21, 12, 6, 7, 14, 25, 28,
                                25, 14, 7, 6, 12, 21, 25, 21, 12, 6, 4, 8, 12, 14, 12, 8, 4, 2, 4, 6, 7, 6, 4, 2};
-__constant__ int c_nb3[8][2] = {{-1, 1}, {0, 1}, {1, 1}, {-1, 0}, {1, 0}, {-1, -1}, {0, -1}, {1, -1}};
-__constant__ int c_nb5[24][2] = {{-2, 2}, {-1, 2}, {0, 2},   {1, 2},   {2, 2},   {-2, 1},  {-1, 1}, {0, 1},
-                                 {1, 1},  {2, 1},  {-2, 0},  {-1, 0},  {1, 0},   {2, 0},   {-2, -1}, {-1, -1},
-                                 {0, -1}, {1, -1}, {2, -1},  {-2, -2}, {-1, -2}, {0, -2},  {1, -2}, {2, -2}};
 
 constexpr int kUFLimit = 1 << 22;
 
@@ -465,6 +459,7 @@ __device__ __forceinline__ void coop_scan(const TickParams& P, bool want, int m,
                                           uint64_t ovGood, ScanSt& st) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & 7;
+    __syncwarp();
     if (m == 8) {
         if (want) lane_scan<C, REC>(P.streams[si], p, vals, curr, intra, th, ovMask, ovGood, st);
         return;
@@ -506,6 +501,7 @@ __device__ __forceinline__ void coop_scan(const TickParams& P, bool want, int m,
         uint32_t mins = 0xffffffffu;  // descriptor minimum | summed minimum, 16 bits each
         uint32_t first = 0xffffffffu, second = 0xffffffffu;  // this lane's good samples: index, distances
         while (__any_sync(kAll, ng < nreq && s < N)) {
+            __syncwarp();
             const bool act = ng < nreq && s < N;
             uint64_t dn = 0;
             uint32_t cn = 0;
@@ -648,15 +644,10 @@ __device__ uint32_t eval_tail(const StreamDev& S, const FrameK& F, int x, int y,
         const bool use3 = F.use3x3 && !uNew;
         const uint32_t rn = draw_k(S.seed, seedFrame, (uint32_t)p, k++, ds);
         int nx, ny;
-        if (use3) {
-            const int r = (int)(rn % 8u);
-            nx = x + c_nb3[r][0];
-            ny = y + c_nb3[r][1];
-        } else {
-            const int r = (int)(rn % 24u);
-            nx = x + c_nb5[r][0];
-            ny = y + c_nb5[r][1];
-        }
+        if (use3) nb3_offset((int)(rn % 8u), nx, ny);
+        else nb5_offset((int)(rn % 24u), nx, ny);
+        nx += x;
+        ny += y;
         clamp_xy(nx, ny, S.W, S.H);
         const uint32_t code = (uint32_t)((ny - y + 2) * 5 + (nx - x + 2));
         const uint32_t nrand = draw_k(S.seed, seedFrame, (uint32_t)p, k++, ds);
@@ -748,31 +739,6 @@ __device__ __forceinline__ void block_add_stats(unsigned long long* a, unsigned 
     }
 }
 
-// block-aggregated list reservation: every thread of the block calls it; returns this thread's slot
-// (or ~0u when it does not want one). One counter atomic per block: the lists' counters are shared by
-// all streams of the batch, and same-address atomics serialize.
-__device__ __forceinline__ unsigned int block_reserve(bool want, unsigned int* count) {
-    __shared__ unsigned int sWarp[32];
-    __shared__ unsigned int sBase;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned m = __ballot_sync(0xffffffffu, want);
-    if (lane == 0) sWarp[warp] = __popc(m);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int run = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-            const unsigned int v = sWarp[i];
-            sWarp[i] = run;
-            run += v;
-        }
-        sBase = run ? atomicAdd(count, run) : 0u;
-    }
-    __syncthreads();
-    const unsigned int r = want ? sBase + sWarp[warp] + (unsigned int)__popc(m & ((1u << lane) - 1u)) : ~0u;
-    __syncthreads();  // the shared slots are reused by the next call
-    return r;
-}
-
 // gathers the 16 LBSP taps of channel c at (x, y) from a byte image (tile or frame)
 template <int C>
 __device__ __forceinline__ void gather_taps(const uint8_t* base, int rowStride, int c, uint32_t (&v)[4]) {
@@ -782,7 +748,7 @@ __device__ __forceinline__ void gather_taps(const uint8_t* base, int rowStride, 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int n = j * 4 + i;
-            w |= (uint32_t)base[c_lbsp_dy[n] * rowStride + c_lbsp_dx[n] * C + c] << (8 * i);
+            w |= (uint32_t)base[lbsp_dy(n) * rowStride + lbsp_dx(n) * C + c] << (8 * i);
         }
         v[j] = w;
     }
@@ -1034,45 +1000,74 @@ __device__ void phaseB_tiles(const TickParams& P, int t0) {
             if (qs[j] > ps[j]) wq[j] = __ldcg(&S.intent[qs[j]]);
         }
     }
+    // one list item per target and stamp generation. The four tiles' items are reserved together: one
+    // counter atomic per block (the counter is shared by all streams, and same-address atomics serialize)
+    bool ok[kResolveTiles];
 #pragma unroll
     for (int j = 0; j < kResolveTiles; ++j) {
-        if (t0 + j >= P.totalTiles) break;  // uniform over the block
         const bool want = (w[j] & kInValid) && in_nb_writes(w[j]) && qs[j] > ps[j] && (wq[j] & kInValid) &&
                           in_snb(w[j]) < in_e(wq[j]);
-        // one list item per target and stamp generation; slots reserved once per block
-        const bool ok = want && atomicExch(&P.streams[sSi[j]].stampD[qs[j]], sStamp[j]) != sStamp[j];
-        const unsigned int i = block_reserve(ok, &P.work->dcount[0]);
-        if (ok) {
-            if (i < P.listCap) P.dlist[0][i] = ((unsigned long long)sSi[j] << 40) | (unsigned long long)(unsigned)qs[j];
-            else atomicOr(&P.work->err, ERR_REPAIR_LIMIT);
+        ok[j] = want && atomicExch(&P.streams[sSi[j]].stampD[qs[j]], sStamp[j]) != sStamp[j];
+    }
+    __shared__ unsigned int sWarp[kThreads / 32], sBase;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int mine[kResolveTiles], cnt = 0;
+#pragma unroll
+    for (int j = 0; j < kResolveTiles; ++j) {
+        const unsigned m = __ballot_sync(0xffffffffu, ok[j]);
+        mine[j] = cnt + (unsigned)__popc(m & ((1u << lane) - 1u));
+        cnt += (unsigned)__popc(m);
+    }
+    if (lane == 0) sWarp[warp] = cnt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned int run = 0;
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; ++i) {
+            const unsigned int v = sWarp[i];
+            sWarp[i] = run;
+            run += v;
         }
+        sBase = run ? atomicAdd(&P.work->dcount[0], run) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kResolveTiles; ++j) {
+        if (!ok[j]) continue;
+        const unsigned int i = sBase + sWarp[warp] + mine[j];
+        if (i < P.listCap) P.dlist[0][i] = ((unsigned long long)sSi[j] << 40) | (unsigned long long)(unsigned)qs[j];
+        else atomicOr(&P.work->err, ERR_REPAIR_LIMIT);
     }
 }
 
-// frame down-sampling for the frame-level analysis (:568-584): one output pixel per thread
+// frame down-sampling for the frame-level analysis (:568-584): one output pixel by a group of eight lanes;
+// the averages of channel c are on lane c
+template <int C>
 __device__ void ds_item(const StreamDev& S, int i) {
-    const int C = S.C;
-    const int dx = i % S.dsW, dy = i / S.dsW;
-    const FrameK F = frame_consts(S);
-    uint32_t dmax = 0;
-    for (int c = 0; c < C; ++c) {
-        const uint8_t* fr = S.frame;
-        const int W = S.W;
-        const int v = area_resample(S.W, S.H, S.dsW, S.dsH, dx, dy,
-                                    [&](int sx, int sy) { return (int)__ldg(fr + ((size_t)sy * W + sx) * C + c); });
-        const size_t k = (size_t)i * C + c;
+    const int sub = threadIdx.x & 7;
+    const unsigned mask = 0xffu << (threadIdx.x & 24);
+    uint32_t v[C];
+    area_resample_group<C>(S.frame, S.W, S.H, S.dsW, S.dsH, i % S.dsW, i / S.dsW, v);
+    uint32_t d = 0;
+    if (sub < C) {
+        const FrameK F = frame_consts(S);
+        uint32_t vc = v[0];
+#pragma unroll
+        for (int c = 1; c < C; ++c) vc = sub == c ? v[c] : vc;
+        const size_t k = (size_t)i * C + sub;
         // accumulateWeighted: dst = src*a + dst*(1-a)
         const float aL = F.fLT, bL = 1.0f - aL, aS = F.fST, bS = 1.0f - aS;
-        const float lt = (float)v * aL + S.dsLT[k] * bL;
-        const float st = (float)v * aS + S.dsST[k] * bS;
+        const float lt = (float)vc * aL + S.dsLT[k] * bL;
+        const float st = (float)vc * aS + S.dsST[k] * bS;
         S.dsLT[k] = lt;
         S.dsST[k] = st;
-        const uint32_t d = (uint32_t)__float2ull_rz(fabsf(st - lt));
-        if (C == 1) dmax = d / 2u;
-        else dmax = c == 0 ? d : (d > dmax ? d : dmax);
+        d = (uint32_t)__float2ull_rz(fabsf(st - lt));
+        if (C == 1) d /= 2u;
     }
-    // reference order: max(d0, max(d1, d2)) -- identical to the running max for integers
-    if (dmax) atomicAdd(&S.ctl->colordiff_acc, (unsigned long long)dmax);
+    // the largest difference of the channels (lanes 0-3 of the group hold them)
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) d = max(d, __shfl_xor_sync(mask, d, o, 8));
+    if (sub == 0 && d) atomicAdd(&S.ctl->colordiff_acc, (unsigned long long)d);
 }
 
 // Place of the length of round i's list: the lists themselves alternate, but a round without re-resolutions
@@ -1129,7 +1124,7 @@ __device__ bool rematch_items(const TickParams& P, bool own, int m, int si, int 
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int n = j * 4 + i;
-                    wv |= (uint32_t)__ldg(base + (c_lbsp_dy[n] * W + c_lbsp_dx[n]) * C + c) << (8 * i);
+                    wv |= (uint32_t)__ldg(base + (lbsp_dy(n) * W + lbsp_dx(n)) * C + c) << (8 * i);
                 }
                 vals[c][j] = wv;
             }
@@ -2079,7 +2074,7 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParam
         phaseB_tiles(P, blockIdx.x * kResolveTiles);
         return;
     }
-    const unsigned long long i = (unsigned long long)(blockIdx.x - tileBlocks) * blockDim.x + threadIdx.x;
+    const unsigned long long i = ((unsigned long long)(blockIdx.x - tileBlocks) * blockDim.x + threadIdx.x) >> 3;
     if (i >= dsTotal) return;
     int lo = 0, hi = P.nStreams - 1;
     while (lo < hi) {
@@ -2087,7 +2082,9 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParam
         if (P.streams[mid].dsBase <= i) lo = mid;
         else hi = mid - 1;
     }
-    ds_item(P.streams[lo], (int)(i - P.streams[lo].dsBase));
+    const StreamDev& S = P.streams[lo];
+    if (S.C == 3) ds_item<3>(S, (int)(i - S.dsBase));
+    else ds_item<1>(S, (int)(i - S.dsBase));
 }
 
 // Repair to the raster-order fixed point (cooperative launch: all CTAs resident). Every round re-matches
@@ -2256,11 +2253,13 @@ extern "C" __global__ void lvbgs_init_maps(StreamDev S, const uint8_t* img, floa
             if (desc) {
                 uint32_t vals[4];
                 const uint8_t* base = img + (size_t)p * C;
+#pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint32_t wv = 0;
+#pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int n = j * 4 + i;
-                        wv |= (uint32_t)base[(c_lbsp_dy[n] * S.W + c_lbsp_dx[n]) * C + c] << (8 * i);
+                        wv |= (uint32_t)base[(lbsp_dy(n) * S.W + lbsp_dx(n)) * C + c] << (8 * i);
                     }
                     vals[j] = wv;
                 }
@@ -2366,11 +2365,13 @@ extern "C" __global__ void lvbgs_lbsp_dense(const uint8_t* img, int W, int H, in
         for (int c = 0; c < C; ++c) {
             const uint8_t* base = img + (size_t)p * C;
             uint32_t vals[4];
+#pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t wv = 0;
+#pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int n = j * 4 + i;
-                    wv |= (uint32_t)base[(c_lbsp_dy[n] * W + c_lbsp_dx[n]) * C + c] << (8 * i);
+                    wv |= (uint32_t)base[(lbsp_dy(n) * W + lbsp_dx(n)) * C + c] << (8 * i);
                 }
                 vals[j] = wv;
             }

@@ -49,3 +49,11 @@ def test_ordered_scans_by_groups_and_by_lanes(N, nreq, channels):
     frames[5] = rng.integers(0, 256, frames[5].shape, dtype=np.uint8)
     lrs = [1.0 if t in (2, 3, 4, 6, 7) else 0.0 for t in range(len(frames))]
     run_pair(frames, seed=nreq + 3, lrs=lrs, nBGSamples=N, nRequiredBGSamples=nreq)
+
+
+@pytest.mark.parametrize("W,H,channels", [(641, 243, 3), (328, 241, 1), (329, 240, 3), (320, 248, 1), (15, 5200, 1),
+                                          (15, 5201, 3)])
+def test_area_down_sampling_at_ragged_sizes(W, H, channels):
+    """The frame-level down-sampling by groups of lanes: integral scales (8 and 15) with and without aligned
+    rows, fractional scales in one or both directions (the averages are part of the compared state)."""
+    run_pair(hollow_frames(W, H, channels, 3, W + H), seed=2)
