@@ -57,7 +57,7 @@ extern "C" __global__ void pw_k_blink_close(PwParams P);
 extern "C" __global__ void pw_k_epilogue(PwParams P);
 extern "C" __global__ void pw_k_ds(PwParams P);
 extern "C" __global__ void pw_k_reset_decide(PwParams P);
-extern "C" __global__ void pw_k_motion_bg(PwParams P, int buf);
+extern "C" __global__ void pw_k_motion_bg(PwParams P);
 extern "C" __global__ void pw_k_motion_decide(PwParams P);
 extern "C" __global__ void pw_k_compact_count(PwParams P, int mode);
 extern "C" __global__ void pw_k_compact_offsets(PwParams P, int ncat);
@@ -69,7 +69,7 @@ extern "C" __global__ void pw_k_refresh_global(PawcsDev S, uint32_t t, int buf, 
 extern "C" __global__ void pw_k_reset_T(PawcsDev S, int buf);
 extern "C" __global__ void pw_k_init(PawcsDev S);
 extern "C" __global__ void pw_k_init_last(PawcsDev S, const uint8_t* img);
-extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc);
+extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc, int ahead);
 // PAWCS, three channels (pawcs3_kernels.cu)
 extern "C" __global__ void pw3_k_local(PwParams P);
 extern "C" __global__ void pw3_k_gscan_seg(PwParams P);
@@ -80,13 +80,13 @@ extern "C" __global__ void pw3_k_dirty(PwParams P);
 extern "C" __global__ void pw3_k_later(PwParams P);
 extern "C" __global__ void pw3_k_commit(PwParams P);
 extern "C" __global__ void pw3_k_ds(PwParams P);
-extern "C" __global__ void pw3_k_motion_bg(PwParams P, int buf);
+extern "C" __global__ void pw3_k_motion_bg(PwParams P);
 extern "C" __global__ void pw3_k_refresh_local(PawcsDev S, uint32_t t, int buf, int baseOcc, float decr, int force,
                                                int onlyPending, int useDil);
 extern "C" __global__ void pw3_k_refresh_global(PawcsDev S, uint32_t t, int buf, int force, int onlyPending, int useDil);
 extern "C" __global__ void pw3_k_init(PawcsDev S);
 extern "C" __global__ void pw3_k_init_last(PawcsDev S, const uint8_t* img);
-extern "C" __global__ void pw3_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc);
+extern "C" __global__ void pw3_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc, int ahead);
 }  // namespace lvbgs
 
 using namespace lvbgs;
@@ -575,7 +575,7 @@ extern "C" {
 namespace {
 
 enum {
-    PL_CTL = 0, PL_PCTL, PL_FM, PL_WCOLOR, PL_WDESC, PL_WOCC, PL_WFIRST, PL_WLAST, PL_ILLUM, PL_UNST, PL_ROI,
+    PL_CTL = 0, PL_PCTL, PL_FM, PL_WA, PL_WLAST, PL_WC2, PL_ILLUM, PL_UNST, PL_ROI,
     PL_BLINKS, PL_LASTRAWFG, PL_LASTFG, PL_DILINV, PL_LASTRAWBLINK, PL_LASTCOL, PL_LASTDESC, PL_KCTR, PL_GLUT,
     PL_GMAP, PL_DSLT, PL_DSST, PL_DSROI,
     // scratch (not part of the model)
@@ -592,10 +592,10 @@ PwLayout pw_layout(int W, int H, int C, int L, int G) {
     sz[PL_CTL] = sizeof(StreamCtl);
     sz[PL_PCTL] = sizeof(PawcsCtl);
     sz[PL_FM] = 2 * kNumFloatMaps * npx * 4;
-    // word colours / descriptors: [2][L][npx] one channel, [2][L][npx][3] three (channel-minor)
-    sz[PL_WCOLOR] = 2 * (size_t)L * npx * C;
-    sz[PL_WDESC] = 2 * (size_t)L * npx * 2 * C;
-    sz[PL_WOCC] = sz[PL_WFIRST] = sz[PL_WLAST] = 2 * (size_t)L * npx * 4;
+    // the words (pawcs_internal.h): [2][L][npx], three channels in three planes
+    sz[PL_WA] = 2 * (size_t)L * npx * 16;
+    sz[PL_WLAST] = C == 3 ? 2 * (size_t)L * npx * 4 : 0;
+    sz[PL_WC2] = C == 3 ? 2 * (size_t)L * npx : 0;
     sz[PL_ILLUM] = sz[PL_UNST] = sz[PL_ROI] = sz[PL_BLINKS] = sz[PL_LASTRAWFG] = sz[PL_LASTFG] = sz[PL_DILINV] =
         sz[PL_LASTRAWBLINK] = npx;
     sz[PL_LASTCOL] = npx * C;
@@ -709,11 +709,9 @@ void pw_fill(lvbgs_ctx* h, const PwLayout& Lo, int L, int G) {
     D.nmv = (unsigned)h->prm.samples_for_moving_avgs;
     D.relThr = h->prm.rel_lbsp_threshold;
     D.lbspOff = (unsigned)h->prm.lbsp_threshold_offset;
-    D.wColor = b + Lo.off[PL_WCOLOR];
-    D.wDesc = (uint16_t*)(b + Lo.off[PL_WDESC]);
-    D.wOcc = (uint32_t*)(b + Lo.off[PL_WOCC]);
-    D.wFirst = (uint32_t*)(b + Lo.off[PL_WFIRST]);
+    D.wA = (uint4*)(b + Lo.off[PL_WA]);
     D.wLast = (uint32_t*)(b + Lo.off[PL_WLAST]);
+    D.wC2 = b + Lo.off[PL_WC2];
     D.illum = b + Lo.off[PL_ILLUM];
     D.unstable = b + Lo.off[PL_UNST];
     D.glut = b + Lo.off[PL_GLUT];
@@ -1059,9 +1057,16 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool& motion) {
         // camera-motion comparison (:1480-1501): the host waits for the decision, which may switch the
         // local word weight offset and run refreshModel(1, 1, true)
         const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
-        if (c3) pw3_k_motion_bg<<<(nds + 255) / 256, 256, 0, st>>>(P, nxt);
-        else pw_k_motion_bg<<<(nds + 255) / 256, 256, 0, st>>>(P, nxt);
-        pw_k_motion_decide<<<1, 32, 0, st>>>(P);
+        // the frame's background image goes to the label buffer (free after the hole filling, 4 bytes a pixel)
+        uint8_t* bg = (uint8_t*)h->sd.label;
+        if (c3) {
+            pw3_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
+            pw3_k_motion_bg<<<(nds + 31) / 32, 256, 0, st>>>(P);
+        } else {
+            pw_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
+            pw_k_motion_bg<<<(nds + 31) / 32, 256, 0, st>>>(P);
+        }
+        pw_k_motion_decide<<<1, 256, 0, st>>>(P);
         LV_CUDA(h, cudaGetLastError(), "PAWCS camera-motion launch");
         LV_CUDA(h, cudaMemcpyAsync(h->h_flags + 1, h->d_flags + 1, 8, cudaMemcpyDeviceToHost, st), "flag read-back");
     }
@@ -1854,8 +1859,8 @@ lvbgs_status lvbgs_get_background(lvbgs_handle h, uint8_t* out) {
     if (h->algo == LVBGS_ALGO_PAWCS) {
         const bool dev = is_device_ptr(out);
         uint8_t* d = dev ? out : h->d_frame;
-        if (h->C == 3) pw3_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), d, nullptr);
-        else pw_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), d, nullptr);
+        if (h->C == 3) pw3_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), d, nullptr, 0);
+        else pw_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), d, nullptr, 0);
         LV_CUDA(h, cudaGetLastError(), "background kernel");
         if (!dev) LV_CUDA(h, cudaMemcpyAsync(out, d, h->npx * h->C, cudaMemcpyDeviceToHost, h->stream), "download");
         LV_CUDA(h, cudaStreamSynchronize(h->stream), "background image");
@@ -1884,9 +1889,9 @@ lvbgs_status lvbgs_get_background_descriptors(lvbgs_handle h, uint16_t* out) {
     uint16_t* d = nullptr;
     LV_CUDA(h, cudaMallocAsync((void**)&d, h->npx * h->C * 2, h->stream), "temporary allocation");
     if (h->algo == LVBGS_ALGO_PAWCS && h->C == 3)
-        pw3_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), nullptr, d);
+        pw3_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), nullptr, d, 0);
     else if (h->algo == LVBGS_ALGO_PAWCS)
-        pw_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), nullptr, d);
+        pw_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), nullptr, d, 0);
     else lvbgs_background<<<512, 256, 0, h->stream>>>(h->sd, nullptr, d);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, h->npx * h->C * 2, cudaMemcpyDefault, h->stream);
@@ -2437,30 +2442,43 @@ lvbgs_status lvbgs_pawcs_debug_export(lvbgs_handle h, int which, void* out, size
         case LVBGS_PAWCS_MAP_LW_COLOR: case LVBGS_PAWCS_MAP_LW_DESC: case LVBGS_PAWCS_MAP_LW_OCC:
         case LVBGS_PAWCS_MAP_LW_FIRST: case LVBGS_PAWCS_MAP_LW_LAST: {
             // model-major (ROI pixels in raster order), slot-minor, as the reference's dictionary
-            const size_t es = which == LVBGS_PAWCS_MAP_LW_COLOR  ? (size_t)h->C
-                              : which == LVBGS_PAWCS_MAP_LW_DESC ? 2 * (size_t)h->C
-                                                                 : 4;
-            const void* src = which == LVBGS_PAWCS_MAP_LW_COLOR  ? (const void*)h->pd.wColor
-                              : which == LVBGS_PAWCS_MAP_LW_DESC ? (const void*)h->pd.wDesc
-                              : which == LVBGS_PAWCS_MAP_LW_OCC  ? (const void*)h->pd.wOcc
-                              : which == LVBGS_PAWCS_MAP_LW_FIRST ? (const void*)h->pd.wFirst
-                                                                  : (const void*)h->pd.wLast;
-            std::vector<uint8_t> planes(L * npx * es);
-            e = dl(planes.data(), (const uint8_t*)src + (size_t)buf * L * npx * es, planes.size());
+            const size_t n = L * npx, o = (size_t)buf * n;
+            std::vector<uint4> wa(n);
+            std::vector<uint32_t> wl(h->C == 3 ? n : 0);
+            std::vector<uint8_t> wc2(h->C == 3 ? n : 0);
+            e = dl(wa.data(), h->pd.wA + o, n * sizeof(uint4));
+            if (e == cudaSuccess && h->C == 3) e = dl(wl.data(), h->pd.wLast + o, n * 4);
+            if (e == cudaSuccess && h->C == 3) e = dl(wc2.data(), h->pd.wC2 + o, n);
             size_t m = 0;
-            for (size_t i = 0; i < npx; ++i) {
+            for (size_t i = 0; i < npx && e == cudaSuccess; ++i) {
                 if (!h->roi[i]) continue;
                 for (size_t j = 0; j < L; ++j) {
-                    const size_t k = m * L + j;
-                    const uint8_t* v = planes.data() + (j * npx + i) * es;
-                    if (es == 4) {
-                        uint32_t u;
-                        std::memcpy(&u, v, 4);
-                        const uint64_t u64 = u;
-                        std::memcpy((uint8_t*)out + k * 8, &u64, 8);
+                    const size_t k = m * L + j, v = j * npx + i;
+                    const uint4 w = wa[v];
+                    uint8_t col[3];
+                    uint16_t desc[3];
+                    uint64_t occ, first, last;
+                    if (h->C == 3) {
+                        col[0] = (uint8_t)(w.y >> 16);
+                        col[1] = (uint8_t)(w.y >> 24);
+                        col[2] = wc2[v];
+                        desc[0] = (uint16_t)w.x;
+                        desc[1] = (uint16_t)(w.x >> 16);
+                        desc[2] = (uint16_t)w.y;
+                        occ = w.z;
+                        first = w.w;
+                        last = wl[v];
                     } else {
-                        std::memcpy((uint8_t*)out + k * es, v, es);
+                        col[0] = (uint8_t)(w.w >> 16);
+                        desc[0] = (uint16_t)w.w;
+                        occ = w.x;
+                        first = w.y;
+                        last = w.z;
                     }
+                    uint8_t* d = (uint8_t*)out;
+                    if (which == LVBGS_PAWCS_MAP_LW_COLOR) std::memcpy(d + k * h->C, col, h->C);
+                    else if (which == LVBGS_PAWCS_MAP_LW_DESC) std::memcpy(d + k * 2 * h->C, desc, 2 * h->C);
+                    else std::memcpy(d + k * 8, which == LVBGS_PAWCS_MAP_LW_OCC ? &occ : which == LVBGS_PAWCS_MAP_LW_FIRST ? &first : &last, 8);
                 }
                 ++m;
             }

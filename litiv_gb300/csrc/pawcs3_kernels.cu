@@ -25,41 +25,6 @@
 
 namespace lvbgs {
 
-// one local word of a three-channel dictionary
-struct Pw3Word {
-    uint32_t col;   // packed colour
-    uint32_t d01;   // descriptors of channels 0 and 1
-    uint32_t d2;    // descriptor of channel 2
-    uint32_t occ, first, last;
-};
-
-__device__ __forceinline__ Pw3Word pw3_load(const PawcsDev& S, int buf, int j, int p) {
-    const size_t a = pw_slot(S, buf, j, p);
-    const uint8_t* c = S.wColor + a * 3;
-    const uint16_t* d = S.wDesc + a * 3;
-    Pw3Word w;
-    w.col = (uint32_t)c[0] | ((uint32_t)c[1] << 8) | ((uint32_t)c[2] << 16);
-    w.d01 = (uint32_t)d[0] | ((uint32_t)d[1] << 16);
-    w.d2 = d[2];
-    w.occ = S.wOcc[a];
-    w.first = S.wFirst[a];
-    w.last = S.wLast[a];
-    return w;
-}
-__device__ __forceinline__ void pw3_store(const PawcsDev& S, int buf, int j, int p, const Pw3Word& w) {
-    const size_t a = pw_slot(S, buf, j, p);
-    uint8_t* c = S.wColor + a * 3;
-    uint16_t* d = S.wDesc + a * 3;
-    c[0] = (uint8_t)w.col;
-    c[1] = (uint8_t)(w.col >> 8);
-    c[2] = (uint8_t)(w.col >> 16);
-    d[0] = (uint16_t)w.d01;
-    d[1] = (uint16_t)(w.d01 >> 16);
-    d[2] = (uint16_t)w.d2;
-    S.wOcc[a] = w.occ;
-    S.wFirst[a] = w.first;
-    S.wLast[a] = w.last;
-}
 __device__ __forceinline__ void pw3_desc(const uint16_t* base, int p, uint32_t& d01, uint32_t& d2) {
     const uint16_t* d = base + (size_t)p * 3;
     d01 = (uint32_t)d[0] | ((uint32_t)d[1] << 16);
@@ -109,44 +74,61 @@ __device__ __forceinline__ Pw3Upd pw3_updater(const PawcsDev& S, int p, int cur,
     return u;
 }
 
-// the neighbour-update loop of updater u over the target's words wd (:1197-1262, three channels: the
-// words are edited in place); rawQ is the target's raw decision as the updater sees it, (lq01, lq2)
-// its last descriptor; k advances by the loop's draws
-__device__ void pw3_loop(Pw3Word* wd, int L, const Pw3Upd& u, int boot, unsigned long long seed, uint32_t t,
-                         unsigned long long off, int rawQ, uint32_t lq01, uint32_t lq2, uint32_t& k) {
-    const uint32_t nlastDist = pw3_hd(u.d01, u.d2, lq01, lq2);
-    const bool nlastFlat = pw3_bits(lq01, lq2) < kPw3Flat;
-    float nsum = 0.0f;
-    for (int j = 0; j < L && nsum < u.thrW; ++j) {
-        Pw3Word& w = wd[j];
+// The neighbour-update loop of an updater over its target's words (:1197-1262, three channels: the words are
+// edited in place), one word at a time. An updater's loop touches words in slot order, and what it does to a
+// word depends on that word and on its own sum and draws so far, so the loops of several updaters (in raster
+// order) can run word by word: word j after all of them, then word j + 1. The dictionary thus streams through
+// registers once, where a pixel's 50 words had to be held in memory for loop after loop.
+struct Pw3Loop {
+    Pw3Upd u;
+    uint32_t nlastDist, k;
+    float nsum;
+    int nlastFlat;
+};
+// (lq01, lq2): the target's last descriptor as the updater sees it; k: the loop's first draw
+__device__ __forceinline__ void pw3_loop_init(Pw3Loop& l, const Pw3Upd& u, uint32_t lq01, uint32_t lq2, uint32_t k) {
+    l.u = u;
+    l.nlastDist = pw3_hd(u.d01, u.d2, lq01, lq2);
+    l.nlastFlat = pw3_bits(lq01, lq2) < kPw3Flat;
+    l.nsum = 0.0f;
+    l.k = k;
+}
+// rawQ is the target's raw decision as the updater sees it; last: word L - 1, where a loop that found too
+// little weight puts its own word
+__device__ __forceinline__ void pw3_loop_word(Pw3Word& w, Pw3Loop& l, bool last, int boot, unsigned long long seed,
+                                              uint32_t t, unsigned long long off, int rawQ) {
+    const Pw3Upd& u = l.u;
+    if (l.nsum < u.thrW) {
         const uint32_t l1 = pw3_l1(u.col, w.col), ncd = pw3_cdist(u.col, w.col);
         const uint32_t ncolorDist = l1 / 2u + ncd * 4u;
         const uint32_t nintra = pw3_hd(u.d01, u.d2, w.d01, w.d2);
         const uint32_t nincr = pw3_bits(w.d01, w.d2) < kPw3Flat ? u.incr * 2u : u.incr;
+        bool seen = false;
         if (ncolorDist <= u.th.color && nintra <= u.th.desc) {
+            seen = true;
+        } else if (!rawQ && u.flat && (boot || pw_mod(pw_draw(seed, t, u.p, l.k++), u.rate) == 0u)) {
+            if (ncolorDist <= u.th.color && l.nlastDist <= u.th.desc / 2u) {
+                seen = true;
+            } else if (l.nlastFlat && u.flat && l.nlastDist + nintra <= u.th.desc && ncd <= u.th.color / 4u) {
+                seen = true;
+            }
+        }
+        if (seen) {
             const float nwW = pw3_weight(w, t, off);
-            nsum += nwW;
+            l.nsum += nwW;
             w.last = t;
             if (nwW < 1.0f) w.occ += nincr;
-        } else if (!rawQ && u.flat && (boot || pw_mod(pw_draw(seed, t, u.p, k++), u.rate) == 0u)) {
-            if (ncolorDist <= u.th.color && nlastDist <= u.th.desc / 2u) {
-                const float nwW = pw3_weight(w, t, off);
-                nsum += nwW;
-                w.last = t;
-                if (nwW < 1.0f) w.occ += nincr;
-                w.d01 = u.d01;
-                w.d2 = u.d2;
-            } else if (nlastFlat && u.flat && nlastDist + nintra <= u.th.desc && ncd <= u.th.color / 4u) {
-                const float nwW = pw3_weight(w, t, off);
-                nsum += nwW;
-                w.last = t;
-                if (nwW < 1.0f) w.occ += nincr;
-                w.col = u.col;
+            if (!(ncolorDist <= u.th.color && nintra <= u.th.desc)) {
+                if (ncolorDist <= u.th.color && l.nlastDist <= u.th.desc / 2u) {
+                    w.d01 = u.d01;
+                    w.d2 = u.d2;
+                } else {
+                    w.col = u.col;
+                }
             }
         }
     }
-    if (nsum < 1.0f / (float)off) {
-        Pw3Word& w = wd[L - 1];
+    if (last && l.nsum < 1.0f / (float)off) {
         w.col = u.col;
         w.d01 = u.d01;
         w.d2 = u.d2;
@@ -170,9 +152,12 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // ------------------------------------------------------------------------------------------
 // local pass (:1011-1126): the dictionary at the pixel's turn (frame-start words after its earlier
 // updaters' loops, in raster order), then its word scan. Writes the scanned dictionary (next-frame
-// buffer; illumination updates as marks) and the record.
+// buffer; illumination updates as marks) and the record. The words stream through registers: a word is
+// read, edited by the updaters' loops, matched, and written one slot later (the scan's bubble pass holds
+// back one word, the lightest so far), so a pixel needs no copy of its 50 words. The copy took 1.2 KB of
+// local memory a pixel, three times what the L1 caches hold, and a word nine accesses.
 // ------------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
+extern "C" __global__ void __launch_bounds__(256, 2) pw3_k_local(PwParams P) {
     PW_ROUND_GUARD(P);
     PW3_PIXEL_PROLOGUE
     if (x >= D.W || y >= D.H) return;
@@ -187,34 +172,36 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
     const int L = S.L;
     const unsigned long long off = pc->lword_offset;
     const int boot = t <= (uint32_t)kBootWin;
-    Pw3Word wd[kPw3MaxLocal];
-    for (int j = 0; j < L; ++j) wd[j] = pw3_load(S, cur, j, q);
-    // earlier updaters' loops (from the previous round's outcomes; none known in round 0)
+    const size_t npx = (size_t)D.npx;
+    size_t src = pw_slot(S, cur, 0, q), dst = pw_slot(S, nxt, 0, q);
+    Pw3Raw next = pw3_fetch(S, src);
+    // earlier updaters (from the previous round's outcomes; none known in round 0)
+    Pw3Loop up[12];
+    int nu = 0;
     if (P.round > 0) {
         uint32_t lq01, lq2;
         pw3_desc(D.lastDesc, q, lq01, lq2);
-        for (int dy = -2; dy <= 0; ++dy)
-            for (int dx = -2; dx <= 2; ++dx) {
-                if (dy == 0 && dx >= 0) break;
-                const int px = x + dx, py = y + dy;
-                if (px < 0 || py < 0 || px >= D.W) continue;
-                const int p = py * D.W + px;
-                if (!D.roi[p] || S.out[p].q != (uint32_t)q) continue;
-                const Pw3Upd u = pw3_updater(S, p, cur, t, P.lr);
-                uint32_t k = S.out[p].kLoop;
-                pw3_loop(wd, L, u, boot, D.seed, t, off, 0, lq01, lq2, k);
-                S.out[p].kEnd = (uint16_t)k;
-            }
+        uint32_t tq[12];
+#pragma unroll
+        for (int j = 0; j < 12; ++j) {
+            const int px = x + j % 5 - 2, py = y + j / 5 - 2;
+            tq[j] = (px >= 0 && py >= 0 && px < D.W && D.roi[py * D.W + px]) ? S.out[py * D.W + px].q : kPwNone;
+        }
+#pragma unroll 1
+        for (int j = 0; j < 12; ++j) {
+            if (tq[j] != (uint32_t)q) continue;
+            const int p = (y + j / 5 - 2) * D.W + x + j % 5 - 2;
+            pw3_loop_init(up[nu++], pw3_updater(S, p, cur, t, P.lr), lq01, lq2, S.out[p].kLoop);
+        }
     }
     // current descriptor (:1003-1010)
-    uint8_t taps[3][16];
-    pw3_taps(D.frame, D.W, x, y, taps);
+    uint32_t taps[3][4], dsc[3];
     const uint32_t col = pw3_color(D.frame, q);
-    uint32_t dsc[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
+        pw_taps<3>(D.frame, D.W, x, y, c, taps[c]);
         const uint32_t v = pw3_ch(col, c);
-        dsc[c] = pw_lbsp(taps[c], v, ctl->lut[v]);
+        dsc[c] = lbsp_thr(taps[c], v, ctl->lut[v]);
     }
     const uint32_t d01 = dsc[0] | (dsc[1] << 16), d2 = dsc[2];
     const uint32_t bits = pw3_bits(d01, d2);
@@ -232,84 +219,92 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
         const float T = fm[FM_T * D.npx + q];
         rate = flat ? (unsigned long long)ceilf(T + kTLower) / 2ull : (unsigned long long)ceilf(T);
     }
-    uint8_t ord[kPw3MaxLocal];
-    for (int j = 0; j < L; ++j) ord[j] = (uint8_t)j;
-    const uint32_t lastFG = D.lastFG[q];
-    const int moving = pc->moving_cam;
-    const float bestW = pw3_weight(wd[0], t, off);
-    const float thrW = bestW / (Rr * 2.0f);
+    const int occOn = !D.lastFG[q] || pc->moving_cam;
+    float thrW = 0.0f;
     uint32_t k = 0;
     float sumW = 0.0f, lastW = FLT_MAX;
     uint32_t minColor = 765, minDesc = 48;
-    unsigned long long mark0 = 0, mark1 = 0, matched = 0;
-    int any0 = 0;
+    unsigned long long m0 = 0, m1 = 0;  // illumination marks by final slot
+    int any0 = 0, any1 = 0;
     const unsigned long long rateHalf = rate / 2ull + 1ull;
-    int i = 0;
-    for (; i < L && sumW < thrW; ++i) {
-        const Pw3Word& w = wd[i];
-        const float cw = pw3_weight(w, t, off);
-        const uint32_t l1 = pw3_l1(col, w.col);
-        const uint32_t cd = l1 / 2u + pw3_cdist(col, w.col) * 4u;
-        const uint32_t intra = pw3_hd(d01, d2, w.d01, w.d2);
-        uint32_t inter = 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const uint32_t wc = pw3_ch(w.col, c);
-            const uint32_t wdc = c == 0 ? (w.d01 & 0xffffu) : c == 1 ? (w.d01 >> 16) : (w.d2 & 0xffffu);
-            inter += (uint32_t)__popc(pw_lbsp(taps[c], wc, ctl->lut[wc]) ^ wdc);
+    const bool illumOn = !unst || flat || border;
+    Pw3Word held;
+    held.col = held.d01 = held.d2 = held.occ = held.first = held.last = 0u;
+    unsigned heldMarks = 0;
+    for (int i = 0; i < L; ++i) {
+        Pw3Word w = pw3_unpack(next);
+        if (i + 1 < L) {
+            src += npx;
+            next = pw3_fetch(S, src);
         }
-        const uint32_t dd = (intra + inter) / 2u;
-        if ((!unst || flat || border) && cd <= th.color && l1 >= th.color / 2u && intra <= th.desc / 2u) {
-            // illumination update test (:1054): modulus halves (+1) once the mask is non-zero
-            const uint32_t r = pw_draw(D.seed, t, (uint32_t)q, k++);
-            if (pw_mod(r, rateHalf) == 0u) mark1 |= 1ull << i;
-            if (pw_mod(r, any0 ? rateHalf : rate) == 0u) {
-                mark0 |= 1ull << i;
-                any0 = 1;
+        for (int j = 0; j < nu; ++j) pw3_loop_word(w, up[j], i == L - 1, boot, D.seed, t, off, 0);
+        const float cw = pw3_weight(w, t, off);
+        if (i == 0) thrW = cw / (Rr * 2.0f);
+        unsigned marks = 0;
+        bool matched = false;
+        if (sumW < thrW) {
+            const uint32_t l1 = pw3_l1(col, w.col);
+            const uint32_t cd = l1 / 2u + pw3_cdist(col, w.col) * 4u;
+            if (cd <= th.color) {
+                const uint32_t intra = pw3_hd(d01, d2, w.d01, w.d2);
+                if (illumOn && l1 >= th.color / 2u && intra <= th.desc / 2u) {
+                    // illumination update test (:1054): modulus halves (+1) once the mask is non-zero
+                    const uint32_t r = pw_draw(D.seed, t, (uint32_t)q, k++);
+                    if (pw_mod(r, rateHalf) == 0u) marks |= 2u;
+                    if (pw_mod(r, any0 ? rateHalf : rate) == 0u) {
+                        marks |= 1u;
+                        any0 = 1;
+                    }
+                    any1 |= (int)(marks >> 1);
+                }
+                uint32_t inter = 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const uint32_t wc = pw3_ch(w.col, c);
+                    const uint32_t wdc = c == 0 ? w.d01 : c == 1 ? (w.d01 >> 16) : w.d2;
+                    inter += (uint32_t)__popc((lbsp_thr_raw(taps[c], wc, ctl->lut[wc]) ^ wdc) & 0xffffu);
+                }
+                const uint32_t dd = (intra + inter) / 2u;
+                if (dd <= th.desc) {
+                    sumW += cw;
+                    matched = true;
+                    minColor = min(minColor, cd);
+                    minDesc = min(minDesc, dd);
+                }
             }
         }
-        if (dd <= th.desc && cd <= th.color) {
-            sumW += cw;
-            matched |= 1ull << i;
-            minColor = min(minColor, cd);
-            minDesc = min(minDesc, dd);
-        }
-        if (cw > lastW) {
-            const uint8_t tmp = ord[i];
-            ord[i] = ord[i - 1];
-            ord[i - 1] = tmp;
-        } else {
-            lastW = cw;
-        }
-    }
-    for (; i < L; ++i) {
-        const float cw = pw3_weight(wd[i], t, off);
-        if (cw > lastW) {
-            const uint8_t tmp = ord[i];
-            ord[i] = ord[i - 1];
-            ord[i - 1] = tmp;
-        } else {
-            lastW = cw;
-        }
-    }
-    const int bg = sumW >= thrW || border;
-    const int occOn = !lastFG || moving;
-    unsigned long long m0 = 0, m1 = 0;
-    for (int s = 0; s < L; ++s) {
-        const int o = ord[s];
-        Pw3Word w = wd[o];
-        if (matched & (1ull << o)) {
-            const float cw = pw3_weight(w, t, off);
+        if (matched) {
             w.last = t;
             if (occOn && cw < 1.0f) w.occ += incr;
         }
-        pw3_store(S, nxt, s, q, w);
-        if (mark0 & (1ull << o)) m0 |= 1ull << s;
-        if (mark1 & (1ull << o)) m1 |= 1ull << s;
+        if (cw > lastW) {  // heavier than the held word: it takes the slot before it
+            pw3_put(S, dst, w);
+            if (marks) {
+                m0 |= (unsigned long long)(marks & 1u) << (i - 1);
+                m1 |= (unsigned long long)(marks >> 1) << (i - 1);
+            }
+            dst += npx;
+        } else {
+            if (i > 0) {
+                pw3_put(S, dst, held);
+                if (heldMarks) {
+                    m0 |= (unsigned long long)(heldMarks & 1u) << (i - 1);
+                    m1 |= (unsigned long long)(heldMarks >> 1) << (i - 1);
+                }
+                dst += npx;
+            }
+            held = w;
+            heldMarks = marks;
+            lastW = cw;
+        }
     }
+    m0 |= (unsigned long long)(heldMarks & 1u) << (L - 1);
+    m1 |= (unsigned long long)(heldMarks >> 1) << (L - 1);
+    for (int j = 0; j < nu; ++j) S.out[up[j].u.p].kEnd = (uint16_t)up[j].k;
+    const int bg = sumW >= thrW || border;
     const float initW = 1.0f / (float)off;
     uint8_t flags = (uint8_t)((bg ? kRfBG : 0) | (flat ? kRfFlat : 0) | (border ? kRfBorder : 0) |
-                              (mark0 ? kRfU0 : 0) | (mark1 ? kRfU1 : 0));
+                              (any0 ? kRfU0 : 0) | (any1 ? kRfU1 : 0));
     if (bg) {
         if (pw_mod(pw_draw(D.seed, t, (uint32_t)q, k), rate) == 0u) {
             flags |= kRfItem | kRfEvent;
@@ -319,21 +314,20 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
         if (flat || pw_mod(pw_draw(D.seed, t, (uint32_t)q, k), rate) == 0u) flags |= kRfItem;
         if (sumW < initW) {
             // new local word in the last slot (:1160-1168)
-            Pw3Word w;
-            w.col = col;
-            w.d01 = d01;
-            w.d2 = d2;
-            w.occ = incr;
-            w.first = t;
-            w.last = t;
-            pw3_store(S, nxt, L - 1, q, w);
+            held.col = col;
+            held.d01 = d01;
+            held.d2 = d2;
+            held.occ = incr;
+            held.first = t;
+            held.last = t;
         }
     }
+    pw3_put(S, dst, held);
     uint16_t* dt = S.descT + (size_t)q * 3;
     dt[0] = (uint16_t)dsc[0];
     dt[1] = (uint16_t)dsc[1];
     dt[2] = (uint16_t)dsc[2];
-    S.uv[q] = (uint8_t)((mark0 ? 1 : 0) | (mark1 ? 2 : 0));
+    S.uv[q] = (uint8_t)((any0 ? 1 : 0) | (any1 ? 2 : 0));
     PwRec& R = S.rec[q];
     R.sumW = sumW;
     R.thrW = thrW;
@@ -377,9 +371,10 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
             wrPos = g;
             continue;
         }
-        if (fixedPos == G && pw_absdiff(bits, pc->gw_bits[w]) <= th.desc / 4u && pw3_cmix(col, pc->gw_color[w]) <= th.color) {
-            fixedPos = g;
+        if (pw_absdiff(bits, pc->gw_bits[w]) <= th.desc / 4u && pw3_cmix(col, pc->gw_color[w]) <= th.color) {
+            fixedPos = g;  // a replaceable word further on is behind it
             fixedWord = w;
+            break;
         }
     }
     const int critical = wrPos < fixedPos;
@@ -777,52 +772,63 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
     const uint8_t u = S.uFinal[q];
     const unsigned long long m = (u & 2) ? (((unsigned long long)R.m1hi << 32) | R.m1)
                                          : (((unsigned long long)R.m0hi << 32) | R.m0);
-    // any later updater?
+    // later updaters: the pixel itself and the twelve later pixels of its window
     bool any = false;
-    for (int dy = 0; dy <= 2 && !any; ++dy)
-        for (int dx = -2; dx <= 2; ++dx) {
-            if (dy == 0 && dx < 0) continue;
-            const int px = x + dx, py = y + dy;
-            if (px < 0 || px >= D.W || py >= D.H) continue;
-            const int p = py * D.W + px;
-            if (D.roi[p] && S.out[p].q == (uint32_t)q) {
-                any = true;
-                break;
-            }
-        }
+    uint32_t tq[13];
+#pragma unroll
+    for (int j = 12; j < 25; ++j) {
+        const int px = x + j % 5 - 2, py = y + j / 5 - 2;
+        tq[j - 12] = (px >= 0 && px < D.W && py < D.H && D.roi[py * D.W + px]) ? S.out[py * D.W + px].q : kPwNone;
+        any |= tq[j - 12] == (uint32_t)q;
+    }
     if (!m && !any) return;
     const uint32_t col = pw3_color(D.frame, q);
     uint32_t d01, d2;
     pw3_desc(S.descT, q, d01, d2);
-    Pw3Word wd[kPw3MaxLocal];
-    for (int j = 0; j < L; ++j) {
-        wd[j] = pw3_load(S, nxt, j, q);
-        if (m & (1ull << j)) {
-            wd[j].col = col;
-            wd[j].d01 = d01;
-            wd[j].d2 = d2;
-        }
-    }
+    Pw3Loop up[13];
+    int nu = 0;
+    int rawQ = 0;
     if (any) {
-        const int rawQ = S.out[q].segm != 0;
+        rawQ = S.out[q].segm != 0;
         uint32_t pl01, pl2;
         pw3_desc(D.lastDesc, q, pl01, pl2);
-        for (int dy = 0; dy <= 2; ++dy)
-            for (int dx = -2; dx <= 2; ++dx) {
-                if (dy == 0 && dx < 0) continue;
-                const int px = x + dx, py = y + dy;
-                if (px < 0 || px >= D.W || py >= D.H) continue;
-                const int p = py * D.W + px;
-                if (!D.roi[p] || S.out[p].q != (uint32_t)q) continue;
-                const Pw3Upd up = pw3_updater(S, p, cur, t, P.lr);
-                uint32_t k = S.out[p].kLoop;
-                // the target's last descriptor is updated at the end of its own processing (:1290-1293)
-                if (p == q) pw3_loop(wd, L, up, boot, D.seed, t, off, rawQ, pl01, pl2, k);
-                else pw3_loop(wd, L, up, boot, D.seed, t, off, rawQ, d01, d2, k);
-                S.out[p].kEnd = (uint16_t)k;
-            }
+#pragma unroll 1
+        for (int j = 12; j < 25; ++j) {
+            if (tq[j - 12] != (uint32_t)q) continue;
+            const int p = (y + j / 5 - 2) * D.W + x + j % 5 - 2;
+            // the target's last descriptor is updated at the end of its own processing (:1290-1293)
+            const bool self = p == q;
+            pw3_loop_init(up[nu++], pw3_updater(S, p, cur, t, P.lr), self ? pl01 : d01, self ? pl2 : d2, S.out[p].kLoop);
+        }
     }
-    for (int j = 0; j < L; ++j) pw3_store(S, nxt, j, q, wd[j]);
+    // the words stream through registers up to the last one that a mark or a loop can still change; only
+    // changed words are written
+    const float initW = 1.0f / (float)off;
+    size_t slot = pw_slot(S, nxt, 0, q);
+    for (int i = 0; i < L; ++i, slot += (size_t)D.npx) {
+        bool scan = false, tail = false;
+        for (int j = 0; j < nu; ++j) {
+            scan |= up[j].nsum < up[j].u.thrW;
+            tail |= up[j].nsum < initW;
+        }
+        const bool mark = (m >> i) & 1ull;
+        if (!mark && !scan && !(tail && i == L - 1)) {
+            if (!tail && !(m >> i)) break;
+            continue;
+        }
+        Pw3Word w = pw3_load(S, nxt, i, q);
+        const Pw3Word before = w;
+        if (mark) {
+            w.col = col;
+            w.d01 = d01;
+            w.d2 = d2;
+        }
+        for (int j = 0; j < nu; ++j) pw3_loop_word(w, up[j], i == L - 1, boot, D.seed, t, off, rawQ);
+        if (w.col != before.col || w.d01 != before.d01 || w.d2 != before.d2 || w.occ != before.occ ||
+            w.first != before.first || w.last != before.last)
+            pw3_put(S, slot, w);
+    }
+    for (int j = 0; j < nu; ++j) S.out[up[j].u.p].kEnd = (uint16_t)up[j].k;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -953,39 +959,26 @@ extern "C" __global__ void pw3_k_ds(PwParams P) {
     S.dsAbs[i] = S.dsRoi[i] ? e : 0.0f;
 }
 
-// camera-motion comparison (:1480-1501), three channels: the background image of the words of buffer
-// buf, area-down-sampled, against the long-term means: L1 over the channels into dsAbs and the float
+// camera-motion comparison (:1480-1501), three channels: the background image (left in the label buffer by
+// the background kernel, a pixel per thread), area-down-sampled, against the long-term means: L1 over the channels into dsAbs and the float
 // colour distortion (lv::cdist<3>, math.hpp:499-527) into contrib; 0 outside the fully covered blocks
-extern "C" __global__ void pw3_k_motion_bg(PwParams P, int buf) {
+extern "C" __global__ void pw3_k_motion_bg(PwParams P) {
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per output
     if (i >= nds) return;
     if (S.dsRoi[i] != 255) {
         S.dsAbs[i] = 0.0f;
         S.contrib[i] = 0.0f;
         return;
     }
-    const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
-    const unsigned long long off = S.pc->lword_offset;
-    const int bx = i % D.dsW, by = i / D.dsW;
+    uint32_t vb[3];
+    area_resample_group<3>((const uint8_t*)D.label, D.W, D.H, D.dsW, D.dsH, i % D.dsW, i / D.dsW, vb);
+    if (threadIdx.x & 7) return;
     float a[3], b[3], e = 0.0f;
     for (int c = 0; c < 3; ++c) {
-        // channel c of the background image (0 outside the ROI), area-down-sampled
-        b[c] = (float)area_resample(D.W, D.H, D.dsW, D.dsH, bx, by, [&](int sx, int sy) {
-            const int p = sy * D.W + sx;
-            if (!D.roi[p]) return 0;
-            float tw = 0.0f, tc = 0.0f;
-            for (int j = 0; j < S.L; ++j) {
-                const size_t a = pw_slot(S, buf, j, p);
-                const float w = pw_weight(S.wOcc[a], S.wFirst[a], S.wLast[a], t, off);
-                tc = tc + (float)S.wColor[a * 3 + c] * w;
-                tw = tw + w;
-            }
-            const int r = __float2int_rn(tc / tw);
-            return r < 0 ? 0 : r > 255 ? 255 : r;
-        });
+        b[c] = (float)vb[c];
         a[c] = D.dsLT[(size_t)i * 3 + c];
         e = e + fabsf(a[c] - b[c]);
     }
@@ -1209,9 +1202,11 @@ extern "C" __global__ void pw3_k_init_last(PawcsDev S, const uint8_t* img) {
         if (D.roi[p]) {
             for (int k = 0; k < 3; ++k) c[k] = img[(size_t)p * 3 + k];
             if (x > 2 && y > 2 && x < D.W - 2 && y < D.H - 2) {
-                uint8_t taps[3][16];
-                pw3_taps(img, D.W, x, y, taps);
-                for (int k = 0; k < 3; ++k) d[k] = (uint16_t)pw_lbsp(taps[k], c[k], D.ctl->lut[c[k]]);
+                for (int k = 0; k < 3; ++k) {
+                    uint32_t taps[4];
+                    pw_taps<3>(img, D.W, x, y, k, taps);
+                    d[k] = (uint16_t)lbsp_thr(taps, c[k], D.ctl->lut[c[k]]);
+                }
             }
         }
         for (int k = 0; k < 3; ++k) {
@@ -1222,9 +1217,9 @@ extern "C" __global__ void pw3_k_init_last(PawcsDev S, const uint8_t* img) {
 }
 
 // background image / descriptors (:1518-1594), three channels
-extern "C" __global__ void pw3_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc) {
+extern "C" __global__ void pw3_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc, int ahead) {
     const StreamDev& D = S.sd;
-    const uint32_t t = (uint32_t)D.ctl->frame_idx;
+    const uint32_t t = (uint32_t)D.ctl->frame_idx + (uint32_t)ahead;
     const unsigned long long off = S.pc->lword_offset;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.npx; p += gridDim.x * blockDim.x) {
         if (!D.roi[p]) {
@@ -1236,11 +1231,12 @@ extern "C" __global__ void pw3_k_background(PawcsDev S, int buf, uint8_t* outCol
         }
         float tw = 0.0f, tc[3] = {0.0f, 0.0f, 0.0f}, td[3] = {0.0f, 0.0f, 0.0f};
         for (int j = 0; j < S.L; ++j) {
-            const size_t a = pw_slot(S, buf, j, p);
-            const float w = pw_weight(S.wOcc[a], S.wFirst[a], S.wLast[a], t, off);
+            const Pw3Word wj = pw3_load(S, buf, j, p);
+            const float w = pw3_weight(wj, t, off);
+            const uint32_t dj[3] = {wj.d01 & 0xffffu, wj.d01 >> 16, wj.d2};
             for (int c = 0; c < 3; ++c) {
-                tc[c] = tc[c] + (float)S.wColor[a * 3 + c] * w;
-                td[c] = td[c] + (float)S.wDesc[a * 3 + c] * w;
+                tc[c] = tc[c] + (float)pw3_ch(wj.col, c) * w;
+                td[c] = td[c] + (float)dj[c] * w;
             }
             tw = tw + w;
         }

@@ -48,11 +48,13 @@ __device__ __forceinline__ uint32_t pw_mod(uint32_t r, unsigned long long m) {
     return m > 0xffffffffull ? r : r % (uint32_t)m;
 }
 
-// GetLocalWordWeight (:1596-1598): (float)occ / (float)((last-first) + (t-last)*2 + offset)
+// GetLocalWordWeight (:1596-1598): (float)occ / (float)((last-first) + (t-last)*2 + offset). The denominator
+// nearly always fits 32 bits, whose conversion is the same number and a quarter of the work.
 __device__ __forceinline__ float pw_weight(uint32_t occ, uint32_t first, uint32_t last, uint32_t t,
                                            unsigned long long off) {
     const unsigned long long den = (unsigned long long)(last - first) + (unsigned long long)(t - last) * 2ull + off;
-    return (float)occ / (float)den;
+    const float fd = (den >> 32) ? (float)den : (float)(uint32_t)den;
+    return (float)occ / fd;
 }
 
 struct PwThr {
@@ -90,16 +92,20 @@ __device__ __forceinline__ PwThr pw_thresholds(float R, uint32_t unstable, uint3
 
 __device__ __forceinline__ uint32_t pw_absdiff(uint32_t a, uint32_t b) { return a > b ? a - b : b - a; }
 
-// current frame: LBSP lookups of pixel (x, y) and its descriptor
-__device__ __forceinline__ void pw_taps(const uint8_t* img, int W, int x, int y, uint8_t taps[16]) {
+// the 16 LBSP taps of channel c at pixel (x, y) of a dense C-channel image, four to a word (lbsp_thr's packing)
+template <int C>
+__device__ __forceinline__ void pw_taps(const uint8_t* img, int W, int x, int y, int c, uint32_t (&v)[4]) {
+    const uint8_t* base = img + ((size_t)y * W + x) * C + c;
 #pragma unroll
-    for (int n = 0; n < 16; ++n) taps[n] = __ldg(img + (size_t)(y + lbsp_dy(n)) * W + (x + lbsp_dx(n)));
-}
-__device__ __forceinline__ uint32_t pw_lbsp(const uint8_t taps[16], uint32_t ref, uint32_t thr) {
-    uint32_t d = 0;
+    for (int j = 0; j < 4; ++j) {
+        uint32_t w = 0;
 #pragma unroll
-    for (int n = 0; n < 16; ++n) d |= (uint32_t)(pw_absdiff(taps[n], ref) > thr) << n;
-    return d;
+        for (int i = 0; i < 4; ++i) {
+            const int n = 4 * j + i;
+            w |= (uint32_t)__ldg(base + (lbsp_dy(n) * W + lbsp_dx(n)) * C) << (8 * i);
+        }
+        v[j] = w;
+    }
 }
 
 // rolling-average factors of frame f (:570-573)
@@ -112,6 +118,46 @@ __device__ __forceinline__ void pw_factors(unsigned long long f, int nmv, float*
 
 __device__ __forceinline__ size_t pw_slot(const PawcsDev& S, int buf, int j, int p) {
     return ((size_t)buf * S.L + j) * S.sd.npx + p;
+}
+
+// one local word of a one-channel dictionary
+struct PwWord {
+    uint32_t occ, first, last, desc, col;
+};
+__device__ __forceinline__ PwWord pw_load(const PawcsDev& S, size_t slot) {
+    const uint4 v = S.wA[slot];
+    return {v.x, v.y, v.z, v.w & 0xffffu, v.w >> 16};
+}
+__device__ __forceinline__ void pw_store(const PawcsDev& S, size_t slot, const PwWord& w) {
+    S.wA[slot] = make_uint4(w.occ, w.first, w.last, w.desc | (w.col << 16));
+}
+// one local word of a three-channel dictionary
+struct Pw3Word {
+    uint32_t col;   // packed colour
+    uint32_t d01;   // descriptors of channels 0 and 1
+    uint32_t d2;    // descriptor of channel 2
+    uint32_t occ, first, last;
+};
+struct Pw3Raw {  // as stored
+    uint4 a;
+    uint32_t last, c2;
+};
+__device__ __forceinline__ Pw3Raw pw3_fetch(const PawcsDev& S, size_t slot) {
+    return {S.wA[slot], S.wLast[slot], S.wC2[slot]};
+}
+__device__ __forceinline__ Pw3Word pw3_unpack(const Pw3Raw& r) {
+    return {(r.a.y >> 16) | (r.c2 << 16), r.a.x, r.a.y & 0xffffu, r.a.z, r.a.w, r.last};
+}
+__device__ __forceinline__ Pw3Word pw3_load(const PawcsDev& S, int buf, int j, int p) {
+    return pw3_unpack(pw3_fetch(S, pw_slot(S, buf, j, p)));
+}
+__device__ __forceinline__ void pw3_put(const PawcsDev& S, size_t slot, const Pw3Word& w) {
+    S.wA[slot] = make_uint4(w.d01, (w.d2 & 0xffffu) | (w.col << 16), w.occ, w.first);
+    S.wLast[slot] = w.last;
+    S.wC2[slot] = (uint8_t)(w.col >> 16);
+}
+__device__ __forceinline__ void pw3_store(const PawcsDev& S, int buf, int j, int p, const Pw3Word& w) {
+    pw3_put(S, pw_slot(S, buf, j, p), w);
 }
 
 }  // namespace lvbgs
@@ -134,36 +180,35 @@ __device__ __forceinline__ uint32_t pw3_ch(uint32_t c, int k) { return (c >> (8 
 // the type of L1dist(uchar, uchar), unsigned char, so it wraps modulo 256 (every three-channel colour
 // L1 of PAWCS goes through it, directly or through cmixdist)
 __device__ __forceinline__ uint32_t pw3_l1(uint32_t a, uint32_t b) {
-    return (pw_absdiff(pw3_ch(a, 0), pw3_ch(b, 0)) + pw_absdiff(pw3_ch(a, 1), pw3_ch(b, 1)) +
-            pw_absdiff(pw3_ch(a, 2), pw3_ch(b, 2))) & 0xffu;
+    return __dp4a(__vabsdiffu4(a, b), 0x00010101u, 0u) & 0xffu;
 }
 // lv::cdist<3> of two byte colours (math.hpp:474-496): sqrt of the colour distortion, 0 for a grey
-// pair or identical colours
+// pair or identical colours: floor(sqrt(|a|^2 - floor((a.b)^2 / |b|^2))). The products are byte dot products;
+// the quotient is at most |a|^2 < 2^18 (Cauchy-Schwarz), so a single-precision estimate is off by less than
+// one and the remainder corrects it (it lies within one divisor of its range, so 32-bit arithmetic holds it);
+// the root of an integer below 2^18 likewise. 64-bit division and the rounded square root cost ~100
+// instructions for each word, of ~250 in all.
 __device__ __forceinline__ uint32_t pw3_cdist(uint32_t a, uint32_t b) {
-    const uint32_t a0 = pw3_ch(a, 0), a1 = pw3_ch(a, 1), a2 = pw3_ch(a, 2);
-    const uint32_t b0 = pw3_ch(b, 0), b1 = pw3_ch(b, 1), b2 = pw3_ch(b, 2);
-    const bool nonconst = a1 != a0 || b1 != b0 || a2 != a1 || b2 != b1;
-    const bool nonnull = a0 != b0 || a1 != b1 || a2 != b2;
-    if (!nonconst || !nonnull) return 0u;
-    const unsigned long long cs = a0 * a0 + a1 * a1 + a2 * a2, bs = b0 * b0 + b1 * b1 + b2 * b2;
-    const unsigned long long mix = a0 * b0 + a1 * b1 + a2 * b2;
-    const float sq = (float)(cs - (mix * mix) / (bs > 1ull ? bs : 1ull));
-    return (uint32_t)__fsqrt_rn(sq);
+    const bool grey = a == (a & 0xffu) * 0x010101u && b == (b & 0xffu) * 0x010101u;
+    if (grey || a == b) return 0u;
+    const uint32_t cs = __dp4a(a, a, 0u), bs = max(__dp4a(b, b, 0u), 1u), mix = __dp4a(a, b, 0u);
+    const float fm = (float)mix;
+    uint32_t q = (uint32_t)(fm * __fdividef(fm, (float)bs));
+    const int r = (int)(mix * mix - q * bs);
+    if (r < 0) --q;
+    else if (r >= (int)bs) ++q;
+    const uint32_t n = cs - q;
+    float root;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"((float)n));
+    uint32_t k = (uint32_t)root;
+    if (k * k > n) --k;
+    else if ((k + 1u) * (k + 1u) <= n) ++k;
+    return k;
 }
 // lv::cmixdist (math.hpp:596-605)
 __device__ __forceinline__ uint32_t pw3_cmix(uint32_t a, uint32_t b) { return pw3_l1(a, b) / 2u + pw3_cdist(a, b) * 4u; }
 __device__ __forceinline__ uint32_t pw3_hd(uint32_t a01, uint32_t a2, uint32_t b01, uint32_t b2) {
     return (uint32_t)__popc(a01 ^ b01) + (uint32_t)__popc((a2 ^ b2) & 0xffffu);
-}
-// the 16 taps of each channel of pixel (x, y) of an interleaved BGR frame
-__device__ __forceinline__ void pw3_taps(const uint8_t* img, int W, int x, int y, uint8_t taps[3][16]) {
-#pragma unroll
-    for (int n = 0; n < 16; ++n) {
-        const uint8_t* q = img + ((size_t)(y + lbsp_dy(n)) * W + (x + lbsp_dx(n))) * 3;
-        taps[0][n] = q[0];
-        taps[1][n] = q[1];
-        taps[2][n] = q[2];
-    }
 }
 __device__ __forceinline__ uint32_t pw3_color(const uint8_t* img, int p) {
     const uint8_t* q = img + (size_t)p * 3;

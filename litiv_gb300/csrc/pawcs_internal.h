@@ -97,10 +97,13 @@ struct PawcsDev {
     unsigned int minColor, descOff, nmv;  // m_nMinColorDistThreshold, m_nDescDistThresholdOffset, samples for averages
     float relThr;
     unsigned int lbspOff;
-    // local dictionaries, slot-major planes [2][L][npx] by frame parity
-    uint8_t* wColor;
-    uint16_t* wDesc;
-    uint32_t *wOcc, *wFirst, *wLast;
+    // local dictionaries, slot-major planes [2][L][npx] by frame parity. One channel: a word is one uint4
+    // (occurrences, first frame, last frame, descriptor | colour << 16). Three: a uint4 (descriptors 0 and 1,
+    // descriptor 2 | colours 0 and 1 << 16, occurrences, first frame), the last frame and the byte of colour 2,
+    // 21 bytes in three accesses that a warp makes in whole lines.
+    uint4* wA;
+    uint32_t* wLast;
+    uint8_t* wC2;
     uint8_t* illum;            // m_oIllumUpdtRegionMask
     uint8_t* unstable;         // m_oUnstableRegionMask
     uint8_t* glut;             // [npx][16] per-pixel global word order (pool indices)

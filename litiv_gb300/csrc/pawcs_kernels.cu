@@ -24,32 +24,22 @@ struct PwWordSrc {
     int repl;          // last slot replaced by source rsrc
     uint32_t rcol, rdesc, rincr, t;
 };
-__device__ __forceinline__ void pw_word(const PwWordSrc& s, int j, uint32_t& c, uint32_t& d, uint32_t& o, uint32_t& f,
-                                        uint32_t& l) {
-    if (s.repl && j == s.L - 1) {
-        c = s.rcol;
-        d = s.rdesc;
-        o = s.rincr;
-        f = s.t;
-        l = s.t;
-        return;
-    }
-    const size_t a = pw_slot(*s.S, s.buf, j, s.q);
-    c = s.S->wColor[a];
-    d = s.S->wDesc[a];
-    o = s.S->wOcc[a];
-    f = s.S->wFirst[a];
-    l = s.S->wLast[a];
+__device__ __forceinline__ PwWord pw_word(const PwWordSrc& s, int j) {
+    if (s.repl && j == s.L - 1) return {s.rincr, s.t, s.t, s.rdesc, s.rcol};
+    PwWord w = pw_load(*s.S, pw_slot(*s.S, s.buf, j, s.q));
     if (s.m & (1u << j)) {
-        c = s.qcol;
-        d = s.qdesc;
+        w.col = s.qcol;
+        w.desc = s.qdesc;
     }
+    return w;
 }
 
 // ------------------------------------------------------------------------------------------
 // local pass: the pixel's word scan (:632-748) against its dictionary at its turn -- the frame-start
 // dictionary with the last slot replaced by the latest earlier neighbour update, if any. Writes the
-// scanned dictionary (next-frame buffer, illumination updates not yet applied) and the record.
+// scanned dictionary (next-frame buffer, illumination updates not yet applied) and the record. The words
+// stream through registers: each is read once and written one slot later (the scan's bubble pass holds back
+// one word, the lightest so far), where every word was read again, in its new order, to be written.
 // ------------------------------------------------------------------------------------------
 __device__ void pw_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t col);
 
@@ -77,10 +67,10 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_local(PwParams P) {
     const unsigned long long off = pc->lword_offset;
     const int boot = t <= (uint32_t)kBootWin;
     // current descriptor
-    uint8_t taps[16];
-    pw_taps(D.frame, D.W, x, y, taps);
+    uint32_t taps[4];
+    pw_taps<1>(D.frame, D.W, x, y, 0, taps);
     const uint32_t col = D.frame[p];
-    const uint32_t desc = pw_lbsp(taps, col, ctl->lut[col]);
+    const uint32_t desc = lbsp_thr(taps, col, ctl->lut[col]);
     const uint32_t bits = __popc(desc);
     const int flat = bits < 2u;
     const int border = roi < 255;
@@ -99,103 +89,91 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_local(PwParams P) {
     }
     // the dictionary at the pixel's turn: the frame-start words (read-only in this pass), the last
     // one replaced by an earlier neighbour update (its colour and descriptor, occurrences = its incr)
-    PwWordSrc ws;
-    ws.S = &S;
-    ws.q = p;
-    ws.buf = cur;
-    ws.L = L;
-    ws.m = 0;
-    ws.repl = rsrc != kPwNone;
-    ws.t = t;
-    if (ws.repl) {
-        ws.rcol = D.frame[rsrc];
-        ws.rdesc = S.descT[rsrc];
-        ws.rincr = S.rec[rsrc].incr;
+    PwWord repl = {0u, t, t, 0u, 0u};
+    if (rsrc != kPwNone) {
+        repl.col = D.frame[rsrc];
+        repl.desc = S.descT[rsrc];
+        repl.occ = S.rec[rsrc].incr;
     }
-    uint8_t ord[kPwMaxLocal];
-    for (int j = 0; j < L; ++j) ord[j] = (uint8_t)j;
-    const uint32_t lastFG = D.lastFG[p];
-    const int moving = pc->moving_cam;
-    uint32_t c0, d0, o0, f0, l0;
-    pw_word(ws, 0, c0, d0, o0, f0, l0);
-    const float bestW = pw_weight(o0, f0, l0, t, off);
-    const float thrW = bestW / (Rr * 2.0f);
+    const int occOn = !D.lastFG[p] || pc->moving_cam;
+    float thrW = 0.0f;
     // word scan with one bubble pass
     uint32_t k = 0;
     float sumW = 0.0f, lastW = FLT_MAX;
     uint32_t minColor = 255, minDesc = 16;
-    uint32_t mark0 = 0, mark1 = 0, matched = 0;
-    int any0 = 0;
+    uint32_t m0 = 0, m1 = 0;  // illumination marks by final slot
+    int any0 = 0, any1 = 0;
     const unsigned long long rateHalf = rate / 2ull + 1ull;
-    int i = 0;
-    for (; i < L && sumW < thrW; ++i) {
-        uint32_t wci, wdi, woi, wfi, wli;
-        pw_word(ws, i, wci, wdi, woi, wfi, wli);
-        const float w = pw_weight(woi, wfi, wli, t, off);
-        const uint32_t cd = pw_absdiff(col, wci);
-        const uint32_t intra = __popc(desc ^ wdi);
-        const uint32_t inter = __popc(pw_lbsp(taps, wci, ctl->lut[wci]) ^ wdi);
-        const uint32_t dd = (intra + inter) / 2u;
-        if ((!unst || flat || border) && cd <= th.color && cd >= th.color / 2u && intra <= th.desc / 2u) {
-            // illumination update test (:684): modulus halves (+1) once the mask is non-zero
-            const uint32_t r = pw_draw(D.seed, t, (uint32_t)p, k++);
-            if (pw_mod(r, rateHalf) == 0u) mark1 |= 1u << i;
-            if (pw_mod(r, any0 ? rateHalf : rate) == 0u) {
-                mark0 |= 1u << i;
-                any0 = 1;
+    const bool illumOn = !unst || flat || border;
+    const size_t npx = (size_t)D.npx;
+    size_t src = pw_slot(S, cur, 0, p), dst = pw_slot(S, nxt, 0, p);
+    PwWord held = {0u, 0u, 0u, 0u, 0u}, next = pw_load(S, src);
+    uint32_t heldMarks = 0;
+    for (int i = 0; i < L; ++i) {
+        PwWord w = next;
+        if (i + 1 < L) {
+            src += npx;
+            next = pw_load(S, src);
+        } else if (rsrc != kPwNone) {
+            w = repl;
+        }
+        const float cw = pw_weight(w.occ, w.first, w.last, t, off);
+        if (i == 0) thrW = cw / (Rr * 2.0f);
+        uint32_t marks = 0;
+        bool matched = false;
+        if (sumW < thrW) {
+            const uint32_t cd = pw_absdiff(col, w.col);
+            if (cd <= th.color) {
+                const uint32_t intra = __popc(desc ^ w.desc);
+                const uint32_t inter = __popc((lbsp_thr_raw(taps, w.col, ctl->lut[w.col]) ^ w.desc) & 0xffffu);
+                const uint32_t dd = (intra + inter) / 2u;
+                if (illumOn && cd >= th.color / 2u && intra <= th.desc / 2u) {
+                    // illumination update test (:684): modulus halves (+1) once the mask is non-zero
+                    const uint32_t r = pw_draw(D.seed, t, (uint32_t)p, k++);
+                    if (pw_mod(r, rateHalf) == 0u) {
+                        marks |= 2u;
+                        any1 = 1;
+                    }
+                    if (pw_mod(r, any0 ? rateHalf : rate) == 0u) {
+                        marks |= 1u;
+                        any0 = 1;
+                    }
+                }
+                if (dd <= th.desc) {
+                    sumW += cw;
+                    matched = true;
+                    minColor = min(minColor, cd);
+                    minDesc = min(minDesc, dd);
+                }
             }
         }
-        if (dd <= th.desc && cd <= th.color) {
-            sumW += w;
-            matched |= 1u << i;
-            minColor = min(minColor, cd);
-            minDesc = min(minDesc, dd);
+        if (matched) {  // seen now, occurrences incremented
+            w.last = t;
+            if (occOn && cw < 1.0f) w.occ += incr;
         }
-        if (w > lastW) {
-            const uint8_t tmp = ord[i];
-            ord[i] = ord[i - 1];
-            ord[i - 1] = tmp;
+        if (cw > lastW) {  // heavier than the held word: it takes the slot before it
+            pw_store(S, dst, w);
+            m0 |= (marks & 1u) << (i - 1);
+            m1 |= (marks >> 1) << (i - 1);
+            dst += npx;
         } else {
-            lastW = w;
+            if (i > 0) {
+                pw_store(S, dst, held);
+                m0 |= (heldMarks & 1u) << (i - 1);
+                m1 |= (heldMarks >> 1) << (i - 1);
+                dst += npx;
+            }
+            held = w;
+            heldMarks = marks;
+            lastW = cw;
         }
     }
-    for (; i < L; ++i) {
-        uint32_t wci, wdi, woi, wfi, wli;
-        pw_word(ws, i, wci, wdi, woi, wfi, wli);
-        const float w = pw_weight(woi, wfi, wli, t, off);
-        if (w > lastW) {
-            const uint8_t tmp = ord[i];
-            ord[i] = ord[i - 1];
-            ord[i - 1] = tmp;
-        } else {
-            lastW = w;
-        }
-    }
+    m0 |= (heldMarks & 1u) << (L - 1);
+    m1 |= (heldMarks >> 1) << (L - 1);
     const int bg = sumW >= thrW || border;
-    // the scanned dictionary in its new order: matched words seen now, occurrences incremented
-    const int occOn = !lastFG || moving;
-    uint32_t m0 = 0, m1 = 0;
-    for (int s = 0; s < L; ++s) {
-        const int o = ord[s];
-        uint32_t wco, wdo, woo, wfo, wlo;
-        pw_word(ws, o, wco, wdo, woo, wfo, wlo);
-        uint32_t occ = woo, last = wlo;
-        if (matched & (1u << o)) {
-            last = t;
-            if (occOn && pw_weight(woo, wfo, wlo, t, off) < 1.0f) occ += incr;
-        }
-        const size_t d = pw_slot(S, nxt, s, p);
-        S.wColor[d] = (uint8_t)wco;
-        S.wDesc[d] = (uint16_t)wdo;
-        S.wOcc[d] = occ;
-        S.wFirst[d] = wfo;
-        S.wLast[d] = last;
-        if (mark0 & (1u << o)) m0 |= 1u << s;
-        if (mark1 & (1u << o)) m1 |= 1u << s;
-    }
     const float initW = 1.0f / (float)off;
     uint8_t flags = (uint8_t)((bg ? kRfBG : 0) | (flat ? kRfFlat : 0) | (border ? kRfBorder : 0) |
-                              (mark0 ? kRfU0 : 0) | (mark1 ? kRfU1 : 0));
+                              (any0 ? kRfU0 : 0) | (any1 ? kRfU1 : 0));
     if (bg) {
         // global dictionary event (:774) and, when nothing matches, the replacement draw (:785)
         if (pw_mod(pw_draw(D.seed, t, (uint32_t)p, k), rate) == 0u) {
@@ -204,18 +182,11 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_local(PwParams P) {
         }
     } else {
         if (flat || pw_mod(pw_draw(D.seed, t, (uint32_t)p, k), rate) == 0u) flags |= kRfItem;
-        if (sumW < initW) {
-            // new local word in the last slot (:822-830)
-            const size_t d = pw_slot(S, nxt, L - 1, p);
-            S.wColor[d] = (uint8_t)col;
-            S.wDesc[d] = (uint16_t)desc;
-            S.wOcc[d] = incr;
-            S.wFirst[d] = t;
-            S.wLast[d] = t;
-        }
+        if (sumW < initW) held = {incr, t, t, desc, col};  // new local word in the last slot (:822-830)
     }
+    pw_store(S, dst, held);
     S.descT[p] = (uint16_t)desc;
-    S.uv[p] = (uint8_t)((mark0 ? 1 : 0) | (mark1 ? 2 : 0));
+    S.uv[p] = (uint8_t)((any0 ? 1 : 0) | (any1 ? 2 : 0));
     R.sumW = sumW;
     R.thrW = thrW;
     R.rate = rate;
@@ -303,9 +274,10 @@ __device__ void pw_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t
             wrPos = g;
             continue;
         }
-        if (fixedPos == G && pw_absdiff(pc->gw_color[w], col) <= th.color && pw_absdiff(bits, pc->gw_bits[w]) <= th.desc / 4u) {
-            fixedPos = g;
+        if (pw_absdiff(pc->gw_color[w], col) <= th.color && pw_absdiff(bits, pc->gw_bits[w]) <= th.desc / 4u) {
+            fixedPos = g;  // a replaceable word further on is behind it
             fixedWord = w;
+            break;
         }
     }
     const int critical = wrPos < fixedPos;
@@ -641,13 +613,13 @@ __device__ float pw_nbr_loop(const PawcsDev& S, uint32_t t, int cur, int nxt, in
     reachedLast = false;
     for (int j = 0; j < S.L && nsum < R.thrW; ++j) {
         if (j == S.L - 1) reachedLast = true;
-        uint32_t c, d, o, f, l;
-        pw_word(ws, j, c, d, o, f, l);
-        const uint32_t cd = pw_absdiff(col, c);
-        if (cd <= th.color && (uint32_t)__popc(desc ^ d) <= th.desc) {
-            nsum += pw_weight(o, f, l, t, off);
+        const PwWord w = pw_word(ws, j);
+        const uint32_t cd = pw_absdiff(col, w.col);
+        if (cd <= th.color && (uint32_t)__popc(desc ^ w.desc) <= th.desc) {
+            nsum += pw_weight(w.occ, w.first, w.last, t, off);
         } else if (!segmQ && flat && (boot || pw_mod(pw_draw(D.seed, t, (uint32_t)p, k++), R.rate) == 0u)) {
-            if (cd <= th.color && (uint32_t)__popc(desc ^ lastDescQ) <= th.desc / 2u) nsum += pw_weight(o, f, l, t, off);
+            if (cd <= th.color && (uint32_t)__popc(desc ^ lastDescQ) <= th.desc / 2u)
+                nsum += pw_weight(w.occ, w.first, w.last, t, off);
         }
     }
     return nsum;
@@ -786,21 +758,11 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_commit(PwParams P) {
         // dictionary: illumination updates, then a later neighbour's replacement of the last slot
         const uint8_t u = S.uFinal[p];
         const uint32_t m = (u & 2) ? R.m1 : R.m0;
-        for (int s = 0; s < S.L; ++s)
-            if (m & (1u << s)) {
-                const size_t a = pw_slot(S, nxt, s, p);
-                S.wColor[a] = (uint8_t)col;
-                S.wDesc[a] = (uint16_t)desc;
-            }
+        for (uint32_t rest = m; rest; rest &= rest - 1u)
+            S.wA[pw_slot(S, nxt, __ffs(rest) - 1, p)].w = desc | (col << 16);
         const uint32_t ra = S.repAfter[p];
-        if (ra != kPwNone) {
-            const size_t a = pw_slot(S, nxt, S.L - 1, p);
-            S.wColor[a] = D.frame[ra];
-            S.wDesc[a] = S.descT[ra];
-            S.wOcc[a] = S.rec[ra].incr;
-            S.wFirst[a] = t;
-            S.wLast[a] = t;
-        }
+        if (ra != kPwNone)
+            pw_store(S, pw_slot(S, nxt, S.L - 1, p), {S.rec[ra].incr, t, t, S.descT[ra], D.frame[ra]});
         // illumination mask at the end of the frame (:686-690, :889-890): the right neighbour's
         // update sets 1 & ROI; else the own update leaves 2-1 = 1; else the start value (1 & ROI
         // after the left neighbour's update) minus one
@@ -1150,52 +1112,67 @@ extern "C" __global__ void pw_k_ds(PwParams P) {
 // frame level (:1462-1516): LBSP threshold LUT, camera-motion analysis, automatic model reset
 // decision; one block per stream
 // ------------------------------------------------------------------------------------------
-extern "C" __global__ void pw_k_epilogue(PwParams P) {
+// acc + v[0] + v[1] + ... in that order, from shared memory at a 16-byte boundary. The chain of additions is
+// the bound (four cycles each); four vector loads are in flight ahead of it.
+__device__ float pw_ordered_sum(const float* v, int n, float acc) {
+    const float4* q = (const float4*)v;
+    int i = 0;
+    for (; i + 16 <= n; i += 16) {
+        const float4 a = q[i / 4], b = q[i / 4 + 1], c = q[i / 4 + 2], d = q[i / 4 + 3];
+        acc = acc + a.x; acc = acc + a.y; acc = acc + a.z; acc = acc + a.w;
+        acc = acc + b.x; acc = acc + b.y; acc = acc + b.z; acc = acc + b.w;
+        acc = acc + c.x; acc = acc + c.y; acc = acc + c.z; acc = acc + c.w;
+        acc = acc + d.x; acc = acc + d.y; acc = acc + d.z; acc = acc + d.w;
+    }
+    for (; i < n; ++i) acc = acc + v[i];
+    return acc;
+}
+
+// the ordered sum of n floats by the block: the block stages the terms in shared memory, one thread (of the
+// warp `warp`) adds them in order; the sum is valid on that thread
+__device__ float pw_block_ordered_sum(const float* v, int n, float* terms, int warp) {
+    float acc = 0.0f;
+    for (int c0 = 0; c0 < n; c0 += 2048) {
+        const int cnt = min(2048, n - c0);
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x) terms[i] = v[c0 + i];
+        __syncthreads();
+        if (threadIdx.x == 32 * warp) acc = pw_ordered_sum(terms, cnt, acc);
+        __syncthreads();
+    }
+    return acc;
+}
+
+extern "C" __global__ void __launch_bounds__(256) pw_k_epilogue(PwParams P) {
     const int si = blockIdx.x;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
     const StreamDev& D = S.sd;
     StreamCtl* ctl = D.ctl;
     PawcsCtl* pc = S.pc;
-    const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
-    const int boot = t <= (uint32_t)kBootWin;
-    float fLT, fST;
-    pw_factors(t, (int)S.nmv, &fLT, &fST);
-    (void)fST;
-    const int nds = D.dsW * D.dsH;
-    // ordered float sum of |LT - ST| over the down-sampled ROI (lv::L1dist, math.hpp:255-268): the
-    // block stages the terms in shared memory, one thread adds them in order
-    __shared__ float terms[2048];
-    float l1 = 0.0f;
-    for (int c0 = 0; c0 < nds; c0 += 2048) {
-        const int cnt = min(2048, nds - c0);
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x) terms[i] = S.dsAbs[c0 + i];
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int i = 0; i < cnt; ++i) l1 = l1 + terms[i];
-        __syncthreads();
-    }
-    if (threadIdx.x != 0) return;
-    const float ratio = l1 / (float)pc->ds_roi_count;
-    pc->frame_ratio = ratio;
-    // LBSP threshold LUT (:1462-1473)
+    // LBSP threshold LUT (:1462-1473), an entry per thread
     const float nonflat = (float)(ctl->n_rel - pc->nflat_acc) / (float)ctl->n_rel;
+    const float lastNonflat = pc->last_nonflat_ratio;
     const float rel = S.relThr;
     const float offs = (float)S.lbspOff;
-    if (nonflat < 0.1f && pc->last_nonflat_ratio < 0.1f) {
-        for (int k = 0; k <= 255; ++k) {
-            const float v = (offs + (float)k * rel) / 4;
-            const int r = __float2int_rn(v);
-            const int lim = r < 0 ? 0 : r > 255 ? 255 : r;
-            if ((int)ctl->lut[k] > lim) --ctl->lut[k];
-        }
-    } else if (nonflat > 0.5f && pc->last_nonflat_ratio > 0.5f) {
+    const int k = threadIdx.x;
+    if (nonflat < 0.1f && lastNonflat < 0.1f) {
+        const float v = (offs + (float)k * rel) / 4;
+        const int r = __float2int_rn(v);
+        const int lim = r < 0 ? 0 : r > 255 ? 255 : r;
+        if ((int)ctl->lut[k] > lim) --ctl->lut[k];
+    } else if (nonflat > 0.5f && lastNonflat > 0.5f) {
         const float v = offs + 255 * rel;
         const int r = __float2int_rn(v);
         const int lim = r < 0 ? 0 : r > 255 ? 255 : r;
-        for (int k = 0; k <= 255; ++k)
-            if ((int)ctl->lut[k] < lim) ++ctl->lut[k];
+        if ((int)ctl->lut[k] < lim) ++ctl->lut[k];
     }
+    // ordered float sum of |LT - ST| over the down-sampled ROI (lv::L1dist, math.hpp:255-268)
+    __shared__ __align__(16) float terms[2048];
+    const float l1 = pw_block_ordered_sum(S.dsAbs, D.dsW * D.dsH, terms, 0);
+    __syncthreads();  // every thread has read the ratios
+    if (threadIdx.x != 0) return;
+    const float ratio = l1 / (float)pc->ds_roi_count;
+    pc->frame_ratio = ratio;
     pc->last_nonflat_ratio = nonflat;
     pc->nflat_acc = 0;
     pc->reset_pending = 0;
@@ -1278,12 +1255,12 @@ extern "C" __global__ void __launch_bounds__(128) pw_k_refresh_local(PawcsDev S,
     uint16_t wd[kPwMaxLocal];
     uint32_t wo[kPwMaxLocal], wf[kPwMaxLocal], wl[kPwMaxLocal];
     for (int j = 0; j < L; ++j) {
-        const size_t a = pw_slot(S, buf, j, p);
-        wc[j] = S.wColor[a];
-        wd[j] = S.wDesc[a];
-        wo[j] = S.wOcc[a];
-        wf[j] = S.wFirst[a];
-        wl[j] = S.wLast[a];
+        const PwWord w = pw_load(S, pw_slot(S, buf, j, p));
+        wc[j] = (uint8_t)w.col;
+        wd[j] = (uint16_t)w.desc;
+        wo[j] = w.occ;
+        wf[j] = w.first;
+        wl[j] = w.last;
     }
     // empty slots carry first == kPwNone (initialization only)
     if (decr > 0.0f)
@@ -1346,14 +1323,7 @@ extern "C" __global__ void __launch_bounds__(128) pw_k_refresh_local(PawcsDev S,
         wf[i] = t;
         wl[i] = t;
     }
-    for (int j = 0; j < L; ++j) {
-        const size_t a = pw_slot(S, buf, j, p);
-        S.wColor[a] = wc[j];
-        S.wDesc[a] = wd[j];
-        S.wOcc[a] = wo[j];
-        S.wFirst[a] = wf[j];
-        S.wLast[a] = wl[j];
-    }
+    for (int j = 0; j < L; ++j) pw_store(S, pw_slot(S, buf, j, p), {wo[j], wf[j], wl[j], wd[j], wc[j]});
     D.kctr[p] = (uint16_t)k;
 }
 
@@ -1377,9 +1347,9 @@ extern "C" __global__ void pw_k_refresh_global(PawcsDev S, uint32_t t, int buf, 
             const int x = (int)(p % D.W), y = (int)(p / D.W);
             const size_t cidx = (size_t)(y / 2) * S.gwW + (x / 2);
             const PwThr th = pw_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff);
-            const size_t a = pw_slot(S, buf, 0, (int)p);
-            const uint32_t bc = S.wColor[a], bd = S.wDesc[a];
-            const float bw = pw_weight(S.wOcc[a], S.wFirst[a], S.wLast[a], t, off);
+            const PwWord best = pw_load(S, pw_slot(S, buf, 0, (int)p));
+            const uint32_t bc = best.col, bd = best.desc;
+            const float bw = pw_weight(best.occ, best.first, best.last, t, off);
             const uint32_t bb = __popc(bd);
             int uninit = 0, g;
             for (g = 0; g < G; ++g) {
@@ -1446,14 +1416,7 @@ extern "C" __global__ void pw_k_init(PawcsDev S) {
             f[FM_T * D.npx + p] = kTLower;
             f[FM_R * D.npx + p] = 2.0f;
             f[FM_V * D.npx + p] = kVIncr * 10;
-            for (int j = 0; j < S.L; ++j) {
-                const size_t a = pw_slot(S, b, j, p);
-                S.wColor[a] = 0;
-                S.wDesc[a] = 0;
-                S.wOcc[a] = 0;
-                S.wFirst[a] = kPwNone;
-                S.wLast[a] = 0;
-            }
+            for (int j = 0; j < S.L; ++j) pw_store(S, pw_slot(S, b, j, p), {0u, kPwNone, 0u, 0u, 0u});
         }
         S.illum[p] = 0;
         S.unstable[p] = 0;
@@ -1478,9 +1441,9 @@ extern "C" __global__ void pw_k_init_last(PawcsDev S, const uint8_t* img) {
         if (D.roi[p]) {
             c = img[p];
             if (x > 2 && y > 2 && x < D.W - 2 && y < D.H - 2) {
-                uint8_t taps[16];
-                pw_taps(img, D.W, x, y, taps);
-                d = (uint16_t)pw_lbsp(taps, c, D.ctl->lut[c]);
+                uint32_t taps[4];
+                pw_taps<1>(img, D.W, x, y, 0, taps);
+                d = (uint16_t)lbsp_thr(taps, c, D.ctl->lut[c]);
             }
         }
         D.lastCol[p] = c;
@@ -1488,63 +1451,49 @@ extern "C" __global__ void pw_k_init_last(PawcsDev S, const uint8_t* img) {
     }
 }
 
-// camera-motion comparison (:1480-1501), frames t with t % 500 == 0: the background image of the words
-// of buffer buf, area-down-sampled like the frame, against the long-term mean of the down-sampled
-// frames; one thread per down-sampled pixel writes |LT - BG| (0 outside the fully covered blocks)
-extern "C" __global__ void pw_k_motion_bg(PwParams P, int buf) {
+// camera-motion comparison (:1480-1501), frames t with t % 500 == 0: the background image (left in the label
+// buffer by the background kernel), area-down-sampled like the frame, against the long-term mean of the
+// down-sampled frames: |LT - BG| per down-sampled pixel (0 outside the fully covered blocks)
+extern "C" __global__ void pw_k_motion_bg(PwParams P) {
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per output
     if (i >= nds) return;
     if (S.dsRoi[i] != 255) {
         S.dsAbs[i] = 0.0f;
         return;
     }
-    const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
-    const unsigned long long off = S.pc->lword_offset;
-    const int bx = i % D.dsW, by = i / D.dsW;
-    // the background image (0 outside the ROI), area-down-sampled
-    const uint8_t v = area_resample(D.W, D.H, D.dsW, D.dsH, bx, by, [&](int sx, int sy) {
-        const int p = sy * D.W + sx;
-        if (!D.roi[p]) return 0;
-        float tw = 0.0f, tc = 0.0f;
-        for (int j = 0; j < S.L; ++j) {
-            const size_t a = pw_slot(S, buf, j, p);
-            const float w = pw_weight(S.wOcc[a], S.wFirst[a], S.wLast[a], t, off);
-            tc = tc + (float)S.wColor[a] * w;
-            tw = tw + w;
-        }
-        const int r = __float2int_rn(tc / tw);
-        return r < 0 ? 0 : r > 255 ? 255 : r;
-    });
-    S.dsAbs[i] = fabsf(D.dsLT[i] - (float)v);
+    uint32_t v[1];
+    area_resample_group<1>((const uint8_t*)D.label, D.W, D.H, D.dsW, D.dsH, i % D.dsW, i / D.dsW, v);
+    if (threadIdx.x & 7) return;
+    S.dsAbs[i] = fabsf(D.dsLT[i] - (float)v[0]);
 }
 
 // camera-motion decision: ordered L1 sum, then switch the mode on (during the bootstrap window, ratio
 // >= 45) or off (ratio < 45/4) with the local word weight offset (5 / 1000); flags[1] tells the host
 // to run refreshModel(1, 1, true), flags[2] carries the new offset. One grayscale channel: the colour
 // distance ratio is 0; three channels: the mean colour distortion of pw3_k_motion_bg.
-extern "C" __global__ void pw_k_motion_decide(PwParams P) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+extern "C" __global__ void __launch_bounds__(256) pw_k_motion_decide(PwParams P) {
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     PawcsCtl* pc = S.pc;
+    __shared__ __align__(16) float terms[2048];
+    float l1 = 0.0f, cs = 0.0f;
+    if (pc->reset_block) {
+        const int nds = D.dsW * D.dsH;
+        l1 = pw_block_ordered_sum(S.dsAbs, nds, terms, 0);
+        // three channels: the ordered sum of the colour distortions (written beside the L1 terms)
+        if (D.C == 3) cs = pw_block_ordered_sum(S.contrib, nds, terms, 0);
+    }
+    __syncthreads();  // reset_block has been read
+    if (threadIdx.x != 0) return;
     pc->motion_pending = 0;
     if (pc->reset_block) {
         const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
         const int boot = t <= (uint32_t)kBootWin;
-        const int nds = D.dsW * D.dsH;
-        float l1 = 0.0f;
-        for (int i = 0; i < nds; ++i) l1 = l1 + S.dsAbs[i];
         const float mr = l1 / (float)pc->ds_roi_count;
-        float cr = 0.0f;
-        if (D.C == 3) {
-            // three channels: the ordered sum of the colour distortions (written beside the L1 terms)
-            float cs = 0.0f;
-            for (int i = 0; i < nds; ++i) cs = cs + S.contrib[i];
-            cr = cs / (float)pc->ds_roi_count;
-        }
+        const float cr = D.C == 3 ? cs / (float)pc->ds_roi_count : 0.0f;
         if (pc->moving_cam && mr < (float)(45 / 4) && cr < (float)(45 / 10 / 4)) {
             pc->lword_offset = (unsigned long long)kBootWin * 2;
             pc->moving_cam = 0;
@@ -1559,10 +1508,11 @@ extern "C" __global__ void pw_k_motion_decide(PwParams P) {
     P.flags[2] = (unsigned int)pc->lword_offset;
 }
 
-// background image (:1518-1545) / descriptors (:1547-1594) from the words of buffer buf
-extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc) {
+// background image (:1518-1545) / descriptors (:1547-1594) from the words of buffer buf; ahead: 1 inside the
+// frame step, before the frame index advances
+extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc, int ahead) {
     const StreamDev& D = S.sd;
-    const uint32_t t = (uint32_t)D.ctl->frame_idx;
+    const uint32_t t = (uint32_t)D.ctl->frame_idx + (uint32_t)ahead;
     const unsigned long long off = S.pc->lword_offset;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.npx; p += gridDim.x * blockDim.x) {
         if (!D.roi[p]) {
@@ -1572,10 +1522,10 @@ extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol,
         }
         float tw = 0.0f, tc = 0.0f, td = 0.0f;
         for (int j = 0; j < S.L; ++j) {
-            const size_t a = pw_slot(S, buf, j, p);
-            const float w = pw_weight(S.wOcc[a], S.wFirst[a], S.wLast[a], t, off);
-            tc = tc + (float)S.wColor[a] * w;
-            td = td + (float)S.wDesc[a] * w;
+            const PwWord wj = pw_load(S, pw_slot(S, buf, j, p));
+            const float w = pw_weight(wj.occ, wj.first, wj.last, t, off);
+            tc = tc + (float)wj.col * w;
+            td = td + (float)wj.desc * w;
             tw = tw + w;
         }
         if (outCol) {

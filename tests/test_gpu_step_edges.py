@@ -1,8 +1,9 @@
-"""SuBSENSE's frame step at the edges of its kernels' tiles, words and chunks, against the oracle (bit-exact)."""
+"""SuBSENSE's and PAWCS's frame steps at the edges of their kernels' tiles, words and chunks, against the oracle (bit-exact)."""
 import numpy as np
 import pytest
 
 from tests.test_gpu_parity import run_pair
+from tests.test_gpu_pawcs import run_pair as pawcs_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,16 @@ def test_area_down_sampling_at_ragged_sizes(W, H, channels):
     """The frame-level down-sampling by groups of lanes: integral scales (8 and 15) with and without aligned
     rows, fractional scales in one or both directions (the averages are part of the compared state)."""
     run_pair(hollow_frames(W, H, channels, 3, W + H), seed=2)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("words", [2, 3, 7, 50])
+def test_pawcs_word_streams(words, channels):
+    """Dictionaries of one word (the held word alone) up to the full count, through the local pass's bubble
+    order, the updaters' loops at the last word and the later updaters, on a frame of partial tiles with border
+    pixels that update themselves."""
+    roi = np.zeros((43, 61), np.uint8)
+    roi[3:40, 4:58] = 255
+    frames = hollow_frames(61, 43, channels, 9, 7 * words)
+    lrs = [1.0 if t in (3, 4, 7) else 0.0 for t in range(len(frames))]
+    pawcs_pair(frames, seed=words, lrs=lrs, roi=roi, nMaxNbWords=words)
