@@ -608,8 +608,8 @@ PwLayout pw_layout(int W, int H, int C, int L, int G) {
     sz[PL_BITS] = bit_planes_bytes(W, H);
     sz[PL_LABEL] = sz[PL_INTENT] = npx * 4;
     sz[PL_DESCT] = npx * 2 * C;
-    sz[PL_REC] = npx * sizeof(PwRec);
-    sz[PL_OUT] = npx * sizeof(PwOut);
+    sz[PL_REC] = npx * PwRecPlanes::kBytes;
+    sz[PL_OUT] = npx * PwOutPlanes::kBytes;
     sz[PL_REPB] = sz[PL_REPA] = npx * 4;
     sz[PL_UFINAL] = npx;
     sz[PL_UV] = npx;
@@ -717,8 +717,8 @@ void pw_fill(lvbgs_ctx* h, const PwLayout& Lo, int L, int G) {
     D.glut = b + Lo.off[PL_GLUT];
     D.gmap = (float*)(b + Lo.off[PL_GMAP]);
     D.descT = (uint16_t*)(b + Lo.off[PL_DESCT]);
-    D.rec = (PwRec*)(b + Lo.off[PL_REC]);
-    D.out = (PwOut*)(b + Lo.off[PL_OUT]);
+    D.rec = {b + Lo.off[PL_REC], h->npx};
+    D.out = {b + Lo.off[PL_OUT], h->npx};
     D.repBefore = (uint32_t*)(b + Lo.off[PL_REPB]);
     D.repAfter = (uint32_t*)(b + Lo.off[PL_REPA]);
     D.uFinal = b + Lo.off[PL_UFINAL];

@@ -185,7 +185,7 @@ extern "C" __global__ void __launch_bounds__(256, 2) pw3_k_local(PwParams P) {
 #pragma unroll
         for (int j = 0; j < 12; ++j) {
             const int px = x + j % 5 - 2, py = y + j / 5 - 2;
-            tq[j] = (px >= 0 && py >= 0 && px < D.W && D.roi[py * D.W + px]) ? S.out[py * D.W + px].q : kPwNone;
+            tq[j] = (px >= 0 && py >= 0 && px < D.W) ? S.out[py * D.W + px].q : kPwNone;
         }
 #pragma unroll 1
         for (int j = 0; j < 12; ++j) {
@@ -328,7 +328,7 @@ extern "C" __global__ void __launch_bounds__(256, 2) pw3_k_local(PwParams P) {
     dt[1] = (uint16_t)dsc[1];
     dt[2] = (uint16_t)dsc[2];
     S.uv[q] = (uint8_t)((any0 ? 1 : 0) | (any1 ? 2 : 0));
-    PwRec& R = S.rec[q];
+    const PwRec R = S.rec[q];
     R.sumW = sumW;
     R.thrW = thrW;
     R.rate = rate;
@@ -352,7 +352,7 @@ extern "C" __global__ void __launch_bounds__(256, 2) pw3_k_local(PwParams P) {
 // ------------------------------------------------------------------------------------------
 __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t col) {
     const StreamDev& D = S.sd;
-    PwOut& O = S.out[p];
+    const PwOut O = S.out[p];
     O.gflags = 0;
     O.epoch = 0;
     O.gword = kPwNone;
@@ -432,7 +432,7 @@ __device__ __forceinline__ bool pw3_gmatch(const Pw3Item& it, const Pw3GFeat& f,
     return pw_absdiff(it.bits, f.bits) <= it.dq && pw3_cmix(it.col, f.col) <= it.cthr;
 }
 __device__ __forceinline__ void pw3_set_out(const PawcsDev& S, uint32_t p, uint32_t word, uint32_t epoch, uint32_t repl) {
-    PwOut& O = S.out[p];
+    const PwOut O = S.out[p];
     O.gword = word;
     O.epoch = epoch;
     O.gflags = (uint8_t)((O.gflags & ~1u) | repl);
@@ -732,18 +732,18 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
     if (x < D.W && y < D.H) {
         const int q = y * D.W + x;
         if (D.roi[q]) {
-            for (int dy = -2; dy <= 0 && !dirty; ++dy)
-                for (int dx = -2; dx <= 2; ++dx) {
-                    if (dy == 0 && dx >= 0) break;
-                    const int px = x + dx, py = y + dy;
-                    if (px < 0 || py < 0 || px >= D.W) continue;
-                    const int p = py * D.W + px;
-                    if (!D.roi[p]) continue;
-                    const PwOut& O = S.out[p];
-                    if (O.chg && (O.q == (uint32_t)q || O.qPrev == (uint32_t)q)) {
-                        dirty = true;
-                        break;
-                    }
+            // the changed flags of the window first; the targets only where one is set
+            bool chg[12];
+#pragma unroll
+            for (int j = 0; j < 12; ++j) {
+                const int px = x + j % 5 - 2, py = y + j / 5 - 2;
+                chg[j] = px >= 0 && py >= 0 && px < D.W && S.out[py * D.W + px].chg;
+            }
+#pragma unroll
+            for (int j = 0; j < 12; ++j)
+                if (chg[j]) {
+                    const PwOut O = S.out[(y + j / 5 - 2) * D.W + x + j % 5 - 2];
+                    dirty = dirty || O.q == (uint32_t)q || O.qPrev == (uint32_t)q;
                 }
             S.dirty[q] = dirty ? 1 : 0;
         }
@@ -768,7 +768,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
     const int boot = t <= (uint32_t)kBootWin;
     const unsigned long long off = S.pc->lword_offset;
     const int L = S.L;
-    const PwRec& R = S.rec[q];
+    const PwRec R = S.rec[q];
     const uint8_t u = S.uFinal[q];
     const unsigned long long m = (u & 2) ? (((unsigned long long)R.m1hi << 32) | R.m1)
                                          : (((unsigned long long)R.m0hi << 32) | R.m0);
@@ -778,7 +778,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
 #pragma unroll
     for (int j = 12; j < 25; ++j) {
         const int px = x + j % 5 - 2, py = y + j / 5 - 2;
-        tq[j - 12] = (px >= 0 && px < D.W && py < D.H && D.roi[py * D.W + px]) ? S.out[py * D.W + px].q : kPwNone;
+        tq[j - 12] = (px >= 0 && px < D.W && py < D.H) ? S.out[py * D.W + px].q : kPwNone;
         any |= tq[j - 12] == (uint32_t)q;
     }
     if (!m && !any) return;
@@ -846,8 +846,8 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_commit(PwParams P) {
         const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
         const int cur = (int)(ctl->frame_idx & 1ull), nxt = cur ^ 1;
         const int boot = t <= (uint32_t)kBootWin;
-        const PwRec& R = S.rec[p];
-        const PwOut& O = S.out[p];
+        const PwRec R = S.rec[p];
+        const PwOut O = S.out[p];
         flat = (R.flags & kRfFlat) != 0;
         const uint8_t u = S.uFinal[p];
         // the neighbours' updates write 1 & ROI (:1025-1026): 0 in the ROI's edge band of 128

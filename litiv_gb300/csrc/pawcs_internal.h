@@ -58,36 +58,62 @@ struct PawcsCtl {
     int motion_pending;                  // camera-motion mode switched this frame (refreshModel(1, 1, true))
 };
 
-// per-pixel record of the local pass of one frame
+// Per-pixel records, one plane per field. Most kernels read one or two fields of a pixel or of its window, so
+// records side by side moved 48 and 28 bytes for each four that were used. A reference bundle stands for one
+// pixel's record: rec[p].field is the element of that field's plane (unused references cost nothing).
 struct PwRec {
-    float sumW;               // fPotentialLocalWordsWeightSum
-    float thrW;               // fLocalWordsWeightSumThreshold
-    unsigned long long rate;  // nCurrLocalWordUpdateRate (size_t; SIZE_MAX for an infinite override)
-    uint32_t m0, m1;          // final slots illumination-updated when the mask is zero / non-zero
-    uint32_t m0hi, m1hi;      // the same for slots 32..63 (three channels)
-    uint32_t rsrc;            // replacement source of the own last slot used by the local pass
-    uint16_t kScan;           // draw counter after the word scan
-    uint16_t incr;            // nCurrWordOccIncr
-    uint16_t minColor, minDesc;
-    uint8_t flags;            // kRf*
-    uint8_t bits;             // popcount of the current descriptor
+    unsigned long long& rate;       // nCurrLocalWordUpdateRate (size_t; SIZE_MAX for an infinite override)
+    float &sumW, &thrW;             // fPotentialLocalWordsWeightSum, fLocalWordsWeightSumThreshold
+    uint32_t &m0, &m1;              // final slots illumination-updated when the mask is zero / non-zero
+    uint32_t &m0hi, &m1hi;          // the same for slots 32..63 (three channels)
+    uint32_t& rsrc;                 // replacement source of the own last slot used by the local pass
+    uint16_t& kScan;                // draw counter after the word scan
+    uint16_t& incr;                 // nCurrWordOccIncr
+    uint16_t &minColor, &minDesc;
+    uint8_t& flags;                 // kRf*
+    uint8_t& bits;                  // popcount of the current descriptor
+};
+struct PwRecPlanes {
+    static constexpr size_t kBytes = 8 + 7 * 4 + 4 * 2 + 2;  // of one pixel
+    uint8_t* base;
+    size_t n;  // pixels
+    template <typename T>
+    LV_HD T& at(size_t off, int p) const { return ((T*)(base + off * n))[p]; }
+    LV_HD PwRec operator[](int p) const {
+        return {at<unsigned long long>(0, p), at<float>(8, p),     at<float>(12, p),    at<uint32_t>(16, p),
+                at<uint32_t>(20, p),          at<uint32_t>(24, p), at<uint32_t>(28, p), at<uint32_t>(32, p),
+                at<uint16_t>(36, p),          at<uint16_t>(38, p), at<uint16_t>(40, p), at<uint16_t>(42, p),
+                at<uint8_t>(44, p),           at<uint8_t>(45, p)};
+    }
 };
 constexpr uint8_t kRfBG = 1, kRfFlat = 2, kRfBorder = 4, kRfU0 = 8, kRfU1 = 16, kRfItem = 32, kRfEvent = 64,
                   kRfRepDraw = 128;
 
 // per-pixel outcome of the global stage / neighbour stage
 struct PwOut {
-    uint32_t gword;      // matched pool word (kPwNone: none)
-    uint32_t epoch;      // replacements of the replaceable word at or before this pixel
-    uint32_t q;          // neighbour-update target (kPwNone: no update)
-    uint16_t kLoop;      // draw counter at the start of the neighbour loop
-    uint8_t segm;        // raw decision (0/255)
-    uint8_t gflags;      // bit0 replaced the replaceable word, bit1 contributed to the word weight, bit2 critical
-    uint16_t kEnd;       // draw counter after the neighbour loop
-    uint8_t rflags;      // neighbour loop: bit0 replaces the target's last word, bit1 reached the last word
-    uint8_t chg;         // three channels: the loop inputs (target, kLoop, thrW) changed this round
-    float thrW;          // weight threshold of the loop (snapshot of the round's local pass)
-    uint32_t qPrev;      // target of the previous round
+    uint32_t& gword;      // matched pool word (kPwNone: none)
+    uint32_t& epoch;      // replacements of the replaceable word at or before this pixel
+    uint32_t& q;          // neighbour-update target (kPwNone: no update; 0 outside the ROI, which is no target)
+    uint32_t& qPrev;      // target of the previous round
+    float& thrW;          // weight threshold of the loop (snapshot of the round's local pass)
+    uint16_t& kLoop;      // draw counter at the start of the neighbour loop
+    uint16_t& kEnd;       // draw counter after the neighbour loop
+    uint8_t& segm;        // raw decision (0/255)
+    uint8_t& gflags;      // bit0 replaced the replaceable word, bit1 contributed to the word weight, bit2 critical
+    uint8_t& rflags;      // neighbour loop: bit0 replaces the target's last word, bit1 reached the last word
+    uint8_t& chg;         // three channels: the loop inputs (target, kLoop, thrW) changed this round
+};
+struct PwOutPlanes {
+    static constexpr size_t kBytes = 5 * 4 + 2 * 2 + 4;  // of one pixel
+    uint8_t* base;
+    size_t n;
+    template <typename T>
+    LV_HD T& at(size_t off, int p) const { return ((T*)(base + off * n))[p]; }
+    LV_HD PwOut operator[](int p) const {
+        return {at<uint32_t>(0, p),  at<uint32_t>(4, p),  at<uint32_t>(8, p), at<uint32_t>(12, p), at<float>(16, p),
+                at<uint16_t>(20, p), at<uint16_t>(22, p), at<uint8_t>(24, p), at<uint8_t>(25, p),  at<uint8_t>(26, p),
+                at<uint8_t>(27, p)};
+    }
 };
 
 struct PawcsDev {
@@ -109,8 +135,8 @@ struct PawcsDev {
     uint8_t* glut;             // [npx][16] per-pixel global word order (pool indices)
     float* gmap;               // [G][gwW*gwH] spatial occurrence maps, by pool word
     uint16_t* descT;           // current-frame descriptors
-    PwRec* rec;
-    PwOut* out;
+    PwRecPlanes rec;
+    PwOutPlanes out;
     uint32_t* repBefore;       // latest replacement source before the pixel (kPwNone: none)
     uint32_t* repAfter;        // latest replacement source after the pixel
     uint8_t* uFinal;           // resolved illumination-update bit per pixel

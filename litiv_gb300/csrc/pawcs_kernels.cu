@@ -56,7 +56,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_local(PwParams P) {
     const int p = y * D.W + x;
     const uint8_t roi = D.roi[p];
     if (!roi) return;
-    PwRec& R = S.rec[p];
+    const PwRec R = S.rec[p];
     const uint32_t rsrc = S.repBefore[p];
     if (P.round > 0 && R.rsrc == rsrc) return;  // inputs unchanged since its last local pass
     const StreamCtl* ctl = D.ctl;
@@ -255,7 +255,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_illum(PwParams P) {
 // ------------------------------------------------------------------------------------------
 __device__ void pw_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t col) {
     const StreamDev& D = S.sd;
-    PwOut& O = S.out[p];
+    const PwOut O = S.out[p];
     O.gflags = 0;
     O.epoch = 0;
     O.gword = kPwNone;
@@ -293,7 +293,7 @@ __device__ void pw_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ int pw_category(const PawcsDev& S, int p, int mode, int wr, uint32_t nrep) {
     if (!S.sd.roi[p]) return -1;
-    const PwOut& O = S.out[p];
+    const PwOut O = S.out[p];
     if (mode == 0) return ((S.rec[p].flags & kRfItem) && (O.gflags & 4)) ? 0 : -1;
     if (mode == 2) return O.q != kPwNone ? 0 : -1;
     if (S.contrib[p] < 0.0f) return -1;
@@ -403,7 +403,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams 
             if (mode == 0) {
                 // two records per item (pixel, colour|bits, thresholds, descriptors 0-1; descriptor 2|event
                 // flags, fixed position|word, and the global scan's speculative outcome)
-                const PwRec& R = S.rec[p];
+                const PwRec R = S.rec[p];
                 const bool c3 = D.C == 3;
                 const PwThr th = c3 ? pw3_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff)
                                     : pw_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff);
@@ -457,12 +457,12 @@ extern "C" __global__ void pw_k_cells(PwParams P, int final) {
         if (x >= D.W || y >= D.H) continue;
         const int p = y * D.W + x;
         if (!D.roi[p]) continue;
-        const PwRec& R = S.rec[p];
+        const PwRec R = S.rec[p];
         if (!(R.flags & kRfItem)) {
             if (final) S.contrib[p] = -1.0f;
             continue;
         }
-        PwOut& O = S.out[p];
+        const PwOut O = S.out[p];
         const uint32_t w = O.gword;
         float contrib = -1.0f;
         if (w == kPwNone) {
@@ -522,8 +522,8 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_nbr(PwParams P) {
     if (x >= D.W || y >= D.H) return;
     const int p = y * D.W + x;
     if (!D.roi[p]) return;
-    const PwRec& R = S.rec[p];
-    PwOut& O = S.out[p];
+    const PwRec R = S.rec[p];
+    const PwOut O = S.out[p];
     const uint32_t t = (uint32_t)(D.ctl->frame_idx + 1ull);
     uint32_t k = R.kScan;
     uint8_t segm;
@@ -577,7 +577,7 @@ __device__ float pw_nbr_loop(const PawcsDev& S, uint32_t t, int cur, int nxt, in
                              int q, uint32_t rs, uint32_t& k, bool& reachedLast) {
     const StreamDev& D = S.sd;
     const float* fm = D.fm + (size_t)cur * kNumFloatMaps * D.npx;
-    const PwRec& R = S.rec[p];
+    const PwRec R = S.rec[p];
     const uint32_t col = D.frame[p], desc = S.descT[p];
     const PwThr th = pw_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff);
     const int flat = (R.flags & kRfFlat) != 0;
@@ -596,7 +596,7 @@ __device__ float pw_nbr_loop(const PawcsDev& S, uint32_t t, int cur, int nxt, in
         segmQ = 0;
         lastDescQ = D.lastDesc[q];
     } else {
-        const PwRec& Rq = S.rec[q];
+        const PwRec Rq = S.rec[q];
         ws.buf = nxt;
         ws.m = (S.uFinal[q] & 2) ? Rq.m1 : Rq.m0;
         segmQ = S.out[q].segm;
@@ -639,7 +639,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_nbr_loops(PwParams P) {
     const float initW = 1.0f / (float)off;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = (int)S.updList[i];
-        PwOut& O = S.out[p];
+        const PwOut O = S.out[p];
         uint32_t k = O.kLoop;
         bool reachedLast;
         const float nsum = pw_nbr_loop(S, t, cur, nxt, boot, off, p, (int)O.q, kPwNone, k, reachedLast);
@@ -670,31 +670,33 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_replace(PwParams P) {
     const unsigned long long off = S.pc->lword_offset;
     const float initW = 1.0f / (float)off;
     uint32_t before = kPwNone, after = kPwNone;
-    for (int dy = -2; dy <= 2; ++dy)
-        for (int dx = -2; dx <= 2; ++dx) {
-            const int px = qx + dx, py = qy + dy;
-            if (px < 0 || py < 0 || px >= D.W || py >= D.H) continue;
-            const int p = py * D.W + px;
-            if (!D.roi[p]) continue;
-            // p == q happens when the clamped neighbour position falls back onto the pixel itself (at
-            // the ROI's outer rows and columns): the update then follows the pixel's own processing
-            PwOut& O = S.out[p];
-            if (O.q != (uint32_t)q) continue;
-            const uint32_t rs = p < q ? before : after;
-            uint8_t rf = O.rflags;
-            if (rs != kPwNone && (rf & 2)) {
-                uint32_t k = O.kLoop;
-                bool reachedLast;
-                const float nsum = pw_nbr_loop(S, t, cur, nxt, boot, off, p, q, rs, k, reachedLast);
-                rf = (uint8_t)((nsum < initW ? 1 : 0) | (reachedLast ? 2 : 0));
-                O.kEnd = (uint16_t)k;
-                O.rflags = rf;
-            }
-            if (rf & 1) {
-                if (p < q) before = (uint32_t)p;
-                else after = (uint32_t)p;
-            }
+    uint32_t hits = 0;  // window slots whose pixel updates q
+#pragma unroll
+    for (int j = 0; j < 25; ++j) {
+        const int px = qx + j % 5 - 2, py = qy + j / 5 - 2;
+        if (px >= 0 && py >= 0 && px < D.W && py < D.H && S.out[py * D.W + px].q == (uint32_t)q) hits |= 1u << j;
+    }
+    for (; hits; hits &= hits - 1u) {
+        const int j = __ffs(hits) - 1;
+        const int p = (qy + j / 5 - 2) * D.W + qx + j % 5 - 2;
+        // p == q happens when the clamped neighbour position falls back onto the pixel itself (at
+        // the ROI's outer rows and columns): the update then follows the pixel's own processing
+        const PwOut O = S.out[p];
+        const uint32_t rs = p < q ? before : after;
+        uint8_t rf = O.rflags;
+        if (rs != kPwNone && (rf & 2)) {
+            uint32_t k = O.kLoop;
+            bool reachedLast;
+            const float nsum = pw_nbr_loop(S, t, cur, nxt, boot, off, p, q, rs, k, reachedLast);
+            rf = (uint8_t)((nsum < initW ? 1 : 0) | (reachedLast ? 2 : 0));
+            O.kEnd = (uint16_t)k;
+            O.rflags = rf;
         }
+        if (rf & 1) {
+            if (p < q) before = (uint32_t)p;
+            else after = (uint32_t)p;
+        }
+    }
     S.repBefore[q] = before;
     S.repAfter[q] = after;
 }
@@ -751,8 +753,8 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_commit(PwParams P) {
         const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
         const int cur = (int)(ctl->frame_idx & 1ull), nxt = cur ^ 1;
         const int boot = t <= (uint32_t)kBootWin;
-        const PwRec& R = S.rec[p];
-        const PwOut& O = S.out[p];
+        const PwRec R = S.rec[p];
+        const PwOut O = S.out[p];
         const uint32_t col = D.frame[p], desc = S.descT[p];
         flat = (R.flags & kRfFlat) != 0;
         // dictionary: illumination updates, then a later neighbour's replacement of the last slot
