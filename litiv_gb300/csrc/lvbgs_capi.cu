@@ -630,7 +630,7 @@ PwLayout pw_layout(int W, int H, int C, int L, int G) {
     sz[PL_PDEV] = sizeof(PawcsDev);
     sz[PL_SDEV] = sizeof(StreamDev);
     sz[PL_DIRTY] = npx;
-    sz[PL_GSEG] = (npx / 512 + 2) * 24 * 4;
+    sz[PL_GSEG] = pw_gseg_max(npx, C) * kPwGsegWords * 4;
     sz[PL_GCAND] = npx * 4;
     sz[PL_GTRUE] = npx;
     PwLayout Lo;
@@ -936,6 +936,8 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
     const dim3 blk(kThreads);
     const int tiles = h->sd.nTiles;
     const int cblocks = (int)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk);
+    const size_t gseg4 = 4 * (size_t)pw_gseg_items(h->C);  // items of a block of four segments
+    const int gsegBlocks = (int)((h->npx + gseg4 - 1) / gseg4);
     for (int r = 0; r < n && w.enq < w.maxRounds; ++r, ++w.enq) {
         w.PR.round = w.enq;
         const PwParams& P = w.PR;
@@ -944,10 +946,10 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
             pw3_k_local<<<tiles, blk, 0, st>>>(P);
             pw_k_illum<<<(h->H + 7) / 8, 256, 0, st>>>(P);
             pw_compact(h, P, 0, st);
-            pw3_k_gscan_seg<<<(int)((h->npx + 4 * 512 - 1) / (4 * 512)), 128, 0, st>>>(P);
+            pw3_k_gscan_seg<<<gsegBlocks, 128, 0, st>>>(P);
             pw3_k_gscan_walk<<<1, 32, 0, st>>>(P);
             pw3_k_gscan_fix<<<(int)((h->npx + 255) / 256), 256, 0, st>>>(P);
-            pw3_k_gscan_fix_walked<<<(int)((h->npx + 4 * 512 - 1) / (4 * 512)), 128, 0, st>>>(P);
+            pw3_k_gscan_fix_walked<<<gsegBlocks, 128, 0, st>>>(P);
             pw_k_cells<<<(P.totalCells + 255) / 256, 256, 0, st>>>(P, 0);
             pw_k_nbr<<<tiles, blk, 0, st>>>(P);
             LV_CUDA(h, cudaMemsetAsync(h->d_flags, 0, 4, st), "flag reset");
@@ -956,10 +958,10 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
             pw_k_local<<<tiles, blk, 0, st>>>(P);
             pw_k_illum<<<(h->H + 7) / 8, 256, 0, st>>>(P);
             pw_compact(h, P, 0, st);
-            pw3_k_gscan_seg<<<(int)((h->npx + 4 * 512 - 1) / (4 * 512)), 128, 0, st>>>(P);
+            pw3_k_gscan_seg<<<gsegBlocks, 128, 0, st>>>(P);
             pw3_k_gscan_walk<<<1, 32, 0, st>>>(P);
             pw3_k_gscan_fix<<<(int)((h->npx + 255) / 256), 256, 0, st>>>(P);
-            pw3_k_gscan_fix_walked<<<(int)((h->npx + 4 * 512 - 1) / (4 * 512)), 128, 0, st>>>(P);
+            pw3_k_gscan_fix_walked<<<gsegBlocks, 128, 0, st>>>(P);
             pw_k_cells<<<(P.totalCells + 255) / 256, 256, 0, st>>>(P, 0);
             pw_k_nbr<<<tiles, blk, 0, st>>>(P);
             pw_compact(h, P, 2, st);

@@ -157,7 +157,7 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // back one word, the lightest so far), so a pixel needs no copy of its 50 words. The copy took 1.2 KB of
 // local memory a pixel, three times what the L1 caches hold, and a word nine accesses.
 // ------------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(256, 2) pw3_k_local(PwParams P) {
+extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
     PW_ROUND_GUARD(P);
     PW3_PIXEL_PROLOGUE
     if (x >= D.W || y >= D.H) return;
@@ -387,8 +387,8 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // ordered scan of the critical items (:776-786 one channel, :1139-1150 three), segment-parallel. The
 // scan's state is only the replaceable word's features (those of its last replacement), only
 // candidates (events with the replacement draw and no fixed match) can replace it, and two scans that
-// both see an item replace it agree from there on. So each segment of kPw3Seg items is scanned by its
-// own warp from kPw3Warm items before its start, from a guessed state (the first of those items'
+// both see an item replace it agree from there on. So each segment of pw_gseg_items items is scanned by its
+// own warp from pw_gseg_warm items before its start, from a guessed state (the first of those items'
 // features): with replacements frequent, the scan reaches the segment in the true state. One warp
 // then walks the segments in order: a segment whose speculative state at its start equals the true
 // incoming features keeps its speculative outcomes (one comparison); otherwise its candidates are
@@ -397,8 +397,6 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // Records: two uint4 per item (pixel, colour|bits, thresholds, descriptors 0-1; descriptor 2|event
 // flags, fixed position|word, speculative word, speculative epoch | replaced << 31).
 // ------------------------------------------------------------------------------------------
-constexpr int kPw3Seg = 512;
-constexpr int kPw3Warm = 128;
 struct Pw3GFeat {
     uint32_t col, d01, d2, bits;
 };
@@ -437,13 +435,20 @@ __device__ __forceinline__ void pw3_set_out(const PawcsDev& S, uint32_t p, uint3
     O.epoch = epoch;
     O.gflags = (uint8_t)((O.gflags & ~1u) | repl);
 }
-// per-segment scratch (PawcsDev::gseg, kPw3SegWords words a segment): [0] replacements of the
+// per-segment scratch (PawcsDev::gseg, kPwGsegWords words a segment): [0] replacements of the
 // speculative scan in the segment, [1..4] its state at the segment's start, [5..8] its state at the
 // end, [9] candidates of the segment (listed in gcand from the segment's first item on); from the
 // walk: [10] mode (1 kept, 2 walked), [11] true epoch at the segment's start, [12] synchronization
 // item (kPwNone: none), [13] epoch shift after it, [14..17] true incoming features
-constexpr int kPw3SegWords = 24;
-__device__ __forceinline__ uint32_t* pw3_segw(const PawcsDev& S, int s) { return S.gseg + (size_t)s * kPw3SegWords; }
+// One plane per scratch word, so that a warp reads 32 segments' words in whole lines.
+struct Pw3SegRef {
+    uint32_t* p;
+    size_t stride;
+    __device__ __forceinline__ uint32_t& operator[](int j) const { return p[(size_t)j * stride]; }
+};
+__device__ __forceinline__ Pw3SegRef pw3_segw(const PawcsDev& S, int s) {
+    return {S.gseg + s, (size_t)pw_gseg_max(S.sd.npx, S.sd.C)};
+}
 __device__ __forceinline__ bool pw3_is_cand(const Pw3Item& it, int G) { return (int)it.fixedPos >= G && it.evRep; }
 
 // the speculative warp scan of items [a, b) from features f and epoch e, 32 items at a time;
@@ -490,19 +495,19 @@ __device__ void pw3_gscan_range(const PawcsDev& S, int G, int wr, uint32_t a, ui
 }
 
 // phase 1: one warp per segment: its candidates listed, then its speculative scan from a guessed
-// state kPw3Warm items before it
+// state pw_gseg_warm items before it
 extern "C" __global__ void __launch_bounds__(128) pw3_k_gscan_seg(PwParams P) {
     PW_ROUND_GUARD(P);
     const PawcsDev& S = P.streams[0];
     const uint32_t n = S.catInfo[0];
     const int s = blockIdx.x * 4 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const uint32_t a = (uint32_t)s * kPw3Seg;
+    const uint32_t seg = (uint32_t)pw_gseg_items(S.sd.C), a = (uint32_t)s * seg;
     if (a >= n) return;
-    const uint32_t b = min(n, a + (uint32_t)kPw3Seg);
+    const uint32_t b = min(n, a + seg);
     const PawcsCtl* pc = S.pc;
     const int G = S.G;
     const int wr = pc->gdict[G - 1];
-    uint32_t* sw = pw3_segw(S, s);
+    const Pw3SegRef sw = pw3_segw(S, s);
     uint32_t nc = 0;
     for (uint32_t base = a; base < b; base += 32) {
         const bool cand = base + lane < b && pw3_is_cand(pw3_item(S, base + lane), G);
@@ -518,7 +523,7 @@ extern "C" __global__ void __launch_bounds__(128) pw3_k_gscan_seg(PwParams P) {
         f.d2 = pc->gw_desc2[wr];
         f.bits = pc->gw_bits[wr];
     } else {
-        const uint32_t w0 = a > (uint32_t)kPw3Warm ? a - (uint32_t)kPw3Warm : 0u;
+        const uint32_t warm = (uint32_t)pw_gseg_warm(S.sd.C), w0 = a > warm ? a - warm : 0u;
         const Pw3Item g = pw3_item(S, w0);
         f.col = g.col;
         f.d01 = g.d01;
@@ -563,34 +568,63 @@ extern "C" __global__ void pw3_k_gscan_walk(PwParams P) {
     f.d2 = pc->gw_desc2[wr];
     f.bits = pc->gw_bits[wr];
     uint32_t e = 0;
-    const int nseg = (int)((n + kPw3Seg - 1) / kPw3Seg);
-    for (int s0 = 0; s0 < nseg; s0 += 32) {
-        const int sl = s0 + lane;
-        uint32_t v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (sl < nseg) {
-            const uint32_t* sw = pw3_segw(S, sl);
+    const uint32_t seg = (uint32_t)pw_gseg_items(S.sd.C);
+    const int nseg = (int)((n + seg - 1) / seg);
+    uint32_t ahead[10];
+    auto fetch = [&](int i) {
+        const Pw3SegRef sw = pw3_segw(S, i < nseg ? i : 0);
 #pragma unroll
-            for (int j = 0; j < 10; ++j) v[j] = sw[j];
-        }
+        for (int j = 0; j < 10; ++j) ahead[j] = i < nseg ? sw[j] : 0u;
+    };
+    fetch(lane);
+    for (int s0 = 0; s0 < nseg; s0 += 32) {
+        // 32 segments at a time, one per lane. Segments whose speculative start equals the speculative end of
+        // the one before follow on it without a look: a run of them is kept at once, by one ballot and a prefix
+        // sum of the replacements; only the breaks are walked one after the other.
+        const int sl = s0 + lane;
+        uint32_t v[10];
+#pragma unroll
+        for (int j = 0; j < 10; ++j) v[j] = ahead[j];
+        fetch(sl + 32);  // the next 32 segments while these are walked
         const int cnt = min(32, nseg - s0);
-        for (int k = 0; k < cnt; ++k) {
-            const int s = s0 + k;
+        bool follows = true;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) follows &= __shfl_up_sync(0xffffffffu, v[5 + j], 1) == v[1 + j];
+        const unsigned breaks = __ballot_sync(0xffffffffu, !follows);
+        uint32_t incl = v[0];  // replacements up to and with this segment
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        for (int k = 0; k < cnt;) {
             uint32_t w[10];
 #pragma unroll
             for (int j = 0; j < 10; ++j) w[j] = __shfl_sync(0xffffffffu, v[j], k);
+            if (w[1] == f.col && w[2] == f.d01 && w[3] == f.d2 && w[4] == f.bits) {
+                // the speculative scan entered segment k in the true state, and so those that follow on it
+                const unsigned after = k < 31 ? breaks >> (k + 1) : 0u;
+                const int stop = min(cnt, after ? k + __ffs(after) : 32);
+                const uint32_t before = __shfl_sync(0xffffffffu, incl - v[0], k);
+                if (lane >= k && lane < stop) {
+                    const Pw3SegRef sw = pw3_segw(S, sl);
+                    sw[10] = 1;
+                    sw[11] = e + incl - v[0] - before;
+                }
+                e += __shfl_sync(0xffffffffu, incl, stop - 1) - before;
+                f.col = __shfl_sync(0xffffffffu, v[5], stop - 1);
+                f.d01 = __shfl_sync(0xffffffffu, v[6], stop - 1);
+                f.d2 = __shfl_sync(0xffffffffu, v[7], stop - 1);
+                f.bits = __shfl_sync(0xffffffffu, v[8], stop - 1);
+                k = stop;
+                continue;
+            }
+            const int s = s0 + k;
             const Pw3GFeat fin = f;
             const uint32_t ein = e;
-            uint32_t mode, sync = kPwNone, offset = 0;
-            if (w[1] == f.col && w[2] == f.d01 && w[3] == f.d2 && w[4] == f.bits) {
-                mode = 1;  // the speculative scan entered the segment in the true state
-                e += w[0];
-                f.col = w[5];
-                f.d01 = w[6];
-                f.d2 = w[7];
-                f.bits = w[8];
-            } else {
-                mode = 2;
-                const uint32_t a = (uint32_t)s * kPw3Seg, nc = w[9];
+            uint32_t sync = kPwNone, offset = 0;
+            {
+                const uint32_t a = (uint32_t)s * seg, nc = w[9];
                 for (uint32_t base = 0; base < nc && sync == kPwNone; base += 32) {
                     const int cn = (int)min(32u, nc - base);
                     const bool valid = lane < cn;
@@ -630,8 +664,8 @@ extern "C" __global__ void pw3_k_gscan_walk(PwParams P) {
                 }
             }
             if (lane == 0) {
-                uint32_t* sw = pw3_segw(S, s);
-                sw[10] = mode;
+                const Pw3SegRef sw = pw3_segw(S, s);
+                sw[10] = 2;
                 sw[11] = ein;
                 sw[12] = sync;
                 sw[13] = offset;
@@ -640,6 +674,7 @@ extern "C" __global__ void pw3_k_gscan_walk(PwParams P) {
                 sw[16] = fin.d2;
                 sw[17] = fin.bits;
             }
+            ++k;
         }
     }
     if (lane == 0) {
@@ -659,7 +694,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_gscan_fix(PwParams P) {
     const uint32_t n = S.catInfo[0];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t* sw = pw3_segw(S, (int)(i / kPw3Seg));
+    const Pw3SegRef sw = pw3_segw(S, (int)(i / (uint32_t)pw_gseg_items(S.sd.C)));
     const uint32_t mode = sw[10], sync = sw[12];
     if (mode == 2 && (sync == kPwNone || i <= sync)) return;
     const uint32_t shift = mode == 1 ? sw[11] : sw[13];
@@ -674,11 +709,11 @@ extern "C" __global__ void __launch_bounds__(128) pw3_k_gscan_fix_walked(PwParam
     const PawcsDev& S = P.streams[0];
     const uint32_t n = S.catInfo[0];
     const int s = blockIdx.x * 4 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const uint32_t a = (uint32_t)s * kPw3Seg;
+    const uint32_t seg = (uint32_t)pw_gseg_items(S.sd.C), a = (uint32_t)s * seg;
     if (a >= n) return;
-    const uint32_t* sw = pw3_segw(S, s);
+    const Pw3SegRef sw = pw3_segw(S, s);
     if (sw[10] != 2u) return;
-    const uint32_t b = min(n, a + (uint32_t)kPw3Seg);
+    const uint32_t b = min(n, a + seg);
     const uint32_t end = sw[12] == kPwNone ? b : sw[12] + 1;
     const int G = S.G;
     const int wr = S.pc->gdict[G - 1];

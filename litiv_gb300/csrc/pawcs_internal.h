@@ -159,6 +159,16 @@ struct PawcsDev {
     uint8_t* gtrue;            // global-word scan: walked candidates that replace the word
 };
 
+// Items per segment of the ordered global-word scan, one warp each, and the warm-up items before it. On three
+// channels every second item replaces the word, each replacement is a step of its warp, and 128 items of
+// warm-up nearly always reach the true start: short segments keep all SMs busy (scan and walk of a 640x480
+// round: 66 + 46 us at 512 items, 29 + 18 at 128, 19 + 32 at 64 with 64 of warm-up). On one channel
+// replacements are rare, a segment seldom starts in the true state, and more segments are more of a walk
+// (33 + 5 us at 512, 19 + 10 at 256).
+LV_HD constexpr int pw_gseg_items(int C) { return C == 3 ? 128 : 256; }
+LV_HD constexpr int pw_gseg_warm(int C) { return C == 3 ? 128 : 64; }
+constexpr int kPwGsegWords = 24;  // scratch words of a segment
+LV_HD constexpr size_t pw_gseg_max(size_t npx, int C) { return npx / pw_gseg_items(C) + 2; }  // segments
 constexpr int kPwCompactBlk = 1024;  // pixels per block of the ordered compactions
 constexpr int kPwCats = kPwMaxGlobal + 1;  // compaction categories: the global words, or the critical items
 constexpr int kPwCatBase = 64;       // catInfo: [0, kPwCats) category totals, [kPwCatBase, +kPwCats) bases

@@ -218,30 +218,45 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_illum(PwParams P) {
     const StreamDev& D = S.sd;
     const int y = gr - D.rowBase;
     uint32_t carry = 0;  // outcome of the pixel before the chunk
-    for (int x0 = 0; x0 < D.W; x0 += 32) {
-        const int x = x0 + lane;
-        const int p = y * D.W + x;
-        const bool in = x < D.W && D.roi[p];
-        uint32_t f = 0, m0 = 0, mL = 0;  // f: bit0 = outcome if the left neighbour made no update, bit1 = if it did
-        if (in) {
-            const uint32_t uvp = S.uv[p];
-            m0 = S.illum[p] != 0;
-            mL = D.roi[p] & 1u;  // the mask after the left neighbour's update
-            const uint32_t u0 = uvp & 1u, u1 = (uvp >> 1) & 1u;
-            f = (m0 ? u1 : u0) | ((mL ? u1 : u0) << 1);
-        }
-        // inclusive scan: F = f_lane o f_lane-1 o ... o f_x0
-        uint32_t F = f;
+    const int row = y * D.W;
+    // four chunks a step: their loads are requested before the first is scanned
+    for (int xb = 0; xb < D.W; xb += 128) {
+        uint32_t roi[4], uvp[4], il[4];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, F, d);
-            if (lane >= d) F = ((F >> (o & 1u)) & 1u) | (((F >> ((o >> 1) & 1u)) & 1u) << 1);
+        for (int j = 0; j < 4; ++j) {
+            const int x = xb + 32 * j + lane;
+            roi[j] = uvp[j] = il[j] = 0u;
+            if (x < D.W) {
+                roi[j] = D.roi[row + x];
+                uvp[j] = S.uv[row + x];
+                il[j] = S.illum[row + x];
+            }
         }
-        const uint32_t u = (F >> carry) & 1u;
-        uint32_t prevU = __shfl_up_sync(0xffffffffu, u, 1);
-        if (lane == 0) prevU = carry;
-        if (x < D.W) S.uFinal[p] = in ? (uint8_t)(u | ((prevU ? mL : m0) ? 2u : 0u)) : (uint8_t)0;
-        carry = __shfl_sync(0xffffffffu, u, 31);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int x = xb + 32 * j + lane;
+            if (xb + 32 * j >= D.W) break;
+            const bool in = roi[j] != 0u;
+            uint32_t f = 0, m0 = 0, mL = 0;  // f: bit0 = outcome if the left neighbour made no update, bit1 = if it did
+            if (in) {
+                m0 = il[j] != 0u;
+                mL = roi[j] & 1u;  // the mask after the left neighbour's update
+                const uint32_t u0 = uvp[j] & 1u, u1 = (uvp[j] >> 1) & 1u;
+                f = (m0 ? u1 : u0) | ((mL ? u1 : u0) << 1);
+            }
+            // inclusive scan: F = f_lane o f_lane-1 o ... o f_x0
+            uint32_t F = f;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, F, d);
+                if (lane >= d) F = ((F >> (o & 1u)) & 1u) | (((F >> ((o >> 1) & 1u)) & 1u) << 1);
+            }
+            const uint32_t u = (F >> carry) & 1u;
+            uint32_t prevU = __shfl_up_sync(0xffffffffu, u, 1);
+            if (lane == 0) prevU = carry;
+            if (x < D.W) S.uFinal[row + x] = in ? (uint8_t)(u | ((prevU ? mL : m0) ? 2u : 0u)) : (uint8_t)0;
+            carry = __shfl_sync(0xffffffffu, u, 31);
+        }
     }
 }
 
