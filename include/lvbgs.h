@@ -277,9 +277,9 @@ int lvbgs_debug_repair_phases(lvbgs_handle h, int batched, double* out_us, int m
 enum { LVBGS_FAULT_NONE = 0, LVBGS_FAULT_BARRIER_TIMEOUT = 1, LVBGS_FAULT_REPAIR_LIMIT = 2, LVBGS_FAULT_PAWCS_ROUNDS = 3 };
 lvbgs_status lvbgs_debug_inject_fault(lvbgs_handle h, int kind);
 /* Host time (ms) of the last PAWCS frame step's parts (inspection; no reference counterpart):
- * [0] enqueueing the fixed-point rounds (the first batch and any further ones), [1] the waits for
- * the rounds, [2] enqueueing the rest of the frame step (with the camera-motion decision's wait every
- * 8 or 16 frames), [3] the final wait, [4] the status read-back. */
+ * [0] enqueueing the fixed-point rounds and the rest of the frame behind them, [1] the waits for them,
+ * [2] enqueueing what follows a camera-motion decision or an automatic model reset, [3] the waits for that,
+ * [4] the status. */
 lvbgs_status lvbgs_debug_pawcs_host_timing(lvbgs_handle h, double* out_ms);
 
 /* ---- PAWCS (BackgroundSubtractorPAWCS, modules/video/src/BackgroundSubtractorPAWCS.cpp) ----

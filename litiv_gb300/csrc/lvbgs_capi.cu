@@ -45,7 +45,6 @@ extern "C" __global__ void pw_k_nbr(PwParams P);
 extern "C" __global__ void pw_k_replace(PwParams P);
 extern "C" __global__ void pw_k_nbr_loops(PwParams P);
 extern "C" __global__ void pw_k_dirty(PwParams P);
-extern "C" __global__ void pw_k_round_end(PwParams P);
 extern "C" __global__ void pw_k_commit(PwParams P);
 extern "C" __global__ void pw_k_weights(PwParams P);
 extern "C" __global__ void pw_k_gw_recalc(PwParams P);
@@ -54,15 +53,15 @@ extern "C" __global__ void pw_k_gw_blur(PwParams P, const double* rowsum);
 extern "C" __global__ void pw_k_gw_sort(PwParams P);
 extern "C" __global__ void pw_k_lut_sort(PwParams P, int mode);
 extern "C" __global__ void pw_k_blink_close(PwParams P);
-extern "C" __global__ void pw_k_epilogue(PwParams P);
+extern "C" __global__ void pw_k_epilogue(PwParams P, int decide);
 extern "C" __global__ void pw_k_ds(PwParams P);
-extern "C" __global__ void pw_k_reset_decide(PwParams P);
 extern "C" __global__ void pw_k_motion_bg(PwParams P);
 extern "C" __global__ void pw_k_motion_decide(PwParams P);
-extern "C" __global__ void pw_k_compact_count(PwParams P, int mode);
+extern "C" __global__ void pw_k_compact(PwParams P, int mode);
+extern "C" __global__ void pw_k_compact_count(PwParams P);
 extern "C" __global__ void pw_k_compact_offsets(PwParams P, int ncat);
-extern "C" __global__ void pw_k_compact_scatter(PwParams P, int mode);
-extern "C" __global__ void pw_k_close(PwParams P);
+extern "C" __global__ void pw_k_compact_scatter(PwParams P);
+extern "C" __global__ void pw_k_close(PwParams P, int resetDone);
 extern "C" __global__ void pw_k_refresh_local(PawcsDev S, uint32_t t, int buf, int baseOcc, float decr, int force,
                                               int onlyPending, int useDil);
 extern "C" __global__ void pw_k_refresh_global(PawcsDev S, uint32_t t, int buf, int force, int onlyPending, int useDil);
@@ -154,13 +153,15 @@ struct Workspace {
 }  // namespace
 
 // a PAWCS frame step in flight: its stream, launch parameters and the stage of its host waits (0: the
-// fixed-point rounds, 1: the camera-motion decision, 2: the end of the frame)
+// fixed-point rounds with the rest of the frame behind them, 1: the frame's end after the camera-motion
+// decision, 2: its end after an automatic model reset)
 struct PwStep {
     cudaStream_t st = nullptr;
     PwParams P{}, PR{};
     int enq = 0, maxRounds = 64, stage = 0;
     uint8_t* mask = nullptr;
     bool devMask = false, active = false;
+    bool motion = false;  // this frame takes the camera-motion decision, for which the host waits
 };
 
 struct lvbgs_ctx {
@@ -424,6 +425,7 @@ lvbgs_status launch_tick(lvbgs_handle errh, Workspace& ws, int n, cudaStream_t s
     P.dbgFault = fault;
     P.barrierNs = fault == LVBGS_FAULT_BARRIER_TIMEOUT ? kDebugBarrierNs : kBarrierNs;
     P.maxRepairIters = fault == LVBGS_FAULT_REPAIR_LIMIT ? 0 : kRepairIterLimit;
+    P.gate = nullptr;
     P.streams = ws.d_streams;
     P.nStreams = n;
     P.totalTiles = totalTiles;
@@ -580,7 +582,7 @@ enum {
     PL_GMAP, PL_DSLT, PL_DSST, PL_DSROI,
     // scratch (not part of the model)
     PL_BITS, PL_LABEL, PL_INTENT, PL_DESCT, PL_REC, PL_OUT, PL_REPB, PL_REPA, PL_UFINAL, PL_UV,
-    PL_ITEMLIST, PL_CONTRIBLIST, PL_BLKCOUNTS, PL_CATINFO, PL_DSABS, PL_UPDLIST, PL_GITEM, PL_CONTRIB, PL_DSFRAME, PL_FRAME, PL_MASK, PL_ROWSUM, PL_WORK, PL_FLAGS, PL_PDEV, PL_SDEV, PL_DIRTY, PL_GSEG, PL_GCAND, PL_GTRUE, PL_COUNT
+    PL_ITEMLIST, PL_CONTRIBLIST, PL_BLKCOUNTS, PL_CHAIN, PL_CATINFO, PL_DSABS, PL_UPDLIST, PL_GITEM, PL_CONTRIB, PL_DSFRAME, PL_FRAME, PL_MASK, PL_ROWSUM, PL_WORK, PL_FLAGS, PL_PDEV, PL_SDEV, PL_DIRTY, PL_GSEG, PL_GCAND, PL_GTRUE, PL_COUNT
 };
 struct PwLayout {
     size_t off[PL_COUNT];
@@ -616,6 +618,7 @@ PwLayout pw_layout(int W, int H, int C, int L, int G) {
     sz[PL_ITEMLIST] = npx * 32;
     sz[PL_CONTRIBLIST] = npx * 4;
     sz[PL_BLKCOUNTS] = ((npx + kPwCompactBlk - 1) / kPwCompactBlk) * kPwCats * 4;
+    sz[PL_CHAIN] = ((npx + kPwCompactBlk - 1) / kPwCompactBlk) * 8 + 256;
     sz[PL_CATINFO] = 2 * kPwCatBase * 4;
     sz[PL_DSABS] = std::max<size_t>(nds, 1) * 4;
     sz[PL_UPDLIST] = npx * 4;
@@ -726,6 +729,8 @@ void pw_fill(lvbgs_ctx* h, const PwLayout& Lo, int L, int G) {
     D.itemList = (uint4*)(b + Lo.off[PL_ITEMLIST]);
     D.contribList = (float*)(b + Lo.off[PL_CONTRIBLIST]);
     D.blkCounts = (uint32_t*)(b + Lo.off[PL_BLKCOUNTS]);
+    D.ticket = (unsigned int*)(b + Lo.off[PL_CHAIN]);
+    D.chain = (unsigned long long*)(b + Lo.off[PL_CHAIN] + 256);
     D.catInfo = (uint32_t*)(b + Lo.off[PL_CATINFO]);
     D.dsAbs = (float*)(b + Lo.off[PL_DSABS]);
     D.updList = (uint32_t*)(b + Lo.off[PL_UPDLIST]);
@@ -754,6 +759,9 @@ PwParams pw_params(lvbgs_ctx* h, double lr) {
     P.round = 0;
     P.lr = lr;
     P.flags = h->d_flags;
+    P.hflags = h->h_flags;
+    P.err = &h->d_work->err;
+    P.gate = nullptr;
     P.conv = nullptr;
     return P;
 }
@@ -768,16 +776,12 @@ lvbgs_status pw_upload_desc(lvbgs_ctx* h, cudaStream_t st) {
 // refreshModel(nBaseOccCount, fOccDecrFrac, bForceFGUpdate) of the dictionaries in buffer buf at frame t
 lvbgs_status pw_refresh(lvbgs_ctx* h, uint32_t t, int buf, int baseOcc, float decr, int force, int onlyPending,
                         int useDil, cudaStream_t st) {
-    const int npx = (int)h->npx;
-    if (h->C == 3) {
-        pw3_k_refresh_local<<<(npx + 127) / 128, 128, 0, st>>>(h->pd, t, buf, baseOcc, decr, force, onlyPending, useDil);
-        pw3_k_refresh_global<<<1, 1, 0, st>>>(h->pd, t, buf, force, onlyPending, useDil);
-    } else {
-        pw_k_refresh_local<<<(npx + 127) / 128, 128, 0, st>>>(h->pd, t, buf, baseOcc, decr, force, onlyPending, useDil);
-        pw_k_refresh_global<<<1, 1, 0, st>>>(h->pd, t, buf, force, onlyPending, useDil);
-    }
-    PwParams P = pw_params(h, 0.0);
-    pw_k_lut_sort<<<h->sd.nTiles, kThreads, 0, st>>>(P, onlyPending ? 2 : 1);
+    const dim3 g((unsigned)((h->npx + 127) / 128));
+    launch_chained(h->C == 3 ? pw3_k_refresh_local : pw_k_refresh_local, g, dim3(128), st, h->pd, t, buf, baseOcc, decr, force,
+                   onlyPending, useDil);
+    launch_chained(h->C == 3 ? pw3_k_refresh_global : pw_k_refresh_global, dim3(1), dim3(1), st, h->pd, t, buf, force,
+                   onlyPending, useDil);
+    launch_chained(pw_k_lut_sort, dim3(h->sd.nTiles), dim3(kThreads), st, pw_params(h, 0.0), onlyPending ? 2 : 1);
     LV_CUDA(h, cudaGetLastError(), "refresh kernel launch");
     return LVBGS_OK;
 }
@@ -836,7 +840,7 @@ lvbgs_status pw_initialize(lvbgs_ctx* h, const uint8_t* img, int W, int H, int C
     h->spilled = false;
     const PwLayout Lo = pw_layout(W, H, C, g.L, g.G);
     LV_CUDA(h, cudaMalloc(&h->dmem, Lo.total), "model allocation");
-    if (!h->h_flags) LV_CUDA(h, cudaHostAlloc((void**)&h->h_flags, 64, cudaHostAllocDefault), "pinned allocation");
+    if (!h->h_flags) LV_CUDA(h, cudaHostAlloc((void**)&h->h_flags, 64, cudaHostAllocMapped), "pinned allocation");
     h->persistBytes = Lo.persist;
     h->totalBytes = Lo.total;
     h->W = W;
@@ -917,65 +921,132 @@ double pw_ms_since(std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
-// ordered compaction: mode 0 lists the critical global items, mode 1 the word weight contributions,
-// mode 2 the neighbour-update loops
-void pw_compact(lvbgs_ctx* h, const PwParams& Pc, int mode, cudaStream_t st) {
-    const int cblocks = (int)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk);
-    pw_k_compact_count<<<cblocks, 256, 0, st>>>(Pc, mode);
-    const int ncat = mode == 1 ? h->pd.G : 1;
-    pw_k_compact_offsets<<<1, 32 * std::min(ncat, 32), 0, st>>>(Pc, ncat);
-    pw_k_compact_scatter<<<cblocks, 256, 0, st>>>(Pc, mode);
-}
-
-// enqueues fixed-point rounds enq .. enq+n-1 (each ends with pw_k_round_end; once a round finds no dirty
-// pixel every later kernel of the rounds returns at once, PW_ROUND_GUARD) and the read-back of the
-// converged flag and round count
+// enqueues fixed-point rounds enq .. enq+n-1 (once a round finds no dirty pixel every later kernel of the rounds
+// returns at once, PW_ROUND_GUARD)
 lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
     PwStep& w = h->pws;
     const cudaStream_t st = w.st;
-    const dim3 blk(kThreads);
-    const int tiles = h->sd.nTiles;
-    const int cblocks = (int)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk);
+    const dim3 blk(kThreads), tiles(h->sd.nTiles), warps4(128);
+    const dim3 cblocks((unsigned)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk));
     const size_t gseg4 = 4 * (size_t)pw_gseg_items(h->C);  // items of a block of four segments
-    const int gsegBlocks = (int)((h->npx + gseg4 - 1) / gseg4);
+    const dim3 gseg((unsigned)((h->npx + gseg4 - 1) / gseg4));
+    const bool c3 = h->C == 3;
     for (int r = 0; r < n && w.enq < w.maxRounds; ++r, ++w.enq) {
         w.PR.round = w.enq;
         const PwParams& P = w.PR;
-        if (h->C == 3) {
-            // three channels: the local pass applies the earlier updaters' loops itself
-            pw3_k_local<<<tiles, blk, 0, st>>>(P);
-            pw_k_illum<<<(h->H + 7) / 8, 256, 0, st>>>(P);
-            pw_compact(h, P, 0, st);
-            pw3_k_gscan_seg<<<gsegBlocks, 128, 0, st>>>(P);
-            pw3_k_gscan_walk<<<1, 32, 0, st>>>(P);
-            pw3_k_gscan_fix<<<(int)((h->npx + 255) / 256), 256, 0, st>>>(P);
-            pw3_k_gscan_fix_walked<<<gsegBlocks, 128, 0, st>>>(P);
-            pw_k_cells<<<(P.totalCells + 255) / 256, 256, 0, st>>>(P, 0);
-            pw_k_nbr<<<tiles, blk, 0, st>>>(P);
-            LV_CUDA(h, cudaMemsetAsync(h->d_flags, 0, 4, st), "flag reset");
-            pw3_k_dirty<<<tiles, blk, 0, st>>>(P);
-        } else {
-            pw_k_local<<<tiles, blk, 0, st>>>(P);
-            pw_k_illum<<<(h->H + 7) / 8, 256, 0, st>>>(P);
-            pw_compact(h, P, 0, st);
-            pw3_k_gscan_seg<<<gsegBlocks, 128, 0, st>>>(P);
-            pw3_k_gscan_walk<<<1, 32, 0, st>>>(P);
-            pw3_k_gscan_fix<<<(int)((h->npx + 255) / 256), 256, 0, st>>>(P);
-            pw3_k_gscan_fix_walked<<<gsegBlocks, 128, 0, st>>>(P);
-            pw_k_cells<<<(P.totalCells + 255) / 256, 256, 0, st>>>(P, 0);
-            pw_k_nbr<<<tiles, blk, 0, st>>>(P);
-            pw_compact(h, P, 2, st);
-            pw_k_nbr_loops<<<std::max(1, std::min(cblocks * 4, 1216)), 256, 0, st>>>(P);
-            pw_k_replace<<<tiles, blk, 0, st>>>(P);
-            LV_CUDA(h, cudaMemsetAsync(h->d_flags, 0, 4, st), "flag reset");
-            pw_k_dirty<<<tiles, blk, 0, st>>>(P);
+        // three channels: the local pass applies the earlier updaters' loops itself
+        launch_chained(c3 ? pw3_k_local : pw_k_local, tiles, blk, st, P);
+        launch_chained(pw_k_illum, dim3((h->H + 7) / 8), blk, st, P);
+        launch_chained(pw_k_compact, cblocks, blk, st, P, 0);
+        launch_chained(pw3_k_gscan_seg, gseg, warps4, st, P);
+        launch_chained(pw3_k_gscan_walk, dim3(1), dim3(32), st, P);
+        launch_chained(pw3_k_gscan_fix, dim3((unsigned)((h->npx + 255) / 256)), blk, st, P);
+        launch_chained(pw3_k_gscan_fix_walked, gseg, warps4, st, P);
+        launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 0);
+        launch_chained(pw_k_nbr, tiles, blk, st, P);
+        if (!c3) {
+            launch_chained(pw_k_compact, cblocks, blk, st, P, 2);
+            launch_chained(pw_k_nbr_loops, dim3(std::max(1u, std::min(cblocks.x * 4, 1216u))), blk, st, P);
+            launch_chained(pw_k_replace, tiles, blk, st, P);
         }
-        pw_k_round_end<<<1, 1, 0, st>>>(P);
+        launch_chained(c3 ? pw3_k_dirty : pw_k_dirty, tiles, blk, st, P);
     }
     LV_CUDA(h, cudaGetLastError(), "PAWCS round launch");
-    LV_CUDA(h, cudaMemcpyAsync(h->h_flags + 3, h->d_flags + 3, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st),
-            "flag read-back");
     return LVBGS_OK;
+}
+
+// opens a PAWCS frame step: the descriptors as kernel arguments, the work area and the flags cleared and, one
+// channel, no replacement known yet (one launch where two uploads and three memsets were enqueued)
+__global__ void __launch_bounds__(256) pw_k_begin(const __grid_constant__ PawcsDev D, PawcsDev* dst, StreamDev* sdst,
+                                                  TickWork* work, unsigned int* flags) {
+    static_assert(sizeof(PawcsDev) % 4 == 0 && sizeof(PawcsDev) < 4000, "copied as words");
+    if (blockIdx.x == 0) {
+        const uint32_t* src = (const uint32_t*)&D;
+        for (int i = threadIdx.x; i < (int)(sizeof(PawcsDev) / 4); i += blockDim.x) ((uint32_t*)dst)[i] = src[i];
+        const uint32_t* ssrc = (const uint32_t*)&D.sd;
+        for (int i = threadIdx.x; i < (int)(sizeof(StreamDev) / 4); i += blockDim.x) ((uint32_t*)sdst)[i] = ssrc[i];
+        for (int i = threadIdx.x; i < (int)(sizeof(TickWork) / 4); i += blockDim.x) ((uint32_t*)work)[i] = 0u;
+        if (threadIdx.x < PWF_COUNT) flags[threadIdx.x] = 0u;
+    }
+    if (D.sd.C == 1)
+        for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.sd.npx; p += gridDim.x * blockDim.x) D.repBefore[p] = kPwNone;
+}
+
+// the rest of the frame after the fixed point, enqueued with the rounds and gated on it; motion frames end at
+// the camera-motion decision
+lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
+    PwStep& w = h->pws;
+    const cudaStream_t st = w.st;
+    const PwParams& P = w.P;
+    const dim3 blk(kThreads), tiles(h->sd.nTiles);
+    const dim3 cblocks((unsigned)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk));
+    const bool c3 = h->C == 3;
+    if (c3) launch_chained(pw3_k_later, tiles, blk, st, P);
+    launch_chained(c3 ? pw3_k_commit : pw_k_commit, tiles, blk, st, P);
+    launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 1);
+    launch_chained(pw_k_compact_count, cblocks, blk, st, P);
+    launch_chained(pw_k_compact_offsets, dim3(1), dim3(32 * std::min(h->pd.G, 32)), st, P, h->pd.G);
+    launch_chained(pw_k_compact_scatter, cblocks, blk, st, P);
+    launch_chained(pw_k_weights, dim3(kPwMaxGlobal), blk, st, P);
+    // global-word upkeep: the kernels of frames without one would return at once
+    const uint32_t t = (uint32_t)(h->pw_frames + 1);
+    const uint32_t rate = t <= (uint32_t)kPwBootWin ? 8u : 16u;
+    if (t % (rate << 5) == 0) launch_chained(pw_k_gw_recalc, dim3(kPwMaxGlobal), blk, st, P);
+    if (t % rate == 0) {
+        launch_chained(pw_k_gw_decay, dim3(64, kPwMaxGlobal), blk, st, P, h->d_rowsum);
+        launch_chained(pw_k_gw_blur, dim3(64, kPwMaxGlobal), blk, st, P, (const double*)h->d_rowsum);
+    }
+    launch_chained(pw_k_gw_sort, dim3(1), dim3(32), st, P);
+    if (t % rate == 0) launch_chained(pw_k_lut_sort, tiles, blk, st, P, 0);
+    launch_chained(pw_k_blink_close, tiles, blk, st, P);
+    TickParams TP;
+    std::memset(&TP, 0, sizeof(TP));
+    TP.streams = h->d_sd;
+    TP.nStreams = 1;
+    TP.totalTiles = h->sd.nTiles;
+    TP.totalRows = h->H;
+    TP.work = h->d_work;
+    TP.totalSegs = h->sd.nSegs;
+    TP.gate = P.gate;
+    const dim3 rowBlocks((h->H + 7) / 8);
+    launch_chained(lvbgs_k_unite, rowBlocks, blk, st, TP);
+    launch_chained(lvbgs_k_fill, rowBlocks, blk, st, TP);
+    launch_chained(lvbgs_k_final, dim3(TP.totalSegs), blk, st, TP);
+    const int nds = (h->W / 8) * (h->H / 8);
+    if (nds > 0) launch_chained(c3 ? pw3_k_ds : pw_k_ds, dim3((nds + 31) / 32), blk, st, P);
+    launch_chained(pw_k_epilogue, dim3(1), blk, st, P, motion ? 0 : 1);
+    if (motion) {
+        // camera-motion comparison (:1480-1501): the host waits for the decision, which may switch the
+        // local word weight offset and run refreshModel(1, 1, true). The frame's background image goes to the
+        // label buffer (free after the hole filling, 4 bytes a pixel).
+        const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
+        uint8_t* bg = (uint8_t*)h->sd.label;
+        if (c3) pw3_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
+        else pw_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
+        launch_chained(c3 ? pw3_k_motion_bg : pw_k_motion_bg, dim3((nds + 31) / 32), blk, st, P);
+        launch_chained(pw_k_motion_decide, dim3(1), blk, st, P);
+    }
+    LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
+    return LVBGS_OK;
+}
+
+// the end of the frame: its close (which a pending automatic reset holds back) and the mask download
+lvbgs_status pw_enqueue_close(lvbgs_ctx* h, int resetDone) {
+    PwStep& w = h->pws;
+    launch_chained(pw_k_close, dim3(1), dim3(32), w.st, w.P, resetDone);
+    LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
+    if (w.mask && !w.devMask)
+        LV_CUDA(h, cudaMemcpyAsync(w.mask, h->d_mask, h->npx, cudaMemcpyDeviceToHost, w.st), "mask download");
+    return LVBGS_OK;
+}
+
+// rounds, then the tail behind their gate: the whole frame in one enqueue when the rounds suffice
+lvbgs_status pw_enqueue_frame(lvbgs_ctx* h, int rounds) {
+    PwStep& w = h->pws;
+    lvbgs_status s = pw_enqueue_rounds(h, rounds);
+    if (s == LVBGS_OK) s = pw_enqueue_tail_a(h, w.motion);
+    if (s == LVBGS_OK && !w.motion) s = pw_enqueue_close(h, 0);
+    return s;
 }
 
 // one PAWCS frame step: local passes to the raster-order fixed point (enqueued ahead, as many rounds as
@@ -994,104 +1065,23 @@ lvbgs_status pw_begin(lvbgs_ctx* h, const uint8_t* img, size_t stride, uint8_t* 
     w.devMask = mask_writable_by_device(mask);
     h->sd.frame = dimg;
     h->sd.maskOut = w.devMask ? mask : h->d_mask;
-    if ((s = pw_upload_desc(h, st)) != LVBGS_OK) return s;
+    h->pd.sd = h->sd;
+    for (int i = 0; i < PWF_COUNT; ++i) h->h_flags[i] = 0u;
+    pw_k_begin<<<h->C == 1 ? (unsigned)((h->npx + 1023) / 1024) : 1u, 256, 0, st>>>(h->pd, h->d_pd, h->d_sd, h->d_work,
+                                                                                  h->d_flags);
     w.P = pw_params(h, lr);
-    LV_CUDA(h, cudaMemsetAsync(h->pd.repBefore, 0xff, h->npx * 4, st), "scratch reset");
-    LV_CUDA(h, cudaMemsetAsync(h->d_work, 0, sizeof(TickWork), st), "scratch reset");
     w.maxRounds = h->dbg_fault == LVBGS_FAULT_PAWCS_ROUNDS ? 1 : 64;
     h->dbg_fault = 0;
-    LV_CUDA(h, cudaMemsetAsync(h->d_flags, 0, 5 * sizeof(unsigned int), st), "flag reset");
     w.PR = w.P;
-    w.PR.conv = h->d_flags + 3;
+    w.PR.conv = h->d_flags + PWF_CONV;
+    w.P.gate = h->d_flags + PWF_CONV;
     w.enq = 0;
-    s = pw_enqueue_rounds(h, std::max(1, std::min(h->pw_rounds_last, w.maxRounds)));
+    w.motion = h->W >= 8 && h->H >= 8 && (uint32_t)(h->pw_frames + 1) % kPwBootWin == 0;
+    s = pw_enqueue_frame(h, std::max(1, std::min(h->pw_rounds_last, w.maxRounds)));
     w.stage = 0;
     w.active = s == LVBGS_OK;
     h->pw_host_ms[0] += pw_ms_since(t0);
     return s;
-}
-
-// the rest of the frame after the fixed point, up to the camera-motion decision (enqueued with its
-// read-back on frames that take it: returns true) or to the end (returns false)
-lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool& motion) {
-    PwStep& w = h->pws;
-    const cudaStream_t st = w.st;
-    const PwParams& P = w.P;
-    const dim3 blk(kThreads);
-    const int tiles = h->sd.nTiles;
-    const bool c3 = h->C == 3;
-    if (c3) {
-        pw3_k_later<<<tiles, blk, 0, st>>>(P);
-        pw3_k_commit<<<tiles, blk, 0, st>>>(P);
-    } else {
-        pw_k_commit<<<tiles, blk, 0, st>>>(P);
-    }
-    pw_k_cells<<<(P.totalCells + 255) / 256, 256, 0, st>>>(P, 1);
-    pw_compact(h, P, 1, st);
-    pw_k_weights<<<kPwMaxGlobal, 256, 0, st>>>(P);
-    pw_k_gw_recalc<<<kPwMaxGlobal, 256, 0, st>>>(P);
-    pw_k_gw_decay<<<dim3(64, kPwMaxGlobal), 256, 0, st>>>(P, h->d_rowsum);
-    pw_k_gw_blur<<<dim3(64, kPwMaxGlobal), 256, 0, st>>>(P, h->d_rowsum);
-    pw_k_gw_sort<<<1, 32, 0, st>>>(P);
-    pw_k_lut_sort<<<tiles, blk, 0, st>>>(P, 0);
-    pw_k_blink_close<<<tiles, blk, 0, st>>>(P);
-    TickParams TP;
-    std::memset(&TP, 0, sizeof(TP));
-    TP.streams = h->d_sd;
-    TP.nStreams = 1;
-    TP.totalTiles = tiles;
-    TP.totalRows = h->H;
-    TP.work = h->d_work;
-    TP.totalSegs = h->sd.nSegs;
-    const int rowBlocks = (h->H + 7) / 8;
-    lvbgs_k_unite<<<rowBlocks, blk, 0, st>>>(TP);
-    lvbgs_k_fill<<<rowBlocks, blk, 0, st>>>(TP);
-    lvbgs_k_final<<<TP.totalSegs, blk, 0, st>>>(TP);
-    const int nds = (h->W / 8) * (h->H / 8);
-    if (nds > 0) {
-        if (c3) pw3_k_ds<<<(nds + 31) / 32, 256, 0, st>>>(P);
-        else pw_k_ds<<<(nds + 31) / 32, 256, 0, st>>>(P);
-    }
-    pw_k_epilogue<<<1, 256, 0, st>>>(P);
-    const uint32_t t = (uint32_t)(h->pw_frames + 1);
-    motion = nds > 0 && t % kPwBootWin == 0;
-    if (motion) {
-        // camera-motion comparison (:1480-1501): the host waits for the decision, which may switch the
-        // local word weight offset and run refreshModel(1, 1, true)
-        const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
-        // the frame's background image goes to the label buffer (free after the hole filling, 4 bytes a pixel)
-        uint8_t* bg = (uint8_t*)h->sd.label;
-        if (c3) {
-            pw3_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
-            pw3_k_motion_bg<<<(nds + 31) / 32, 256, 0, st>>>(P);
-        } else {
-            pw_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
-            pw_k_motion_bg<<<(nds + 31) / 32, 256, 0, st>>>(P);
-        }
-        pw_k_motion_decide<<<1, 256, 0, st>>>(P);
-        LV_CUDA(h, cudaGetLastError(), "PAWCS camera-motion launch");
-        LV_CUDA(h, cudaMemcpyAsync(h->h_flags + 1, h->d_flags + 1, 8, cudaMemcpyDeviceToHost, st), "flag read-back");
-    }
-    return LVBGS_OK;
-}
-
-// the end of the frame: the automatic model reset and the mask download
-lvbgs_status pw_enqueue_tail_b(lvbgs_ctx* h) {
-    PwStep& w = h->pws;
-    const cudaStream_t st = w.st;
-    const PwParams& P = w.P;
-    const uint32_t t = (uint32_t)(h->pw_frames + 1);
-    const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
-    pw_k_reset_decide<<<1, 32, 0, st>>>(P);
-    // automatic model reset (:1503-1508): refreshModel(offset/8, 0, true) and T(x) := 1
-    lvbgs_status s = pw_refresh(h, t, nxt, (int)(h->pw_offset / 8), 0.0f, 1, 1, 1, st);
-    if (s != LVBGS_OK) return s;
-    pw_k_reset_T<<<256, 256, 0, st>>>(h->pd, nxt);
-    pw_k_close<<<1, 32, 0, st>>>(P);
-    LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
-    if (w.mask && !w.devMask)
-        LV_CUDA(h, cudaMemcpyAsync(w.mask, h->d_mask, h->npx, cudaMemcpyDeviceToHost, st), "mask download");
-    return LVBGS_OK;
 }
 
 // waits for the step's latest read-back and enqueues what follows; done is set when the step is over
@@ -1109,50 +1099,47 @@ lvbgs_status pw_advance(lvbgs_ctx* h, bool& done) {
         return s;
     };
     cudaError_t e = cudaStreamSynchronize(w.st);
-    h->pw_host_ms[w.stage == 0 ? 1 : w.stage == 1 ? 2 : 3] += pw_ms_since(t0);
-    if (e != cudaSuccess) return finish(cuda_fail(h, e, w.stage == 0 ? "PAWCS rounds" : "PAWCS frame step"));
+    h->pw_host_ms[w.stage == 0 ? 1 : 3] += pw_ms_since(t0);
+    if (e != cudaSuccess) return finish(cuda_fail(h, e, "PAWCS frame step"));
     t0 = std::chrono::steady_clock::now();
     lvbgs_status s = LVBGS_OK;
+    volatile unsigned int* hf = h->h_flags;
+    const uint32_t t = (uint32_t)(h->pw_frames + 1);
+    const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
     if (w.stage == 0) {
-        if (!h->h_flags[3]) {
+        if (!hf[PWF_CONV]) {
             if (w.enq >= w.maxRounds)
                 return finish(fail(h, LVBGS_DEVICE_ERROR, "PAWCS raster-order fixed point did not converge in the round limit"));
-            s = pw_enqueue_rounds(h, 1);
+            s = pw_enqueue_frame(h, 1);
             h->pw_host_ms[0] += pw_ms_since(t0);
             return s == LVBGS_OK ? s : finish(s);
         }
-        h->pw_rounds_last = (int)h->h_flags[4];
-        bool motion = false;
-        if ((s = pw_enqueue_tail_a(h, motion)) != LVBGS_OK) return finish(s);
-        if (motion) {
+        h->pw_rounds_last = (int)hf[PWF_ROUNDS];
+        if (w.motion) {
+            if (hf[PWF_MOTION]) {
+                h->pw_offset = hf[PWF_OFFSET];
+                if ((s = pw_refresh(h, t, nxt, 1, 1.0f, 1, 0, 1, w.st)) != LVBGS_OK) return finish(s);
+            }
+            s = pw_enqueue_close(h, 0);
             w.stage = 1;
             h->pw_host_ms[2] += pw_ms_since(t0);
-            return LVBGS_OK;
+            return s == LVBGS_OK ? s : finish(s);
         }
-        s = pw_enqueue_tail_b(h);
+    }
+    if (!hf[PWF_CLOSED]) {
+        if (w.stage == 2 || !hf[PWF_RESET]) return finish(fail(h, LVBGS_DEVICE_ERROR, "PAWCS frame step did not close"));
+        // automatic model reset (:1503-1508): refreshModel(offset/8, 0, true) and T(x) := 1
+        if ((s = pw_refresh(h, t, nxt, (int)(h->pw_offset / 8), 0.0f, 1, 1, 1, w.st)) != LVBGS_OK) return finish(s);
+        launch_chained(pw_k_reset_T, dim3(256), dim3(256), w.st, h->pd, nxt);
+        s = pw_enqueue_close(h, 1);
         w.stage = 2;
         h->pw_host_ms[2] += pw_ms_since(t0);
         return s == LVBGS_OK ? s : finish(s);
     }
-    if (w.stage == 1) {
-        if (h->h_flags[1]) {
-            h->pw_offset = h->h_flags[2];
-            const uint32_t t = (uint32_t)(h->pw_frames + 1);
-            const int nxt = (int)((h->pw_frames & 1ull) ^ 1ull);
-            if ((s = pw_refresh(h, t, nxt, 1, 1.0f, 1, 0, 1, w.st)) != LVBGS_OK) return finish(s);
-        }
-        s = pw_enqueue_tail_b(h);
-        w.stage = 2;
-        h->pw_host_ms[2] += pw_ms_since(t0);
-        return s == LVBGS_OK ? s : finish(s);
-    }
-    // stage 2: the frame step is over
+    // the frame step is over
     h->pw_frames += 1;
-    TickWork tw;
-    e = cudaMemcpy(&tw, h->d_work, sizeof(TickWork), cudaMemcpyDeviceToHost);
     h->pw_host_ms[4] += pw_ms_since(t0);
-    if (e != cudaSuccess) return finish(cuda_fail(h, e, "status read-back"));
-    return finish(status_from_flags(h, tw.err));
+    return finish(status_from_flags(h, hf[PWF_STATUS]));
 }
 
 lvbgs_status pw_apply(lvbgs_ctx* h, const uint8_t* img, size_t stride, uint8_t* mask, double lr, cudaStream_t st) {

@@ -190,6 +190,7 @@ struct TickParams {
     int maxRepairIters;            // repair rounds before ERR_REPAIR_LIMIT
     int dbgFault;                  // injected fault (lvbgs_debug_inject_fault), 0: none
     unsigned int* hostErr;         // page-locked host copy of the tick's error flags, written by its last kernel
+    const unsigned int* gate;      // PAWCS: the post-processing waits for the fixed point (0 there: return at once)
 };
 constexpr unsigned long long kBarrierNs = 2000000000ull;  // 2 s
 constexpr unsigned long long kDebugBarrierNs = 2000000ull;  // 2 ms, for the injected barrier timeout

@@ -783,8 +783,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
             S.dirty[q] = dirty ? 1 : 0;
         }
     }
-    const unsigned b = __ballot_sync(0xffffffffu, dirty);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(&P.flags[0], (unsigned)__popc(b));
+    pw_round_end(P, dirty);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -793,6 +792,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
 // in raster order, on the scanned dictionary; each loop's final draw count goes to its updater
 // ------------------------------------------------------------------------------------------
 extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
+    PW_TAIL_GATE(P);
     PW3_PIXEL_PROLOGUE
     if (x >= D.W || y >= D.H) return;
     const int q = y * D.W + x;
@@ -871,6 +871,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
 // draw counters (the dictionaries are final after pw3_k_later)
 // ------------------------------------------------------------------------------------------
 extern "C" __global__ void __launch_bounds__(256) pw3_k_commit(PwParams P) {
+    PW_TAIL_GATE(P);
     PW3_PIXEL_PROLOGUE
     const bool in = x < D.W && y < D.H;
     const int p = in ? y * D.W + x : 0;
@@ -969,6 +970,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_commit(PwParams P) {
 // down-sampled frame per channel (INTER_AREA, integral scale), its rolling averages and the
 // per-pixel L1 |LT - ST| over the channels (:1475-1478)
 extern "C" __global__ void pw3_k_ds(PwParams P) {
+    PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
@@ -998,6 +1000,7 @@ extern "C" __global__ void pw3_k_ds(PwParams P) {
 // the background kernel, a pixel per thread), area-down-sampled, against the long-term means: L1 over the channels into dsAbs and the float
 // colour distortion (lv::cdist<3>, math.hpp:499-527) into contrib; 0 outside the fully covered blocks
 extern "C" __global__ void pw3_k_motion_bg(PwParams P) {
+    PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
@@ -1044,6 +1047,7 @@ extern "C" __global__ void pw3_k_motion_bg(PwParams P) {
 extern "C" __global__ void __launch_bounds__(128) pw3_k_refresh_local(PawcsDev S, uint32_t t, int buf, int baseOcc,
                                                                        float decr, int force, int onlyPending,
                                                                        int useDil) {
+    pdl_entry();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const StreamDev& D = S.sd;
     if (p >= D.npx) return;
@@ -1128,6 +1132,7 @@ extern "C" __global__ void __launch_bounds__(128) pw3_k_refresh_local(PawcsDev S
 
 extern "C" __global__ void pw3_k_refresh_global(PawcsDev S, uint32_t t, int buf, int force, int onlyPending,
                                                 int useDil) {
+    pdl_entry();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     PawcsCtl* pc = S.pc;
     if (onlyPending && pc->reset_pending == 0) return;

@@ -160,6 +160,25 @@ __device__ __forceinline__ void pw3_store(const PawcsDev& S, int buf, int j, int
     pw3_put(S, pw_slot(S, buf, j, p), w);
 }
 
+// End of a fixed-point round, called by every thread of the dirty pass: counts the pixels to rerun; the block
+// that finishes last closes the round. No dirty pixel means the fixed point is reached: its round count and
+// flag are set, here for the rounds and the tail enqueued after this one, and in host memory.
+__device__ __forceinline__ void pw_round_end(const PwParams& P, bool dirty) {
+    const int any = __syncthreads_count(dirty);
+    if (threadIdx.x != 0) return;
+    if (any) atomicAdd(&P.flags[PWF_DIRTY], (unsigned)any);
+    __threadfence();
+    if (atomicAdd(&P.flags[PWF_DONE], 1u) != gridDim.x - 1u) return;
+    P.flags[PWF_DONE] = 0u;
+    if (atomicExch(&P.flags[PWF_DIRTY], 0u) == 0u) {
+        P.flags[PWF_ROUNDS] = (unsigned)P.round + 1u;
+        P.hflags[PWF_ROUNDS] = (unsigned)P.round + 1u;
+        P.hflags[PWF_CONV] = 1u;
+        __threadfence();
+        P.flags[PWF_CONV] = 1u;
+    }
+}
+
 }  // namespace lvbgs
 
 namespace lvbgs {

@@ -150,6 +150,8 @@ struct PawcsDev {
                                // event flags << 16, fixed position|fixed word << 8, speculative word and epoch
     float* contribList;        // word weight contributions, word-major, raster order within a word
     uint32_t* blkCounts;       // ordered compaction: per block and category counts, then offsets
+    unsigned long long* chain; // one-pass compaction: per block, generation << 34 | state << 32 | count
+    unsigned int* ticket;      // one-pass compaction: next block, generation
     uint32_t* catInfo;         // [0..16] category totals, [32..48] category bases
     float* dsAbs;              // |LT - ST| per down-sampled pixel (0 outside the down-sampled ROI)
     uint32_t* updList;         // pixels that update a neighbour this round, raster order
@@ -183,12 +185,25 @@ struct PwParams {
     int totalCells;
     int round;            // fixed-point round of the local pass (0: every pixel)
     double lr;            // learningRateOverride of the tick (<= 0: internal, inf: never)
-    unsigned int* flags;  // [0] dirty pixels of the round, [3] fixed point reached, [4] its round count
+    unsigned int* flags;  // PWF_* (device)
+    unsigned int* hflags; // PWF_* results in page-locked host memory, written by the kernels that know them
+    unsigned int* err;    // error flags of the frame step (TickWork::err)
+    // set for the launches of the frame's tail, which are enqueued with the rounds before the host knows that
+    // these suffice: while the fixed point is not reached every kernel of the tail returns at once
+    const unsigned int* gate;
     // set for the launches of a fixed-point round: the rounds of a frame are enqueued ahead, and
     // every kernel of a round returns at once when an earlier round reached the fixed point
     const unsigned int* conv;
 };
 #define PW_ROUND_GUARD(P) \
+    pdl_entry();          \
     if ((P).conv && *(const volatile unsigned int*)(P).conv) return
+#define PW_TAIL_GATE(P) \
+    pdl_entry();        \
+    if ((P).gate && *(const volatile unsigned int*)(P).gate == 0u) return
+// flags: dirty pixels of the round; camera-motion switch and the new weight offset; fixed point reached and
+// its round count; blocks of the dirty pass that are done; status (host: error flags of the finished frame);
+// automatic model reset pending (host: the frame waits for it)
+enum { PWF_DIRTY = 0, PWF_MOTION, PWF_OFFSET, PWF_CONV, PWF_ROUNDS, PWF_DONE, PWF_STATUS, PWF_RESET, PWF_CLOSED, PWF_COUNT };
 
 }  // namespace lvbgs

@@ -303,8 +303,8 @@ __device__ void pw_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_t
 
 // ------------------------------------------------------------------------------------------
 // ordered compactions (raster order kept): mode 0 lists the critical global items, mode 1 the word
-// weight contributions per word, mode 2 the pixels that update a neighbour. Blocks of kPwCompactBlk
-// pixels: counts, offsets, scatter.
+// weight contributions per word, mode 2 the pixels that update a neighbour. Mode 1 has a list per word, so it
+// counts, makes offsets and scatters in three launches, over blocks of kPwCompactBlk pixels.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ int pw_category(const PawcsDev& S, int p, int mode, int wr, uint32_t nrep) {
     if (!S.sd.roi[p]) return -1;
@@ -318,8 +318,9 @@ __device__ __forceinline__ int pw_category(const PawcsDev& S, int p, int mode, i
     return (int)O.gword;
 }
 
-extern "C" __global__ void __launch_bounds__(256) pw_k_compact_count(PwParams P, int mode) {
+extern "C" __global__ void __launch_bounds__(256) pw_k_compact_count(PwParams P) {
     PW_ROUND_GUARD(P);
+    if (P.gate && *(const volatile unsigned int*)P.gate == 0u) return;
     const PawcsDev& S = P.streams[0];
     const int nb = (S.sd.npx + kPwCompactBlk - 1) / kPwCompactBlk;
     if ((int)blockIdx.x >= nb) return;
@@ -331,7 +332,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_count(PwParams P,
     for (int k = 0; k < kPwCompactBlk / 256; ++k) {
         const int p = blockIdx.x * kPwCompactBlk + k * 256 + threadIdx.x;
         if (p < S.sd.npx) {
-            const int c = pw_category(S, p, mode, wr, nrep);
+            const int c = pw_category(S, p, 1, wr, nrep);
             if (c >= 0) atomicAdd(&cnt[c], 1u);
         }
     }
@@ -343,6 +344,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_count(PwParams P,
 // bases of the word-major list; the compaction uses categories [0, ncat), the others are left empty
 extern "C" __global__ void __launch_bounds__(1024) pw_k_compact_offsets(PwParams P, int ncat) {
     PW_ROUND_GUARD(P);
+    if (P.gate && *(const volatile unsigned int*)P.gate == 0u) return;
     const PawcsDev& S = P.streams[0];
     const int nb = (S.sd.npx + kPwCompactBlk - 1) / kPwCompactBlk;
     __shared__ uint32_t tot[kPwCats];
@@ -377,8 +379,9 @@ extern "C" __global__ void __launch_bounds__(1024) pw_k_compact_offsets(PwParams
     }
 }
 
-extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams P, int mode) {
+extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams P) {
     PW_ROUND_GUARD(P);
+    if (P.gate && *(const volatile unsigned int*)P.gate == 0u) return;
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nb = (D.npx + kPwCompactBlk - 1) / kPwCompactBlk;
@@ -390,12 +393,11 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams 
     const uint32_t nrep = S.pc->n_repl;
     if (threadIdx.x < kPwCats)
         run[threadIdx.x] = S.catInfo[kPwCatBase + threadIdx.x] + S.blkCounts[(size_t)blockIdx.x * kPwCats + threadIdx.x];
-    const float* fm = D.fm + (size_t)(D.ctl->frame_idx & 1ull) * kNumFloatMaps * D.npx;
     for (int k = 0; k < kPwCompactBlk / 256; ++k) {
         const int p = blockIdx.x * kPwCompactBlk + k * 256 + threadIdx.x;
-        const int c = p < D.npx ? pw_category(S, p, mode, wr, nrep) : -1;
+        const int c = p < D.npx ? pw_category(S, p, 1, wr, nrep) : -1;
         uint32_t rank = 0;
-        const int ncat = mode == 1 ? S.G : 1;
+        const int ncat = S.G;
         for (int j = 0; j < ncat; ++j) {
             const unsigned m = __ballot_sync(0xffffffffu, c == j);
             if (c == j) rank = __popc(m & ((1u << lane) - 1u));
@@ -415,27 +417,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams 
         __syncthreads();
         if (c >= 0) {
             const uint32_t pos = run[c] + warpCnt[w][c] + rank;
-            if (mode == 0) {
-                // two records per item (pixel, colour|bits, thresholds, descriptors 0-1; descriptor 2|event
-                // flags, fixed position|word, and the global scan's speculative outcome)
-                const PwRec R = S.rec[p];
-                const bool c3 = D.C == 3;
-                const PwThr th = c3 ? pw3_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff)
-                                    : pw_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff);
-                const uint32_t g = S.gitem[p];
-                const uint16_t* dt = S.descT + (size_t)p * (c3 ? 3 : 1);
-                const uint32_t a = (c3 ? pw3_color(D.frame, p) : (uint32_t)D.frame[p]) | ((uint32_t)R.bits << 24);
-                const uint32_t b = min(th.color, 65535u) | (min(th.desc / 4u, 65535u) << 16);
-                const uint32_t d01 = c3 ? (uint32_t)dt[0] | ((uint32_t)dt[1] << 16) : (uint32_t)dt[0];
-                const uint32_t d2 = c3 ? (uint32_t)dt[2] : 0u;
-                S.itemList[2 * pos] = make_uint4((uint32_t)p, a, b, d01);
-                S.itemList[2 * pos + 1] = make_uint4(d2 | ((uint32_t)(R.flags & (kRfEvent | kRfRepDraw)) << 16),
-                                                     ((g >> 6) & 63u) | ((g & 63u) << 8), 0u, 0u);
-            } else if (mode == 2) {
-                S.updList[pos] = (uint32_t)p;
-            } else {
-                S.contribList[pos] = S.contrib[p];
-            }
+            S.contribList[pos] = S.contrib[p];
         }
         __syncthreads();
         if (threadIdx.x < ncat) run[threadIdx.x] += passTot[threadIdx.x];
@@ -443,10 +425,125 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams 
     }
 }
 
+// The ordered compactions of one category (modes 0 and 2) in one pass: a block takes the next kPwCompactBlk
+// pixels (by ticket, so that the blocks before it are running or done), counts its members, publishes the
+// count, and finds its offset by looking back over the blocks before it, a warp's width at a time, until one
+// that has published its total. Count, offsets and scatter were three launches (7 + 8 + 9 us of a 640x480
+// frame, up to eleven times a frame). The wait is bounded (ERR_BARRIER_TIMEOUT). The generation tells this launch's entries from
+// the last one's; the block with the last ticket advances it.
+__device__ __forceinline__ void pw_list_item(const PawcsDev& S, int mode, int p, uint32_t pos) {
+    if (mode == 2) {
+        S.updList[pos] = (uint32_t)p;
+        return;
+    }
+    const StreamDev& D = S.sd;
+    const float* fm = D.fm + (size_t)(D.ctl->frame_idx & 1ull) * kNumFloatMaps * D.npx;
+    // two records per item (pixel, colour|bits, thresholds, descriptors 0-1; descriptor 2|event
+    // flags, fixed position|word, and the global scan's speculative outcome)
+    const PwRec R = S.rec[p];
+    const bool c3 = D.C == 3;
+    const PwThr th = c3 ? pw3_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff)
+                        : pw_thresholds(fm[FM_R * D.npx + p], S.unstable[p], S.minColor, S.descOff);
+    const uint32_t g = S.gitem[p];
+    const uint16_t* dt = S.descT + (size_t)p * (c3 ? 3 : 1);
+    const uint32_t a = (c3 ? pw3_color(D.frame, p) : (uint32_t)D.frame[p]) | ((uint32_t)R.bits << 24);
+    const uint32_t b = min(th.color, 65535u) | (min(th.desc / 4u, 65535u) << 16);
+    const uint32_t d01 = c3 ? (uint32_t)dt[0] | ((uint32_t)dt[1] << 16) : (uint32_t)dt[0];
+    const uint32_t d2 = c3 ? (uint32_t)dt[2] : 0u;
+    S.itemList[2 * pos] = make_uint4((uint32_t)p, a, b, d01);
+    S.itemList[2 * pos + 1] = make_uint4(d2 | ((uint32_t)(R.flags & (kRfEvent | kRfRepDraw)) << 16),
+                                         ((g >> 6) & 63u) | ((g & 63u) << 8), 0u, 0u);
+}
+extern "C" __global__ void __launch_bounds__(256) pw_k_compact(PwParams P, int mode) {
+    PW_ROUND_GUARD(P);
+    const PawcsDev& S = P.streams[0];
+    const int npx = S.sd.npx, nb = (npx + kPwCompactBlk - 1) / kPwCompactBlk;
+    constexpr int K = kPwCompactBlk / 256;
+    __shared__ uint32_t sBid, sGen, sCnt[K][8], sBase;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        sBid = atomicAdd(&S.ticket[0], 1u);
+        sGen = *(volatile unsigned int*)&S.ticket[1] & 0x3fffffffu;
+    }
+    __syncthreads();
+    const int bid = (int)sBid;
+    bool in[K];
+    uint32_t rank[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int p = bid * kPwCompactBlk + k * 256 + (int)threadIdx.x;
+        in[k] = p < npx && pw_category(S, p, mode, 0, 0u) == 0;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const unsigned m = __ballot_sync(0xffffffffu, in[k]);
+        rank[k] = (uint32_t)__popc(m & ((1u << lane) - 1u));
+        if (lane == 0) sCnt[k][warp] = (uint32_t)__popc(m);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        static_assert(K * 8 == 32, "one count per lane");
+        // offsets of the warps in raster order and the block's total
+        const uint32_t v = sCnt[lane >> 3][lane & 7];
+        uint32_t inc = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
+        }
+        sCnt[lane >> 3][lane & 7] = inc - v;
+        const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+        const unsigned long long tag = (unsigned long long)sGen << 34, kCount = 1ull << 32, kTotal = 2ull << 32;
+        volatile unsigned long long* chain = S.chain;
+        uint32_t base = 0;
+        if (bid > 0) {
+            if (lane == 0) chain[bid] = tag | kCount | total;
+            for (int at = bid - 1; at >= 0;) {
+                const int b = at - lane;
+                unsigned long long e = tag | kTotal;  // before the first block: a total of 0
+                for (int spin = 0; b >= 0; ++spin) {
+                    e = chain[b];
+                    if ((e >> 34) == (unsigned long long)sGen && ((e >> 32) & 3ull) != 0ull) break;
+                    if (spin > (1 << 22)) {
+                        atomicOr(P.err, ERR_BARRIER_TIMEOUT);
+                        e = tag | kTotal;
+                        break;
+                    }
+                    __nanosleep(20);
+                }
+                __syncwarp();
+                const unsigned done = __ballot_sync(0xffffffffu, ((e >> 32) & 3ull) == 2ull);
+                const int stop = done ? __ffs(done) - 1 : 31;  // the nearest block with a total
+                base += __reduce_add_sync(0xffffffffu, lane <= stop ? (uint32_t)e : 0u);
+                if (done) break;
+                at -= 32;
+            }
+        }
+        if (lane == 0) {
+            __threadfence();
+            chain[bid] = tag | kTotal | (base + total);
+            sBase = base;
+            if (bid == nb - 1) {
+                S.catInfo[0] = base + total;
+                S.catInfo[kPwCatBase] = 0u;
+                S.ticket[0] = 0u;
+                *(volatile unsigned int*)&S.ticket[1] = (sGen + 1u) & 0x3fffffffu;
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t base = sBase;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (in[k])
+            pw_list_item(S, mode, bid * kPwCompactBlk + k * 256 + (int)threadIdx.x, base + sCnt[k][warp] + rank[k]);
+}
+
 // per 2x2 cell of the spatial maps: the cell's (at most four) items in raster order (:786-791,
 // :805-812); final = 1 also writes the frame's map values and word contributions
 extern "C" __global__ void pw_k_cells(PwParams P, int final) {
     PW_ROUND_GUARD(P);
+    if (P.gate && *(const volatile unsigned int*)P.gate == 0u) return;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.totalCells) return;
     int si = 0;
@@ -731,19 +828,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_dirty(PwParams P) {
         const int p = y * D.W + x;
         dirty = D.roi[p] && S.repBefore[p] != S.rec[p].rsrc;
     }
-    const unsigned b = __ballot_sync(0xffffffffu, dirty);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(&P.flags[0], (unsigned)__popc(b));
-}
-
-// end of a fixed-point round (one thread): no dirty pixel means the fixed point is reached; the
-// round count is recorded and the flag makes the rounds enqueued after this one return at once
-extern "C" __global__ void pw_k_round_end(PwParams P) {
-    PW_ROUND_GUARD(P);
-    if (P.flags[0] == 0u) {
-        P.flags[4] = (unsigned)P.round + 1u;
-        __threadfence();
-        P.flags[3] = 1u;
-    }
+    pw_round_end(P, dirty);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -752,6 +837,7 @@ extern "C" __global__ void pw_k_round_end(PwParams P) {
 // descriptor, raw mask (as the post-processing "intent" word) and draw counters
 // ------------------------------------------------------------------------------------------
 extern "C" __global__ void __launch_bounds__(256) pw_k_commit(PwParams P) {
+    PW_TAIL_GATE(P);
     const int t0 = blockIdx.x;
     if (t0 >= P.totalTiles) return;
     const PawcsDev& S = P.streams[pw_stream_by_tile(P, t0)];
@@ -863,6 +949,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_commit(PwParams P) {
 // (stream, word) over the word's compacted list; the replaceable word restarts from zero at the
 // frame's last replacement (its list holds only the contributions after it)
 extern "C" __global__ void __launch_bounds__(256) pw_k_weights(PwParams P) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.x / kPwMaxGlobal, w = blockIdx.x % kPwMaxGlobal;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -905,6 +992,7 @@ __device__ __forceinline__ void pw_gw_rates(uint32_t t, int* recalc, int* update
 }
 
 extern "C" __global__ void pw_k_gw_recalc(PwParams P) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.x / kPwMaxGlobal, w = blockIdx.x % kPwMaxGlobal;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -930,6 +1018,7 @@ extern "C" __global__ void pw_k_gw_recalc(PwParams P) {
 // decay (accumulateProduct with the INTER_NEAREST down-scaled previous inverted dilated mask) and the
 // first half of the blur (row sums, double); one block row per map row
 extern "C" __global__ void pw_k_gw_decay(PwParams P, double* rowsum) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.y / kPwMaxGlobal, w = blockIdx.y % kPwMaxGlobal;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -966,6 +1055,7 @@ extern "C" __global__ void pw_k_gw_decay(PwParams P, double* rowsum) {
 // second half of the blur (column sums * 1/9, to float), the weight decay and, in the last block,
 // the one-pass dictionary sort by weight
 extern "C" __global__ void pw_k_gw_blur(PwParams P, const double* rowsum) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.y / kPwMaxGlobal, w = blockIdx.y % kPwMaxGlobal;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -988,6 +1078,7 @@ extern "C" __global__ void pw_k_gw_blur(PwParams P, const double* rowsum) {
 
 // weight decay and the dictionary's bubble step (after all maps are final)
 extern "C" __global__ void pw_k_gw_sort(PwParams P) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.x * blockDim.x + threadIdx.x;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -1008,6 +1099,7 @@ extern "C" __global__ void pw_k_gw_sort(PwParams P) {
 // per-pixel global word order: one bubble pass on the local map weights (:1318-1330, :415-427);
 // mode 0: only on update frames (apply), 1: always (refreshModel), 2: when an automatic reset is pending
 extern "C" __global__ void __launch_bounds__(256) pw_k_lut_sort(PwParams P, int mode) {
+    PW_TAIL_GATE(P);
     const int t0 = blockIdx.x;
     if (t0 >= P.totalTiles) return;
     const PawcsDev& S = P.streams[pw_stream_by_tile(P, t0)];
@@ -1046,6 +1138,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_lut_sort(PwParams P, int 
 
 // blinks (:1443-1446) and the 3x3 closing of the raw mask (:1447)
 extern "C" __global__ void __launch_bounds__(256) pw_k_blink_close(PwParams P) {
+    PW_TAIL_GATE(P);
     const int t0 = blockIdx.x;
     if (t0 >= P.totalTiles) return;
     const PawcsDev& S = P.streams[pw_stream_by_tile(P, t0)];
@@ -1105,6 +1198,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_blink_close(PwParams P) {
 // down-sampled frame (INTER_AREA, integral scale), its rolling averages (accumulateWeighted) and the
 // per-pixel |LT - ST| of the motion analysis (:1475-1478); one thread per down-sampled pixel
 extern "C" __global__ void pw_k_ds(PwParams P) {
+    PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
@@ -1159,7 +1253,28 @@ __device__ float pw_block_ordered_sum(const float* v, int n, float* terms, int w
     return acc;
 }
 
-extern "C" __global__ void __launch_bounds__(256) pw_k_epilogue(PwParams P) {
+// reset decision of the frame-level block (:1509-1513)
+__device__ void pw_reset_decide(const PawcsDev& S) {
+    StreamCtl* ctl = S.sd.ctl;
+    PawcsCtl* pc = S.pc;
+    const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
+    const int boot = t <= (uint32_t)kBootWin;
+    const float ratio = pc->frame_ratio;
+    if (pc->reset_block) {
+        if (ctl->frames_since_reset > (unsigned long long)kBootWin * 2) {
+            ctl->auto_reset = 0;
+        } else if (ratio >= 45.0f && ctl->cooldown == 0) {
+            ctl->frames_since_reset = 0;
+            pc->reset_pending = 1;
+        } else if (!boot) {
+            ++ctl->frames_since_reset;
+        }
+    }
+}
+
+// the frame level; decide: the reset decision too (frames without a camera-motion comparison before it)
+extern "C" __global__ void __launch_bounds__(256) pw_k_epilogue(PwParams P, int decide) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.x;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
@@ -1198,37 +1313,25 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_epilogue(PwParams P) {
     // (pw_k_reset_decide) follow
     if (!ctl->auto_reset && ratio >= 45.0f * 2) ctl->auto_reset = 1;
     pc->reset_block = ctl->auto_reset || pc->moving_cam;
-}
-
-// reset decision of the frame-level block (:1509-1513)
-extern "C" __global__ void pw_k_reset_decide(PwParams P) {
-    const int si = blockIdx.x;
-    if (si >= P.nStreams || threadIdx.x != 0) return;
-    const PawcsDev& S = P.streams[si];
-    StreamCtl* ctl = S.sd.ctl;
-    PawcsCtl* pc = S.pc;
-    const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
-    const int boot = t <= (uint32_t)kBootWin;
-    const float ratio = pc->frame_ratio;
-    if (pc->reset_block) {
-        if (ctl->frames_since_reset > (unsigned long long)kBootWin * 2) {
-            ctl->auto_reset = 0;
-        } else if (ratio >= 45.0f && ctl->cooldown == 0) {
-            ctl->frames_since_reset = 0;
-            pc->reset_pending = 1;
-        } else if (!boot) {
-            ++ctl->frames_since_reset;
-        }
-    }
+    if (decide) pw_reset_decide(S);
 }
 
 // closes the frame: frame index, cooldown, factors of the next frame's final-segmentation averages
-extern "C" __global__ void pw_k_close(PwParams P) {
+// and, for the host, the error flags. resetDone 0: a pending automatic reset leaves the frame open, and the host
+// runs it and closes the frame after it.
+extern "C" __global__ void pw_k_close(PwParams P, int resetDone) {
+    PW_TAIL_GATE(P);
     const int si = blockIdx.x * blockDim.x + threadIdx.x;
     if (si >= P.nStreams) return;
     const PawcsDev& S = P.streams[si];
     StreamCtl* ctl = S.sd.ctl;
     PawcsCtl* pc = S.pc;
+    if (!resetDone && pc->reset_pending) {
+        P.hflags[PWF_RESET] = 1u;
+        return;
+    }
+    P.hflags[PWF_STATUS] = *(const volatile unsigned int*)P.err;
+    P.hflags[PWF_CLOSED] = 1u;
     const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
     if (pc->reset_pending == 1) {
         float fLT, fST;
@@ -1256,6 +1359,7 @@ extern "C" __global__ void pw_k_close(PwParams P) {
 extern "C" __global__ void __launch_bounds__(128) pw_k_refresh_local(PawcsDev S, uint32_t t, int buf, int baseOcc,
                                                                       float decr, int force, int onlyPending,
                                                                       int useDil) {
+    pdl_entry();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const StreamDev& D = S.sd;
     if (p >= D.npx) return;
@@ -1348,6 +1452,7 @@ extern "C" __global__ void __launch_bounds__(128) pw_k_refresh_local(PawcsDev S,
 // slots; one thread per stream (it visits about 4 G pixels)
 extern "C" __global__ void pw_k_refresh_global(PawcsDev S, uint32_t t, int buf, int force, int onlyPending,
                                                int useDil) {
+    pdl_entry();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     PawcsCtl* pc = S.pc;
     if (onlyPending && pc->reset_pending == 0) return;
@@ -1417,6 +1522,7 @@ extern "C" __global__ void pw_k_refresh_global(PawcsDev S, uint32_t t, int buf, 
 
 // the automatic reset's T(x) := 1 (:1508)
 extern "C" __global__ void pw_k_reset_T(PawcsDev S, int buf) {
+    pdl_entry();
     if (S.pc->reset_pending == 0) return;
     const StreamDev& D = S.sd;
     float* T = D.fm + (size_t)buf * kNumFloatMaps * D.npx + FM_T * D.npx;
@@ -1472,6 +1578,7 @@ extern "C" __global__ void pw_k_init_last(PawcsDev S, const uint8_t* img) {
 // buffer by the background kernel), area-down-sampled like the frame, against the long-term mean of the
 // down-sampled frames: |LT - BG| per down-sampled pixel (0 outside the fully covered blocks)
 extern "C" __global__ void pw_k_motion_bg(PwParams P) {
+    PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     const int nds = D.dsW * D.dsH;
@@ -1488,10 +1595,11 @@ extern "C" __global__ void pw_k_motion_bg(PwParams P) {
 }
 
 // camera-motion decision: ordered L1 sum, then switch the mode on (during the bootstrap window, ratio
-// >= 45) or off (ratio < 45/4) with the local word weight offset (5 / 1000); flags[1] tells the host
-// to run refreshModel(1, 1, true), flags[2] carries the new offset. One grayscale channel: the colour
+// >= 45) or off (ratio < 45/4) with the local word weight offset (5 / 1000); PWF_MOTION tells the
+// host to run refreshModel(1, 1, true), PWF_OFFSET carries the new offset. One grayscale channel: the colour
 // distance ratio is 0; three channels: the mean colour distortion of pw3_k_motion_bg.
 extern "C" __global__ void __launch_bounds__(256) pw_k_motion_decide(PwParams P) {
+    PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];
     const StreamDev& D = S.sd;
     PawcsCtl* pc = S.pc;
@@ -1521,8 +1629,9 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_motion_decide(PwParams P)
             pc->motion_pending = 1;
         }
     }
-    P.flags[1] = (unsigned int)pc->motion_pending;
-    P.flags[2] = (unsigned int)pc->lword_offset;
+    pw_reset_decide(S);
+    P.hflags[PWF_OFFSET] = (unsigned int)pc->lword_offset;
+    P.hflags[PWF_MOTION] = (unsigned int)pc->motion_pending;
 }
 
 // background image (:1518-1545) / descriptors (:1547-1594) from the words of buffer buf; ahead: 1 inside the

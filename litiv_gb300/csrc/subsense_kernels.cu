@@ -1534,6 +1534,7 @@ __device__ void stream_epilogue(const TickParams& P, const StreamDev& S);
 // Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
     pdl_entry();
+    if (P.gate && ld_volatile(P.gate) == 0u) return;
     const int rowBlocks = (P.totalRows + 7) / 8;
     if ((int)blockIdx.x >= rowBlocks) {
         stream_epilogue(P, P.streams[blockIdx.x - rowBlocks]);
@@ -1585,6 +1586,7 @@ extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
 // hole words took a pass of their own through memory: 20 + 6 us on a 1920x1080 frame before.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_fill(TickParams P) {
     pdl_entry();
+    if (P.gate && ld_volatile(P.gate) == 0u) return;
     const int gr = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (gr >= P.totalRows) return;
     const StreamDev& S = P.streams[find_stream_by_row(P, gr)];
@@ -1736,6 +1738,7 @@ __device__ __forceinline__ void median_words(FinSmem& sm, int r, int half, int y
 // when it is in host memory. Bound by the 22 B/px of maps and by the latency of the short word phases.
 extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams P) {
     pdl_entry();
+    if (P.gate && ld_volatile(P.gate) == 0u) return;
     __shared__ FinSmem sm;
     const int gt = blockIdx.x;
     if (gt >= P.totalSegs) return;
