@@ -928,6 +928,7 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
     const cudaStream_t st = w.st;
     const dim3 blk(kThreads), tiles(h->sd.nTiles), warps4(128);
     const dim3 cblocks((unsigned)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk));
+    const dim3 oneBlocks((unsigned)((h->npx + kPwOneBlk - 1) / kPwOneBlk));
     const size_t gseg4 = 4 * (size_t)pw_gseg_items(h->C);  // items of a block of four segments
     const dim3 gseg((unsigned)((h->npx + gseg4 - 1) / gseg4));
     const bool c3 = h->C == 3;
@@ -937,7 +938,7 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
         // three channels: the local pass applies the earlier updaters' loops itself
         launch_chained(c3 ? pw3_k_local : pw_k_local, tiles, blk, st, P);
         launch_chained(pw_k_illum, dim3((h->H + 7) / 8), blk, st, P);
-        launch_chained(pw_k_compact, cblocks, blk, st, P, 0);
+        launch_chained(pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 0);
         launch_chained(pw3_k_gscan_seg, gseg, warps4, st, P);
         launch_chained(pw3_k_gscan_walk, dim3(1), dim3(32), st, P);
         launch_chained(pw3_k_gscan_fix, dim3((unsigned)((h->npx + 255) / 256)), blk, st, P);
@@ -945,7 +946,7 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
         launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 0);
         launch_chained(pw_k_nbr, tiles, blk, st, P);
         if (!c3) {
-            launch_chained(pw_k_compact, cblocks, blk, st, P, 2);
+            launch_chained(pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 2);
             launch_chained(pw_k_nbr_loops, dim3(std::max(1u, std::min(cblocks.x * 4, 1216u))), blk, st, P);
             launch_chained(pw_k_replace, tiles, blk, st, P);
         }

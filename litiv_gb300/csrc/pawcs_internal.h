@@ -171,6 +171,7 @@ LV_HD constexpr int pw_gseg_items(int C) { return C == 3 ? 128 : 256; }
 LV_HD constexpr int pw_gseg_warm(int C) { return C == 3 ? 128 : 64; }
 constexpr int kPwGsegWords = 24;  // scratch words of a segment
 LV_HD constexpr size_t pw_gseg_max(size_t npx, int C) { return npx / pw_gseg_items(C) + 2; }  // segments
+constexpr int kPwOneThreads = 1024, kPwOneBlk = 2048;  // block of the one-pass compactions, its pixels (256 and 1024: 15 us on 640x480 gray, 1024 and 4096: 13, these: 12)
 constexpr int kPwCompactBlk = 1024;  // pixels per block of the ordered compactions
 constexpr int kPwCats = kPwMaxGlobal + 1;  // compaction categories: the global words, or the critical items
 constexpr int kPwCatBase = 64;       // catInfo: [0, kPwCats) category totals, [kPwCatBase, +kPwCats) bases

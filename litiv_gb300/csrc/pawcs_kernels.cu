@@ -425,7 +425,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact_scatter(PwParams 
     }
 }
 
-// The ordered compactions of one category (modes 0 and 2) in one pass: a block takes the next kPwCompactBlk
+// The ordered compactions of one category (modes 0 and 2) in one pass: a block takes the next kPwOneBlk
 // pixels (by ticket, so that the blocks before it are running or done), counts its members, publishes the
 // count, and finds its offset by looking back over the blocks before it, a warp's width at a time, until one
 // that has published its total. Count, offsets and scatter were three launches (7 + 8 + 9 us of a 640x480
@@ -454,12 +454,12 @@ __device__ __forceinline__ void pw_list_item(const PawcsDev& S, int mode, int p,
     S.itemList[2 * pos + 1] = make_uint4(d2 | ((uint32_t)(R.flags & (kRfEvent | kRfRepDraw)) << 16),
                                          ((g >> 6) & 63u) | ((g & 63u) << 8), 0u, 0u);
 }
-extern "C" __global__ void __launch_bounds__(256) pw_k_compact(PwParams P, int mode) {
+extern "C" __global__ void __launch_bounds__(kPwOneThreads) pw_k_compact(PwParams P, int mode) {
     PW_ROUND_GUARD(P);
     const PawcsDev& S = P.streams[0];
-    const int npx = S.sd.npx, nb = (npx + kPwCompactBlk - 1) / kPwCompactBlk;
-    constexpr int K = kPwCompactBlk / 256;
-    __shared__ uint32_t sBid, sGen, sCnt[K][8], sBase;
+    const int npx = S.sd.npx, nb = (npx + kPwOneBlk - 1) / kPwOneBlk;
+    constexpr int K = kPwOneBlk / kPwOneThreads, WARPS = kPwOneThreads / 32, PER = K * WARPS / 32;
+    __shared__ uint32_t sBid, sGen, sCnt[K * WARPS], sBase;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         sBid = atomicAdd(&S.ticket[0], 1u);
@@ -471,27 +471,33 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact(PwParams P, int m
     uint32_t rank[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const int p = bid * kPwCompactBlk + k * 256 + (int)threadIdx.x;
+        const int p = bid * kPwOneBlk + k * kPwOneThreads + (int)threadIdx.x;
         in[k] = p < npx && pw_category(S, p, mode, 0, 0u) == 0;
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         const unsigned m = __ballot_sync(0xffffffffu, in[k]);
         rank[k] = (uint32_t)__popc(m & ((1u << lane) - 1u));
-        if (lane == 0) sCnt[k][warp] = (uint32_t)__popc(m);
+        if (lane == 0) sCnt[k * WARPS + warp] = (uint32_t)__popc(m);
     }
     __syncthreads();
     if (warp == 0) {
-        static_assert(K * 8 == 32, "one count per lane");
+        static_assert(PER * 32 == K * WARPS, "whole lanes");
         // offsets of the warps in raster order and the block's total
-        const uint32_t v = sCnt[lane >> 3][lane & 7];
-        uint32_t inc = v;
+        uint32_t v[PER], sum = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            v[i] = sum;
+            sum += sCnt[lane * PER + i];
+        }
+        uint32_t inc = sum;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
             if (lane >= d) inc += o;
         }
-        sCnt[lane >> 3][lane & 7] = inc - v;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) sCnt[lane * PER + i] = inc - sum + v[i];
         const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
         const unsigned long long tag = (unsigned long long)sGen << 34, kCount = 1ull << 32, kTotal = 2ull << 32;
         volatile unsigned long long* chain = S.chain;
@@ -536,7 +542,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_compact(PwParams P, int m
 #pragma unroll
     for (int k = 0; k < K; ++k)
         if (in[k])
-            pw_list_item(S, mode, bid * kPwCompactBlk + k * 256 + (int)threadIdx.x, base + sCnt[k][warp] + rank[k]);
+            pw_list_item(S, mode, bid * kPwOneBlk + k * kPwOneThreads + (int)threadIdx.x, base + sCnt[k * WARPS + warp] + rank[k]);
 }
 
 // per 2x2 cell of the spatial maps: the cell's (at most four) items in raster order (:786-791,
