@@ -28,6 +28,7 @@
 
 #include "lbsp_device.cuh"
 #include "lobster_internal.h"
+#include "staging.h"
 
 namespace lvbgs {
 
@@ -1117,6 +1118,12 @@ inline uint8_t sat_round_u8f(float v) {
         }                                                                         \
     } while (0)
 
+inline cudaError_t staging(void** p, size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e == cudaSuccess ? staging_alloc(dev, p, bytes, st) : e;
+}
+
 inline int blocks_for(size_t n) { return (int)((n + kThreadsL - 1) / kThreadsL); }
 
 }  // namespace
@@ -1438,7 +1445,7 @@ lvbgs_status lob_background(LobState& L, void* hostOut, bool descriptors, cudaSt
     LOB_CUDA(cudaEventSynchronize(L.meanDone), "frame step");  // the last frame step may run on another stream
     const size_t n = (size_t)D.npx * D.C * (descriptors ? 2 : 1);
     void* tmp = nullptr;
-    LOB_CUDA(cudaMallocAsync(&tmp, n, st), "staging allocation");
+    LOB_CUDA(staging(&tmp, n, st), "staging allocation");
     if (D.C == 3) lob_k_background<3><<<1024, 256, 0, st>>>(D, tmp, descriptors ? 1 : 0);
     else lob_k_background<1><<<1024, 256, 0, st>>>(D, tmp, descriptors ? 1 : 0);
     cudaError_t e = cudaGetLastError();
@@ -1514,7 +1521,7 @@ lvbgs_status lob_get_map(LobState& L, int which, void* hostOut, size_t bytes, cu
         return LVBGS_OK;
     }
     void* tmp = nullptr;
-    LOB_CUDA(cudaMallocAsync(&tmp, need, st), "staging allocation");
+    LOB_CUDA(staging(&tmp, need, st), "staging allocation");
     const int desc = which == LVBGS_MAP_SAMPLE_DESC ? 1 : 0;
     if (D.C == 3) lob_k_export_samples<3><<<1024, 256, 0, st>>>(D, tmp, desc);
     else lob_k_export_samples<1><<<1024, 256, 0, st>>>(D, tmp, desc);

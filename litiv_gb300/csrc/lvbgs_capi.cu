@@ -18,6 +18,7 @@
 #include "lobster_internal.h"
 #include "lvbgs_internal.h"
 #include "pawcs_internal.h"
+#include "staging.h"
 
 namespace lvbgs {
 extern "C" __global__ void lvbgs_k_eval(TickParams P);
@@ -1877,7 +1878,7 @@ lvbgs_status lvbgs_get_background_descriptors(lvbgs_handle h, uint16_t* out) {
         return s == LVBGS_OK ? s : fail(h, s, err);
     }
     uint16_t* d = nullptr;
-    LV_CUDA(h, cudaMallocAsync((void**)&d, h->npx * h->C * 2, h->stream), "temporary allocation");
+    LV_CUDA(h, staging_alloc(h->device, (void**)&d, h->npx * h->C * 2, h->stream), "temporary allocation");
     if (h->algo == LVBGS_ALGO_PAWCS && h->C == 3)
         pw3_k_background<<<512, 256, 0, h->stream>>>(h->pd, (int)(h->pw_frames & 1ull), nullptr, d, 0);
     else if (h->algo == LVBGS_ALGO_PAWCS)
@@ -2075,21 +2076,55 @@ lvbgs_status lvbgs_lbsp_compute2(const uint8_t* img, int W, int H, int C, long a
     if (C != 1 && C != 3) return fail(nullptr, LVBGS_BAD_TYPE, "input image must be of type 8UC1/8UC3");
     if (absThr < 0 && !(rel >= 0)) return fail(nullptr, LVBGS_BAD_ARG, "relative LBSP threshold must be non-negative");
     if (cudaSetDevice(device_id) != cudaSuccess) return fail(nullptr, LVBGS_DEVICE_ERROR, "cannot select the CUDA device");
-    const size_t n = (size_t)W * H * C;
-    uint8_t* di = nullptr;
-    uint16_t* dd = nullptr;
-    LV_CUDA(nullptr, cudaMalloc(&di, n), "allocation");
-    cudaError_t e = cudaMalloc(&dd, n * 2);
-    if (e == cudaSuccess) e = cudaMemcpy(di, img, n, cudaMemcpyDefault);
-    if (e == cudaSuccess) e = cudaMemcpy(dd, desc, n * 2, cudaMemcpyDefault);  // border keeps the caller's content
+    // Device buffers are used in place. Host buffers are staged; the 2-pixel border of a host result keeps the
+    // caller's content, which is saved and put back on the host (the whole result was uploaded for it before).
+    const size_t n = (size_t)W * H * C, row = (size_t)W * C;
+    const bool devImg = is_device_ptr(img), devDesc = is_device_ptr(desc);
+    const size_t needImg = devImg ? 0 : align256(n), needDesc = devDesc ? 0 : align256(n * 2);
+    uint8_t* tmp = nullptr;
+    if (needImg + needDesc)
+        LV_CUDA(nullptr, staging_alloc(device_id, (void**)&tmp, needImg + needDesc, nullptr), "allocation");
+    const uint8_t* di = devImg ? img : tmp;
+    uint16_t* dd = devDesc ? desc : (uint16_t*)(tmp + needImg);
+    cudaError_t e = cudaSuccess;
+    if (!devImg) e = cudaMemcpyAsync(tmp, img, n, cudaMemcpyHostToDevice, nullptr);
+    const int edge = std::min(kBorder, H);  // full border rows at the top and at the bottom
+    const int side = std::min(kBorder * C, (int)row);
+    std::vector<uint16_t> keep;
+    if (!devDesc) {
+        keep.reserve(2 * edge * row + 2 * (size_t)side * H);
+        for (int y = 0; y < H; ++y) {
+            const uint16_t* r = desc + (size_t)y * row;
+            if (y < edge || y >= H - edge) {
+                keep.insert(keep.end(), r, r + row);
+            } else {
+                keep.insert(keep.end(), r, r + side);
+                keep.insert(keep.end(), r + row - side, r + row);
+            }
+        }
+    }
     if (e == cudaSuccess) {
         const int thr = absThr < 0 ? -1 : (int)std::min<long>(absThr, 255);
-        lvbgs_lbsp_dense<<<256, 256>>>(di, W, H, C, thr, rel, (unsigned)off, dd);
+        const size_t blocks = ((size_t)W * H + 255) / 256;
+        lvbgs_lbsp_dense<<<(unsigned)std::min<size_t>(blocks, 1u << 20), 256>>>(di, W, H, C, thr, rel, (unsigned)off, dd);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(desc, dd, n * 2, cudaMemcpyDefault);
-    cudaFree(di);
-    cudaFree(dd);
+    if (e == cudaSuccess && !devDesc) e = cudaMemcpyAsync(desc, dd, n * 2, cudaMemcpyDeviceToHost, nullptr);
+    if (tmp) cudaFreeAsync(tmp, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    const uint16_t* k = keep.data();
+    if (!devDesc)
+        for (int y = 0; y < H; ++y) {
+            uint16_t* r = desc + (size_t)y * row;
+            if (y < edge || y >= H - edge) {
+                std::memcpy(r, k, row * 2);
+                k += row;
+            } else {
+                std::memcpy(r, k, (size_t)side * 2);
+                std::memcpy(r + row - side, k + side, (size_t)side * 2);
+                k += 2 * side;
+            }
+        }
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "LBSP extraction");
     return LVBGS_OK;
 }

@@ -1,7 +1,12 @@
 """SuBSENSE's and PAWCS's frame steps at the edges of their kernels' tiles, words and chunks, against the oracle (bit-exact)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from litiv_gb300 import _lib as L
+from litiv_gb300.metrics import BinClassif
+from oracle import metrics as oracle_metrics, pyoracle
 from tests.test_gpu_parity import run_pair
 from tests.test_gpu_pawcs import run_pair as pawcs_pair
 
@@ -71,3 +76,52 @@ def test_pawcs_word_streams(words, channels):
     frames = hollow_frames(61, 43, channels, 9, 7 * words)
     lrs = [1.0 if t in (3, 4, 7) else 0.0 for t in range(len(frames))]
     pawcs_pair(frames, seed=words, lrs=lrs, roi=roi, nMaxNbWords=words)
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4095, 4097, 70001])
+def test_classification_counters_at_packed_byte_edges(n, offset):
+    """Sizes around the 16-pixel packs and the 4,096-pixel blocks, images at and off 16-byte boundaries, with
+    and without a region of interest, against the restatement."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    codes = np.array([0, 50, 85, 170, 255, 17], np.uint8)
+    mask, gt = (rng.choice(codes, n) for _ in range(2))
+    roi = rng.choice(np.array([0, 255], np.uint8), n)
+
+    def on_device(a):
+        buf = torch.zeros(n + offset, dtype=torch.uint8, device="cuda")
+        buf[offset:] = torch.from_numpy(a).cuda()
+        return buf[offset:].view(1, n)
+
+    for r in (None, roi):
+        got = BinClassif().accumulate(on_device(mask), on_device(gt), None if r is None else on_device(r))
+        assert list(got.counts) == oracle_metrics.accumulate(mask[None], gt[None], None if r is None else r[None])
+
+
+@pytest.mark.parametrize("where", ["host", "device"])
+@pytest.mark.parametrize("W,H,channels", [(3, 9, 1), (4, 4, 3), (5, 5, 3), (61, 3, 1), (67, 53, 3), (640, 360, 1)])
+def test_lbsp_descriptors_keep_the_border(W, H, channels, where):
+    """Dense descriptors into host and device buffers: the interior against the oracle, the 2-pixel border as the
+    caller left it."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(W * H)
+    img = rng.integers(0, 256, (H, W, channels), dtype=np.uint8)
+    mark = rng.integers(0, 65536, (H, W, channels), dtype=np.uint16)
+    want = mark.copy()
+    if W > 4 and H > 4:
+        want[2:-2, 2:-2] = pyoracle.lbsp_compute2(img if channels == 3 else img[:, :, 0], rel_threshold=0.333,
+                                                  offset=2).reshape(H, W, channels)[2:-2, 2:-2]
+    if where == "host":
+        out = mark.copy()
+        ptrs = (img.ctypes.data, out.ctypes.data)
+    else:
+        di = torch.from_numpy(img).cuda()
+        do = torch.from_numpy(mark.view(np.uint8).reshape(-1).copy()).cuda()
+        torch.cuda.synchronize()
+        ptrs = (di.data_ptr(), do.data_ptr())
+    st = L.lib().lvbgs_lbsp_compute2(C.c_void_p(ptrs[0]), W, H, channels, -1, 0.333, 2, C.c_void_p(ptrs[1]), 0)
+    assert st == L.OK
+    if where == "device":
+        out = do.cpu().numpy().view(np.uint16).reshape(H, W, channels)
+    assert np.array_equal(out, want)
