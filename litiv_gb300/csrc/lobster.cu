@@ -12,15 +12,20 @@
 // they do not depend on the scan order. A frame step therefore
 //   1. evaluates every pixel against the frame-start samples (lob_k_eval): decision, samples scanned
 //      e, and the model writes it makes (own sample, neighbour target and sample), in an intent word;
-//   2. marks the pixels whose scan read a sample that an earlier neighbour writes (lob_k_mark);
-//   3. re-evaluates the marked pixels with the samples the raster scan would see (the latest earlier
-//      writer of each sample), and marks the later pixels whose incoming writes changed, round after
-//      round until nothing changes (lob_k_round; the dependencies follow raster order, so this is the
-//      raster-order fixed point). Rounds are enqueued ahead; a converged flag makes the rest return;
+//   2. re-evaluates the pixels whose scan read a sample that an earlier neighbour writes, with the samples
+//      the raster scan would see (the latest earlier writer of each sample; lob_k_first);
+//   3. repeats that for the later pixels whose incoming writes changed, round after round until nothing
+//      changes (lob_k_round; the dependencies follow raster order, so this is the raster-order fixed
+//      point). Rounds are enqueued ahead; a converged flag makes the rest return;
 //   4. commits every sample write in raster order, each pixel gathering the writes aimed at it from
 //      its 3x3 neighbourhood (lob_k_commit), then the median blur of the mask (:577-579).
 // The writers of a pixel are within one pixel of it: getNeighborPosition_3x3 moves one step and
 // clamps into the LBSP border, and ROI pixels lie inside that border.
+//
+// A scan that ends within a few samples (most of a background) stays with its pixel's lane; a longer one is
+// finished by eight lanes, eight samples a step, whose ballots give the samples scanned before the stop, so that
+// one long scan does not hold 31 lanes for N steps. The samples of a pixel are one aligned word or word pair
+// (load_sample), and a frame's launches are chained (each starts while the one before drains).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -34,25 +39,10 @@ namespace lvbgs {
 
 namespace {
 
-// LBSP 16-bit double-cross pattern (LBSP.hpp:297-298) as compile-time offsets: (offset + 2) in three
-// bits per tap, so that unrolled tap loops fold the offsets into immediates
-constexpr unsigned long long pack3(const int (&a)[16]) {
-    unsigned long long v = 0;
-    for (int i = 0; i < 16; ++i) v |= (unsigned long long)(a[i] + 2) << (3 * i);
-    return v;
-}
-constexpr int kDx[16] = {-2, 2, 0, 0, -2, 2, 2, -2, 0, -1, 0, 1, -1, 1, 1, -1};
-constexpr int kDy[16] = {0, 0, -2, 2, 2, -2, 2, -2, 1, 0, -1, 0, -1, 1, -1, 1};
-constexpr unsigned long long kDx3 = pack3(kDx), kDy3 = pack3(kDy);
-__device__ __forceinline__ constexpr int tap_dx(int n) { return (int)((kDx3 >> (3 * n)) & 7ull) - 2; }
-__device__ __forceinline__ constexpr int tap_dy(int n) { return (int)((kDy3 >> (3 * n)) & 7ull) - 2; }
-
-// 7x7 Gaussian sampling weights (opencv.hpp:915-923) and the 3x3 neighbour table (opencv.hpp:945-953)
+// 7x7 Gaussian sampling weights (opencv.hpp:915-923)
 __constant__ int c_lob_pat7[49] = {2,  4,  6,  7,  6,  4,  2,  4,  8,  12, 14, 12, 8,  4,  6, 12, 21,
                                    25, 21, 12, 6,  7,  14, 25, 28, 25, 14, 7,  6,  12, 21, 25, 21, 12,
                                    6,  4,  8,  12, 14, 12, 8,  4,  2,  4,  6,  7,  6,  4,  2};
-__constant__ int c_lob_nb3[8][2] = {{-1, 1}, {0, 1}, {1, 1}, {-1, 0}, {1, 0}, {-1, -1}, {0, -1}, {1, -1}};
-
 constexpr int kThreadsL = 256;
 constexpr int kMaxRoundsL = 4096;  // repair rounds of one frame step before LVBGS_DEVICE_ERROR
 
@@ -111,31 +101,62 @@ __device__ __forceinline__ void taps(const uint8_t* img, int W, int p, int c, ui
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int n = 4 * j + i;
-            w |= (uint32_t)__ldg(base + (tap_dy(n) * W + tap_dx(n)) * C) << (8 * i);
+            w |= (uint32_t)__ldg(base + (lbsp_dy(n) * W + lbsp_dx(n)) * C) << (8 * i);
         }
         v[j] = w;
     }
 }
 
-// sample s of pixel p: LOBSTER, the packed word and the colour byte; ViBe, the colour bytes packed into d
+// Sample s of pixel p as (d, c2): LOBSTER, the packed word and the colour byte; ViBe, colour c at bits 8c of
+// d; PBAS, also gradient c at bits 24 + 8c. A sample is one or two accesses that a warp makes in whole lines:
+// LOBSTER u64 + u8 (one channel u16 + u8); PBAS u32 (colours, gradient 0) + u16 (gradients 1 and 2), one
+// channel u16; ViBe u16 + u8, one channel u8. With a byte plane per value a PBAS sample took six accesses.
 template <int C, int ALG>
 __device__ __forceinline__ void load_sample(const LobDev& D, int s, int p, unsigned long long& d, uint32_t& c2) {
-    if (ALG == ALG_VIBE || ALG == ALG_PBAS) {
-        // colour c at bits 8c; PBAS: gradient c at bits 24 + 8c
-        const size_t o = ((size_t)s * D.npx + p) * C;
-        d = 0;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            d |= (unsigned long long)__ldg(D.sC + o + c) << (8 * c);
-            if (ALG == ALG_PBAS) d |= (unsigned long long)__ldg(D.sG + o + c) << (24 + 8 * c);
+    const size_t o = (size_t)s * D.npx + p;
+    c2 = 0;
+    if (ALG == ALG_PBAS) {
+        if (C == 3) {
+            d = (unsigned long long)__ldg((const uint32_t*)D.sC + o) | ((unsigned long long)__ldg((const uint16_t*)D.sG + o) << 32);
+        } else {
+            const uint32_t v = __ldg((const uint16_t*)D.sC + o);
+            d = (v & 0xffu) | ((unsigned long long)(v >> 8) << 24);
         }
-        c2 = 0;
-        return;
+    } else if (ALG == ALG_VIBE) {
+        if (C == 3) d = (uint32_t)__ldg((const uint16_t*)D.sC + o) | ((uint32_t)__ldg(D.sG + o) << 16);
+        else d = __ldg(D.sC + o);
+    } else {
+        if (C == 3) d = __ldg((const unsigned long long*)D.sD + o);
+        else d = __ldg((const uint16_t*)D.sD + o);
+        c2 = __ldg(D.sC + o);
     }
-    if (C == 3) d = __ldg((const unsigned long long*)D.sD + (size_t)s * D.npx + p);
-    else d = __ldg((const uint16_t*)D.sD + (size_t)s * D.npx + p);
-    c2 = __ldg(D.sC + (size_t)s * D.npx + p);
 }
+template <int C, int ALG>
+__device__ __forceinline__ void store_sample(const LobDev& D, int s, int p, unsigned long long d, uint32_t c2) {
+    const size_t o = (size_t)s * D.npx + p;
+    if (ALG == ALG_PBAS) {
+        if (C == 3) {
+            ((uint32_t*)D.sC)[o] = (uint32_t)d;
+            ((uint16_t*)D.sG)[o] = (uint16_t)(d >> 32);
+        } else {
+            ((uint16_t*)D.sC)[o] = (uint16_t)((d & 0xffu) | ((d >> 16) & 0xff00u));
+        }
+    } else if (ALG == ALG_VIBE) {
+        if (C == 3) {
+            ((uint16_t*)D.sC)[o] = (uint16_t)d;
+            D.sG[o] = (uint8_t)(d >> 16);
+        } else {
+            D.sC[o] = (uint8_t)d;
+        }
+    } else {
+        if (C == 3) ((unsigned long long*)D.sD)[o] = d;
+        else ((uint16_t*)D.sD)[o] = (uint16_t)d;
+        D.sC[o] = (uint8_t)c2;
+    }
+}
+// bytes of the two sample planes (sC, sG) per sample and pixel
+inline size_t sample_bytes_lo(int alg, int C) { return alg == ALG_PBAS ? (C == 3 ? 4 : 2) : alg == ALG_VIBE ? (C == 3 ? 2 : 1) : 1; }
+inline size_t sample_bytes_hi(int alg, int C) { return C != 3 ? 0 : alg == ALG_PBAS ? 2 : alg == ALG_VIBE ? 1 : 0; }
 
 // one sample against the pixel: LOBSTER (:479-494 / :522-541); ViBe (BackgroundSubtractorViBe.cpp:87 /
 // :165-170): |in - bg| < R on one channel; on three, lv::L2dist<3>(uchar*, uchar*) < 3R, whose squared
@@ -180,127 +201,267 @@ __device__ __forceinline__ bool match(const LobDev& D, const uint32_t (&vals)[C]
     }
 }
 
-// overrides of a re-evaluation: the samples that earlier neighbours write (latest writer last)
-struct LobOvr {
-    int n;
-    int s[4];
-    unsigned long long d[4];
-    uint32_t c[4];
-    unsigned long long mask;
+// what the scan needs of a pixel: its colour, LOBSTER its LBSP taps, PBAS its gradient, its threshold
+// R(x) * R0 and the weight of gradient distances BGSPBAS_GRAD_WEIGHT_ALPHA / m_fFormerMeanGradDist
+template <int C, int ALG>
+struct PxIn {
+    uint32_t vals[C][4];
+    uint32_t curr[C], g[ALG == ALG_PBAS ? C : 1];
+    float thr, gw;
 };
-
-// the evaluation of pixel p (x, y): ordered scan (with overrides), then the decision and the model
-// writes with their draws (:497-513 / :545-575); returns the intent word
-template <int C, int ALG, bool OVR>
-__device__ uint32_t eval_px(const LobDev& D, int p, int x, int y, const uint32_t (&vals)[C][4],
-                            const uint32_t (&curr)[C], const LobOvr& ov, unsigned long long* scanned) {
-    int nGood = 0, s = 0;
-    unsigned long long dB = 0;
-    uint32_t cB = 0;
-    if (D.N > 0) load_sample<C, ALG>(D, 0, p, dB, cB);
-    while (nGood < D.nreq && s < D.N) {
-        unsigned long long d = dB;
-        uint32_t c2 = cB;
-        if (s + 1 < D.N) load_sample<C, ALG>(D, s + 1, p, dB, cB);
-        if (OVR && ((ov.mask >> s) & 1ull)) {
-            for (int k = 0; k < ov.n; ++k)
-                if (ov.s[k] == s) {
-                    d = ov.d[k];
-                    c2 = ov.c[k];
-                }
-        }
-        if (match<C, ALG>(D, vals, curr, d, c2)) ++nGood;
-        ++s;
+template <int C, int ALG>
+__device__ __forceinline__ void pixel_inputs(const LobDev& D, int p, bool on, PxIn<C, ALG>& in) {
+    in.thr = in.gw = 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        in.curr[c] = 0u;
+        if (ALG == ALG_PBAS) in.g[c] = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) in.vals[c][j] = 0u;
     }
-    *scanned += (unsigned long long)s;
-    uint32_t w = kIValid | ((uint32_t)s << 2);
-    if (nGood < D.nreq) return w | kIFG;
-    Draws ds;
-    ds.blk = 0xffffffffu;
-    uint32_t k = 0;
-    if (mod64(draw(D, (uint32_t)p, k++, ds), D.nLR) == 0ull) {
-        const uint32_t so = draw(D, (uint32_t)p, k++, ds) % (uint32_t)D.N;
-        w |= kIOwn | (so << 10);
+    if (!on) return;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        if constexpr (ALG == ALG_LOBSTER) taps<C>(D.frame, D.W, p, c, in.vals[c]);
+        in.curr[c] = __ldg(D.frame + (size_t)p * C + c);
+        if (ALG == ALG_PBAS) in.g[c] = __ldg(D.grad + (size_t)p * C + c);
     }
-    if (mod64(draw(D, (uint32_t)p, k++, ds), D.nLR) == 0ull) {
-        // getNeighborPosition_3x3 (opencv.hpp:945-953), clamped into the LBSP border (LOBSTER) or the frame (ViBe)
-        constexpr int bord = ALG == ALG_VIBE ? 0 : kBorder;
-        const int r = (int)(draw(D, (uint32_t)p, k++, ds) % 8u);
-        const int nx = clampi(x + c_lob_nb3[r][0], bord, D.W - bord - 1);
-        const int ny = clampi(y + c_lob_nb3[r][1], bord, D.H - bord - 1);
-        const uint32_t sn = draw(D, (uint32_t)p, k++, ds) % (uint32_t)D.N;
-        const uint32_t code = (uint32_t)((ny - y + 1) * 3 + (nx - x + 1));
-        w |= kINb | (code << 17) | (sn << 21);
+    if (ALG == ALG_PBAS) {
+        in.thr = D.fm[(size_t)D.cur * 3 * D.npx + p] * D.R0;
+        in.gw = 10.0f / *D.meanGrad;
     }
-    return w | (k << 27);
+}
+// The sample word the pixel writes: LOBSTER, its descriptors (:499-500 / :548-550) and colour; ViBe, its colour;
+// PBAS, its colour and gradient (also what a neighbour update writes into it)
+template <int C, int ALG>
+__device__ __forceinline__ unsigned long long sample_word(const LobDev& D, const PxIn<C, ALG>& in) {
+    unsigned long long wd = 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        if constexpr (ALG == ALG_LOBSTER)
+            wd |= (unsigned long long)lbsp_thr(in.vals[c], in.curr[c], __ldg(D.lut + in.curr[c])) << (16 * c);
+        else wd |= (unsigned long long)in.curr[c] << (8 * c);
+        if (ALG == ALG_PBAS) wd |= (unsigned long long)in.g[c] << (24 + 8 * c);
+    }
+    if (ALG == ALG_LOBSTER && C == 3) wd |= ((unsigned long long)in.curr[0] << 48) | ((unsigned long long)in.curr[1] << 56);
+    return wd;
 }
 
-// PBAS's evaluation of pixel p (:146-231 / :365-458): the ordered scan with the colour + weighted
-// gradient distance against the threshold R(x) * R0, the bad samples' gradient distances for the frame
-// level, then the D(x), T(x) and R(x) updates (written to the maps of the next parity) and the model
-// updates with their draws. g holds the pixel's gradient. Three-channel distances: (float)sqrt((double)s)
-// of the uint16 sum s equals sqrtf((float)s), since double rounding through double is innocuous for the
-// square root (53 >= 2 * 24 + 2 bits).
-template <int C, bool OVR>
-__device__ uint32_t pbas_eval_px(const LobDev& D, int p, int x, int y, const uint32_t (&curr)[C], const uint32_t (&g)[C],
-                                 const LobOvr& ov, unsigned long long* scanned) {
-    const size_t npx = (size_t)D.npx;
-    const float* fc = D.fm + (size_t)D.cur * 3 * npx;
-    float* fn = D.fm + (size_t)(D.cur ^ 1) * 3 * npx;
-    const float R = fc[p], T = fc[npx + p], Dm = fc[2 * npx + p];
-    const float thr = R * D.R0;
-    const float gw = 10.0f / *D.meanGrad;  // BGSPBAS_GRAD_WEIGHT_ALPHA / m_fFormerMeanGradDist
-    float fMin = 255.0f;
-    int nGood = 0, s = 0, nb = 0;
-    uint32_t badSum = 0;
+// One sample against the pixel. PBAS (:146-166 / :365-394): the colour distance plus the weighted gradient
+// distance, at most 255, against the threshold; grad is the gradient distance (one channel) or its square
+// modulo 65536, with dist its root (three: lv::L2dist of two Vec3b adds in uint16_t). (float)sqrt((double)s) of that integer
+// equals sqrtf((float)s), since double rounding through double is innocuous for the square root
+// (53 >= 2 * 24 + 2 bits).
+template <int C, int ALG>
+__device__ __forceinline__ bool judge(const LobDev& D, const PxIn<C, ALG>& in, unsigned long long d, uint32_t c2, float& fSum,
+                                      uint32_t& grad, float& dist) {
+    if constexpr (ALG != ALG_PBAS) {
+        return match<C, ALG>(D, in.vals, in.curr, d, c2);
+    } else if constexpr (C == 1) {
+        const uint32_t nCol = (uint32_t)abs((int)in.curr[0] - (int)(d & 0xffu));
+        grad = (uint32_t)abs((int)in.g[0] - (int)((d >> 24) & 0xffu));
+        fSum = in.gw * (float)grad + (float)nCol;
+    } else {
+        uint32_t aC = 0, aG = 0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const int dc = (int)in.curr[c] - (int)((d >> (8 * c)) & 0xffu);
+            const int dg = (int)in.g[c] - (int)((d >> (24 + 8 * c)) & 0xffu);
+            aC += (uint32_t)(dc * dc);
+            aG += (uint32_t)(dg * dg);
+        }
+        grad = aG & 0xffffu;
+        dist = __fsqrt_rn((float)grad);
+        fSum = in.gw * dist + __fsqrt_rn((float)(aC & 0xffffu));
+    }
+    if (fSum > 255.0f) fSum = 255.0f;
+    return fSum <= in.thr;
+}
+
+// Samples that earlier neighbours write this frame (repair): which, and which of them match the pixel now. PBAS
+// writes the pixel's own values into them (self diffusion): distance 0, always good.
+struct Over {
+    unsigned long long mask, good;
+};
+// state of a pixel's ordered scan; PBAS: smallest good distance, bad samples and the sum of their gradient
+// distances (one channel: exact; three: about, it only predicts where the ordered sum will be)
+struct Scan {
+    int s, nGood, nb;
+    uint32_t badSum;
+    float badAbout, fMin;
+};
+__device__ __forceinline__ Scan scan_start() { return {0, 0, 0, 0u, 0.0f, 255.0f}; }
+// the gradient distance of the pixel's i-th bad sample, three channels, as its square in 16 bits
+__device__ __forceinline__ uint16_t& bad_value(const LobDev& D, int i, int p) { return D.badVals[(size_t)p * D.N + i]; }
+
+// the ordered scan by the pixel's own lane, from st up to sample end
+template <int C, int ALG>
+__device__ __forceinline__ void lane_scan(const LobDev& D, int p, const PxIn<C, ALG>& in, const Over& ov, int end, Scan& st) {
     unsigned long long dB = 0;
     uint32_t cB = 0;
-    if (D.N > 0) load_sample<C, ALG_PBAS>(D, 0, p, dB, cB);
-    while (nGood < D.nreq && s < D.N) {
-        unsigned long long d = dB;
-        if (s + 1 < D.N) load_sample<C, ALG_PBAS>(D, s + 1, p, dB, cB);
-        if (OVR && ((ov.mask >> s) & 1ull)) d = ov.d[0];  // self diffusion: the pixel's own values
-        float fSum, fGrad = 0.0f;
-        uint32_t nGrad = 0;
-        if (C == 1) {
-            const uint32_t nCol = (uint32_t)abs((int)curr[0] - (int)(d & 0xffu));
-            nGrad = (uint32_t)abs((int)g[0] - (int)((d >> 24) & 0xffu));
-            fSum = gw * (float)nGrad + (float)nCol;
-        } else {
-            uint32_t aC = 0, aG = 0;
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int dc = (int)curr[c] - (int)((d >> (8 * c)) & 0xffu);
-                const int dg = (int)g[c] - (int)((d >> (24 + 8 * c)) & 0xffu);
-                aC += (uint32_t)(dc * dc);
-                aG += (uint32_t)(dg * dg);
-            }
-            fGrad = __fsqrt_rn((float)(aG & 0xffffu));
-            fSum = gw * fGrad + __fsqrt_rn((float)(aC & 0xffffu));
+    if (st.s < end && st.nGood < D.nreq) load_sample<C, ALG>(D, st.s, p, dB, cB);
+    while (st.nGood < D.nreq && st.s < end) {
+        const unsigned long long d = dB;
+        const uint32_t c2 = cB;
+        if (st.s + 1 < end) load_sample<C, ALG>(D, st.s + 1, p, dB, cB);
+        float fSum = 0.0f, dist = 0.0f;
+        uint32_t grad = 0u;
+        const bool good = ((ov.mask >> st.s) & 1ull) ? (ov.good >> st.s) & 1ull : judge<C, ALG>(D, in, d, c2, fSum, grad, dist);
+        if (good) {
+            if (ALG == ALG_PBAS && st.fMin > fSum) st.fMin = fSum;
+            ++st.nGood;
+        } else if (ALG == ALG_PBAS) {
+            if (C == 1) st.badSum += grad;
+            else bad_value(D, st.nb, p) = (uint16_t)grad;
+            st.badAbout += dist;
+            ++st.nb;
         }
-        if (fSum > 255.0f) fSum = 255.0f;
-        if (fSum <= thr) {
-            if (fMin > fSum) fMin = fSum;
-            ++nGood;
-        } else {
-            if (C == 1) badSum += nGrad;
-            else D.badVals[(size_t)p * D.N + nb] = fGrad;
-            ++nb;
-        }
-        ++s;
+        ++st.s;
     }
-    *scanned += (unsigned long long)s;
-    const float Nf = (float)D.N;
-    const float Dn = (Dm * (Nf - 1.0f) + fMin / 255.0f) / Nf;
-    uint32_t w = kIValid | ((uint32_t)s << 2);
-    float Tn;
-    uint32_t k = 0;
-    if (nGood < D.nreq) {
+}
+
+// The rest of the scans of a warp's pixels (on: this lane's pixel p may need more), by groups of eight lanes: a
+// group takes the next unsettled pixel, broadcasts its inputs and judges eight samples a step; the ballot gives
+// the ordered result (the scan stops at the nreq-th good sample). A warp whose lanes scan alone runs to its
+// slowest lane, all N samples as soon as one lane is foreground, and a single scan is a chain of ~0.4 us a
+// sample. Every lane of the warp calls it.
+template <int C, int ALG>
+__device__ __forceinline__ void group_scan(const LobDev& D, bool on, int p, const PxIn<C, ALG>& in, const Over& ov, Scan& st) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7, N = D.N, nreq = D.nreq;
+    unsigned todo = __ballot_sync(kAll, on && st.nGood < nreq && st.s < N);
+    while (todo) {
+        unsigned own = todo;
+        for (int i = 0; i < grp; ++i) own &= own - 1u;
+        const bool go = own != 0u;
+        const int src = go ? __ffs(own) - 1 : lane;
+        unsigned taken = todo;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) todo &= todo - 1u;
+        taken ^= todo;
+        __syncwarp();
+        PxIn<C, ALG> b;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            b.curr[c] = __shfl_sync(kAll, in.curr[c], src);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b.vals[c][j] = ALG == ALG_LOBSTER ? __shfl_sync(kAll, in.vals[c][j], src) : 0u;
+            if constexpr (ALG == ALG_PBAS) b.g[c] = __shfl_sync(kAll, in.g[c], src);
+        }
+        b.thr = b.gw = 0.0f;
+        if (ALG == ALG_PBAS) {
+            b.thr = __shfl_sync(kAll, in.thr, src);
+            b.gw = __shfl_sync(kAll, in.gw, src);
+        }
+        const int bp = __shfl_sync(kAll, p, src);
+        Over bo;
+        bo.mask = __shfl_sync(kAll, ov.mask, src);
+        bo.good = __shfl_sync(kAll, ov.good, src);
+        Scan t;
+        t.s = __shfl_sync(kAll, st.s, src);
+        t.nGood = __shfl_sync(kAll, st.nGood, src);
+        t.nb = ALG == ALG_PBAS ? __shfl_sync(kAll, st.nb, src) : 0;
+        t.badSum = 0u;
+        t.badAbout = 0.0f;
+        t.fMin = 255.0f;
+        int k = t.s + sub;
+        unsigned long long d = 0;
+        uint32_t c2 = 0;
+        if (go && k < N) load_sample<C, ALG>(D, k, bp, d, c2);
+        while (__any_sync(kAll, go && t.nGood < nreq && t.s < N)) {
+            __syncwarp();
+            const bool act = go && t.nGood < nreq && t.s < N;
+            unsigned long long dn = 0;
+            uint32_t cn = 0;
+            if (act && k + 8 < N) load_sample<C, ALG>(D, k + 8, bp, dn, cn);
+            float fSum = 0.0f, dist = 0.0f;
+            uint32_t grad = 0u;
+            bool good = false;
+            if (act && k < N)
+                good = ((bo.mask >> k) & 1ull) ? (bo.good >> k) & 1ull : judge<C, ALG>(D, b, d, c2, fSum, grad, dist);
+            __syncwarp();
+            const uint32_t m = (__ballot_sync(kAll, good) >> (8 * grp)) & 0xffu;
+            if (act) {
+                const int need = nreq - t.nGood, cnt = __popc(m);
+                int stop = min(8, N - t.s);
+                if (cnt >= need) {
+                    uint32_t r = m;
+                    for (int i = 1; i < need; ++i) r &= r - 1u;
+                    stop = __ffs(r);
+                    t.nGood = nreq;
+                } else {
+                    t.nGood += cnt;
+                }
+                if (ALG == ALG_PBAS && sub < stop) {
+                    if (good) {
+                        if (t.fMin > fSum) t.fMin = fSum;
+                    } else if (C == 1) {
+                        t.badSum += grad;
+                    } else {
+                        t.badAbout += dist;
+                        bad_value(D, t.nb + __popc(~m & ((1u << sub) - 1u)), bp) = (uint16_t)grad;
+                    }
+                }
+                if (ALG == ALG_PBAS) t.nb += __popc(~m & ((1u << stop) - 1u));
+                t.s += stop;
+            }
+            d = dn;
+            c2 = cn;
+            k += 8;
+        }
+        if (ALG == ALG_PBAS) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                t.badSum += __shfl_xor_sync(kAll, t.badSum, o);
+                t.badAbout += __shfl_xor_sync(kAll, t.badAbout, o);
+                const float f = __shfl_xor_sync(kAll, t.fMin, o);
+                if (t.fMin > f) t.fMin = f;
+            }
+        }
+        // back to the owners: the r-th owner's scan was done by group r
+        const bool mine = (taken >> lane) & 1u;
+        const int from = mine ? 8 * __popc(taken & ((1u << lane) - 1u)) : lane;
+        const int rs = __shfl_sync(kAll, t.s, from), rg = __shfl_sync(kAll, t.nGood, from);
+        if (mine) {
+            st.s = rs;
+            st.nGood = rg;
+        }
+        if (ALG == ALG_PBAS) {
+            const int rb = __shfl_sync(kAll, t.nb, from);
+            const uint32_t rq = __shfl_sync(kAll, t.badSum, from);
+            const float rf = __shfl_sync(kAll, t.fMin, from), ra = __shfl_sync(kAll, t.badAbout, from);
+            if (mine) {
+                st.nb = rb;
+                st.badSum += rq;
+                st.badAbout += ra;
+                if (st.fMin > rf) st.fMin = rf;
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// The decision of a scanned pixel p (x, y) and its model writes with their draws (:497-513 / :545-575; PBAS
+// :174-194 / :402-424): returns the intent word. PBAS also writes its D(x), T(x) and R(x) of the next parity
+// (:198-231 / :427-458) and the bad samples for the frame level.
+template <int C, int ALG>
+__device__ uint32_t decide(const LobDev& D, int p, int x, int y, const Scan& st) {
+    uint32_t w = kIValid | ((uint32_t)st.s << 2), k = 0;
+    const bool fg = st.nGood < D.nreq;
+    const size_t npx = (size_t)D.npx;
+    float R = 0.0f, T = 0.0f, Dn = 0.0f;
+    if (ALG == ALG_PBAS) {
+        const float* fc = D.fm + (size_t)D.cur * 3 * npx;
+        R = fc[p];
+        T = fc[npx + p];
+        const float Dm = fc[2 * npx + p], Nf = (float)D.N;
+        Dn = (Dm * (Nf - 1.0f) + st.fMin / 255.0f) / Nf;
+    }
+    if (fg) {
         w |= kIFG;
-        Tn = T + 1.0000f / (Dn * 255.00f + 1.0000f);
-        if (Tn > 200.00f) Tn = 200.00f;
     } else {
-        const unsigned long long nLR = D.lrOverride ? D.nLR : (unsigned long long)__float2uint_rz(ceilf(T));
+        const unsigned long long nLR =
+            ALG == ALG_PBAS && !D.lrOverride ? (unsigned long long)__float2uint_rz(ceilf(T)) : D.nLR;
         Draws ds;
         ds.blk = 0xffffffffu;
         if (mod64(draw(D, (uint32_t)p, k++, ds), nLR) == 0ull) {
@@ -308,43 +469,58 @@ __device__ uint32_t pbas_eval_px(const LobDev& D, int p, int x, int y, const uin
             w |= kIOwn | (so << 10);
         }
         if (mod64(draw(D, (uint32_t)p, k++, ds), nLR) == 0ull) {
-            const int r = (int)(draw(D, (uint32_t)p, k++, ds) % 8u);
-            const int nx = clampi(x + c_lob_nb3[r][0], 0, D.W - 1);
-            const int ny = clampi(y + c_lob_nb3[r][1], 0, D.H - 1);
+            // getNeighborPosition_3x3 (opencv.hpp:945-953), clamped into the LBSP border (LOBSTER) or the frame
+            constexpr int bord = ALG == ALG_LOBSTER ? kBorder : 0;
+            int dx, dy;
+            nb3_offset((int)(draw(D, (uint32_t)p, k++, ds) % 8u), dx, dy);
+            const int nx = clampi(x + dx, bord, D.W - bord - 1), ny = clampi(y + dy, bord, D.H - bord - 1);
             const uint32_t sn = draw(D, (uint32_t)p, k++, ds) % (uint32_t)D.N;
             w |= kINb | ((uint32_t)((ny - y + 1) * 3 + (nx - x + 1)) << 17) | (sn << 21);
         }
-        Tn = T - 0.0500f / (Dn * 255.00f + 1.0000f);
-        if (Tn < 2.0000f) Tn = 2.0000f;
     }
-    float Rn = R;
-    if (R < 0.6000f + Dn * 5.0000f + 0.0000f) {
-        if (R < 99.0000f) Rn = R * 1.0500f;
-    } else if (R > 0.6000f) {
-        Rn = R * 0.9500f;
+    if (ALG == ALG_PBAS) {
+        float Tn;
+        if (fg) {
+            Tn = T + 1.0000f / (Dn * 255.00f + 1.0000f);
+            if (Tn > 200.00f) Tn = 200.00f;
+        } else {
+            Tn = T - 0.0500f / (Dn * 255.00f + 1.0000f);
+            if (Tn < 2.0000f) Tn = 2.0000f;
+        }
+        float Rn = R;
+        if (R < 0.6000f + Dn * 5.0000f + 0.0000f) {
+            if (R < 99.0000f) Rn = R * 1.0500f;
+        } else if (R > 0.6000f) {
+            Rn = R * 0.9500f;
+        }
+        float* fn = D.fm + (size_t)(D.cur ^ 1) * 3 * npx;
+        fn[p] = Rn;
+        fn[npx + p] = Tn;
+        fn[2 * npx + p] = Dn;
+        D.badSum[p] = C == 1 ? st.badSum : __float_as_uint(st.badAbout);  // three channels keep the values too (badVals)
+        D.badCnt[p] = (uint8_t)st.nb;
     }
-    fn[p] = Rn;
-    fn[npx + p] = Tn;
-    fn[2 * npx + p] = Dn;
-    if (C == 1) D.badSum[p] = badSum;  // three channels keep the values themselves (badVals)
-    D.badCnt[p] = (uint8_t)nb;
     return w | (k << 27);
 }
 
-// the pixel's colour and (LOBSTER) its LBSP taps
-template <int C, int ALG>
-__device__ __forceinline__ void pixel_inputs(const LobDev& D, int p, uint32_t (&vals)[C][4], uint32_t (&curr)[C]) {
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-        if (ALG == ALG_LOBSTER) taps<C>(D.frame, D.W, p, c, vals[c]);
-        curr[c] = __ldg(D.frame + (size_t)p * C + c);
+// per-thread counts (each below 2^24) into one or two 64-bit counters, one atomic each per block: the counters
+// are shared by the whole frame, and same-address atomics serialize. Every thread of the block calls it.
+__device__ __forceinline__ void block_add(unsigned long long* a, unsigned int va, unsigned long long* b = nullptr,
+                                          unsigned int vb = 0u) {
+    __shared__ unsigned int red[2][kThreadsL / 32];
+    const unsigned int sa = __reduce_add_sync(0xffffffffu, va), sb = b ? __reduce_add_sync(0xffffffffu, vb) : 0u;
+    __syncthreads();  // an earlier call's values have been read
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = sa;
+        red[1][threadIdx.x >> 5] = sb;
     }
-}
-
-// warp-aggregated count of a per-thread value into a 64-bit counter
-__device__ __forceinline__ void warp_add(unsigned long long* ctr, unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(ctr, v);
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long t = 0;
+        for (int w = 0; w < kThreadsL / 32; ++w) t += red[threadIdx.x][w];
+        unsigned long long* c = threadIdx.x ? b : a;
+        if (t) atomicAdd(c, t);
+    }
 }
 
 // list push with per-round dedupe; the lanes that push together share one counter atomic
@@ -362,140 +538,102 @@ __device__ __forceinline__ void push(const LobDev& D, uint32_t* list, unsigned i
 
 }  // namespace
 
-// 1. every ROI pixel (ViBe: every pixel) against the frame-start samples
+// 1. every ROI pixel (ViBe, PBAS: every pixel) against the frame-start samples: the lane itself up to lane_cap
+// samples, which settle most pixels, the others by groups. Block 0 opens the frame step's flags. Caps of 2, 4, 8
+// and none: LOBSTER 1277x719 BGR 53 / 45 / 42 / 46 us; PBAS 1920x1080 BGR 177 / 140 / 149 / 164 us; ViBe, whose
+// judgements are too cheap for the broadcasts, 320x240 BGR 11.7 / 10.8 / 10.5 / 9.9 us.
+LV_HD constexpr int lane_cap(int alg) { return alg == ALG_LOBSTER ? 8 : alg == ALG_PBAS ? 4 : kMaxSamples; }
 template <int C, int ALG>
 __global__ void __launch_bounds__(kThreadsL) lob_k_eval(LobDev D) {
+    pdl_entry();
+    if (blockIdx.x == 0 && threadIdx.x < LOB_F_WORDS) D.flags[threadIdx.x] = 0u;
+    if (ALG == ALG_PBAS && blockIdx.x == 0 && threadIdx.x < 2) D.stats[2 + threadIdx.x] = 0ull;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long scanned = 0;
-    if (p < D.npx) {
-        if (ALG == ALG_LOBSTER && !D.roi[p]) {
-            D.intent[p] = 0u;
-        } else {
-            const int x = p % D.W, y = p / D.W;
-            uint32_t vals[C][4], curr[C];
-            pixel_inputs<C, ALG>(D, p, vals, curr);
-            // the sample word this pixel writes: LOBSTER, its descriptors (:499-500 / :548-550) and colour;
-            // ViBe, its colour; PBAS, its colour and gradient (also what a neighbour update writes into it)
-            unsigned long long wd = 0;
-            LobOvr none;
-            none.n = 0;
-            none.mask = 0;
-            if (ALG == ALG_PBAS) {
-                uint32_t g[C];
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    g[c] = __ldg(D.grad + (size_t)p * C + c);
-                    wd |= ((unsigned long long)curr[c] << (8 * c)) | ((unsigned long long)g[c] << (24 + 8 * c));
-                }
-                D.wD[p] = wd;
-                D.intent[p] = pbas_eval_px<C, false>(D, p, x, y, curr, g, none, &scanned);
-            } else {
-                if (ALG == ALG_VIBE) {
-#pragma unroll
-                    for (int c = 0; c < C; ++c) wd |= (unsigned long long)curr[c] << (8 * c);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < C; ++c)
-                        wd |= (unsigned long long)lbsp_thr(vals[c], curr[c], __ldg(D.lut + curr[c])) << (16 * c);
-                    if (C == 3) wd |= ((unsigned long long)curr[0] << 48) | ((unsigned long long)curr[1] << 56);
-                }
-                D.wD[p] = wd;
-                D.intent[p] = eval_px<C, ALG, false>(D, p, x, y, vals, curr, none, &scanned);
-            }
-        }
+    const bool in = p < D.npx;
+    const bool on = in && (ALG != ALG_LOBSTER || D.roi[p]);
+    PxIn<C, ALG> px;
+    pixel_inputs<C, ALG>(D, p, on, px);
+    const Over none = {0ull, 0ull};
+    Scan st = scan_start();
+    if (on) {
+        D.wD[p] = sample_word<C, ALG>(D, px);
+        lane_scan<C, ALG>(D, p, px, none, min(lane_cap(ALG), D.N), st);
     }
-    warp_add(&D.stats[0], scanned);
+    group_scan<C, ALG>(D, on, p, px, none, st);
+    if (in) D.intent[p] = on ? decide<C, ALG>(D, p, p % D.W, p / D.W, st) : 0u;
+    block_add(&D.stats[0], on ? (unsigned int)st.s : 0u);
 }
 
-// 2. the pixels whose scan read a sample that an earlier neighbour writes
-__global__ void __launch_bounds__(kThreadsL) lob_k_mark(LobDev D) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= D.npx) return;
-    const uint32_t w = D.intent[p];
-    if (!(w & kIValid)) return;
-    const int x = p % D.W, y = p / D.W, e = i_e(w);
-    bool dirty = false;
-    // earlier pixels within one step: the row above, then the left neighbour
-    const int q4[4] = {p - D.W - 1, p - D.W, p - D.W + 1, p - 1};
-    const bool ok4[4] = {y > 0 && x > 0, y > 0, y > 0 && x + 1 < D.W, x > 0};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (!ok4[i]) continue;
-        const uint32_t wq = D.intent[q4[i]];
-        if ((wq & kIValid) && (wq & kINb) && nb_target(wq, q4[i], D.W) == p && i_snb(wq) < e) dirty = true;
-    }
-    if (dirty) push(D, D.list0, &D.flags[LOB_F_COUNT0], D.stampBase, p);
+// the four earlier pixels within one step of p (x, y): the row above, then the left neighbour
+struct Earlier {
+    int q[4];
+    bool ok[4];
+};
+__device__ __forceinline__ Earlier earlier(const LobDev& D, int p, int x, int y) {
+    return {{p - D.W - 1, p - D.W, p - D.W + 1, p - 1}, {y > 0 && x > 0, y > 0, y > 0 && x + 1 < D.W, x > 0}};
 }
 
-// 3. one repair round: re-evaluates the pixels of list (round & 1) with the samples their earlier
-// neighbours write now, and lists the later pixels whose incoming writes changed
+// Re-evaluates the pixels of a warp's owner lanes (on: this lane holds pixel p; every lane calls it) with the
+// samples that their earlier neighbours write now, and lists the later pixels whose incoming writes changed.
+// alone: every lane scans its own pixel (a list that fills the machine), otherwise groups of eight lanes do.
 template <int C, int ALG>
-__global__ void __launch_bounds__(kThreadsL) lob_k_round(LobDev D, int round) {
-    if (ld_vol(&D.flags[LOB_F_CONV])) return;
-    const int cur = round & 1;
-    const unsigned int n0 = ld_vol(&D.flags[cur]);
-    const unsigned int n = n0 < D.listCap ? n0 : D.listCap;
-    const uint32_t* in = cur ? D.list1 : D.list0;
-    uint32_t* out = cur ? D.list0 : D.list1;
-    unsigned int* outCount = &D.flags[cur ^ 1];
-    const uint32_t stamp = D.stampBase + (uint32_t)round + 1u;
-    unsigned long long scanned = 0;
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int p = (int)__ldcg(in + i);
-        const int x = p % D.W, y = p / D.W;
-        LobOvr ov;
-        ov.n = 0;
-        ov.mask = 0;
-        const int q4[4] = {p - D.W - 1, p - D.W, p - D.W + 1, p - 1};
-        const bool ok4[4] = {y > 0 && x > 0, y > 0, y > 0 && x + 1 < D.W, x > 0};
-        for (int j = 0; j < 4; ++j) {
-            if (!ok4[j]) continue;
-            const uint32_t wq = ld_vol(&D.intent[q4[j]]);
-            if ((wq & kIValid) && (wq & kINb) && nb_target(wq, q4[j], D.W) == p) {
-                const int s = i_snb(wq);
-                ov.s[ov.n] = s;
-                ov.d[ov.n] = __ldcg(D.wD + q4[j]);
-                ov.c[ov.n] = ALG != ALG_LOBSTER ? 0u : __ldg(D.frame + (size_t)q4[j] * C + (C == 3 ? 2 : 0));
-                ++ov.n;
-                ov.mask |= 1ull << s;
-            }
-        }
-        uint32_t vals[C][4], curr[C];
-        pixel_inputs<C, ALG>(D, p, vals, curr);
-        uint32_t wNew;
-        if (ALG == ALG_PBAS) {
-            // self diffusion: a sample that an earlier neighbour writes holds the pixel's own values
-            uint32_t g[C];
+__device__ void reevaluate(const LobDev& D, bool on, int p, bool alone, uint32_t* out, unsigned int* outCount, uint32_t stamp,
+                           unsigned int& scanned) {
+    const int x = on ? p % D.W : 0, y = on ? p / D.W : 0;
+    PxIn<C, ALG> px;
+    pixel_inputs<C, ALG>(D, p, on, px);
+    Over ov = {0ull, 0ull};
+    if (on) {
+        const Earlier e = earlier(D, p, x, y);
+        uint32_t wq[4];
 #pragma unroll
-            for (int c = 0; c < C; ++c) g[c] = __ldg(D.grad + (size_t)p * C + c);
-            ov.d[0] = __ldcg(D.wD + p);
-            wNew = pbas_eval_px<C, true>(D, p, x, y, curr, g, ov, &scanned);
-        } else {
-            wNew = eval_px<C, ALG, true>(D, p, x, y, vals, curr, ov, &scanned);
-        }
-        const uint32_t wOld = ld_vol(&D.intent[p]);
-        if (wNew == wOld) continue;
-        *(volatile uint32_t*)&D.intent[p] = wNew;
-        if (i_nbpart(wNew) == i_nbpart(wOld)) continue;
-        // the targets of the old and the new neighbour write that come later in raster order
-        if (wOld & kINb) {
-            const int t = nb_target(wOld, p, D.W);
-            if (t > p) push(D, out, outCount, stamp, t);
-        }
-        if (wNew & kINb) {
-            const int t = nb_target(wNew, p, D.W);
-            if (t > p) push(D, out, outCount, stamp, t);
+        for (int j = 0; j < 4; ++j) wq[j] = e.ok[j] ? ld_vol(&D.intent[e.q[j]]) : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!((wq[j] & kIValid) && (wq[j] & kINb) && nb_target(wq[j], e.q[j], D.W) == p)) continue;
+            const unsigned long long bit = 1ull << i_snb(wq[j]);
+            bool good = true;
+            if (ALG != ALG_PBAS) {
+                const uint32_t c = ALG != ALG_LOBSTER ? 0u : __ldg(D.frame + (size_t)e.q[j] * C + (C == 3 ? 2 : 0));
+                float f, dist;
+                uint32_t gr;
+                good = judge<C, ALG>(D, px, __ldcg(D.wD + e.q[j]), c, f, gr, dist);
+            }
+            // the latest writer of a sample decides
+            ov.mask |= bit;
+            ov.good = good ? ov.good | bit : ov.good & ~bit;
         }
     }
-    warp_add(&D.stats[0], scanned);
+    Scan st = scan_start();
+    if (alone && on) lane_scan<C, ALG>(D, p, px, ov, D.N, st);
+    group_scan<C, ALG>(D, on, p, px, ov, st);
+    if (!on) return;
+    scanned += (unsigned int)st.s;
+    const uint32_t wNew = decide<C, ALG>(D, p, x, y, st), wOld = ld_vol(&D.intent[p]);
+    if (wNew == wOld) return;
+    *(volatile uint32_t*)&D.intent[p] = wNew;
+    if (i_nbpart(wNew) == i_nbpart(wOld)) return;
+    // the targets of the old and the new neighbour write that come later in raster order
+    if (wOld & kINb) {
+        const int t = nb_target(wOld, p, D.W);
+        if (t > p) push(D, out, outCount, stamp, t);
+    }
+    if (wNew & kINb) {
+        const int t = nb_target(wNew, p, D.W);
+        if (t > p) push(D, out, outCount, stamp, t);
+    }
 }
 
-// end of repair round `round`: converged when the round listed nothing; otherwise its input list
-// becomes the next round's output
-__global__ void lob_k_round_end(LobDev D, int round) {
-    if (D.flags[LOB_F_CONV]) return;
+// End of repair round `round`, by every block of its kernel; the block that finishes last closes it: converged
+// when the round listed nothing, otherwise its input list becomes the next round's output
+__device__ __forceinline__ void round_end(const LobDev& D, int round) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&D.flags[LOB_F_DONE], 1u) != gridDim.x - 1u) return;
+    D.flags[LOB_F_DONE] = 0u;
     const int cur = round & 1;
-    const unsigned int next = D.flags[cur ^ 1];
+    const unsigned int next = ld_vol(&D.flags[cur ^ 1]);
     D.flags[LOB_F_ROUNDS] = (unsigned int)round + 1u;
     if (next > D.listCap) {
         D.flags[LOB_F_ERR] |= 1u;
@@ -507,69 +645,178 @@ __global__ void lob_k_round_end(LobDev D, int round) {
     }
 }
 
+// 2. Round 0: a block finds the pixels of its own (four a thread) whose scan read a sample that an earlier
+// neighbour writes, and re-evaluates them, with the other blocks' re-evaluations under way: a pixel that changes
+// its neighbour write after a later pixel looked at it lists that pixel for round 1. One launch where the marks
+// went through a list in memory. A block lasts as long as its slowest re-evaluation, so it takes 1,024 pixels:
+// with 256, LOBSTER 1277x719 BGR took 36 us and PBAS 1920x1080 BGR 67 us.
+constexpr int kFirstPer = 4, kFirstPx = kFirstPer * kThreadsL;
+template <int C, int ALG>
+__global__ void __launch_bounds__(kThreadsL) lob_k_first(LobDev D) {
+    pdl_entry();
+    __shared__ int items[kFirstPx];
+    __shared__ int count;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, p0 = blockIdx.x * kFirstPx + (int)threadIdx.x;
+    uint32_t w[kFirstPer], wq[kFirstPer][4];
+#pragma unroll
+    for (int i = 0; i < kFirstPer; ++i) {
+        const int p = p0 + i * kThreadsL;
+        w[i] = p < D.npx ? ld_vol(&D.intent[p]) : 0u;
+        const Earlier e = earlier(D, p, p % D.W, p / D.W);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wq[i][j] = p < D.npx && e.ok[j] ? ld_vol(&D.intent[e.q[j]]) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < kFirstPer; ++i) {
+        const int p = p0 + i * kThreadsL;
+        bool dirty = false;
+        if (w[i] & kIValid) {
+            const int n = i_e(w[i]);
+            // the four earlier neighbours reach p with the codes of one step down right, down, down left, right
+            const int code[4] = {8, 7, 6, 5};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                dirty = dirty || ((wq[i][j] & kIValid) && (wq[i][j] & kINb) && i_code(wq[i][j]) == code[j] && i_snb(wq[i][j]) < n);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, dirty);
+        int base = 0;
+        if (lane == 0 && m) base = atomicAdd(&count, __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (dirty) items[base + __popc(m & ((1u << lane) - 1u))] = p;
+    }
+    __syncthreads();
+    unsigned int scanned = 0;
+    const uint32_t stamp = D.stampBase + 1u;
+    const int n = count;
+    const bool alone = n > kThreadsL / 2;  // more than four pixels a group: every lane its own
+    const int per = alone ? 32 : 4;
+    for (int i0 = (threadIdx.x >> 5) * per; i0 < n; i0 += per * (kThreadsL / 32)) {
+        const int i = alone ? i0 + lane : i0 + (lane >> 3);
+        const bool on = i < n && (alone || (lane & 7) == 0);
+        reevaluate<C, ALG>(D, on, on ? items[i] : 0, alone, D.list1, &D.flags[LOB_F_COUNT1], stamp, scanned);
+    }
+    block_add(&D.stats[0], scanned);
+    round_end(D, 0);
+}
+
+// 3. one later repair round: the pixels of list (round & 1)
+template <int C, int ALG>
+__global__ void __launch_bounds__(kThreadsL) lob_k_round(LobDev D, int round) {
+    pdl_entry();
+    if (ld_vol(&D.flags[LOB_F_CONV])) return;
+    const int cur = round & 1;
+    const unsigned int n0 = ld_vol(&D.flags[cur]);
+    const unsigned int n = n0 < D.listCap ? n0 : D.listCap;
+    const uint32_t* in = cur ? D.list1 : D.list0;
+    uint32_t* out = cur ? D.list0 : D.list1;
+    unsigned int* outCount = &D.flags[cur ^ 1];
+    const uint32_t stamp = D.stampBase + (uint32_t)round + 1u;
+    unsigned int scanned = 0;
+    const int lane = threadIdx.x & 31;
+    const unsigned int warp = blockIdx.x * (kThreadsL / 32) + (threadIdx.x >> 5), warps = gridDim.x * (kThreadsL / 32);
+    const bool alone = n > 16u * warps;  // more than four pixels a group: every lane its own
+    const unsigned int per = alone ? 32u : 4u;
+    for (unsigned int i0 = warp * per; i0 < n; i0 += warps * per) {
+        const unsigned int i = alone ? i0 + lane : i0 + (lane >> 3);
+        const bool on = i < n && (alone || (lane & 7) == 0);
+        reevaluate<C, ALG>(D, on, on ? (int)__ldcg(in + i) : 0, alone, out, outCount, stamp, scanned);
+    }
+    block_add(&D.stats[0], scanned);
+    round_end(D, round);
+}
+
 // 4. every pixel gathers the sample writes aimed at it, in raster order of the writers (own update
 // before neighbour update within a writer); the raw mask (ViBe: the output, :84 / :176) and the draw
-// counters of the frame
+// counters of the frame. The nine intents are requested together; the writes go to a register list of 12 bits
+// each (window slot, sample, own write) that the warp executes together, and more than five (rare) take the
+// slots one by one. A pixel's writes are its own thread's, in order, so the last writer of a sample wins.
 template <int C, int ALG>
 __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
-    if (!ld_vol(&D.flags[LOB_F_CONV])) return;
+    pdl_entry();
+    const unsigned int conv = ld_vol(&D.flags[LOB_F_CONV]);
+    if (blockIdx.x == 0 && threadIdx.x < LOB_F_WORDS) ((volatile unsigned int*)D.hflags)[threadIdx.x] = ld_vol(&D.flags[threadIdx.x]);
+    if (!conv) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long writes = 0;
+    unsigned int writes = 0;
     if (p < D.npx) {
-        const uint32_t wp = D.intent[p];
+        const int x = p % D.W, y = p / D.W;
+        uint32_t w9[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int dx = k % 3 - 1, dy = k / 3 - 1;
+            const bool ok = y + dy >= 0 && y + dy < D.H && x + dx >= 0 && x + dx < D.W;
+            w9[k] = ok ? D.intent[p + dy * D.W + dx] : 0u;
+        }
+        const uint32_t wp = w9[4];
         const bool valid = (wp & kIValid) != 0;
         const uint8_t raw = (valid && (wp & kIFG)) ? 255 : 0;
         if (ALG == ALG_VIBE) D.maskOut[p] = raw;
         else D.rawFG[p] = raw;
-        // PBAS: every write into pixel p holds p's own colour and gradient
-        const unsigned long long wOwn = ALG == ALG_PBAS ? D.wD[p] : 0ull;
         D.kctr[p] = (uint16_t)(valid ? i_draws(wp) : 0);
-        if (valid) writes = ((wp & kIOwn) ? 1ull : 0ull) + ((wp & kINb) ? 1ull : 0ull);
-        const int x = p % D.W, y = p / D.W;
+        if (valid) writes = ((wp & kIOwn) ? 1u : 0u) + ((wp & kINb) ? 1u : 0u);
         // the pixels a write can reach: inside the LBSP border (LOBSTER), the whole frame (ViBe, PBAS)
         constexpr int bord = ALG == ALG_LOBSTER ? kBorder : 0;
-        if (x >= bord && y >= bord && x < D.W - bord && y < D.H - bord) {
-            int ns = 0;
-            int ss[10], sq[10];
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    if (y + dy < 0 || y + dy >= D.H || x + dx < 0 || x + dx >= D.W) continue;
-                    const int q = p + dy * D.W + dx;
-                    const uint32_t wq = D.intent[q];
-                    if (!(wq & kIValid)) continue;
-                    int sv[2], nv = 0;
-                    if (q == p && (wq & kIOwn)) sv[nv++] = i_sown(wq);
-                    if ((wq & kINb) && nb_target(wq, q, D.W) == p) sv[nv++] = i_snb(wq);
-                    for (int v = 0; v < nv; ++v) {
-                        int k = 0;
-                        while (k < ns && ss[k] != sv[v]) ++k;
-                        ss[k] = sv[v];
-                        sq[k] = q;
-                        if (k == ns) ++ns;
-                    }
-                }
-            for (int k = 0; k < ns; ++k) {
-                const size_t o = (size_t)ss[k] * D.npx + p;
-                const int q = sq[k];
-                if (ALG == ALG_PBAS) {
+        const bool reach = x >= bord && y >= bord && x < D.W - bord && y < D.H - bord;
+        unsigned long long list = 0;
+        int nwr = 0;
 #pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        D.sC[o * C + c] = (uint8_t)(wOwn >> (8 * c));
-                        D.sG[o * C + c] = (uint8_t)(wOwn >> (24 + 8 * c));
-                    }
-                } else if (ALG == ALG_VIBE) {
-                    const unsigned long long wq = D.wD[q];
-#pragma unroll
-                    for (int c = 0; c < C; ++c) D.sC[o * C + c] = (uint8_t)(wq >> (8 * c));
-                } else {
-                    if (C == 3) ((unsigned long long*)D.sD)[o] = D.wD[q];
-                    else ((uint16_t*)D.sD)[o] = (uint16_t)D.wD[q];
-                    D.sC[o] = __ldg(D.frame + (size_t)q * C + (C == 3 ? 2 : 0));
-                }
+        for (int k = 0; k < 9; ++k) {
+            const uint32_t w = w9[k];
+            if (!reach || !(w & kIValid)) continue;
+            if (k == 4 && (w & kIOwn)) {
+                if (nwr < 5) list |= (unsigned long long)(2048u | (4u << 6) | (uint32_t)i_sown(w)) << (12 * nwr);
+                ++nwr;
+            }
+            if ((w & kINb) && i_code(w) == 8 - k) {
+                if (nwr < 5) list |= (unsigned long long)(((uint32_t)k << 6) | (uint32_t)i_snb(w)) << (12 * nwr);
+                ++nwr;
+            }
+        }
+        auto write = [&](int k, int s) {
+            // PBAS: every write into pixel p holds p's own colour and gradient
+            const int q = ALG == ALG_PBAS ? p : p + (k / 3 - 1) * D.W + k % 3 - 1;
+            const uint32_t c2 = ALG == ALG_LOBSTER ? __ldg(D.frame + (size_t)q * C + (C == 3 ? 2 : 0)) : 0u;
+            store_sample<C, ALG>(D, s, p, __ldg(D.wD + q), c2);
+        };
+        const int nlist = nwr <= 5 ? nwr : 0;
+        const int iters = (int)__reduce_max_sync(__activemask(), (unsigned)nlist);
+        for (int j = 0; j < iters; ++j)
+            if (j < nlist) {
+                const uint32_t e = (uint32_t)(list >> (12 * j)) & 0xfffu;
+                write((int)((e >> 6) & 15u), (int)(e & 63u));
+            }
+        if (nwr > 5) {
+#pragma unroll 1
+            for (int k = 0; k < 9; ++k) {
+                const int q = p + (k / 3 - 1) * D.W + k % 3 - 1;
+                const int qy = y + k / 3 - 1, qx = x + k % 3 - 1;
+                if (qy < 0 || qy >= D.H || qx < 0 || qx >= D.W) continue;
+                const uint32_t w = D.intent[q];
+                if (!(w & kIValid)) continue;
+                if (k == 4 && (w & kIOwn)) write(4, i_sown(w));
+                if ((w & kINb) && i_code(w) == 8 - k) write(k, i_snb(w));
             }
         }
     }
-    warp_add(&D.stats[1], writes);
+    if (!(ALG == ALG_PBAS && C == 3)) {
+        block_add(&D.stats[1], writes);
+    } else {
+        // this block's pixels are one chunk of the ordered sum below: about how much it adds, and its count
+        __shared__ float sm[kThreadsL / 32];
+        float about = p < D.npx ? __uint_as_float(D.badSum[p]) : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) about += __shfl_xor_sync(0xffffffffu, about, o);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = about;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float c = 0.0f;
+            for (int w = 0; w < kThreadsL / 32; ++w) c += sm[w];
+            D.chunkAbout[blockIdx.x] = c;
+        }
+        block_add(&D.stats[1], writes, &D.stats[3], p < D.npx ? (unsigned int)D.badCnt[p] : 0u);
+    }
 }
 
 // cv::medianBlur(raw mask, k) with replicated borders: 255 where more than half of the k*k window is
@@ -579,6 +826,7 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
 constexpr int kMedTile = 32, kMedMaxR = 15, kMedS = kMedTile + 2 * kMedMaxR;
 template <int C, bool KEEP>
 __global__ void __launch_bounds__(kThreadsL) lob_k_median(LobDev D) {
+    pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
     __shared__ uint8_t raw[kMedS][kMedS];
     __shared__ uint8_t rows[kMedS][kMedTile];
@@ -661,9 +909,10 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_vibe_init(LobDev D, const uin
         sx = clampi(sx + x0 - 3, 0, D.W - 1);
         sy = clampi(sy + y0 - 3, 0, D.H - 1);
         const uint8_t* src = img + ((size_t)sy * D.W + sx) * C;
-        uint8_t* dst = D.sC + ((size_t)s * D.npx + p) * C;
+        unsigned long long d = 0;
 #pragma unroll
-        for (int c = 0; c < C; ++c) dst[c] = __ldg(src + c);
+        for (int c = 0; c < C; ++c) d |= (unsigned long long)__ldg(src + c) << (8 * c);
+        store_sample<C, ALG_VIBE>(D, s, p, d, 0u);
     }
 }
 
@@ -675,45 +924,86 @@ __device__ __forceinline__ int reflect101(int i, int n) {
     return i;
 }
 
-// the gradient image of a frame (:127-135 / :338-346), first pass: GaussianBlur 3x3 (sigma 0), the
-// separable [1 2 1] / 4 kernel in 8-bit fixed point, (sum + 8) >> 4, with BORDER_REFLECT_101
+// The gradient image of a frame (:127-135 / :338-346): GaussianBlur 3x3 (sigma 0), the separable [1 2 1] / 4
+// kernel in 8-bit fixed point, (sum + 8) >> 4; the Scharr derivatives ([-3 0 3; -10 0 10; -3 0 3] and its
+// transpose), convertScaleAbs (|v| saturated to 255) and addWeighted(0.5, 0.5) ((a + b) * 0.5 rounded half to
+// even), all with BORDER_REFLECT_101. One block per tile of kGradW x kGradH pixels: the frame tile with its
+// reflected 2-pixel halo in shared memory, blurred there with a 1-pixel halo (both kernels are symmetric, so
+// the blur of a reflected position is the reflected blur), then the derivatives; four bytes at a time, two per
+// word in 16 bits (the sums are at most 16 * 255). Bytes of a channel are C apart in the interleaved rows. The
+// blur went through memory before, a byte and nine loads a thread: 30 + 38 us on a 1920x1080 BGR frame.
+constexpr int kGradW = 64, kGradH = 16;
 template <int C>
-__global__ void __launch_bounds__(kThreadsL) pbas_k_blur(LobDev D, const uint8_t* img) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.npx * C) return;
-    const int p = i / C, c = i % C, x = p % D.W, y = p / D.W;
-    const int xs[3] = {reflect101(x - 1, D.W), x, reflect101(x + 1, D.W)};
-    const int ys[3] = {reflect101(y - 1, D.H), y, reflect101(y + 1, D.H)};
-    int acc = 0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const uint8_t* row = img + (size_t)ys[j] * D.W * C + c;
-        const int r = __ldg(row + xs[0] * C) + 2 * __ldg(row + xs[1] * C) + __ldg(row + xs[2] * C);
-        acc += (j == 1 ? 2 : 1) * r;
-    }
-    D.blur[i] = (uint8_t)((acc + 8) >> 4);
+struct GradTile {
+    static constexpr int kPad = 8;                                   // bytes before the tile's first pixel
+    static constexpr int kRow = (kPad + (kGradW + 2) * C + 4 + 3) / 4;  // words of a row
+    uint32_t src[kGradH + 4][kRow], blur[kGradH + 2][kRow];
+};
+// bytes b .. b + 3 of a shared row (any byte offset), and their spread to two 16-bit pairs
+__device__ __forceinline__ uint32_t row4(const uint32_t* row, int b) {
+    return __funnelshift_r(row[b >> 2], row[(b >> 2) + 1], 8 * (b & 3));
 }
-
-// second pass: the Scharr derivatives ([-3 0 3; -10 0 10; -3 0 3] and its transpose, int16, no
-// overflow at these magnitudes), convertScaleAbs (|v| saturated to 255) and addWeighted(0.5, 0.5)
-// ((a + b) * 0.5 rounded half to even), BORDER_REFLECT_101
+__device__ __forceinline__ uint32_t even2(uint32_t w) { return w & 0x00ff00ffu; }
+__device__ __forceinline__ uint32_t odd2(uint32_t w) { return (w >> 8) & 0x00ff00ffu; }
 template <int C>
-__global__ void __launch_bounds__(kThreadsL) pbas_k_grad(LobDev D) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.npx * C) return;
-    const int p = i / C, c = i % C, x = p % D.W, y = p / D.W;
-    const int xs[3] = {reflect101(x - 1, D.W), x, reflect101(x + 1, D.W)};
-    const int ys[3] = {reflect101(y - 1, D.H), y, reflect101(y + 1, D.H)};
-    int v[3][3];
+__global__ void __launch_bounds__(kThreadsL) pbas_k_grad(LobDev D, const uint8_t* img) {
+    using T = GradTile<C>;
+    __shared__ T sm;
+    const int x0 = blockIdx.x * kGradW, y0 = blockIdx.y * kGradH, t = threadIdx.x;
+    // frame bytes of rows y0 - 2 .. y0 + 17, pixels x0 - 2 .. x0 + 65, from byte kPad - 2 C of a row on
+    constexpr int kBytes = (kGradW + 4) * C;
+    for (int i = t; i < (kGradH + 4) * kBytes; i += kThreadsL) {
+        const int r = i / kBytes, b = i % kBytes;
+        const int gy = reflect101(y0 - 2 + r, D.H), gx = reflect101(x0 - 2 + b / C, D.W);
+        ((uint8_t*)sm.src[r])[T::kPad - 2 * C + b] = __ldg(img + ((size_t)gy * D.W + gx) * C + b % C);
+    }
+    __syncthreads();
+    // blur of rows y0 - 1 .. y0 + 16, pixels x0 - 1 .. x0 + 64, in words from byte kFirst on
+    constexpr int kFirst = (T::kPad - C) / 4 * 4, kBlurW = (T::kPad + (kGradW + 1) * C - kFirst + 3) / 4;
+    for (int i = t; i < (kGradH + 2) * kBlurW; i += kThreadsL) {
+        const int r = i / kBlurW, b = kFirst + 4 * (i % kBlurW);
+        uint32_t e = 0x00080008u, o = 0x00080008u;
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
+        for (int j = 0; j < 3; ++j) {
+            const uint32_t* row = sm.src[r + j];
+            const uint32_t L = row4(row, b - C), M = row[b >> 2], R = row4(row, b + C);
+            const uint32_t he = even2(L) + 2u * even2(M) + even2(R), ho = odd2(L) + 2u * odd2(M) + odd2(R);
+            e += j == 1 ? 2u * he : he;
+            o += j == 1 ? 2u * ho : ho;
+        }
+        sm.blur[r][b >> 2] = ((e >> 4) & 0x00ff00ffu) | (((o >> 4) & 0x00ff00ffu) << 8);
+    }
+    __syncthreads();
+    constexpr int kOutW = kGradW * C / 4;
+    for (int i = t; i < kGradH * kOutW; i += kThreadsL) {
+        const int r = i / kOutW, k = 4 * (i % kOutW), b = T::kPad + k;
+        if (y0 + r >= D.H) break;
+        uint32_t l[3], c[3], h[3];  // the rows' words to the left, at and to the right of the four bytes
 #pragma unroll
-        for (int k = 0; k < 3; ++k) v[j][k] = __ldg(D.blur + ((size_t)ys[j] * D.W + xs[k]) * C + c);
-    const int gx = 3 * (v[0][2] - v[0][0]) + 10 * (v[1][2] - v[1][0]) + 3 * (v[2][2] - v[2][0]);
-    const int gy = 3 * (v[2][0] - v[0][0]) + 10 * (v[2][1] - v[0][1]) + 3 * (v[2][2] - v[0][2]);
-    const int ax = min(abs(gx), 255), ay = min(abs(gy), 255);
-    const int sum = ax + ay;
-    D.grad[i] = (uint8_t)((sum >> 1) + ((sum & 1) & ((sum >> 1) & 1)));
+        for (int j = 0; j < 3; ++j) {
+            const uint32_t* row = sm.blur[r + j];
+            l[j] = row4(row, b - C);
+            c[j] = row[b >> 2];
+            h[j] = row4(row, b + C);
+        }
+        uint32_t out = 0;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            auto u = [&](uint32_t w) { return half ? odd2(w) : even2(w); };
+            const uint32_t colL = 3u * (u(l[0]) + u(l[2])) + 10u * u(l[1]), colR = 3u * (u(h[0]) + u(h[2])) + 10u * u(h[1]);
+            const uint32_t top = 3u * (u(l[0]) + u(h[0])) + 10u * u(c[0]), bot = 3u * (u(l[2]) + u(h[2])) + 10u * u(c[2]);
+            const uint32_t sum = __vminu2(__vabsdiffu2(colR, colL), 0x00ff00ffu) + __vminu2(__vabsdiffu2(bot, top), 0x00ff00ffu);
+            const uint32_t hf = (sum >> 1) & 0x00ff00ffu;
+            out |= (hf + (sum & hf & 0x00010001u)) << (8 * half);
+        }
+        const int left = (D.W - x0) * C - k;  // bytes of the frame row from here on
+        uint8_t* dst = D.grad + ((size_t)(y0 + r) * D.W + x0) * C + k;
+        if (left >= 4 && ((uintptr_t)dst & 3) == 0) {
+            *(uint32_t*)dst = out;
+        } else {
+            for (int q = 0; q < min(left, 4); ++q) dst[q] = (uint8_t)(out >> (8 * q));
+        }
+    }
 }
 
 // PBAS's initialize() (:61-109 / :287-324): R = 1, T = the default update rate, D = 0 in the maps of
@@ -744,28 +1034,36 @@ __global__ void __launch_bounds__(kThreadsL) pbas_k_init(LobDev D, const uint8_t
         }
         sx = clampi(sx + x0 - 3, 0, D.W - 1);
         sy = clampi(sy + y0 - 3, 0, D.H - 1);
-        const size_t src = ((size_t)sy * D.W + sx) * C, dst = ((size_t)s * npx + p) * C;
+        const size_t src = ((size_t)sy * D.W + sx) * C;
+        unsigned long long d = 0;
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-            D.sC[dst + c] = __ldg(img + src + c);
-            D.sG[dst + c] = D.grad[src + c];
-        }
+        for (int c = 0; c < C; ++c)
+            d |= ((unsigned long long)__ldg(img + src + c) << (8 * c)) | ((unsigned long long)D.grad[src + c] << (24 + 8 * c));
+        store_sample<C, ALG_PBAS>(D, s, p, d, 0u);
     }
 }
 
 // the frame-level mean gradient distance of the bad samples, single channel (:232): the size_t sum
 // of their gradient distances and their count (which starts at 1), per block into two counters
 __global__ void __launch_bounds__(kThreadsL) pbas_k_mean1(LobDev D) {
+    pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
     unsigned long long sum = 0, cnt = 0;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.npx; p += gridDim.x * blockDim.x) {
         sum += D.badSum[p];
         cnt += D.badCnt[p];
     }
-    warp_add(&D.stats[2], sum);
-    warp_add(&D.stats[3], cnt);
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (sum) atomicAdd(&D.stats[2], sum);
+        if (cnt) atomicAdd(&D.stats[3], cnt);
+    }
 }
 __global__ void pbas_k_mean1_end(LobDev D) {
+    pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
     const float mean = (float)D.stats[2] / (float)(D.stats[3] + 1ull);
     *D.meanGrad = mean > 20.0f ? mean : 20.0f;
@@ -778,118 +1076,181 @@ __global__ void pbas_k_mean1_end(LobDev D) {
 // to the even quotient, which depends on the parity of s / u. The sum over a chunk of values is
 // therefore a function of that parity only: a transfer (d0, d1), the increment in ulps for an even or
 // odd start, composed value by value (d'_p = d_p + d2_{(p + d_p) & 1}).
-//   pbas_k_sum_chunks: the count of bad samples, and each chunk's total in double precision;
-//   pbas_k_sum_scan: their exclusive prefix, which predicts the binade of s at each chunk's start;
-//   pbas_k_sum_tr: each chunk's transfers for the predicted binade and the two beside it;
-//   pbas_k_sum_walk: from s = 0, chunk after chunk, applies the chunk's transfer when s is at least 1024,
-//     its binade is one of the chunk's three and the chunk cannot leave it (s / u + increment + 1 < 2^24:
-//     no value of the chunk reaches the next binade), and otherwise adds the chunk's values one by one.
-// The result is the sequential sum bit for bit; only the first chunks, those where s crosses a power of
-// two and those whose binade was mispredicted are summed value by value.
+//   lob_k_commit: the count of bad samples, and about how much each chunk of 256 pixels adds;
+//   pbas_k_sum_scan: the exclusive prefix of that, which predicts the binade of s at each chunk's start;
+//   pbas_k_sum_tr: the transfers of each chunk, and of its 32-pixel granules, for the predicted binade and
+//     the two beside it;
+//   pbas_k_sum_win: those of each window of 32 chunks, composed from its chunks';
+//   pbas_k_sum_walk: from s = 0, one warp over the windows, as many at once as have transfers for the binade of
+//     s and keep s in it; where s crosses into the next binade (or the prediction was off), the same over that
+//     window's chunks, over that chunk's granules, and value by value over that granule.
+// The result is the sequential sum bit for bit. An increment of 2^24 ulps leaves the binade whatever the start,
+// so transfers saturate at 2^25 and fit 32 bits.
 constexpr int kSumChunk = 256, kSumNB = 3, kSumEMin = 10, kSumScan = 1024;
+static_assert(kSumChunk == kThreadsL, "a block of the commit is a chunk");
+constexpr uint32_t kTrSat = 1u << 25;
 struct Tr {
-    unsigned long long d0, d1;
+    uint32_t d0, d1;
 };
 __device__ __forceinline__ Tr tr_then(Tr a, Tr b) {
     Tr r;
-    r.d0 = a.d0 + ((a.d0 & 1ull) ? b.d1 : b.d0);
-    r.d1 = a.d1 + ((a.d1 & 1ull) ? b.d0 : b.d1);
+    r.d0 = min(a.d0 + ((a.d0 & 1u) ? b.d1 : b.d0), kTrSat);
+    r.d1 = min(a.d1 + ((a.d1 & 1u) ? b.d0 : b.d1), kTrSat);
     return r;
 }
-// one value v >= 0 in binade e: its increment in ulps for an even / odd s / u
+// one value v in [0, 256] in binade e >= 10: its increment in ulps for an even / odd s / u
 __device__ __forceinline__ Tr tr_value(float v, int e) {
     const float x = v * __int_as_float((127 + 23 - e) << 23);  // v / u, exact (a power of two)
     const float a = floorf(x), r = x - a;
-    const unsigned long long ai = (unsigned long long)a;
+    const uint32_t ai = (uint32_t)a;
     Tr t;
-    if (r > 0.5f) t.d0 = t.d1 = ai + 1ull;
+    if (r > 0.5f) t.d0 = t.d1 = ai + 1u;
     else if (r < 0.5f) t.d0 = t.d1 = ai;
     else {
-        t.d0 = ai + (ai & 1ull);  // even s/u: s/u + a is even when a is
-        t.d1 = ai + ((ai + 1ull) & 1ull);
+        t.d0 = ai + (ai & 1u);  // even s/u: s/u + a is even when a is
+        t.d1 = ai + ((ai + 1u) & 1u);
     }
     return t;
 }
-__device__ __forceinline__ Tr tr_shfl_down(Tr t, int o) {
-    Tr r;
-    r.d0 = __shfl_down_sync(0xffffffffu, t.d0, o);
-    r.d1 = __shfl_down_sync(0xffffffffu, t.d1, o);
-    return r;
+__device__ __forceinline__ Tr tr_shfl(Tr t, int src) {
+    return {__shfl_sync(0xffffffffu, t.d0, src), __shfl_sync(0xffffffffu, t.d1, src)};
 }
 // binade of a positive float
 __device__ __forceinline__ int binade(float s) { return (int)((__float_as_uint(s) >> 23) & 0xffu) - 127; }
-
-struct SumWork {
-    double* chunkSum;  // [nChunks], then their exclusive prefix
-    Tr* tr;            // [nChunks][kSumNB]
-    Tr* trw;           // [nChunks][kSumChunk / 32][kSumNB]: the transfers of each chunk's 32-pixel granules
-    int* eb;           // [nChunks]: the first of the chunk's binades
-};
-constexpr int kSumGran = kSumChunk / 32;
-
-__global__ void __launch_bounds__(kSumChunk) pbas_k_sum_chunks(LobDev D, SumWork W) {
-    if (!ld_vol(&D.flags[LOB_F_CONV])) return;
-    __shared__ double sm[kSumChunk / 32];
-    const int t = threadIdx.x, p = blockIdx.x * kSumChunk + t;
-    const int n = p < D.npx ? (int)D.badCnt[p] : 0;
-    double acc = 0.0;
-    for (int k = 0; k < n; ++k) acc += (double)__ldg(D.badVals + (size_t)p * D.N + k);
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((t & 31) == 0) sm[t >> 5] = acc;
-    __syncthreads();
-    if (t == 0) {
-        double c = 0.0;
-        for (int w = 0; w < kSumChunk / 32; ++w) c += sm[w];
-        W.chunkSum[blockIdx.x] = c;
-    }
-    warp_add(&D.stats[3], (unsigned long long)n);
+// s after a transfer, when s >= 1024 and the transfer keeps s in its binade
+__device__ __forceinline__ bool tr_apply(float& s, Tr t) {
+    if (s < 1024.0f) return false;
+    const uint32_t bits = __float_as_uint(s), m = (bits & 0x7fffffu) | 0x800000u;
+    const uint32_t m2 = m + ((m & 1u) ? t.d1 : t.d0);
+    if (m2 + 1u >= (1u << 24)) return false;
+    s = __uint_as_float((bits & 0xff800000u) | (m2 & 0x7fffffu));
+    return true;
 }
 
-__global__ void __launch_bounds__(kSumScan) pbas_k_sum_scan(LobDev D, SumWork W, int nChunks) {
-    if (!ld_vol(&D.flags[LOB_F_CONV])) return;
-    __shared__ double sm[kSumScan];
-    const int t = threadIdx.x, per = (nChunks + kSumScan - 1) / kSumScan;
-    const int c0 = min(t * per, nChunks), c1 = min(c0 + per, nChunks);
-    double own = 0.0;
-    for (int c = c0; c < c1; ++c) own += W.chunkSum[c];
-    sm[t] = own;
-    __syncthreads();
-    for (int o = 1; o < kSumScan; o <<= 1) {
-        const double v = t >= o ? sm[t - o] : 0.0;
-        __syncthreads();
-        sm[t] += v;
-        __syncthreads();
+constexpr int kSumGran = kSumChunk / 32;
+struct SumWork {
+    float* about;  // [nChunks], then their exclusive prefix
+    Tr* tr;        // [nChunks][kSumNB]
+    Tr* trw;       // [nChunks][kSumGran][kSumNB]: the transfers of each chunk's 32-pixel granules
+    Tr* win;       // [nWin][kSumNB]: of each window of 32 chunks
+    int* eb;       // [nChunks]: the first of the chunk's binades
+    int* winEb;    // [nWin]: the first of the window's binades << 3 | which of the three all its chunks have
+    static size_t bytes(size_t nChunks) {
+        const size_t nWin = (nChunks + 31) / 32;
+        return nChunks * (2 * 4 + (1 + kSumGran) * kSumNB * sizeof(Tr)) + nWin * (kSumNB * sizeof(Tr) + 4);
     }
-    double run = sm[t] - own;
+};
+inline SumWork sum_work(void* base, size_t nChunks) {
+    const size_t nWin = (nChunks + 31) / 32;
+    SumWork W;
+    W.tr = (Tr*)base;
+    W.trw = W.tr + nChunks * kSumNB;
+    W.win = W.trw + nChunks * kSumGran * kSumNB;
+    W.about = (float*)(W.win + nWin * kSumNB);
+    W.eb = (int*)(W.about + nChunks);
+    W.winEb = W.eb + nChunks;
+    return W;
+}
+// the k-th bad sample's gradient distance of pixel p
+__device__ __forceinline__ float bad_dist(const LobDev& D, int k, int p) { return __fsqrt_rn((float)bad_value(D, k, p)); }
+
+__global__ void __launch_bounds__(kSumScan) pbas_k_sum_scan(LobDev D, SumWork W, int nChunks) {
+    pdl_entry();
+    if (!ld_vol(&D.flags[LOB_F_CONV])) return;
+    __shared__ float sm[kSumScan / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, per = (nChunks + kSumScan - 1) / kSumScan;
+    const int c0 = min(t * per, nChunks), c1 = min(c0 + per, nChunks);
+    float own = 0.0f;
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) own += W.about[c];
+    float inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) sm[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const float v = sm[lane];
+        float i2 = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_up_sync(0xffffffffu, i2, o);
+            if (lane >= o) i2 += y;
+        }
+        sm[lane] = i2 - v;
+    }
+    __syncthreads();
+    float run = sm[warp] + inc - own;
     for (int c = c0; c < c1; ++c) {
-        const double v = W.chunkSum[c];
-        W.chunkSum[c] = run;
+        const float v = W.about[c];
+        W.about[c] = run;
         run += v;
     }
 }
 
+// A warp takes a granule of 32 pixels: their values, in order, are split evenly over its lanes (a foreground pixel
+// has up to N, most have none or a few), each lane composes its own run, and the runs are composed in order.
 __global__ void __launch_bounds__(kSumChunk) pbas_k_sum_tr(LobDev D, SumWork W) {
+    pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
-    __shared__ Tr sm[kSumChunk / 32][kSumNB];
+    __shared__ Tr sm[kSumGran][kSumNB];
+    __shared__ int first[kSumGran][33];
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    const int p = blockIdx.x * kSumChunk + t;
+    const int p0 = blockIdx.x * kSumChunk + 32 * wid, p = p0 + lane;
     const int n = p < D.npx ? (int)D.badCnt[p] : 0;
-    const float* v = D.badVals + (size_t)(p < D.npx ? p : 0) * D.N;
-    const float pre = (float)W.chunkSum[blockIdx.x];
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    first[wid][lane + 1] = inc;
+    if (lane == 0) first[wid][0] = 0;
+    __syncwarp();
+    const int total = __shfl_sync(0xffffffffu, inc, 31), per = (total + 31) / 32;
+    const float pre = W.about[blockIdx.x];
     const int e0 = max(pre >= 1.0f ? binade(pre) - 1 : kSumEMin, kSumEMin);
     Tr acc[kSumNB];
 #pragma unroll
-    for (int j = 0; j < kSumNB; ++j) acc[j].d0 = acc[j].d1 = 0ull;
-    for (int k = 0; k < n; ++k) {
-        const float x = __ldg(v + k);
+    for (int j = 0; j < kSumNB; ++j) acc[j].d0 = acc[j].d1 = 0u;
+    const int i0 = min(lane * per, total), i1 = min(i0 + per, total);
+    if (i0 < i1) {
+        int q = 0;  // the pixel of value i0: the last one whose first value is at most i0
 #pragma unroll
-        for (int j = 0; j < kSumNB; ++j) acc[j] = tr_then(acc[j], tr_value(x, e0 + j));
+        for (int step = 16; step > 0; step >>= 1)
+            if (first[wid][q + step] <= i0) q += step;
+        int k = i0 - first[wid][q], left = first[wid][q + 1] - i0;
+        for (int i = i0; i < i1;) {
+            const int m = min(min(left, i1 - i), 4);  // values of this pixel in flight together
+            float x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = j < m ? bad_dist(D, k + j, p0 + q) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < m)
+#pragma unroll
+                    for (int b = 0; b < kSumNB; ++b) acc[b] = tr_then(acc[b], tr_value(x[j], e0 + b));
+            i += m;
+            k += m;
+            left -= m;
+            while (left == 0 && i < i1) {
+                ++q;
+                k = 0;
+                left = first[wid][q + 1] - first[wid][q];
+            }
+        }
     }
+    __syncwarp();
     // ordered reduction: lane 0 of each warp, then the warps in order
 #pragma unroll
     for (int j = 0; j < kSumNB; ++j) {
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const Tr y = tr_shfl_down(acc[j], o);
+            Tr y;
+            y.d0 = __shfl_down_sync(0xffffffffu, acc[j].d0, o);
+            y.d1 = __shfl_down_sync(0xffffffffu, acc[j].d1, o);
             if ((lane & (2 * o - 1)) == 0) acc[j] = tr_then(acc[j], y);
         }
         if (lane == 0) {
@@ -900,97 +1261,139 @@ __global__ void __launch_bounds__(kSumChunk) pbas_k_sum_tr(LobDev D, SumWork W) 
     __syncthreads();
     if (t < kSumNB) {
         Tr r = sm[0][t];
-        for (int w = 1; w < kSumChunk / 32; ++w) r = tr_then(r, sm[w][t]);
+        for (int w = 1; w < kSumGran; ++w) r = tr_then(r, sm[w][t]);
         W.tr[(size_t)blockIdx.x * kSumNB + t] = r;
         if (t == 0) W.eb[blockIdx.x] = e0;
     }
 }
 
-// s advanced by a transfer when s >= 1024 and the transfer keeps s in its binade; false otherwise
-__device__ __forceinline__ bool tr_apply(float& s, Tr t) {
-    if (s < 1024.0f) return false;
-    const unsigned int bits = __float_as_uint(s);
-    const unsigned long long m = (unsigned long long)((bits & 0x7fffffu) | 0x800000u);
-    const unsigned long long m2 = m + ((m & 1ull) ? t.d1 : t.d0);
-    if (m2 + 1ull >= (1ull << 24)) return false;
-    s = __uint_as_float((bits & 0xff800000u) | ((unsigned int)m2 & 0x7fffffu));
-    return true;
+// the transfers of a window of 32 chunks, one warp each, for three binades from its first chunk's on
+__global__ void __launch_bounds__(256) pbas_k_sum_win(LobDev D, SumWork W, int nChunks) {
+    pdl_entry();
+    if (!ld_vol(&D.flags[LOB_F_CONV])) return;
+    const int w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, c = 32 * w + lane;
+    if (32 * w >= nChunks) return;
+    const bool in = c < nChunks;
+    const int eb = in ? W.eb[c] : 0, e0 = __shfl_sync(0xffffffffu, eb, 0);
+    Tr t[kSumNB];
+#pragma unroll
+    for (int i = 0; i < kSumNB; ++i) t[i] = in ? W.tr[(size_t)c * kSumNB + i] : Tr{0u, 0u};
+    int have = 0;
+#pragma unroll
+    for (int j = 0; j < kSumNB; ++j) {
+        const int k = e0 + j - eb;
+        Tr a = {0u, 0u};
+#pragma unroll
+        for (int i = 0; i < kSumNB; ++i)
+            if (in && k == i) a = t[i];
+        if (__all_sync(0xffffffffu, !in || (k >= 0 && k < kSumNB))) have |= 1 << j;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            Tr y;
+            y.d0 = __shfl_down_sync(0xffffffffu, a.d0, o);
+            y.d1 = __shfl_down_sync(0xffffffffu, a.d1, o);
+            if ((lane & (2 * o - 1)) == 0) a = tr_then(a, y);
+        }
+        if (lane == 0) W.win[(size_t)w * kSumNB + j] = a;
+    }
+    if (lane == 0) W.winEb[w] = (e0 << 3) | have;
 }
 
-// the walk over the chunks (one warp; every lane holds the same sum), then the mean and its floor of 20:
-// 32 chunks at once when all of them have transfers for the binade of s (their ordered composition),
-// else chunk by chunk, else 32-pixel granule by granule, else value by value
+// Advances s over the elements pos .. cnt - 1 of a warp's 32 (element l on lane l: transfers t for the binades eb,
+// eb + 1, eb + 2 as far as `have` says), as far as transfers for the binade of s exist and keep s in it: an
+// inclusive scan composes them, and a ballot finds how many fit. Returns the element it stopped at.
+__device__ int tr_run(float& s, const Tr (&t)[kSumNB], int eb, int have, int cnt, int pos) {
+    const int lane = threadIdx.x & 31;
+    while (pos < cnt && s >= 1024.0f) {
+        const int k = binade(s) - eb;
+        const bool usable = lane >= pos && lane < cnt && k >= 0 && k < kSumNB && ((have >> k) & 1);
+        const unsigned m = __ballot_sync(0xffffffffu, usable) >> pos;
+        const int run = ~m ? __ffs(~m) - 1 : 32;
+        if (run == 0) break;
+        Tr a = {0u, 0u};
+#pragma unroll
+        for (int i = 0; i < kSumNB; ++i)
+            if (lane >= pos && lane < pos + run && k == i) a = t[i];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            Tr y;
+            y.d0 = __shfl_up_sync(0xffffffffu, a.d0, o);
+            y.d1 = __shfl_up_sync(0xffffffffu, a.d1, o);
+            if (lane >= o) a = tr_then(y, a);
+        }
+        float mine = s;
+        const bool fits = lane >= pos && lane < pos + run && tr_apply(mine, a);
+        const unsigned f = __ballot_sync(0xffffffffu, fits) >> pos;  // the increments grow: a prefix fits
+        const int n = ~f ? __ffs(~f) - 1 : 32;
+        if (n == 0) break;
+        s = __shfl_sync(0xffffffffu, mine, pos + n - 1);
+        pos += n;
+        if (n < run) break;
+    }
+    return pos;
+}
+
+// the walk (one warp; every lane holds the same sum), then the mean and its floor of 20
 __global__ void __launch_bounds__(32) pbas_k_sum_walk(LobDev D, SumWork W, int nChunks) {
+    pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
     __shared__ float vals[32 * 64];
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x, nWin = (nChunks + 31) / 32;
     float s = 0.0f;
-    for (int c0 = 0; c0 < nChunks; c0 += 32) {
-        // the window's transfers, one chunk per lane
+    Tr tn[kSumNB];
+    int en = 0;
+    auto fetch = [&](int w) {
+        en = w < nWin ? W.winEb[w] : 0;
+#pragma unroll
+        for (int i = 0; i < kSumNB; ++i) tn[i] = w < nWin ? W.win[(size_t)w * kSumNB + i] : Tr{0u, 0u};
+    };
+    fetch(lane);
+    for (int w0 = 0; w0 < nWin; w0 += 32) {
         Tr tw[kSumNB];
-        int ew = 0;
-        const bool in = c0 + lane < nChunks;
 #pragma unroll
-        for (int i = 0; i < kSumNB; ++i) tw[i].d0 = tw[i].d1 = 0ull;
-        if (in) {
+        for (int i = 0; i < kSumNB; ++i) tw[i] = tn[i];
+        const int ew = en, wcnt = min(32, nWin - w0);
+        fetch(w0 + 32 + lane);  // the next 32 windows while these are walked
+        for (int wp = 0; wp < wcnt; ++wp) {
+            wp = tr_run(s, tw, ew >> 3, ew & 7, wcnt, wp);
+            if (wp >= wcnt) break;
+            // window wp chunk by chunk
+            const int c0 = 32 * (w0 + wp), c = c0 + lane, ccnt = min(32, nChunks - c0);
+            Tr tc[kSumNB];
+            const int ec = c < nChunks ? W.eb[c] : 0;
 #pragma unroll
-            for (int i = 0; i < kSumNB; ++i) tw[i] = W.tr[(size_t)(c0 + lane) * kSumNB + i];
-            ew = W.eb[c0 + lane];
-        }
-        {
-            const int k = binade(s) - ew;
-            Tr t;
-            t.d0 = t.d1 = 0ull;
+            for (int i = 0; i < kSumNB; ++i) tc[i] = c < nChunks ? W.tr[(size_t)c * kSumNB + i] : Tr{0u, 0u};
+            for (int cp = 0; cp < ccnt; ++cp) {
+                cp = tr_run(s, tc, ec, 7, ccnt, cp);
+                if (cp >= ccnt) break;
+                // chunk cp granule by granule
+                const int chunk = c0 + cp, eg = __shfl_sync(0xffffffffu, ec, cp);
+                const int pEnd = min((chunk + 1) * kSumChunk, D.npx);
+                const int gcnt = (pEnd - chunk * kSumChunk + 31) / 32;
+                Tr tg[kSumNB];
 #pragma unroll
-            for (int i = 0; i < kSumNB; ++i)
-                if (k == i) t = tw[i];
-            if (__all_sync(0xffffffffu, !in || (k >= 0 && k < kSumNB))) {
-                for (int o = 1; o < 32; o <<= 1) {
-                    const Tr y = tr_shfl_down(t, o);
-                    if ((lane & (2 * o - 1)) == 0) t = tr_then(t, y);
+                for (int i = 0; i < kSumNB; ++i)
+                    tg[i] = lane < gcnt ? W.trw[((size_t)chunk * kSumGran + lane) * kSumNB + i] : Tr{0u, 0u};
+                for (int g = 0; g < gcnt; ++g) {
+                    g = tr_run(s, tg, eg, 7, gcnt, g);
+                    if (g >= gcnt) break;
+                    // value by value, the granule's values staged in shared memory, every lane adding them in order
+                    const int p = chunk * kSumChunk + 32 * g + lane;
+                    const int n = p < pEnd ? (int)D.badCnt[p] : 0;
+                    int off = n;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, off, o);
+                        if (lane >= o) off += y;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, off, 31);
+                    off -= n;
+#pragma unroll 8
+                    for (int q = 0; q < n; ++q) vals[off + q] = bad_dist(D, q, p);
+                    __syncwarp();
+                    for (int q = 0; q < total; ++q) s += vals[q];
+                    __syncwarp();
                 }
-                Tr tot;
-                tot.d0 = __shfl_sync(0xffffffffu, t.d0, 0);
-                tot.d1 = __shfl_sync(0xffffffffu, t.d1, 0);
-                if (tr_apply(s, tot)) continue;
-            }
-        }
-        for (int j = 0; j < 32 && c0 + j < nChunks; ++j) {
-            const int c = c0 + j;
-            const int eb = __shfl_sync(0xffffffffu, ew, j);
-            int k = binade(s) - eb;
-            Tr tc;
-            tc.d0 = tc.d1 = 0ull;
-#pragma unroll
-            for (int i = 0; i < kSumNB; ++i) {
-                const unsigned long long a = __shfl_sync(0xffffffffu, tw[i].d0, j);
-                const unsigned long long b = __shfl_sync(0xffffffffu, tw[i].d1, j);
-                if (k == i) {
-                    tc.d0 = a;
-                    tc.d1 = b;
-                }
-            }
-            if (k >= 0 && k < kSumNB && tr_apply(s, tc)) continue;
-            const int pEnd = min((c + 1) * kSumChunk, D.npx);
-            for (int g = 0; g < kSumGran; ++g) {
-                const int pg = c * kSumChunk + g * 32;
-                if (pg >= pEnd) break;
-                k = binade(s) - eb;
-                if (k >= 0 && k < kSumNB && tr_apply(s, W.trw[((size_t)c * kSumGran + g) * kSumNB + k])) continue;
-                // value by value, the granule's values staged in shared memory, every lane adding them in order
-                const int p = pg + lane;
-                const int n = p < pEnd ? (int)D.badCnt[p] : 0;
-                int off = n;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, off, o);
-                    if (lane >= o) off += y;
-                }
-                const int total = __shfl_sync(0xffffffffu, off, 31);
-                off -= n;
-                for (int q = 0; q < n; ++q) vals[off + q] = D.badVals[(size_t)p * D.N + q];
-                __syncwarp();
-                for (int q = 0; q < total; ++q) s += vals[q];
-                __syncwarp();
             }
         }
     }
@@ -1063,7 +1466,11 @@ __global__ void lob_k_background(LobDev D, void* out, int descriptors) {
             const size_t o = (size_t)s * D.npx + p;
             uint32_t v;
             if (D.alg != ALG_LOBSTER) {
-                v = D.sC[o * C + c];
+                unsigned long long d;
+                uint32_t c2;
+                if (D.alg == ALG_VIBE) load_sample<C, ALG_VIBE>(D, s, p, d, c2);
+                else load_sample<C, ALG_PBAS>(D, s, p, d, c2);
+                v = (uint32_t)(d >> (8 * c)) & 0xffu;
             } else if (descriptors) {
                 v = C == 3 ? (uint32_t)(((const unsigned long long*)D.sD)[o] >> (16 * c)) & 0xffffu
                            : ((const uint16_t*)D.sD)[o];
@@ -1080,14 +1487,22 @@ __global__ void lob_k_background(LobDev D, void* out, int descriptors) {
     }
 }
 
-// the sample planes in the reference's layout ([N][H*W*C] colours or descriptors)
+// the sample planes in the reference's layout ([N][H*W*C] colours; what 1: descriptors, 2: PBAS's gradients)
 template <int C>
-__global__ void lob_k_export_samples(LobDev D, void* out, int descriptors) {
+__global__ void lob_k_export_samples(LobDev D, void* out, int what) {
+    const int descriptors = what == 1;
     const size_t n = (size_t)D.N * D.npx * C;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t sp = i / C;
         const int c = (int)(i % C);
-        if (descriptors) {
+        if (D.alg != ALG_LOBSTER) {
+            const int smp = (int)(sp / D.npx), p = (int)(sp % D.npx);
+            unsigned long long d;
+            uint32_t c2;
+            if (D.alg == ALG_VIBE) load_sample<C, ALG_VIBE>(D, smp, p, d, c2);
+            else load_sample<C, ALG_PBAS>(D, smp, p, d, c2);
+            ((uint8_t*)out)[i] = (uint8_t)(d >> ((what == 2 ? 24 : 0) + 8 * c));
+        } else if (descriptors) {
             ((uint16_t*)out)[i] = C == 3 ? (uint16_t)(((const unsigned long long*)D.sD)[sp] >> (16 * c))
                                          : ((const uint16_t*)D.sD)[sp];
         } else {
@@ -1163,19 +1578,17 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
     };
     const size_t oRoi = take(npx), oLastColor = take(lob * npx * C), oLastFG = take(lob * npx),
                  oRawFG = take(lob * npx), oLut = take(256), oLastDesc = take(lob * npx * C * 2), oKctr = take(npx * 2),
-                 oSD = take(lob * N * npx * (C == 3 ? 8 : 2)), oSC = take(vibe ? N * npx * C : N * npx),
+                 oSD = take(lob * N * npx * (C == 3 ? 8 : 2)), oSC = take(N * npx * sample_bytes_lo(alg, C)),
                  oIntent = take(npx * 4),
                  oWD = take(npx * 8), oList0 = take(npx * 4), oList1 = take(npx * 4), oStamp = take(npx * 4),
                  oFlags = take(LOB_F_WORDS * 4), oStats = take(32), oFrame = take(npx * C), oMask = take(npx),
-                 oSG = take(pb * N * npx * C), oGrad = take(pb * npx * C), oBlur = take(pb * npx * C),
-                 oFm = take(pb * 6 * npx * 4), oMean = take(pb * 4), oBadSum = take(pb * (C == 1 ? npx * 4 : 0)),
-                 oBadCnt = take(pb * npx), oBadVals = take(pb * (C == 3 ? npx * N * 4 : 0)),
-                 oSumTr = take(pb * (C == 3 ? (npx + kSumChunk - 1) / kSumChunk *
-                                                  (sizeof(double) + (1 + kSumGran) * kSumNB * sizeof(Tr) + sizeof(int))
-                                            : 0)),
+                 oSG = take(N * npx * sample_bytes_hi(alg, C)), oGrad = take(pb * npx * C),
+                 oFm = take(pb * 6 * npx * 4), oMean = take(pb * 4), oBadSum = take(pb * npx * 4),
+                 oBadCnt = take(pb * npx), oBadVals = take(pb * (C == 3 ? npx * N * 2 : 0)),
+                 oSumTr = take(pb * (C == 3 ? SumWork::bytes((npx + kSumChunk - 1) / kSumChunk) : 0)),
                  oRawPb = take(pb * npx);
     LOB_CUDA(cudaMalloc(&L.mem, off), "model allocation");
-    if (!L.h_flags) LOB_CUDA(cudaHostAlloc((void**)&L.h_flags, LOB_F_WORDS * 4, cudaHostAllocDefault), "pinned allocation");
+    if (!L.h_flags) LOB_CUDA(cudaHostAlloc((void**)&L.h_flags, LOB_F_WORDS * 4, cudaHostAllocMapped), "pinned allocation");
     if (!L.done) LOB_CUDA(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming), "event creation");
     if (!L.meanDone) LOB_CUDA(cudaEventCreateWithFlags(&L.meanDone, cudaEventDisableTiming), "event creation");
     L.bytes = off;
@@ -1204,25 +1617,26 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
     D.kctr = (uint16_t*)(b + oKctr);
     D.sD = b + oSD;
     D.sC = b + oSC;
+    D.sG = b + oSG;
     D.intent = (uint32_t*)(b + oIntent);
     D.wD = (unsigned long long*)(b + oWD);
     D.list0 = (uint32_t*)(b + oList0);
     D.list1 = (uint32_t*)(b + oList1);
     D.stamp = (uint32_t*)(b + oStamp);
     D.flags = (unsigned int*)(b + oFlags);
+    D.hflags = L.h_flags;
     D.stats = (unsigned long long*)(b + oStats);
     L.d_frame = b + oFrame;
     L.d_mask = b + oMask;
     if (pbas) {
-        D.sG = b + oSG;
         D.grad = b + oGrad;
-        D.blur = b + oBlur;
         D.fm = (float*)(b + oFm);
         D.meanGrad = (float*)(b + oMean);
         D.badSum = (uint32_t*)(b + oBadSum);
         D.badCnt = b + oBadCnt;
-        D.badVals = (float*)(b + oBadVals);
+        D.badVals = (uint16_t*)(b + oBadVals);
         D.sumTr = b + oSumTr;
+        if (C == 3) D.chunkAbout = sum_work(D.sumTr, (npx + kSumChunk - 1) / kSumChunk).about;
         D.rawFG = b + oRawPb;
         // the constructor's arguments (BackgroundSubtractorPBAS.cpp:21-32) and medianBlur(.., 9) (:266 / :494)
         D.R0 = (float)prm.min_color_dist_threshold;
@@ -1264,45 +1678,40 @@ void launch(const LobDev& D, int blocks, cudaStream_t st, A... args) {
 }
 template <int C, int ALG>
 struct Eval {
-    static void run(int b, cudaStream_t st, const LobDev& D) { lob_k_eval<C, ALG><<<b, kThreadsL, 0, st>>>(D); }
+    static void run(int b, cudaStream_t st, const LobDev& D) { launch_chained(lob_k_eval<C, ALG>, dim3(b), dim3(kThreadsL), st, D); }
+};
+template <int C, int ALG>
+struct First {
+    static void run(int b, cudaStream_t st, const LobDev& D) { launch_chained(lob_k_first<C, ALG>, dim3(b), dim3(kThreadsL), st, D); }
 };
 template <int C, int ALG>
 struct Round {
-    static void run(int b, cudaStream_t st, const LobDev& D, int r) { lob_k_round<C, ALG><<<b, kThreadsL, 0, st>>>(D, r); }
+    static void run(int b, cudaStream_t st, const LobDev& D, int r) { launch_chained(lob_k_round<C, ALG>, dim3(b), dim3(kThreadsL), st, D, r); }
 };
 template <int C, int ALG>
 struct Commit {
-    static void run(int b, cudaStream_t st, const LobDev& D) { lob_k_commit<C, ALG><<<b, kThreadsL, 0, st>>>(D); }
+    static void run(int b, cudaStream_t st, const LobDev& D) { launch_chained(lob_k_commit<C, ALG>, dim3(b), dim3(kThreadsL), st, D); }
 };
 
 // PBAS's gradient image of a device frame into D.grad
 void pbas_gradient(const LobDev& D, const uint8_t* img, cudaStream_t st) {
-    const int nb = blocks_for((size_t)D.npx * D.C);
-    if (D.C == 3) {
-        pbas_k_blur<3><<<nb, kThreadsL, 0, st>>>(D, img);
-        pbas_k_grad<3><<<nb, kThreadsL, 0, st>>>(D);
-    } else {
-        pbas_k_blur<1><<<nb, kThreadsL, 0, st>>>(D, img);
-        pbas_k_grad<1><<<nb, kThreadsL, 0, st>>>(D);
-    }
+    const dim3 g((D.W + kGradW - 1) / kGradW, (D.H + kGradH - 1) / kGradH);
+    if (D.C == 3) pbas_k_grad<3><<<g, kThreadsL, 0, st>>>(D, img);
+    else pbas_k_grad<1><<<g, kThreadsL, 0, st>>>(D, img);
 }
 
 // PBAS's frame-level mean gradient distance, after the commit
 lvbgs_status pbas_mean_launch(const LobDev& D, int sms, cudaStream_t st, std::string& err) {
     if (D.C == 1) {
-        pbas_k_mean1<<<2 * sms, kThreadsL, 0, st>>>(D);
-        pbas_k_mean1_end<<<1, 1, 0, st>>>(D);
+        launch_chained(pbas_k_mean1, dim3(2 * sms), dim3(kThreadsL), st, D);
+        launch_chained(pbas_k_mean1_end, dim3(1), dim3(1), st, D);
     } else {
         const int nChunks = (D.npx + kSumChunk - 1) / kSumChunk;
-        SumWork W;
-        W.chunkSum = (double*)D.sumTr;
-        W.tr = (Tr*)(W.chunkSum + nChunks);
-        W.trw = W.tr + (size_t)nChunks * kSumNB;
-        W.eb = (int*)(W.trw + (size_t)nChunks * kSumGran * kSumNB);
-        pbas_k_sum_chunks<<<nChunks, kSumChunk, 0, st>>>(D, W);
-        pbas_k_sum_scan<<<1, kSumScan, 0, st>>>(D, W, nChunks);
-        pbas_k_sum_tr<<<nChunks, kSumChunk, 0, st>>>(D, W);
-        pbas_k_sum_walk<<<1, 32, 0, st>>>(D, W, nChunks);
+        const SumWork W = sum_work(D.sumTr, nChunks);
+        launch_chained(pbas_k_sum_scan, dim3(1), dim3(kSumScan), st, D, W, nChunks);
+        launch_chained(pbas_k_sum_tr, dim3(nChunks), dim3(kSumChunk), st, D, W);
+        launch_chained(pbas_k_sum_win, dim3((nChunks + 255) / 256), dim3(256), st, D, W, nChunks);
+        launch_chained(pbas_k_sum_walk, dim3(1), dim3(32), st, D, W, nChunks);
     }
     return LVBGS_OK;
 }
@@ -1384,33 +1793,26 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int roundBlocks = 2 * (sms > 0 ? sms : 1);
-    LOB_CUDA(cudaMemsetAsync(D.flags, 0, LOB_F_WORDS * 4, st), "flag reset");
-    if (D.alg == ALG_PBAS) {
-        LOB_CUDA(cudaMemsetAsync(D.stats + 2, 0, 16, st), "counter reset");
-        pbas_gradient(D, dimg, st);
-    }
+    std::memset(L.h_flags, 0, LOB_F_WORDS * 4);  // the commit writes the frame step's flags here
+    if (D.alg == ALG_PBAS) pbas_gradient(D, dimg, st);
     launch<Eval>(D, nb, st);
-    lob_k_mark<<<nb, kThreadsL, 0, st>>>(D);
+    launch<First>(D, (D.npx + kFirstPx - 1) / kFirstPx, st);
     LOB_CUDA(cudaGetLastError(), "evaluation launch");
-    int round = 0, chunk = L.lastRounds + 1;
+    int round = 1, chunk = L.lastRounds;
     for (;;) {
-        for (int i = 0; i < chunk; ++i, ++round) {
-            launch<Round>(D, roundBlocks, st, round);
-            lob_k_round_end<<<1, 1, 0, st>>>(D, round);
-        }
+        for (int i = 0; i < chunk; ++i, ++round) launch<Round>(D, roundBlocks, st, round);
         launch<Commit>(D, nb, st);
         // LOBSTER's median blur, last mask and last colour frame; PBAS's median blur (ViBe outputs its
         // raw mask)
         const dim3 mg((D.W + kMedTile - 1) / kMedTile, (D.H + kMedTile - 1) / kMedTile);
         if (D.alg == ALG_LOBSTER) {
-            if (C == 3) lob_k_median<3, true><<<mg, kThreadsL, 0, st>>>(D);
-            else lob_k_median<1, true><<<mg, kThreadsL, 0, st>>>(D);
+            if (C == 3) launch_chained(lob_k_median<3, true>, mg, dim3(kThreadsL), st, D);
+            else launch_chained(lob_k_median<1, true>, mg, dim3(kThreadsL), st, D);
         } else if (D.alg == ALG_PBAS) {
-            lob_k_median<1, false><<<mg, kThreadsL, 0, st>>>(D);
+            launch_chained(lob_k_median<1, false>, mg, dim3(kThreadsL), st, D);
         }
         LOB_CUDA(cudaGetLastError(), "repair launch");
         if (hostMask) LOB_CUDA(cudaMemcpyAsync(hostMask, dmask, (size_t)D.npx, cudaMemcpyDeviceToHost, st), "mask download");
-        LOB_CUDA(cudaMemcpyAsync(L.h_flags, D.flags, LOB_F_WORDS * 4, cudaMemcpyDeviceToHost, st), "flag read-back");
         // PBAS's frame-level mean gradient distance is only needed by the next frame step: the host does
         // not wait for it
         if (D.alg == ALG_PBAS) {
@@ -1423,16 +1825,17 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
         } else {
             LOB_CUDA(cudaStreamSynchronize(st), "frame step");
         }
-        if (L.h_flags[LOB_F_ERR]) {
+        const volatile unsigned int* hf = L.h_flags;
+        if (hf[LOB_F_ERR]) {
             err = "LOBSTER repair list overflow";
             return LVBGS_DEVICE_ERROR;
         }
-        if (L.h_flags[LOB_F_CONV]) break;
+        if (hf[LOB_F_CONV]) break;
         if (round >= kMaxRoundsL) {
             err = "LOBSTER raster-order repair did not converge";
             return LVBGS_DEVICE_ERROR;
         }
-        chunk *= 2;
+        chunk = std::max(1, chunk * 2);
     }
     L.lastRounds = (int)L.h_flags[LOB_F_ROUNDS];
     D.stampBase += (uint32_t)round + 2u;
@@ -1496,10 +1899,10 @@ lvbgs_status lob_get_map(LobState& L, int which, void* hostOut, size_t bytes, cu
     }
     const void* src = nullptr;
     const float* fm = D.fm ? D.fm + (size_t)D.cur * 3 * D.npx : nullptr;
-    if (D.alg == ALG_VIBE) src = which == LVBGS_MAP_ROI ? (const void*)D.roi : (const void*)D.sC;
+    if (D.alg == ALG_VIBE) src = which == LVBGS_MAP_ROI ? (const void*)D.roi : nullptr;
     else if (D.alg == ALG_PBAS) switch (which) {
-            case LVBGS_MAP_SAMPLE_COLOR: src = D.sC; break;
-            case LVBGS_MAP_SAMPLE_GRAD: src = D.sG; break;
+            case LVBGS_MAP_SAMPLE_COLOR:
+            case LVBGS_MAP_SAMPLE_GRAD: break;
             case LVBGS_MAP_R: src = fm; break;
             case LVBGS_MAP_T: src = fm + D.npx; break;
             case LVBGS_MAP_DMIN_LT: src = fm + 2 * (size_t)D.npx; break;
@@ -1522,7 +1925,7 @@ lvbgs_status lob_get_map(LobState& L, int which, void* hostOut, size_t bytes, cu
     }
     void* tmp = nullptr;
     LOB_CUDA(staging(&tmp, need, st), "staging allocation");
-    const int desc = which == LVBGS_MAP_SAMPLE_DESC ? 1 : 0;
+    const int desc = which == LVBGS_MAP_SAMPLE_DESC ? 1 : which == LVBGS_MAP_SAMPLE_GRAD ? 2 : 0;
     if (D.C == 3) lob_k_export_samples<3><<<1024, 256, 0, st>>>(D, tmp, desc);
     else lob_k_export_samples<1><<<1024, 256, 0, st>>>(D, tmp, desc);
     cudaError_t e = cudaGetLastError();

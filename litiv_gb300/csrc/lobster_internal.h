@@ -26,7 +26,7 @@ namespace lvbgs {
 enum { ALG_LOBSTER = 0, ALG_VIBE = 1, ALG_PBAS = 2 };
 
 // flags of one frame step (device words)
-enum { LOB_F_COUNT0 = 0, LOB_F_COUNT1, LOB_F_CONV, LOB_F_ROUNDS, LOB_F_ERR, LOB_F_WORDS = 8 };
+enum { LOB_F_COUNT0 = 0, LOB_F_COUNT1, LOB_F_CONV, LOB_F_ROUNDS, LOB_F_ERR, LOB_F_DONE, LOB_F_WORDS = 8 };
 
 // kernel parameters (by value)
 struct LobDev {
@@ -49,15 +49,18 @@ struct LobDev {
     unsigned long long* wD;
     uint32_t *list0, *list1, *stamp;
     unsigned int* flags;
+    unsigned int* hflags;  // page-locked copy of the flags, written by the commit
     unsigned long long* stats;  // samples evaluated, sample writes (cumulative); PBAS: bad samples' gradient sum, count
     // PBAS
     int cur;                // parity of the R, T, D maps the frame starts from
     int lrOverride;         // nLR is the override (otherwise ceil(T(x)) per pixel)
     float R0, updateRate;   // m_nDefaultColorDistThreshold, m_fDefaultUpdateRate
-    uint8_t *sG, *grad, *blur;
-    float *fm, *meanGrad, *badVals;
+    uint8_t *sG, *grad;
+    float *fm, *meanGrad;
+    uint16_t* badVals;  // three channels: the bad samples' squared gradient distances, [N][npx]
     uint32_t* badSum;
     uint8_t* badCnt;
+    float* chunkAbout;  // three channels: about what each chunk of the mean's sum adds (in sumTr)
     void* sumTr;  // three channels: the per-chunk transfers of the mean's exact float sum
 };
 
@@ -67,7 +70,7 @@ struct LobState {
     size_t bytes = 0;
     uint8_t* d_frame = nullptr;  // staging of host frames
     uint8_t* d_mask = nullptr;   // mask of the last frame step
-    unsigned int* h_flags = nullptr;  // pinned copy of the flags
+    unsigned int* h_flags = nullptr;  // page-locked copy of the flags (LobDev::hflags)
     cudaEvent_t done = nullptr;       // PBAS: the frame step's mask and flags are on the host
     cudaEvent_t meanDone = nullptr;   // PBAS: the frame step's mean gradient distance is written
     float pbasMean = 20.0f;           // PBAS: m_fFormerMeanGradDist across initialize() calls

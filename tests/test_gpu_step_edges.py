@@ -1,4 +1,4 @@
-"""SuBSENSE's and PAWCS's frame steps at the edges of their kernels' tiles, words and chunks, against the oracle (bit-exact)."""
+"""Every algorithm's frame step at the edges of their kernels' tiles, words and chunks, against the oracle (bit-exact)."""
 import ctypes as C
 
 import numpy as np
@@ -7,8 +7,11 @@ import pytest
 from litiv_gb300 import _lib as L
 from litiv_gb300.metrics import BinClassif
 from oracle import metrics as oracle_metrics, pyoracle
+from tests.test_gpu_lobster import run_pair as lobster_pair
 from tests.test_gpu_parity import run_pair
+from tests.test_gpu_pbas import run_pair as pbas_pair
 from tests.test_gpu_pawcs import run_pair as pawcs_pair
+from tests.test_gpu_vibe import run_pair as vibe_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -125,3 +128,21 @@ def test_lbsp_descriptors_keep_the_border(W, H, channels, where):
     if where == "device":
         out = do.cpu().numpy().view(np.uint16).reshape(H, W, channels)
     assert np.array_equal(out, want)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("W,H,N,nreq", [(96, 64, 4, 1), (97, 61, 5, 2), (65, 33, 8, 3), (64, 17, 9, 2), (130, 16, 20, 1),
+                                        (33, 47, 35, 4), (129, 79, 63, 2)])
+def test_sample_scans_of_the_consensus_models(W, H, N, nreq, channels):
+    """LOBSTER, ViBe and PBAS with sample counts around the lane scans' caps and the groups' steps of eight, frames
+    of ragged gradient tiles and sum chunks, few repairs a block (one a group) and, at learning rate 1, most of a
+    block's pixels (every lane its own)."""
+    frames = hollow_frames(W, H, channels, 8, W * 7 + N)
+    rng = np.random.default_rng(N)
+    frames[5] = rng.integers(0, 256, frames[5].shape, dtype=np.uint8)
+    lrs = [16.0, 1.0, 1.0, 2.0, 16.0, 1.0, 1.0, 3.0]
+    args = dict(nBGSamples=N, nRequiredBGSamples=nreq)
+    lobster_pair(frames, seed=N, lrs=lrs, **args)
+    vibe_pair(frames, N + 1, lrs, **args)
+    pbas_pair(frames, N + 2, lrs, **args)
+    pbas_pair(frames, N + 3, [-1.0] * len(frames), **args)
