@@ -254,7 +254,7 @@ struct Layout {
     size_t persist, total;
 };
 enum {
-    L_CTL = 0, L_FM, L_UNST, L_LASTCOL, L_LASTDESC, L_SD, L_SC, L_ROI, L_BLINKS, L_LASTRAWFG, L_LASTFG, L_DILINV,
+    L_CTL = 0, L_FM, L_UNST, L_LASTCOL, L_LASTDESC, L_SAMPLES, L_ROI, L_BLINKS, L_LASTRAWFG, L_LASTFG, L_DILINV,
     L_LASTRAWBLINK, L_KCTR, L_DSLT, L_DSST,
     // scratch (not spilled)
     L_STAMPD, L_STAMPR, L_GOODREC, L_BITS, L_LABEL, L_INTENT, L_FRAME, L_MASK, L_COUNT
@@ -268,8 +268,7 @@ Layout make_layout(int W, int H, int C, size_t N) {
     sz[L_UNST] = 2 * npx;
     sz[L_LASTCOL] = 2 * npx * C;
     sz[L_LASTDESC] = 2 * npx * C * 2;
-    sz[L_SD] = N * npx * (C == 3 ? 8 : 2);
-    sz[L_SC] = N * npx;
+    sz[L_SAMPLES] = N * sample_stride(npx, C);
     sz[L_ROI] = sz[L_BLINKS] = sz[L_LASTRAWFG] = sz[L_LASTFG] = sz[L_DILINV] = sz[L_LASTRAWBLINK] = npx;
     sz[L_KCTR] = npx * 2;
     sz[L_DSLT] = sz[L_DSST] = std::max<size_t>(nds, 1) * 4;
@@ -298,8 +297,8 @@ void fill_pointers(lvbgs_ctx* h, const Layout& L) {
     S.unst = b + L.off[L_UNST];
     S.lastCol = b + L.off[L_LASTCOL];
     S.lastDesc = (uint16_t*)(b + L.off[L_LASTDESC]);
-    S.sD = b + L.off[L_SD];
-    S.sC = b + L.off[L_SC];
+    S.samples = b + L.off[L_SAMPLES];
+    S.sStride = sample_stride(h->npx, h->C);
     S.roi = b + L.off[L_ROI];
     S.blinks = b + L.off[L_BLINKS];
     S.lastRawFG = b + L.off[L_LASTRAWFG];

@@ -6,10 +6,10 @@
 //                    (BackgroundSubtractorSuBSENSE.hpp:100-115)
 //   unst[2][npx]     unstable-region flags (double-buffered)
 //   lastCol[2][npx*C], lastDesc[2][npx*C]   last colour / LBSP descriptor frames
-//   sD[N][npx]       sample descriptors: for C=3 one uint64 = desc0|desc1<<16|desc2<<32|B<<48|G<<56,
-//                    for C=1 one uint16 descriptor
-//   sC[N][npx]       sample colour byte: R for C=3, the intensity for C=1
-//   (so one sample costs exactly 3*C bytes, the algorithmic minimum)
+//   samples[N][ceil(npx / kSecPx)][32 bytes]   samples, kSecPx pixels to a 32-byte sector: C=3, 3 x uint64
+//                    desc0|desc1<<16|desc2<<32|B<<48|G<<56, 3 x R and 5 spare bytes; C=1, 10 x uint16
+//                    descriptor, 10 x intensity and 2 spare bytes. A write, at a random sample of a pixel, is one
+//                    sector of DRAM and not two.
 //   u8 maps: roi, blinks, last raw mask, last final mask, inverted dilated mask, last raw blinks,
 //   plus per-frame scratch (closed mask, combined mask, union-find labels, intents, draw counters).
 #pragma once
@@ -35,6 +35,9 @@ constexpr int kTileH = 8;
 constexpr int kThreads = kTileW * kTileH;
 constexpr int kBorder = 2;  // LBSP::PATCH_SIZE/2
 constexpr int kMaxSamples = 64;
+template <int C>
+constexpr unsigned kSecPx = C == 3 ? 3u : 10u;  // pixels per sector of samples
+inline size_t sample_stride(size_t npx, int C) { return (npx + (C == 3 ? 2 : 9)) / (C == 3 ? 3 : 10) * 32; }
 constexpr int kNumFloatMaps = 10;
 enum FloatMap { FM_R = 0, FM_V, FM_T, FM_DLAST, FM_DMIN_LT, FM_DMIN_ST, FM_RAW_LT, FM_RAW_ST, FM_FIN_LT, FM_FIN_ST };
 constexpr unsigned kPhilox0 = 0xD2511F53u, kPhilox1 = 0xCD9E8D57u, kWeyl0 = 0x9E3779B9u, kWeyl1 = 0xBB67AE85u;
@@ -146,8 +149,8 @@ struct StreamDev {
     uint8_t* unst;
     uint8_t* lastCol;
     uint16_t* lastDesc;
-    void* sD;
-    uint8_t* sC;
+    uint8_t* samples;
+    size_t sStride;  // bytes from a sample of a pixel to its next one
     uint8_t* roi;
     uint8_t *blinks, *lastRawFG, *lastFG, *dilInv, *lastRawBlink;
     uint32_t* bits;   // mask bit planes (BP_*): rowWords words per row, bit b of word w = pixel 32w + b
