@@ -1797,6 +1797,24 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams 
         sm.dil[dr][dw] = v;
     }
     __syncthreads();
+    if (S.maskOut && y < H) {
+        // The mask bytes of the tile row as aligned words, whatever the frame's width and the buffer's address (32 or
+        // 33 of them, the row's first and last in bytes): single bytes cost a transaction each when the mask
+        // is in host memory, 12 mixed streams with two frames of 1279x719 82 to 157 us.
+        uint8_t* out = S.maskOut + (size_t)y * W + w0 * 32;
+        const int len = min(32 * kFinWords, W - w0 * 32), off = (int)((uintptr_t)out & 3);
+        for (int i = quad; 4 * i - off < len; i += 32) {
+            const int b = 4 * i - off;  // the word's first byte, from -3 on
+            const uint32_t* f = &sm.fg[row + 3][1 + (b >> 5)];
+            const uint32_t bits = __funnelshift_r(f[0], f[1], b & 31) & 15u;
+            const uint32_t v = ((bits * 0x00204081u) & 0x01010101u) * 255u;
+            if (b >= 0 && b + 4 <= len) {
+                *(uint32_t*)(out + b) = v;
+            } else {
+                for (int j = max(0, -b); j < 4 && b + j < len; ++j) out[b + j] = (uint8_t)(v >> (8 * j));
+            }
+        }
+    }
     if (n <= 0) return;
     const uint32_t fg4 = (sm.fg[row + 3][1 + (quad >> 3)] >> ((quad & 7) * 4)) & 15u;
     const uint32_t dl4 = (sm.dil[row][quad >> 3] >> ((quad & 7) * 4)) & 15u;
@@ -1828,15 +1846,6 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams 
                 S.blinks[q + i] = (uint8_t)(nb >> (8 * i));
                 S.dilInv[q + i] = (uint8_t)(inv >> (8 * i));
             }
-    }
-    if (S.maskOut) {
-        if (vec && ((uintptr_t)S.maskOut & 3) == 0) {
-            *(uint32_t*)(S.maskOut + q) = fgb;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (i < n) S.maskOut[q + i] = (uint8_t)(fgb >> (8 * i));
-        }
     }
 }
 
