@@ -536,8 +536,8 @@ def main():
         dev_frames.append(buf)
     torch.cuda.synchronize()
     px_step = sum(s.cfg.width * s.cfg.height for s in synth)
-    # groups the library splits each tick into (lvbgs_batch_apply: >= 8 streams, >= 4 Mi px, >= 4 per group)
-    groups = min(args.batch_groups, n // 4) if n >= 8 and px_step >= (4 << 20) else 1
+    # groups the library splits each tick into (lvbgs_batch_apply: >= 8 streams, >= 3 Mi px, >= 4 per group)
+    groups = min(args.batch_groups, n // 4) if n >= 8 and px_step >= (3 << 20) else 1
     if lib.lvbgs_set_batch_groups(args.batch_groups) != 0:
         raise SystemExit("--batch-groups must be 1..4")
     # a dedicated stream: the library launches on it and the CUDA events are recorded on it (a NULL

@@ -109,7 +109,7 @@ lvbgs_status lvbgs_apply(lvbgs_handle h, const uint8_t* image, size_t stride, ui
  * lvbgs_batch_wait() waits and reports the SuBSENSE part's device errors. Host buffers referenced
  * by `frames` must stay valid until the wait returns. No reference counterpart (the reference runs
  * one subtractor per sequence). */
-/* How lvbgs_batch_apply runs large batches (>= 8 streams and >= 4 Mi pixels): G in 2..4 (default 4)
+/* How lvbgs_batch_apply runs large batches (>= 8 streams and >= 3 Mi pixels): G in 2..4 (default 4)
  * splits them into up to G groups of about equal pixels (at least 4 streams each), run on the
  * caller's stream and on further streams of the first handle (forked and joined with events), so
  * that one group's latency-bound phases overlap the others' work; 1 runs every batch as one group
