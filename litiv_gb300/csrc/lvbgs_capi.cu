@@ -71,12 +71,14 @@ extern "C" __global__ void pw_k_init(PawcsDev S);
 extern "C" __global__ void pw_k_init_last(PawcsDev S, const uint8_t* img);
 extern "C" __global__ void pw_k_background(PawcsDev S, int buf, uint8_t* outCol, uint16_t* outDesc, int ahead);
 // PAWCS, three channels (pawcs3_kernels.cu)
+extern "C" __global__ void pw3_k_local_first(PwParams P);
 extern "C" __global__ void pw3_k_local(PwParams P);
 extern "C" __global__ void pw3_k_gscan_seg(PwParams P);
 extern "C" __global__ void pw3_k_gscan_walk(PwParams P);
 extern "C" __global__ void pw3_k_gscan_fix(PwParams P);
 extern "C" __global__ void pw3_k_gscan_fix_walked(PwParams P);
 extern "C" __global__ void pw3_k_dirty(PwParams P);
+extern "C" __global__ void pw3_k_later_list(PwParams P);
 extern "C" __global__ void pw3_k_later(PwParams P);
 extern "C" __global__ void pw3_k_commit(PwParams P);
 extern "C" __global__ void pw3_k_ds(PwParams P);
@@ -632,7 +634,7 @@ PwLayout pw_layout(int W, int H, int C, int L, int G) {
     sz[PL_FLAGS] = 64;
     sz[PL_PDEV] = sizeof(PawcsDev);
     sz[PL_SDEV] = sizeof(StreamDev);
-    sz[PL_DIRTY] = npx;
+    sz[PL_DIRTY] = C == 3 ? npx * 4 : 4;
     sz[PL_GSEG] = pw_gseg_max(npx, C) * kPwGsegWords * 4;
     sz[PL_GCAND] = npx * 4;
     sz[PL_GTRUE] = npx;
@@ -738,7 +740,7 @@ void pw_fill(lvbgs_ctx* h, const PwLayout& Lo, int L, int G) {
     D.contrib = (float*)(b + Lo.off[PL_CONTRIB]);
     D.dsRoi = b + Lo.off[PL_DSROI];
     D.dsFrame = b + Lo.off[PL_DSFRAME];
-    D.dirty = b + Lo.off[PL_DIRTY];
+    D.dirty = (uint32_t*)(b + Lo.off[PL_DIRTY]);
     D.gseg = (uint32_t*)(b + Lo.off[PL_GSEG]);
     D.gcand = (uint32_t*)(b + Lo.off[PL_GCAND]);
     D.gtrue = b + Lo.off[PL_GTRUE];
@@ -936,7 +938,7 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
         w.PR.round = w.enq;
         const PwParams& P = w.PR;
         // three channels: the local pass applies the earlier updaters' loops itself
-        launch_chained(c3 ? pw3_k_local : pw_k_local, tiles, blk, st, P);
+        launch_chained(!c3 ? pw_k_local : P.round == 0 ? pw3_k_local_first : pw3_k_local, tiles, blk, st, P);
         launch_chained(pw_k_illum, dim3((h->H + 7) / 8), blk, st, P);
         launch_chained(pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 0);
         launch_chained(pw3_k_gscan_seg, gseg, warps4, st, P);
@@ -982,7 +984,10 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
     const dim3 blk(kThreads), tiles(h->sd.nTiles);
     const dim3 cblocks((unsigned)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk));
     const bool c3 = h->C == 3;
-    if (c3) launch_chained(pw3_k_later, tiles, blk, st, P);
+    if (c3) {
+        launch_chained(pw3_k_later_list, tiles, blk, st, P);
+        launch_chained(pw3_k_later, tiles, blk, st, P);
+    }
     launch_chained(c3 ? pw3_k_commit : pw_k_commit, tiles, blk, st, P);
     launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 1);
     launch_chained(pw_k_compact_count, cblocks, blk, st, P);

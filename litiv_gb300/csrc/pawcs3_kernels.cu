@@ -156,15 +156,31 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // read, edited by the updaters' loops, matched, and written one slot later (the scan's bubble pass holds
 // back one word, the lightest so far), so a pixel needs no copy of its 50 words. The copy took 1.2 KB of
 // local memory a pixel, three times what the L1 caches hold, and a word nine accesses.
+// From round 1 on the pixels come from the list of the dirty pass: a lane's chain of 50 words with its updaters' loops
+// holds its warp, however few of the warp's lanes are dirty. Rounds 0 to 4 of a 640x480 frame took 205, 355, 300, 87
+// and 61 us by tiles and take 199, 342, 212, 86 and 59 us (a full warp of listed pixels whatever their number:
+// 214, 321, 236, 233, 108). Bound by DRAM's sectors: 860 MB in round 1, half of them for words beside the listed ones.
 // ------------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
+constexpr unsigned kPwLocalWarps = 152u * 3u * 8u;  // resident at once: three blocks on each of 152 SMs
+template <bool FIRST>
+__device__ __forceinline__ void pw3_local(const PwParams& P) {
     PW_ROUND_GUARD(P);
-    PW3_PIXEL_PROLOGUE
-    if (x >= D.W || y >= D.H) return;
+    const PawcsDev& S = P.streams[0];
+    const StreamDev& D = S.sd;
+    int x, y;
+    if (FIRST) {
+        x = ((int)blockIdx.x % D.tilesX) * kTileW + (int)threadIdx.x % kTileW;
+        y = ((int)blockIdx.x / D.tilesX) * kTileH + (int)threadIdx.x / kTileW;
+        if (x >= D.W || y >= D.H) return;
+    } else {
+        const int i = pw_list_index(P.flags[PWF_NDIRTY], kPwLocalWarps);
+        if (i < 0) return;
+        y = (int)S.dirty[i] / D.W;
+        x = (int)S.dirty[i] - y * D.W;
+    }
     const int q = y * D.W + x;
     const uint8_t roi = D.roi[q];
     if (!roi) return;
-    if (P.round > 0 && !S.dirty[q]) return;
     const StreamCtl* ctl = D.ctl;
     const PawcsCtl* pc = S.pc;
     const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
@@ -176,9 +192,9 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
     size_t src = pw_slot(S, cur, 0, q), dst = pw_slot(S, nxt, 0, q);
     Pw3Raw next = pw3_fetch(S, src);
     // earlier updaters (from the previous round's outcomes; none known in round 0)
-    Pw3Loop up[12];
+    Pw3Loop up[FIRST ? 1 : 12];
     int nu = 0;
-    if (P.round > 0) {
+    if (!FIRST) {
         uint32_t lq01, lq2;
         pw3_desc(D.lastDesc, q, lq01, lq2);
         uint32_t tq[12];
@@ -237,7 +253,8 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
             src += npx;
             next = pw3_fetch(S, src);
         }
-        for (int j = 0; j < nu; ++j) pw3_loop_word(w, up[j], i == L - 1, boot, D.seed, t, off, 0);
+        if (!FIRST)
+            for (int j = 0; j < nu; ++j) pw3_loop_word(w, up[j], i == L - 1, boot, D.seed, t, off, 0);
         const float cw = pw3_weight(w, t, off);
         if (i == 0) thrW = cw / (Rr * 2.0f);
         unsigned marks = 0;
@@ -300,7 +317,8 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
     }
     m0 |= (unsigned long long)(heldMarks & 1u) << (L - 1);
     m1 |= (unsigned long long)(heldMarks >> 1) << (L - 1);
-    for (int j = 0; j < nu; ++j) S.out[up[j].u.p].kEnd = (uint16_t)up[j].k;
+    if (!FIRST)
+        for (int j = 0; j < nu; ++j) S.out[up[j].u.p].kEnd = (uint16_t)up[j].k;
     const int bg = sumW >= thrW || border;
     const float initW = 1.0f / (float)off;
     uint8_t flags = (uint8_t)((bg ? kRfBG : 0) | (flat ? kRfFlat : 0) | (border ? kRfBorder : 0) |
@@ -345,6 +363,10 @@ extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) {
     R.bits = (uint8_t)bits;
     pw3_item_pixel(S, q, R, col);
 }
+
+// round 0 (every pixel, no updaters yet), the later rounds (the dirty pixels)
+extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local_first(PwParams P) { pw3_local<true>(P); }
+extern "C" __global__ void __launch_bounds__(256, 3) pw3_k_local(PwParams P) { pw3_local<false>(P); }
 
 // ------------------------------------------------------------------------------------------
 // global items (:1127-1150): as pw_item_pixel with the three-channel match (descriptor bits, then the
@@ -764,8 +786,8 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
     PW_ROUND_GUARD(P);
     PW3_PIXEL_PROLOGUE
     bool dirty = false;
+    const int q = y * D.W + x;
     if (x < D.W && y < D.H) {
-        const int q = y * D.W + x;
         if (D.roi[q]) {
             // the changed flags of the window first; the targets only where one is set
             bool chg[12];
@@ -780,10 +802,9 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
                     const PwOut O = S.out[(y + j / 5 - 2) * D.W + x + j % 5 - 2];
                     dirty = dirty || O.q == (uint32_t)q || O.qPrev == (uint32_t)q;
                 }
-            S.dirty[q] = dirty ? 1 : 0;
         }
     }
-    pw_round_end(P, dirty);
+    pw_round_end(P, dirty, S.dirty, q);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -791,22 +812,42 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_dirty(PwParams P) {
 // later updaters (the pixel itself first, when its clamped neighbour position falls back onto it)
 // in raster order, on the scanned dictionary; each loop's final draw count goes to its updater
 // ------------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
+// The pixels that have any, listed for the same reason: 219 us by tiles, 9 + 159 us (640x480). The round's list is free
+// by now, its count zero.
+__device__ __forceinline__ unsigned long long pw3_marks(const PawcsDev& S, int q) {
+    const PwRec R = S.rec[q];
+    return (S.uFinal[q] & 2) ? (((unsigned long long)R.m1hi << 32) | R.m1) : (((unsigned long long)R.m0hi << 32) | R.m0);
+}
+extern "C" __global__ void __launch_bounds__(256) pw3_k_later_list(PwParams P) {
     PW_TAIL_GATE(P);
     PW3_PIXEL_PROLOGUE
-    if (x >= D.W || y >= D.H) return;
     const int q = y * D.W + x;
-    if (!D.roi[q]) return;
+    bool any = false;
+    if (x < D.W && y < D.H && D.roi[q]) {
+        any = pw3_marks(S, q) != 0ull;
+#pragma unroll
+        for (int j = 12; j < 25; ++j) {
+            const int px = x + j % 5 - 2, py = y + j / 5 - 2;
+            any |= px >= 0 && px < D.W && py < D.H && S.out[py * D.W + px].q == (uint32_t)q;
+        }
+    }
+    pw_list_append(S.dirty, &P.flags[PWF_NDIRTY], any, q);
+}
+constexpr unsigned kPwLaterWarps = 152u * 4u * 8u;
+extern "C" __global__ void __launch_bounds__(256, 4) pw3_k_later(PwParams P) {
+    PW_TAIL_GATE(P);
+    const PawcsDev& S = P.streams[0];
+    const StreamDev& D = S.sd;
+    const int li = pw_list_index(P.flags[PWF_NDIRTY], kPwLaterWarps);
+    if (li < 0) return;
+    const int q = (int)S.dirty[li], y = q / D.W, x = q - y * D.W;
     const StreamCtl* ctl = D.ctl;
     const uint32_t t = (uint32_t)(ctl->frame_idx + 1ull);
     const int cur = (int)(ctl->frame_idx & 1ull), nxt = cur ^ 1;
     const int boot = t <= (uint32_t)kBootWin;
     const unsigned long long off = S.pc->lword_offset;
     const int L = S.L;
-    const PwRec R = S.rec[q];
-    const uint8_t u = S.uFinal[q];
-    const unsigned long long m = (u & 2) ? (((unsigned long long)R.m1hi << 32) | R.m1)
-                                         : (((unsigned long long)R.m0hi << 32) | R.m0);
+    const unsigned long long m = pw3_marks(S, q);
     // later updaters: the pixel itself and the twelve later pixels of its window
     bool any = false;
     uint32_t tq[13];
@@ -816,7 +857,6 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later(PwParams P) {
         tq[j - 12] = (px >= 0 && px < D.W && py < D.H) ? S.out[py * D.W + px].q : kPwNone;
         any |= tq[j - 12] == (uint32_t)q;
     }
-    if (!m && !any) return;
     const uint32_t col = pw3_color(D.frame, q);
     uint32_t d01, d2;
     pw3_desc(S.descT, q, d01, d2);

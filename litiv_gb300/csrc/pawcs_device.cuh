@@ -41,7 +41,8 @@ __device__ __forceinline__ int pw_stream_by_row(const PwParams& P, int r) {
 __device__ __forceinline__ uint32_t pw_draw(unsigned long long seed, uint32_t f, uint32_t px, uint32_t k) {
     uint32_t c[4] = {k >> 2, px, f, 0u};
     philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-    return c[k & 3u] & 0x7fffffffu;
+    const uint32_t lo = (k & 1u) ? c[1] : c[0], hi = (k & 1u) ? c[3] : c[2];  // registers, not an indexed array
+    return ((k & 2u) ? hi : lo) & 0x7fffffffu;
 }
 // draw % m for the reference's size_t moduli (rand() < 2^31, so a modulus above 2^32 leaves it as is)
 __device__ __forceinline__ uint32_t pw_mod(uint32_t r, unsigned long long m) {
@@ -160,17 +161,55 @@ __device__ __forceinline__ void pw3_store(const PawcsDev& S, int buf, int j, int
     pw3_put(S, pw_slot(S, buf, j, p), w);
 }
 
+// Appends the pixels q of a block of 256 threads (every thread calls it) to a list, one atomic a block.
+__device__ __forceinline__ void pw_list_append(uint32_t* list, unsigned int* count, bool want, int q) {
+    __shared__ unsigned int off[8], base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (lane == 0) off[warp] = (unsigned)__popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned int all = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned int c = off[i];
+            off[i] = all;
+            all += c;
+        }
+        base = all ? atomicAdd(count, all) : 0u;
+    }
+    __syncthreads();
+    if (want) list[base + off[warp] + (unsigned)__popc(m & ((1u << lane) - 1u))] = (uint32_t)q;
+}
+// The place of a thread in a list of n pixels: as few pixels a warp as fill the machine (warps: resident at once),
+// because the updaters' loops diverge and a warp serves its lanes' paths one after the other; -1: none.
+__device__ __forceinline__ int pw_list_index(unsigned int n, unsigned int warps) {
+    warps = min(warps, gridDim.x * (blockDim.x / 32u));  // the grid has a thread for every pixel, so 32 a warp serve all
+    const unsigned int k = min(32u, (n + warps - 1u) / warps), lane = threadIdx.x & 31u;
+    const unsigned int i = (blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * k + lane;
+    return lane < k && i < n ? (int)i : -1;
+}
+
 // End of a fixed-point round, called by every thread of the dirty pass: counts the pixels to rerun; the block
 // that finishes last closes the round. No dirty pixel means the fixed point is reached: its round count and
 // flag are set, here for the rounds and the tail enqueued after this one, and in host memory.
-__device__ __forceinline__ void pw_round_end(const PwParams& P, bool dirty) {
-    const int any = __syncthreads_count(dirty);
-    if (threadIdx.x != 0) return;
-    if (any) atomicAdd(&P.flags[PWF_DIRTY], (unsigned)any);
+// list: the dirty pixels (q), any order, their count in PWF_NDIRTY; null: not listed.
+__device__ __forceinline__ void pw_round_end(const PwParams& P, bool dirty, uint32_t* list = nullptr, int q = 0) {
+    if (list) {
+        pw_list_append(list, &P.flags[PWF_DIRTY], dirty, q);
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+    } else {
+        const int any = __syncthreads_count(dirty);
+        if (threadIdx.x != 0) return;
+        if (any) atomicAdd(&P.flags[PWF_DIRTY], (unsigned)any);
+    }
     __threadfence();
     if (atomicAdd(&P.flags[PWF_DONE], 1u) != gridDim.x - 1u) return;
     P.flags[PWF_DONE] = 0u;
-    if (atomicExch(&P.flags[PWF_DIRTY], 0u) == 0u) {
+    const unsigned int total = atomicExch(&P.flags[PWF_DIRTY], 0u);
+    P.flags[PWF_NDIRTY] = total;
+    if (total == 0u) {
         P.flags[PWF_ROUNDS] = (unsigned)P.round + 1u;
         P.hflags[PWF_ROUNDS] = (unsigned)P.round + 1u;
         P.hflags[PWF_CONV] = 1u;

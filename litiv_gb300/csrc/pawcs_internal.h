@@ -155,7 +155,7 @@ struct PawcsDev {
     uint32_t* catInfo;         // [0..16] category totals, [32..48] category bases
     float* dsAbs;              // |LT - ST| per down-sampled pixel (0 outside the down-sampled ROI)
     uint32_t* updList;         // pixels that update a neighbour this round, raster order
-    uint8_t* dirty;            // three channels: pixels whose local pass reruns next round
+    uint32_t* dirty;           // three channels: list of the pixels whose local pass reruns next round
     uint32_t* gseg;            // global-word scan: per-segment state (pawcs3_kernels.cu)
     uint32_t* gcand;           // global-word scan: candidate items, listed per segment
     uint8_t* gtrue;            // global-word scan: walked candidates that replace the word
@@ -205,6 +205,6 @@ struct PwParams {
 // flags: dirty pixels of the round; camera-motion switch and the new weight offset; fixed point reached and
 // its round count; blocks of the dirty pass that are done; status (host: error flags of the finished frame);
 // automatic model reset pending (host: the frame waits for it)
-enum { PWF_DIRTY = 0, PWF_MOTION, PWF_OFFSET, PWF_CONV, PWF_ROUNDS, PWF_DONE, PWF_STATUS, PWF_RESET, PWF_CLOSED, PWF_COUNT };
+enum { PWF_DIRTY = 0, PWF_MOTION, PWF_OFFSET, PWF_CONV, PWF_ROUNDS, PWF_DONE, PWF_STATUS, PWF_RESET, PWF_CLOSED, PWF_NDIRTY, PWF_COUNT };
 
 }  // namespace lvbgs
