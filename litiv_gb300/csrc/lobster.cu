@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "bitslice.cuh"
 #include "lbsp_device.cuh"
 #include "lobster_internal.h"
 #include "staging.h"
@@ -759,6 +760,7 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
     if (!conv) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned int writes = 0;
+    bool fg = false;
     if (p < D.npx) {
         const int x = p % D.W, y = p / D.W;
         uint32_t w9[9];
@@ -770,9 +772,8 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
         }
         const uint32_t wp = w9[4];
         const bool valid = (wp & kIValid) != 0;
-        const uint8_t raw = (valid && (wp & kIFG)) ? 255 : 0;
-        if (ALG == ALG_VIBE) D.maskOut[p] = raw;
-        else D.rawFG[p] = raw;
+        fg = valid && (wp & kIFG);
+        if (ALG == ALG_VIBE) D.maskOut[p] = fg ? 255 : 0;
         D.kctr[p] = (uint16_t)(valid ? i_draws(wp) : 0);
         if (valid) writes = ((wp & kIOwn) ? 1u : 0u) + ((wp & kINb) ? 1u : 0u);
         // the pixels a write can reach: inside the LBSP border (LOBSTER), the whole frame (ViBe, PBAS)
@@ -819,48 +820,113 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
             }
         }
     }
+    if (ALG != ALG_VIBE) {
+        const uint32_t m = __ballot_sync(0xffffffffu, fg);
+        if ((threadIdx.x & 31) == 0 && p < D.npx) D.rawBits[p >> 5] = m;
+    }
     block_add(&D.stats[1], writes);
 }
 
 // cv::medianBlur(raw mask, k) with replicated borders: 255 where more than half of the k*k window is
 // set (:577), which becomes the last mask and the output (:578); the frame becomes the last colour
-// frame (:580). One block per kMedTile x kMedTile tile: the raw mask with its clamped halo in shared
-// memory, the row-window counts, then the column sums of those.
-constexpr int kMedTile = 32, kMedMaxR = 15, kMedS = kMedTile + 2 * kMedMaxR;
-template <int C, bool KEEP>
+// frame (:580). The raw mask comes as bits of the pixels in order (a warp of the commit writes a word), so a row's
+// word is two loads and a shift; one block per tile of kMedW words x kMedH rows counts the row windows and then
+// their sums on bit planes, 32 pixels an operation, and writes four pixels a store. With a byte and a count a
+// pixel in shared memory and byte copies: 1920x1080 16 us and now 7, 1277x719 BGR 11 us and now 8.
+constexpr int kMedW = 4, kMedH = 16, kMedMaxR = 15, kMedRows = kMedH + 2 * kMedMaxR;
+struct MedSmem {
+    uint32_t raw[kMedRows][kMedW + 2];
+    uint32_t h[5][kMedRows][kMedW];
+    uint32_t fg[kMedH][kMedW];
+};
+template <int HB>
+__device__ __forceinline__ void lob_median_words(MedSmem& sm, int r, int half) {
+    for (int i = threadIdx.x; i < (kMedH + 2 * r) * kMedW; i += kThreadsL) {
+        const int y = i / kMedW, w = i % kMedW;
+        uint32_t h[HB];
+        row_window_planes<HB>(sm.raw[y][w], sm.raw[y][w + 1], sm.raw[y][w + 2], r, h);
+#pragma unroll
+        for (int b = 0; b < HB; ++b) sm.h[b][y][w] = h[b];
+    }
+    __syncthreads();
+    if (threadIdx.x < kMedH * kMedW) {
+        const int y = threadIdx.x / kMedW, w = threadIdx.x % kMedW;
+        uint32_t a[2 * HB];
+#pragma unroll
+        for (int b = 0; b < 2 * HB; ++b) a[b] = 0u;
+        for (int j = 0; j <= 2 * r; ++j) {
+            uint32_t v[HB];
+#pragma unroll
+            for (int b = 0; b < HB; ++b) v[b] = sm.h[b][y + j][w];
+            add_planes<HB>(a, v);
+        }
+        sm.fg[y][w] = planes_above<2 * HB>(a, half);
+    }
+    __syncthreads();
+}
+template <bool KEEP>
 __global__ void __launch_bounds__(kThreadsL) lob_k_median(LobDev D) {
     pdl_entry();
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
-    __shared__ uint8_t raw[kMedS][kMedS];
-    __shared__ uint8_t rows[kMedS][kMedTile];
-    const int r = D.medianK / 2, span = kMedTile + 2 * r;
-    const int x0 = blockIdx.x * kMedTile, y0 = blockIdx.y * kMedTile, t = threadIdx.x;
-    for (int i = t; i < span * span; i += blockDim.x) {
-        const int ty = i / span, tx = i % span;
-        const int gy = clampi(y0 - r + ty, 0, D.H - 1), gx = clampi(x0 - r + tx, 0, D.W - 1);
-        raw[ty][tx] = D.rawFG[(size_t)gy * D.W + gx] != 0;
+    __shared__ MedSmem sm;
+    const int r = D.medianK / 2, t = threadIdx.x, W = D.W;
+    const int x0 = blockIdx.x * 32 * kMedW, y0 = blockIdx.y * kMedH;
+    for (int i = t; i < (kMedH + 2 * r) * (kMedW + 2); i += kThreadsL) {
+        const int ry = i / (kMedW + 2), x = x0 + 32 * (i % (kMedW + 2) - 1);
+        const int row = clampi(y0 - r + ry, 0, D.H - 1) * W;
+        auto bits = [&](int p) {  // 32 pixels from p on (the plane has a word past the frame)
+            return __funnelshift_r(__ldcg(&D.rawBits[p >> 5]), __ldcg(&D.rawBits[(p >> 5) + 1]), p & 31);
+        };
+        uint32_t v;
+        if (x < 0) {
+            v = (bits(row) & 1u) ? 0xffffffffu : 0u;
+        } else {
+            const uint32_t last = (bits(row + W - 1) & 1u) ? 0xffffffffu : 0u, in = x + 32 <= W ? 0xffffffffu : x < W ? (1u << (W - x)) - 1u : 0u;
+            v = x < W ? (bits(row + x) & in) | (last & ~in) : last;
+        }
+        sm.raw[ry][i % (kMedW + 2)] = v;
     }
     __syncthreads();
-    for (int i = t; i < span * kMedTile; i += blockDim.x) {
-        const int ty = i / kMedTile, tx = i % kMedTile;
-        int c = 0;
-        for (int d = 0; d <= 2 * r; ++d) c += raw[ty][tx + d];
-        rows[ty][tx] = (uint8_t)c;
+    // 2 * sum > k * k
+    if (r < 8) lob_median_words<4>(sm, r, D.medianK * D.medianK / 2);
+    else lob_median_words<5>(sm, r, D.medianK * D.medianK / 2);
+    const int y = y0 + t / 16, len = min(32 * kMedW, W - x0);
+    if (y < D.H) {
+        // 16 threads a row; aligned words whatever the width, the row's first and last in bytes
+        auto put = [&](uint8_t* plane) {
+            uint8_t* out = plane + (size_t)y * W + x0;
+            const int off = (int)((uintptr_t)out & 3);
+            for (int i = t % 16; 4 * i - off < len; i += 16) {
+                const int b = 4 * i - off;  // from -3 on
+                const uint32_t lo = b >= 0 ? sm.fg[t / 16][b >> 5] : 0u, hi = b < 32 * (kMedW - 1) ? sm.fg[t / 16][(b >> 5) + 1] : 0u;
+                const uint32_t v = (((__funnelshift_r(lo, hi, b & 31) & 15u) * 0x00204081u) & 0x01010101u) * 255u;
+                if (b >= 0 && b + 4 <= len) {
+                    *(uint32_t*)(out + b) = v;
+                } else {
+                    for (int j = max(0, -b); j < 4 && b + j < len; ++j) out[b + j] = (uint8_t)(v >> (8 * j));
+                }
+            }
+        };
+        put(D.maskOut);
+        if (KEEP) put(D.lastFG);  // PBAS keeps neither
     }
-    __syncthreads();
-    for (int i = t; i < kMedTile * kMedTile; i += blockDim.x) {
-        const int ty = i / kMedTile, tx = i % kMedTile;
-        const int x = x0 + tx, y = y0 + ty;
-        if (x >= D.W || y >= D.H) continue;
-        int cnt = 0;
-        for (int d = 0; d <= 2 * r; ++d) cnt += rows[ty + d][tx];
-        const size_t p = (size_t)y * D.W + x;
-        const uint8_t m = (2 * cnt > D.medianK * D.medianK) ? 255 : 0;
-        D.maskOut[p] = m;
-        if (!KEEP) continue;  // PBAS keeps neither
-        D.lastFG[p] = m;
-#pragma unroll
-        for (int c = 0; c < C; ++c) D.lastColor[p * C + c] = __ldg(D.frame + p * C + c);
+    if (KEEP) {
+        const size_t bytes = (size_t)D.npx * D.C, g = (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kThreadsL + t;
+        const size_t threads = (size_t)gridDim.x * gridDim.y * kThreadsL;
+        // lastColor is aligned; a frame at any address is read as the aligned words that lie wholly inside it
+        const uint32_t sh = 8u * (uint32_t)((uintptr_t)D.frame & 3);
+        const uint32_t* src = (const uint32_t*)((uintptr_t)D.frame & ~(uintptr_t)3);
+        size_t first = 0, end = bytes / 4;  // words of lastColor
+        if (sh) {
+            first = 1;
+            end = bytes >= 12 ? (bytes - 8) / 4 + 1 : 1;
+        }
+        for (size_t i = first + g; i < end; i += threads)
+            ((uint32_t*)D.lastColor)[i] = sh ? __funnelshift_r(__ldg(src + i), __ldg(src + i + 1), sh) : __ldg(src + i);
+        for (size_t i = g; i < 4 * first + (bytes - 4 * end); i += threads) {
+            const size_t j = i < 4 * first ? i : 4 * end + i - 4 * first;
+            if (j < bytes) D.lastColor[j] = __ldg(D.frame + j);
+        }
     }
 }
 
@@ -934,7 +1000,8 @@ __device__ __forceinline__ int reflect101(int i, int n) {
 // reflected 2-pixel halo in shared memory, blurred there with a 1-pixel halo (both kernels are symmetric, so
 // the blur of a reflected position is the reflected blur), then the derivatives; four bytes at a time, two per
 // word in 16 bits (the sums are at most 16 * 255). Bytes of a channel are C apart in the interleaved rows. The
-// blur went through memory before, a byte and nine loads a thread: 30 + 38 us on a 1920x1080 BGR frame.
+// blur went through memory before, a byte and nine loads a thread: 30 + 38 us on a 1920x1080 BGR frame, 34 with tiles
+// loaded by bytes, 25 with words.
 constexpr int kGradW = 64, kGradH = 16;
 template <int C>
 struct GradTile {
@@ -955,10 +1022,20 @@ __global__ void __launch_bounds__(kThreadsL) pbas_k_grad(LobDev D, const uint8_t
     const int x0 = blockIdx.x * kGradW, y0 = blockIdx.y * kGradH, t = threadIdx.x;
     // frame bytes of rows y0 - 2 .. y0 + 17, pixels x0 - 2 .. x0 + 65, from byte kPad - 2 C of a row on
     constexpr int kBytes = (kGradW + 4) * C;
-    for (int i = t; i < (kGradH + 4) * kBytes; i += kThreadsL) {
-        const int r = i / kBytes, b = i % kBytes;
-        const int gy = reflect101(y0 - 2 + r, D.H), gx = reflect101(x0 - 2 + b / C, D.W);
-        ((uint8_t*)sm.src[r])[T::kPad - 2 * C + b] = __ldg(img + ((size_t)gy * D.W + gx) * C + b % C);
+    // inside the frame's width a tile row is kRow aligned words from byte x0 C - kPad on (x0 C is a multiple of 64)
+    const long b0 = (long)x0 * C - T::kPad, rowBytes = (long)D.W * C;
+    const bool words = b0 >= 0 && b0 + 4 * T::kRow <= rowBytes && ((rowBytes | (uintptr_t)img) & 3) == 0;
+    if (words) {
+        for (int i = t; i < (kGradH + 4) * T::kRow; i += kThreadsL) {
+            const int r = i / T::kRow, w = i % T::kRow, gy = reflect101(y0 - 2 + r, D.H);
+            sm.src[r][w] = __ldg((const uint32_t*)(img + (size_t)gy * rowBytes + b0) + w);
+        }
+    } else {
+        for (int i = t; i < (kGradH + 4) * kBytes; i += kThreadsL) {
+            const int r = i / kBytes, b = i % kBytes;
+            const int gy = reflect101(y0 - 2 + r, D.H), gx = reflect101(x0 - 2 + b / C, D.W);
+            ((uint8_t*)sm.src[r])[T::kPad - 2 * C + b] = __ldg(img + ((size_t)gy * D.W + gx) * C + b % C);
+        }
     }
     __syncthreads();
     // blur of rows y0 - 1 .. y0 + 16, pixels x0 - 1 .. x0 + 64, in words from byte kFirst on
@@ -1603,7 +1680,7 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
         return o;
     };
     const size_t oRoi = take(npx), oLastColor = take(lob * npx * C), oLastFG = take(lob * npx),
-                 oRawFG = take(lob * npx), oLut = take(256), oLastDesc = take(lob * npx * C * 2), oKctr = take(npx * 2),
+                 oRawBits = take(vibe && !pbas ? 0 : (npx / 32 + 2) * 4), oLut = take(256), oLastDesc = take(lob * npx * C * 2), oKctr = take(npx * 2),
                  oSD = take(lob * N * npx * (C == 3 ? 8 : 2)), oSC = take(N * npx * sample_bytes_lo(alg, C)),
                  oIntent = take(npx * 4),
                  oWD = take(npx * 8), oList0 = take(npx * 4), oList1 = take(npx * 4), oStamp = take(npx * 4),
@@ -1611,8 +1688,7 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
                  oSG = take(N * npx * sample_bytes_hi(alg, C)), oGrad = take(pb * npx * C),
                  oFm = take(pb * 6 * npx * 4), oMean = take(pb * 4), oBadSum = take(pb * npx * 4),
                  oBadCnt = take(pb * npx), oBadVals = take(pb * (C == 3 ? npx * N * 2 : 0)),
-                 oSumTr = take(pb * (C == 3 ? SumWork::bytes((npx + kSumChunk - 1) / kSumChunk) : 0)),
-                 oRawPb = take(pb * npx);
+                 oSumTr = take(pb * (C == 3 ? SumWork::bytes((npx + kSumChunk - 1) / kSumChunk) : 0));
     LOB_CUDA(cudaMalloc(&L.mem, off), "model allocation");
     if (!L.h_flags) LOB_CUDA(cudaHostAlloc((void**)&L.h_flags, LOB_F_WORDS * 4, cudaHostAllocMapped), "pinned allocation");
     if (!L.done) LOB_CUDA(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming), "event creation");
@@ -1641,7 +1717,7 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
     D.roi = b + oRoi;
     D.lastColor = b + oLastColor;
     D.lastFG = b + oLastFG;
-    D.rawFG = b + oRawFG;
+    D.rawBits = (uint32_t*)(b + oRawBits);
     D.lut = b + oLut;
     D.lastDesc = (uint16_t*)(b + oLastDesc);
     D.kctr = (uint16_t*)(b + oKctr);
@@ -1667,7 +1743,6 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
         D.badVals = (uint16_t*)(b + oBadVals);
         D.sumTr = b + oSumTr;
         if (C == 3) D.chunkAbout = sum_work(D.sumTr, (npx + kSumChunk - 1) / kSumChunk).about;
-        D.rawFG = b + oRawPb;
         // the constructor's arguments (BackgroundSubtractorPBAS.cpp:21-32) and medianBlur(.., 9) (:266 / :494)
         D.R0 = (float)prm.min_color_dist_threshold;
         D.updateRate = prm.update_rate;
@@ -1854,13 +1929,9 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
         launch<Commit>(D, nb, st);
         // LOBSTER's median blur, last mask and last colour frame; PBAS's median blur (ViBe outputs its
         // raw mask)
-        const dim3 mg((D.W + kMedTile - 1) / kMedTile, (D.H + kMedTile - 1) / kMedTile);
-        if (D.alg == ALG_LOBSTER) {
-            if (C == 3) launch_chained(lob_k_median<3, true>, mg, dim3(kThreadsL), st, D);
-            else launch_chained(lob_k_median<1, true>, mg, dim3(kThreadsL), st, D);
-        } else if (D.alg == ALG_PBAS) {
-            launch_chained(lob_k_median<1, false>, mg, dim3(kThreadsL), st, D);
-        }
+        const dim3 mg((D.W + 32 * kMedW - 1) / (32 * kMedW), (D.H + kMedH - 1) / kMedH);
+        if (D.alg == ALG_LOBSTER) launch_chained(lob_k_median<true>, mg, dim3(kThreadsL), st, D);
+        else if (D.alg == ALG_PBAS) launch_chained(lob_k_median<false>, mg, dim3(kThreadsL), st, D);
         LOB_CUDA(cudaGetLastError(), "repair launch");
         if (hostMask) LOB_CUDA(cudaMemcpyAsync(hostMask, dmask, (size_t)D.npx, cudaMemcpyDeviceToHost, st), "mask download");
         if (D.alg == ALG_PBAS) {  // the host does not wait for the mean

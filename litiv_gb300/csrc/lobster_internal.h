@@ -10,7 +10,7 @@
 //   ViBe keeps only its samples, sC[N][npx*C] (the reference's layout: C colour bytes per sample);
 //   PBAS its colour and gradient samples sC / sG[N][npx*C], the R, T and D maps fm[2][3][npx] (by frame
 //   parity), the frame's gradient image and the frame-level mean gradient distance;
-//   scratch of a frame step: intent[npx] (u32), wD[npx] (the sample word a pixel writes), rawFG[npx],
+//   scratch of a frame step: intent[npx] (u32), wD[npx] (the sample word a pixel writes), rawBits (a bit a pixel),
 //   two repair lists and their dedupe stamps, flags and counters, the staged frame and mask.
 #pragma once
 #include <cuda_runtime.h>
@@ -41,7 +41,8 @@ struct LobDev {
     unsigned int listCap;
     const uint8_t* frame;
     uint8_t* maskOut;
-    uint8_t *roi, *lastColor, *lastFG, *rawFG, *lut;
+    uint8_t *roi, *lastColor, *lastFG, *lut;
+    uint32_t* rawBits;  // the raw mask, pixel p at bit p & 31 of word p >> 5
     uint16_t *lastDesc, *kctr;
     void* sD;
     uint8_t* sC;

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "area_device.cuh"
+#include "bitslice.cuh"
 #include "lbsp_device.cuh"
 #include "lvbgs_internal.h"
 
@@ -1607,45 +1608,6 @@ extern "C" __global__ void __launch_bounds__(256) lvbgs_k_fill(TickParams P) {
     }
 }
 
-// bit-sliced arithmetic on 32 pixels at once: carry of a full adder
-__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (a & c) | (b & c); }
-
-// number of set pixels of each pixel's row window [x - r, x + r], r < 2^(HB-1): bit planes h[0..HB-1] of
-// word C with its neighbour words L and R
-template <int HB>
-__device__ __forceinline__ void row_window_planes(uint32_t L, uint32_t C, uint32_t R, int r, uint32_t (&h)[HB]) {
-    h[0] = C;
-#pragma unroll
-    for (int i = 1; i < HB; ++i) h[i] = 0u;
-    int d = 1;
-    for (; d + 1 <= r; d += 2) {
-        const uint32_t a = __funnelshift_r(C, R, d), b = __funnelshift_l(L, C, d);
-        const uint32_t e = __funnelshift_r(C, R, d + 1), f = __funnelshift_l(L, C, d + 1);
-        const uint32_t s = h[0] ^ a ^ b, c1 = maj3(h[0], a, b);
-        h[0] = s ^ e ^ f;
-        const uint32_t c2 = maj3(s, e, f);
-        uint32_t c = maj3(h[1], c1, c2);
-        h[1] ^= c1 ^ c2;
-#pragma unroll
-        for (int i = 2; i < HB; ++i) {
-            const uint32_t t = h[i] & c;
-            h[i] ^= c;
-            c = t;
-        }
-    }
-    if (d <= r) {
-        const uint32_t a = __funnelshift_r(C, R, d), b = __funnelshift_l(L, C, d);
-        uint32_t c = maj3(h[0], a, b);
-        h[0] ^= a ^ b;
-#pragma unroll
-        for (int i = 1; i < HB; ++i) {
-            const uint32_t t = h[i] & c;
-            h[i] ^= c;
-            c = t;
-        }
-    }
-}
-
 // shared memory of one tile of the final-mask kernel: the combined mask's words with their halo, the row
 // window counts as bit planes, the final mask with the dilation's halo, the dilated words
 constexpr int kFinMaxR = 15;                            // median radius (kernel size at most 31)
@@ -1680,24 +1642,12 @@ __device__ __forceinline__ void median_words(FinSmem& sm, int r, int half, int y
 #pragma unroll
             for (int b = 0; b < 2 * HB; ++b) a[b] = b < HB ? sm.h[b < HB ? b : 0][fr][fw] : 0u;
             for (int j = 1; j <= 2 * r; ++j) {
-                uint32_t c = 0u;
+                uint32_t v[HB];
 #pragma unroll
-                for (int b = 0; b < HB; ++b) {
-                    const uint32_t v = sm.h[b][fr + j][fw];
-                    const uint32_t s = a[b] ^ v ^ c;
-                    c = maj3(a[b], v, c);
-                    a[b] = s;
-                }
-#pragma unroll
-                for (int b = HB; b < 2 * HB; ++b) {
-                    const uint32_t t = a[b] & c;
-                    a[b] ^= c;
-                    c = t;
-                }
+                for (int b = 0; b < HB; ++b) v[b] = sm.h[b][fr + j][fw];
+                add_planes<HB>(a, v);
             }
-            // sum > half, from the lowest bit up
-#pragma unroll
-            for (int b = 0; b < 2 * HB; ++b) fg = ((half >> b) & 1) ? (a[b] & fg) : (a[b] | fg);
+            fg = planes_above<2 * HB>(a, half);
             fg &= valid_bits(w, W);
         }
         sm.fg[fr][fw] = fg;

@@ -4,7 +4,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from litiv_gb300 import _lib as L
+from litiv_gb300 import BackgroundSubtractorLOBSTER, _lib as L
 from litiv_gb300.metrics import BinClassif
 from oracle import metrics as oracle_metrics, pyoracle
 from tests.test_gpu_lobster import run_pair as lobster_pair
@@ -146,3 +146,18 @@ def test_sample_scans_of_the_consensus_models(W, H, N, nreq, channels):
     vibe_pair(frames, N + 1, lrs, **args)
     pbas_pair(frames, N + 2, lrs, **args)
     pbas_pair(frames, N + 3, [-1.0] * len(frames), **args)
+
+
+@pytest.mark.parametrize("W,H,k,channels", [(31, 33, 3, 1), (128, 16, 9, 3), (129, 17, 15, 1), (255, 31, 17, 3), (300, 20, 31, 1),
+                                            (67, 53, 1, 3), (640, 35, 9, 1)])
+def test_median_of_bits_and_gradient_tiles(W, H, k, channels):
+    """LOBSTER's median over windows of four and of five bit planes and PBAS's gradient, on frames that end inside a
+    word, a tile and eight pixels, with rows at and off the alignment of the word loads."""
+    frames = hollow_frames(W, H, channels, 5, W * 5 + k)
+    gpu = BackgroundSubtractorLOBSTER(seed=k, nDefaultMedianBlurKernelSize=k)
+    ora = pyoracle.OracleLOBSTER(seed=k, default_median_blur_kernel_size=k)
+    gpu.initialize(frames[0])
+    ora.initialize(frames[0])
+    for f in frames[1:]:
+        assert np.array_equal(gpu.apply(f, learningRate=16.0), ora.apply(f, 16.0))
+    pbas_pair(frames, k + 1, [-1.0] * len(frames))
