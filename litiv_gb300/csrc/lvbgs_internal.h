@@ -165,7 +165,7 @@ struct StreamDev {
 
 // Per-launch work area (reset before every launch).
 struct TickWork {
-    unsigned int bar_count, bar_gen, err, err_info;
+    unsigned int bar_count, err, err_info;
     unsigned int phase_ctr[16];  // repair: re-matched items of rounds 0..15 (phase profile)
     unsigned int dcount[4], rcount[2];  // repair lists' lengths (dcount: by dcount_slot, rcount: by round parity)
     unsigned int done_ctas, iters;

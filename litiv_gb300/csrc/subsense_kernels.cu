@@ -46,36 +46,35 @@ __device__ __forceinline__ unsigned long long gtimer() {
 __device__ __forceinline__ unsigned int ld_volatile(const unsigned int* p) { return *(const volatile unsigned int*)p; }
 
 // Barrier over the first nCtas CTAs of a cooperative launch (all co-resident). The wait is bounded: after
-// timeoutNs the CTA records ERR_BARRIER_TIMEOUT and every CTA leaves at its next check.
-__device__ bool grid_sync(TickWork* w, unsigned int nCtas, unsigned long long timeoutNs) {
+// timeoutNs the CTA records ERR_BARRIER_TIMEOUT and every CTA leaves at its next check. The arrivals only count up
+// (from the tick's start, zero): the due value, kept by the CTA, is what the barriers so far need, so nothing is
+// reset or released, and the error word is read together with the count. With a count that the last
+// arrival resets and a generation that it raises, a barrier was a chain of seven trips to L2.
+__device__ bool grid_sync(TickWork* w, unsigned int nCtas, unsigned long long timeoutNs, unsigned int& due) {
     __shared__ int s_ok;
+    due += nCtas;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned int gen = ld_volatile(&w->bar_gen);
         __threadfence();
-        const unsigned int arrived = atomicAdd(&w->bar_count, 1u) + 1u;
+        atomicAdd(&w->bar_count, 1u);
+        const unsigned long long t0 = gtimer();
         int ok = 1;
-        if (arrived == nCtas) {
-            atomicExch(&w->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&w->bar_gen, 1u);
-        } else {
-            const unsigned long long t0 = gtimer();
-            while (ld_volatile(&w->bar_gen) == gen) {
-                if (ld_volatile(&w->err) != 0u) {
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(40);
-                if (gtimer() - t0 > timeoutNs) {
-                    atomicOr(&w->err, ERR_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
+        for (;;) {
+            const unsigned int arrived = ld_volatile(&w->bar_count), err = ld_volatile(&w->err);
+            if (err != 0u) {
+                ok = 0;
+                break;
             }
+            if ((int)(arrived - due) >= 0) break;
+            if (gtimer() - t0 > timeoutNs) {
+                atomicOr(&w->err, ERR_BARRIER_TIMEOUT);
+                ok = 0;
+                break;
+            }
+            __nanosleep(20);
         }
         __threadfence();
-        s_ok = ok && (ld_volatile(&w->err) == 0u);
+        s_ok = ok;
     }
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0 && w->nts < 40u) w->ts[w->nts++] = gtimer();
@@ -2027,11 +2026,12 @@ extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_resolve(TickParam
 // list has work for (later lists are shorter): a barrier over 28 CTAs costs a third of one over 304.
 extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickParams P) {
     TickWork* w = P.work;
+    unsigned int due = 0u;  // barrier arrivals
     if (blockIdx.x == 0 && threadIdx.x == 0 && w->nts < 40u) w->ts[w->nts++] = gtimer();  // phase profile
     if (P.dbgFault == LVBGS_FAULT_BARRIER_TIMEOUT) {
         // injected fault: every CTA but CTA 0 waits at a barrier CTA 0 never reaches; each wait gives
         // up after P.barrierNs and records ERR_BARRIER_TIMEOUT, and every CTA returns
-        if (blockIdx.x != 0) grid_sync(w, gridDim.x, P.barrierNs);
+        if (blockIdx.x != 0) grid_sync(w, gridDim.x, P.barrierNs, due);
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -2081,7 +2081,7 @@ extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickPar
             const unsigned grp = __match_any_sync(0xffffffffu, counted ? si : -1 - lane);
             if (counted && lane == __ffs(grp) - 1) atomicAdd(&S.ctl->st_rematched, (unsigned long long)__popc(grp));
         }
-        if (!grid_sync(w, ctas, P.barrierNs)) return;
+        if (!grid_sync(w, ctas, P.barrierNs, due)) return;
         const unsigned int nr0 = ld_volatile(&w->rcount[par]);
         const unsigned int nr = nr0 < P.listCap ? nr0 : P.listCap;
         if (nr != 0u) {  // the same value in every CTA: rcount[par] is reset only in the next round, from 0
@@ -2098,7 +2098,7 @@ extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickPar
                     reresolve_item(P, si, S, p, S.ctl->stamp_base + (uint32_t)iter + 2u, iter);
                 }
             }
-            if (!grid_sync(w, ctas, P.barrierNs)) return;
+            if (!grid_sync(w, ctas, P.barrierNs, due)) return;
         }
         ++iter;
     }
