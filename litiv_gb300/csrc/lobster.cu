@@ -663,25 +663,27 @@ __device__ __forceinline__ void round_end(const LobDev& D, int round) {
     }
 }
 
-// 2. Round 0: a block finds the pixels of its own (four a thread) whose scan read a sample that an earlier
+// 2. Round 0: a block finds the pixels of its own (PER a thread) whose scan read a sample that an earlier
 // neighbour writes, and re-evaluates them, with the other blocks' re-evaluations under way: a pixel that changes
 // its neighbour write after a later pixel looked at it lists that pixel for round 1. One launch where the marks
 // went through a list in memory. A block lasts as long as its slowest re-evaluation, so it takes 1,024 pixels:
 // with 256, LOBSTER 1277x719 BGR took 36 us and PBAS 1920x1080 BGR 67 us. A chain of latencies: more blocks at
 // once are worth some spilled registers (3 / 5 / 6 / 8 blocks per SM: LOBSTER 19.6 / 17.8 / 14.6 / 15.4 us, PBAS
-// 34 / 30 / 28 / 24 us).
-constexpr int kFirstPer = 4, kFirstPx = kFirstPer * kThreadsL;
-template <int C, int ALG>
+// 34 / 30 / 28 / 24 us). A frame of which four pixels a thread would make fewer than two blocks an SM takes one a
+// thread: 320x240 BGR ViBe 8.6 -> 7.7 us, 45 -> 40 us a frame.
+constexpr int kFirstSmall = 304 * 1024;
+template <int C, int ALG, int PER>
 __global__ void __launch_bounds__(kThreadsL, ALG == ALG_PBAS ? 8 : 6) lob_k_first(LobDev D) {
     pdl_entry();
+    constexpr int kFirstPx = PER * kThreadsL;
     __shared__ int items[kFirstPx];
     __shared__ int count;
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, p0 = blockIdx.x * kFirstPx + (int)threadIdx.x;
-    uint32_t w[kFirstPer], wq[kFirstPer][4];
+    uint32_t w[PER], wq[PER][4];
 #pragma unroll
-    for (int i = 0; i < kFirstPer; ++i) {
+    for (int i = 0; i < PER; ++i) {
         const int p = p0 + i * kThreadsL;
         w[i] = p < D.npx ? ld_vol(&D.intent[p]) : 0u;
         const Earlier e = earlier(D, p, p % D.W, p / D.W);
@@ -689,7 +691,7 @@ __global__ void __launch_bounds__(kThreadsL, ALG == ALG_PBAS ? 8 : 6) lob_k_firs
         for (int j = 0; j < 4; ++j) wq[i][j] = p < D.npx && e.ok[j] ? ld_vol(&D.intent[e.q[j]]) : 0u;
     }
 #pragma unroll
-    for (int i = 0; i < kFirstPer; ++i) {
+    for (int i = 0; i < PER; ++i) {
         const int p = p0 + i * kThreadsL;
         bool dirty = false;
         if (w[i] & kIValid) {
@@ -1790,7 +1792,10 @@ struct Eval {
 };
 template <int C, int ALG>
 struct First {
-    static void run(int b, cudaStream_t st, const LobDev& D) { launch_chained(lob_k_first<C, ALG>, dim3(b), dim3(kThreadsL), st, D); }
+    static void run(int b, cudaStream_t st, const LobDev& D) {
+        if (D.npx < kFirstSmall) launch_chained(lob_k_first<C, ALG, 1>, dim3(b), dim3(kThreadsL), st, D);
+        else launch_chained(lob_k_first<C, ALG, 4>, dim3((b + 3) / 4), dim3(kThreadsL), st, D);
+    }
 };
 template <int C, int ALG>
 struct Round {
@@ -1914,7 +1919,7 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
         const int nChunks = (D.npx + kSumChunk - 1) / kSumChunk;
         pbas_k_sum_scan<<<1, kSumScan, 0, L.meanStream>>>(sum_work(D.sumTr, nChunks), nChunks);
     }
-    launch<First>(D, (D.npx + kFirstPx - 1) / kFirstPx, st);
+    launch<First>(D, nb, st);
     LOB_CUDA(cudaGetLastError(), "evaluation launch");
     int round = 1, chunk = L.lastRounds;
     for (;;) {
