@@ -201,12 +201,23 @@ struct lvbgs_ctx {
     unsigned long long pw_frames = 0;
     unsigned long long pw_offset = 1000;
     int pw_rounds_last = 0;
+    bool pw_unchained = false;  // PAWCS launches wait for the one before to drain (pw_set_unchained)
     double pw_host_ms[5] = {0, 0, 0, 0, 0};  // last PAWCS frame: lvbgs_debug_pawcs_host_timing
     PwStep pws;  // the PAWCS frame step in flight (pw_begin / pw_advance)
     cudaEvent_t evPw = nullptr;  // fork / join of the handle's PAWCS step in a batch
     int dbg_fault = 0;  // one-shot fault injection of the next frame step (lvbgs_debug_inject_fault)
     LobState* lob = nullptr;  // LOBSTER and ViBe (LVBGS_ALGO_LOBSTER / _VIBE): the stream's device state
 };
+
+// A launch of a PAWCS frame step. Chained, a kernel's blocks take the SMs' places while the one before drains, so a
+// cooperative grid of another stream (a SuBSENSE repair) finds no moment to become resident: in the serving loop,
+// whose PAWCS frames run beside the SuBSENSE ticks, a tick then waited for the end of a PAWCS frame (99th
+// percentile 22-30 ms; unchained 4-9 ms, and 12-17 ms when the host waited between rounds).
+template <typename... KArgs, typename... Args>
+void pw_launch(const lvbgs_ctx* h, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+    if (h->pw_unchained) kernel<<<grid, block, 0, st>>>(KArgs(args)...);
+    else launch_chained(kernel, grid, block, st, args...);
+}
 
 namespace {
 
@@ -570,6 +581,7 @@ uint8_t sat_round_u8(float v) {
 
 // library-level error message (lvbgs_last_error(NULL)) for entry points defined in other files
 lvbgs_status lvbgs::report_error(lvbgs_status st, const char* msg) { return fail(nullptr, st, msg); }
+void lvbgs::pw_set_unchained(lvbgs_handle h, bool on) { h->pw_unchained = on; }
 
 extern "C" {
 
@@ -779,11 +791,11 @@ lvbgs_status pw_upload_desc(lvbgs_ctx* h, cudaStream_t st) {
 lvbgs_status pw_refresh(lvbgs_ctx* h, uint32_t t, int buf, int baseOcc, float decr, int force, int onlyPending,
                         int useDil, cudaStream_t st) {
     const dim3 g((unsigned)((h->npx + 127) / 128));
-    launch_chained(h->C == 3 ? pw3_k_refresh_local : pw_k_refresh_local, g, dim3(128), st, h->pd, t, buf, baseOcc, decr, force,
+    pw_launch(h, h->C == 3 ? pw3_k_refresh_local : pw_k_refresh_local, g, dim3(128), st, h->pd, t, buf, baseOcc, decr, force,
                    onlyPending, useDil);
-    launch_chained(h->C == 3 ? pw3_k_refresh_global : pw_k_refresh_global, dim3(1), dim3(1), st, h->pd, t, buf, force,
+    pw_launch(h, h->C == 3 ? pw3_k_refresh_global : pw_k_refresh_global, dim3(1), dim3(1), st, h->pd, t, buf, force,
                    onlyPending, useDil);
-    launch_chained(pw_k_lut_sort, dim3(h->sd.nTiles), dim3(kThreads), st, pw_params(h, 0.0), onlyPending ? 2 : 1);
+    pw_launch(h, pw_k_lut_sort, dim3(h->sd.nTiles), dim3(kThreads), st, pw_params(h, 0.0), onlyPending ? 2 : 1);
     LV_CUDA(h, cudaGetLastError(), "refresh kernel launch");
     return LVBGS_OK;
 }
@@ -938,21 +950,22 @@ lvbgs_status pw_enqueue_rounds(lvbgs_ctx* h, int n) {
         w.PR.round = w.enq;
         const PwParams& P = w.PR;
         // three channels: the local pass applies the earlier updaters' loops itself
-        launch_chained(!c3 ? pw_k_local : P.round == 0 ? pw3_k_local_first : pw3_k_local, tiles, blk, st, P);
-        launch_chained(pw_k_illum, dim3((h->H + 7) / 8), blk, st, P);
-        launch_chained(pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 0);
-        launch_chained(pw3_k_gscan_seg, gseg, warps4, st, P);
-        launch_chained(pw3_k_gscan_walk, dim3(1), dim3(32), st, P);
-        launch_chained(pw3_k_gscan_fix, dim3((unsigned)((h->npx + 255) / 256)), blk, st, P);
-        launch_chained(pw3_k_gscan_fix_walked, gseg, warps4, st, P);
-        launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 0);
-        launch_chained(pw_k_nbr, tiles, blk, st, P);
+        // not chained: once a round the device drains, and another stream's cooperative grid can become resident
+        (!c3 ? pw_k_local : P.round == 0 ? pw3_k_local_first : pw3_k_local)<<<tiles, blk, 0, st>>>(P);
+        pw_launch(h, pw_k_illum, dim3((h->H + 7) / 8), blk, st, P);
+        pw_launch(h, pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 0);
+        pw_launch(h, pw3_k_gscan_seg, gseg, warps4, st, P);
+        pw_launch(h, pw3_k_gscan_walk, dim3(1), dim3(32), st, P);
+        pw_launch(h, pw3_k_gscan_fix, dim3((unsigned)((h->npx + 255) / 256)), blk, st, P);
+        pw_launch(h, pw3_k_gscan_fix_walked, gseg, warps4, st, P);
+        pw_launch(h, pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 0);
+        pw_launch(h, pw_k_nbr, tiles, blk, st, P);
         if (!c3) {
-            launch_chained(pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 2);
-            launch_chained(pw_k_nbr_loops, dim3(std::max(1u, std::min(cblocks.x * 4, 1216u))), blk, st, P);
-            launch_chained(pw_k_replace, tiles, blk, st, P);
+            pw_launch(h, pw_k_compact, oneBlocks, dim3(kPwOneThreads), st, P, 2);
+            pw_launch(h, pw_k_nbr_loops, dim3(std::max(1u, std::min(cblocks.x * 4, 1216u))), blk, st, P);
+            pw_launch(h, pw_k_replace, tiles, blk, st, P);
         }
-        launch_chained(c3 ? pw3_k_dirty : pw_k_dirty, tiles, blk, st, P);
+        pw_launch(h, c3 ? pw3_k_dirty : pw_k_dirty, tiles, blk, st, P);
     }
     LV_CUDA(h, cudaGetLastError(), "PAWCS round launch");
     return LVBGS_OK;
@@ -985,26 +998,26 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
     const dim3 cblocks((unsigned)((h->npx + kPwCompactBlk - 1) / kPwCompactBlk));
     const bool c3 = h->C == 3;
     if (c3) {
-        launch_chained(pw3_k_later_list, tiles, blk, st, P);
-        launch_chained(pw3_k_later, tiles, blk, st, P);
+        pw_launch(h, pw3_k_later_list, tiles, blk, st, P);
+        pw_launch(h, pw3_k_later, tiles, blk, st, P);
     }
-    launch_chained(c3 ? pw3_k_commit : pw_k_commit, tiles, blk, st, P);
-    launch_chained(pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 1);
-    launch_chained(pw_k_compact_count, cblocks, blk, st, P);
-    launch_chained(pw_k_compact_offsets, dim3(1), dim3(32 * std::min(h->pd.G, 32)), st, P, h->pd.G);
-    launch_chained(pw_k_compact_scatter, cblocks, blk, st, P);
-    launch_chained(pw_k_weights, dim3(kPwMaxGlobal), blk, st, P);
+    pw_launch(h, c3 ? pw3_k_commit : pw_k_commit, tiles, blk, st, P);
+    pw_launch(h, pw_k_cells, dim3((P.totalCells + 255) / 256), blk, st, P, 1);
+    pw_launch(h, pw_k_compact_count, cblocks, blk, st, P);
+    pw_launch(h, pw_k_compact_offsets, dim3(1), dim3(32 * std::min(h->pd.G, 32)), st, P, h->pd.G);
+    pw_launch(h, pw_k_compact_scatter, cblocks, blk, st, P);
+    pw_launch(h, pw_k_weights, dim3(kPwMaxGlobal), blk, st, P);
     // global-word upkeep: the kernels of frames without one would return at once
     const uint32_t t = (uint32_t)(h->pw_frames + 1);
     const uint32_t rate = t <= (uint32_t)kPwBootWin ? 8u : 16u;
-    if (t % (rate << 5) == 0) launch_chained(pw_k_gw_recalc, dim3(kPwMaxGlobal), blk, st, P);
+    if (t % (rate << 5) == 0) pw_launch(h, pw_k_gw_recalc, dim3(kPwMaxGlobal), blk, st, P);
     if (t % rate == 0) {
-        launch_chained(pw_k_gw_decay, dim3(64, kPwMaxGlobal), blk, st, P, h->d_rowsum);
-        launch_chained(pw_k_gw_blur, dim3(64, kPwMaxGlobal), blk, st, P, (const double*)h->d_rowsum);
+        pw_launch(h, pw_k_gw_decay, dim3(64, kPwMaxGlobal), blk, st, P, h->d_rowsum);
+        pw_launch(h, pw_k_gw_blur, dim3(64, kPwMaxGlobal), blk, st, P, (const double*)h->d_rowsum);
     }
-    launch_chained(pw_k_gw_sort, dim3(1), dim3(32), st, P);
-    if (t % rate == 0) launch_chained(pw_k_lut_sort, tiles, blk, st, P, 0);
-    launch_chained(pw_k_blink_close, tiles, blk, st, P);
+    pw_launch(h, pw_k_gw_sort, dim3(1), dim3(32), st, P);
+    if (t % rate == 0) pw_launch(h, pw_k_lut_sort, tiles, blk, st, P, 0);
+    pw_launch(h, pw_k_blink_close, tiles, blk, st, P);
     TickParams TP;
     std::memset(&TP, 0, sizeof(TP));
     TP.streams = h->d_sd;
@@ -1015,12 +1028,12 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
     TP.totalSegs = h->sd.nSegs;
     TP.gate = P.gate;
     const dim3 rowBlocks((h->H + 7) / 8);
-    launch_chained(lvbgs_k_unite, rowBlocks, blk, st, TP);
-    launch_chained(lvbgs_k_fill, rowBlocks, blk, st, TP);
-    launch_chained(lvbgs_k_final, dim3(TP.totalSegs), blk, st, TP);
+    pw_launch(h, lvbgs_k_unite, rowBlocks, blk, st, TP);
+    pw_launch(h, lvbgs_k_fill, rowBlocks, blk, st, TP);
+    pw_launch(h, lvbgs_k_final, dim3(TP.totalSegs), blk, st, TP);
     const int nds = (h->W / 8) * (h->H / 8);
-    if (nds > 0) launch_chained(c3 ? pw3_k_ds : pw_k_ds, dim3((nds + 31) / 32), blk, st, P);
-    launch_chained(pw_k_epilogue, dim3(1), blk, st, P, motion ? 0 : 1);
+    if (nds > 0) pw_launch(h, c3 ? pw3_k_ds : pw_k_ds, dim3((nds + 31) / 32), blk, st, P);
+    pw_launch(h, pw_k_epilogue, dim3(1), blk, st, P, motion ? 0 : 1);
     if (motion) {
         // camera-motion comparison (:1480-1501): the host waits for the decision, which may switch the
         // local word weight offset and run refreshModel(1, 1, true). The frame's background image goes to the
@@ -1029,8 +1042,8 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
         uint8_t* bg = (uint8_t*)h->sd.label;
         if (c3) pw3_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
         else pw_k_background<<<1024, 256, 0, st>>>(h->pd, nxt, bg, nullptr, 1);
-        launch_chained(c3 ? pw3_k_motion_bg : pw_k_motion_bg, dim3((nds + 31) / 32), blk, st, P);
-        launch_chained(pw_k_motion_decide, dim3(1), blk, st, P);
+        pw_launch(h, c3 ? pw3_k_motion_bg : pw_k_motion_bg, dim3((nds + 31) / 32), blk, st, P);
+        pw_launch(h, pw_k_motion_decide, dim3(1), blk, st, P);
     }
     LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
     return LVBGS_OK;
@@ -1039,7 +1052,7 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
 // the end of the frame: its close (which a pending automatic reset holds back) and the mask download
 lvbgs_status pw_enqueue_close(lvbgs_ctx* h, int resetDone) {
     PwStep& w = h->pws;
-    launch_chained(pw_k_close, dim3(1), dim3(32), w.st, w.P, resetDone);
+    pw_launch(h, pw_k_close, dim3(1), dim3(32), w.st, w.P, resetDone);
     LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
     if (w.mask && !w.devMask)
         LV_CUDA(h, cudaMemcpyAsync(w.mask, h->d_mask, h->npx, cudaMemcpyDeviceToHost, w.st), "mask download");
@@ -1136,7 +1149,7 @@ lvbgs_status pw_advance(lvbgs_ctx* h, bool& done) {
         if (w.stage == 2 || !hf[PWF_RESET]) return finish(fail(h, LVBGS_DEVICE_ERROR, "PAWCS frame step did not close"));
         // automatic model reset (:1503-1508): refreshModel(offset/8, 0, true) and T(x) := 1
         if ((s = pw_refresh(h, t, nxt, (int)(h->pw_offset / 8), 0.0f, 1, 1, 1, w.st)) != LVBGS_OK) return finish(s);
-        launch_chained(pw_k_reset_T, dim3(256), dim3(256), w.st, h->pd, nxt);
+        pw_launch(h, pw_k_reset_T, dim3(256), dim3(256), w.st, h->pd, nxt);
         s = pw_enqueue_close(h, 1);
         w.stage = 2;
         h->pw_host_ms[2] += pw_ms_since(t0);

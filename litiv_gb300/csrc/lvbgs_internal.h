@@ -27,6 +27,9 @@
 
 namespace lvbgs {
 
+// PAWCS frame steps of h without chained launches, for a device shared with SuBSENSE ticks: a chained step leaves no
+// moment between its kernels at which a tick's cooperative repair grid could become resident.
+void pw_set_unchained(lvbgs_handle h, bool on);
 // sets the library-level error message returned by lvbgs_last_error(NULL); returns st
 lvbgs_status report_error(lvbgs_status st, const char* msg);
 

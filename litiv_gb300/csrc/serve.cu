@@ -19,6 +19,7 @@
 #include <thread>
 #include <vector>
 
+#include "lvbgs_internal.h"
 #include "../../include/lvbgs.h"
 #include "../../include/lvbgs_synth.h"
 #include "../../include/lvserve.h"
@@ -491,6 +492,7 @@ void pawcs_lane(lvserve_ctx* s) {
                 } else {
                     lvbgs_handle h = nullptr;
                     lvbgs_status rc = lvbgs_create(job->algo, &job->prm, &h);
+                    if (rc == LVBGS_OK) lvbgs::pw_set_unchained(h, true);
                     if (rc == LVBGS_OK)
                         rc = lvbgs_initialize(h, job->init.data(), job->W, job->H, job->C, 0,
                                               job->roi.empty() ? nullptr : job->roi.data());
