@@ -25,10 +25,10 @@ sys.path.insert(0, ROOT)
 METRIC = "SuBSENSE Mpix/s: batched 64-stream vs plain 1-stream on GB300; p99 frame ms"
 # DRAM bytes (read + write) of the evaluation per pixel (lvbgs_k_eval + lvbgs_k_longscan), from an
 # ncu capture of dram__bytes_read.sum + dram__bytes_write.sum on six streams of the mix (indices
-# 52-57: four 1280x720, one of them gray, and two 1920x1080; 7,833,600 px): eval 878,392,064 +
-# 393,505,536 bytes, long scans 435,291,392 + 44,822,016 bytes. roofline.traffic scales it to a tick
+# 52-57: four 1280x720, one of them gray, and two 1920x1080; 7,833,600 px): eval 920,057,088 +
+# 417,870,336 bytes, long scans 369,738,496 + 55,198,720 bytes. roofline.traffic scales it to a tick
 # by pixels.
-EVAL_DRAM_BYTES_PER_PX = (878392064 + 393505536 + 435291392 + 44822016) / 7833600
+EVAL_DRAM_BYTES_PER_PX = (920057088 + 417870336 + 369738496 + 55198720) / 7833600
 WORKLOAD = ("subsense-mix64: 16x320x240 + 24x640x480 + 16x1280x720 + 8x1920x1080, 48 BGR + 16 gray, "
             "default parameters, synthetic seeded scenes")
 # CPU sample: 4 streams of each resolution class
