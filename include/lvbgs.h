@@ -279,7 +279,7 @@ lvbgs_status lvbgs_debug_inject_fault(lvbgs_handle h, int kind);
 /* Host time (ms) of the last PAWCS frame step's parts (inspection; no reference counterpart):
  * [0] enqueueing the fixed-point rounds and the rest of the frame behind them, [1] the waits for them,
  * [2] enqueueing what follows a camera-motion decision or an automatic model reset, [3] the waits for that,
- * [4] the status. */
+ * [4] the copy of a mask that the kernels do not write themselves, and the status. */
 lvbgs_status lvbgs_debug_pawcs_host_timing(lvbgs_handle h, double* out_ms);
 
 /* ---- PAWCS (BackgroundSubtractorPAWCS, modules/video/src/BackgroundSubtractorPAWCS.cpp) ----

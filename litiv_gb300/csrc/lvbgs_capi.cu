@@ -1049,13 +1049,11 @@ lvbgs_status pw_enqueue_tail_a(lvbgs_ctx* h, bool motion) {
     return LVBGS_OK;
 }
 
-// the end of the frame: its close (which a pending automatic reset holds back) and the mask download
+// the end of the frame: its close (which a pending automatic reset holds back)
 lvbgs_status pw_enqueue_close(lvbgs_ctx* h, int resetDone) {
     PwStep& w = h->pws;
     pw_launch(h, pw_k_close, dim3(1), dim3(32), w.st, w.P, resetDone);
     LV_CUDA(h, cudaGetLastError(), "PAWCS frame step launch");
-    if (w.mask && !w.devMask)
-        LV_CUDA(h, cudaMemcpyAsync(w.mask, h->d_mask, h->npx, cudaMemcpyDeviceToHost, w.st), "mask download");
     return LVBGS_OK;
 }
 
@@ -1155,8 +1153,15 @@ lvbgs_status pw_advance(lvbgs_ctx* h, bool& done) {
         h->pw_host_ms[2] += pw_ms_since(t0);
         return s == LVBGS_OK ? s : finish(s);
     }
-    // the frame step is over
+    // The frame step is over. A mask that the kernels cannot write themselves is copied now: enqueued with the frame,
+    // a copy to pageable memory would hold the host until the device is done (so that a batch's steps ran one after
+    // the other), and a frame that fails would leave the mask of the one before.
     h->pw_frames += 1;
+    if (w.mask && !w.devMask) {
+        e = cudaMemcpyAsync(w.mask, h->d_mask, h->npx, cudaMemcpyDeviceToHost, w.st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(w.st);
+        if (e != cudaSuccess) return finish(cuda_fail(h, e, "mask download"));
+    }
     h->pw_host_ms[4] += pw_ms_since(t0);
     return finish(status_from_flags(h, hf[PWF_STATUS]));
 }
