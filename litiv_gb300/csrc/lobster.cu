@@ -1166,8 +1166,9 @@ __global__ void pbas_k_mean1_end(LobDev D) {
 //   pbas_k_sum_walk: from s = 0, one warp over the windows, as many at once as have transfers for the binade of
 //     s and keep s in it; where s crosses into the next binade (or the prediction was off), the same over that
 //     window's chunks, over that chunk's granules, and value by value over that granule.
-// 1920x1080 BGR: 8 + 46 + 3 + 59 us, the first beside the repairs, the others beside the commit, the median and the next
-// gradient; one handle's frames took 395 us back to back with the sums in line and 298 us now.
+// 1920x1080 BGR: 8 + 46 + 3 + 59 us, the first beside the repairs, the others beside the commit, the median and the
+// mask's copy. A frame is over when both streams are: one handle's frames take 289 us back to back (253 us when a frame's
+// mean was left to run beside the next frame's upload and gradient, after the call had returned).
 // The result is the sequential sum bit for bit. An increment of 2^24 ulps leaves the binade whatever the start,
 // so transfers saturate at 2^25 and fit 32 bits.
 constexpr int kSumChunk = 256, kSumNB = 3, kSumEMin = 10, kSumScan = 1024;
@@ -1647,11 +1648,10 @@ inline int blocks_for(size_t n) { return (int)((n + kThreadsL - 1) / kThreadsL);
 
 void lob_release(LobState& L) {
     if (L.meanDone) cudaEventSynchronize(L.meanDone);
-    if (L.done) cudaEventDestroy(L.done);
     if (L.repaired) cudaEventDestroy(L.repaired);
     if (L.meanStream) cudaStreamDestroy(L.meanStream);
     if (L.meanDone) cudaEventDestroy(L.meanDone);
-    L.done = L.meanDone = L.repaired = nullptr;
+    L.meanDone = L.repaired = nullptr;
     L.meanStream = nullptr;
     cudaFree(L.mem);
     L.mem = nullptr;
@@ -1693,7 +1693,6 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
                  oSumTr = take(pb * (C == 3 ? SumWork::bytes((npx + kSumChunk - 1) / kSumChunk) : 0));
     LOB_CUDA(cudaMalloc(&L.mem, off), "model allocation");
     if (!L.h_flags) LOB_CUDA(cudaHostAlloc((void**)&L.h_flags, LOB_F_WORDS * 4, cudaHostAllocMapped), "pinned allocation");
-    if (!L.done) LOB_CUDA(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming), "event creation");
     if (!L.meanDone) LOB_CUDA(cudaEventCreateWithFlags(&L.meanDone, cudaEventDisableTiming), "event creation");
     if (pbas && !L.meanStream) {
         LOB_CUDA(cudaEventCreateWithFlags(&L.repaired, cudaEventDisableTiming), "event creation");
@@ -1786,7 +1785,7 @@ void launch(const LobDev& D, int blocks, cudaStream_t st, A... args) {
 template <int C, int ALG>
 struct Eval {
     static void run(int b, cudaStream_t st, const LobDev& D) {
-        if (ALG == ALG_PBAS) lob_k_eval<C, ALG><<<b, kThreadsL, 0, st>>>(D);  // after another stream's event
+        if (ALG == ALG_PBAS) lob_k_eval<C, ALG><<<b, kThreadsL, 0, st>>>(D);
         else launch_chained(lob_k_eval<C, ALG>, dim3(b), dim3(kThreadsL), st, D);
     }
 };
@@ -1906,12 +1905,9 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
     const int roundBlocks = 2 * (sms > 0 ? sms : 1);
     std::memset(L.h_flags, 0, LOB_F_WORDS * 4);  // the commit writes the frame step's flags here
     // PBAS's frame-level mean gradient distance is only needed by the next evaluation: it runs on a stream of its
-    // own, beside the commit, the median, the mask's copy and the next gradient (its last kernel is one warp's
-    // serial walk). Only the evaluation and the repairs write what it reads.
-    if (D.alg == ALG_PBAS) {
-        pbas_gradient(D, dimg, st);
-        LOB_CUDA(cudaStreamWaitEvent(st, L.meanDone, 0), "event wait");
-    }
+    // own, beside the commit, the median and the mask's copy (its last kernel is one warp's serial walk). The host
+    // waits for both streams. Only the evaluation and the repairs write what the mean reads.
+    if (D.alg == ALG_PBAS) pbas_gradient(D, dimg, st);
     launch<Eval>(D, nb, st);
     if (D.alg == ALG_PBAS && C == 3) {
         LOB_CUDA(cudaEventRecord(L.repaired, st), "event record");
@@ -1939,12 +1935,8 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
         else if (D.alg == ALG_PBAS) launch_chained(lob_k_median<false>, mg, dim3(kThreadsL), st, D);
         LOB_CUDA(cudaGetLastError(), "repair launch");
         if (hostMask) LOB_CUDA(cudaMemcpyAsync(hostMask, dmask, (size_t)D.npx, cudaMemcpyDeviceToHost, st), "mask download");
-        if (D.alg == ALG_PBAS) {  // the host does not wait for the mean
-            LOB_CUDA(cudaEventRecord(L.done, st), "event record");
-            LOB_CUDA(cudaEventSynchronize(L.done), "frame step");
-        } else {
-            LOB_CUDA(cudaStreamSynchronize(st), "frame step");
-        }
+        LOB_CUDA(cudaStreamSynchronize(st), "frame step");
+        if (D.alg == ALG_PBAS) LOB_CUDA(cudaEventSynchronize(L.meanDone), "frame step");
         const volatile unsigned int* hf = L.h_flags;
         if (hf[LOB_F_ERR]) {
             err = "LOBSTER repair list overflow";
@@ -1956,7 +1948,6 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
             return LVBGS_DEVICE_ERROR;
         }
         chunk = std::max(1, chunk * 2);
-        if (D.alg == ALG_PBAS) LOB_CUDA(cudaStreamWaitEvent(st, L.meanDone, 0), "event wait");  // the flags are still read
     }
     L.lastRounds = (int)L.h_flags[LOB_F_ROUNDS];
     D.stampBase += (uint32_t)round + 2u;
@@ -1966,7 +1957,6 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
 
 lvbgs_status lob_background(LobState& L, void* hostOut, bool descriptors, cudaStream_t st, std::string& err) {
     LobDev& D = L.d;
-    LOB_CUDA(cudaEventSynchronize(L.meanDone), "frame step");  // the last frame step may run on another stream
     const size_t n = (size_t)D.npx * D.C * (descriptors ? 2 : 1);
     void* tmp = nullptr;
     LOB_CUDA(staging(&tmp, n, st), "staging allocation");
@@ -2008,7 +1998,6 @@ size_t lob_map_bytes(const LobState& L, int which) {
 
 lvbgs_status lob_get_map(LobState& L, int which, void* hostOut, size_t bytes, cudaStream_t st, std::string& err) {
     LobDev& D = L.d;
-    LOB_CUDA(cudaEventSynchronize(L.meanDone), "frame step");
     const size_t need = lob_map_bytes(L, which);
     if (need == 0) {
         err = "map not kept by LOBSTER";
@@ -2058,7 +2047,6 @@ lvbgs_status lob_get_map(LobState& L, int which, void* hostOut, size_t bytes, cu
 }
 
 lvbgs_status lob_stats(LobState& L, unsigned long long out[2], cudaStream_t st, std::string& err) {
-    LOB_CUDA(cudaEventSynchronize(L.meanDone), "frame step");
     LOB_CUDA(cudaMemcpyAsync(out, L.d.stats, 16, cudaMemcpyDeviceToHost, st), "statistics download");
     LOB_CUDA(cudaStreamSynchronize(st), "statistics download");
     return LVBGS_OK;

@@ -72,7 +72,6 @@ struct LobState {
     uint8_t* d_frame = nullptr;  // staging of host frames
     uint8_t* d_mask = nullptr;   // mask of the last frame step
     unsigned int* h_flags = nullptr;  // page-locked copy of the flags (LobDev::hflags)
-    cudaEvent_t done = nullptr;       // PBAS: the frame step's mask and flags are on the host
     cudaEvent_t repaired = nullptr;  // PBAS: the evaluation, then the repairs of the frame step, for the mean's stream
     cudaStream_t meanStream = nullptr;  // PBAS: the mean's stream
     cudaEvent_t meanDone = nullptr;   // PBAS: the frame step's mean gradient distance is written
