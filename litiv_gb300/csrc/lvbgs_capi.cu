@@ -246,6 +246,14 @@ bool is_device_ptr(const void* p) {
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
+bool in_place(const void* p, int device, size_t align) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return usable_in_place(a, device, p, align);
+}
 // a mask destination the kernels can write themselves: device or managed memory, or page-locked host
 // memory registered with CUDA and mapped at the same address (unified addressing), which the
 // post-processing kernel then writes over the host link while it runs, with no copy after the frame
@@ -2101,30 +2109,34 @@ lvbgs_status lvbgs_lbsp_compute2(const uint8_t* img, int W, int H, int C, long a
     if (C != 1 && C != 3) return fail(nullptr, LVBGS_BAD_TYPE, "input image must be of type 8UC1/8UC3");
     if (absThr < 0 && !(rel >= 0)) return fail(nullptr, LVBGS_BAD_ARG, "relative LBSP threshold must be non-negative");
     if (cudaSetDevice(device_id) != cudaSuccess) return fail(nullptr, LVBGS_DEVICE_ERROR, "cannot select the CUDA device");
-    // Device buffers are used in place. Host buffers are staged; the 2-pixel border of a host result keeps the
-    // caller's content, which is saved and put back on the host (the whole result was uploaded for it before).
+    // Buffers of this device are used in place, unless the descriptors' address is odd or the image lies in the
+    // memory of the descriptors. All others are staged. The 2-pixel border of the result keeps the caller's content: a
+    // host result's is saved and put back on the host, one in another device's memory is copied in with the rest.
     const size_t n = (size_t)W * H * C, row = (size_t)W * C;
-    const bool devImg = is_device_ptr(img), devDesc = is_device_ptr(desc);
-    const size_t needImg = devImg ? 0 : align256(n), needDesc = devDesc ? 0 : align256(n * 2);
+    const bool inDesc = in_place(desc, device_id, alignof(uint16_t)), hostDesc = !is_device_ptr(desc);
+    const bool inImg = in_place(img, device_id, 1) && !(inDesc && ranges_overlap(img, n, desc, n * 2));
+    const size_t needImg = inImg ? 0 : align256(n), needDesc = inDesc ? 0 : align256(n * 2);
     uint8_t* tmp = nullptr;
     if (needImg + needDesc)
         LV_CUDA(nullptr, staging_alloc(device_id, (void**)&tmp, needImg + needDesc, nullptr), "allocation");
-    const uint8_t* di = devImg ? img : tmp;
-    uint16_t* dd = devDesc ? desc : (uint16_t*)(tmp + needImg);
+    const uint8_t* di = inImg ? img : tmp;
+    uint16_t* dd = inDesc ? desc : (uint16_t*)(tmp + needImg);
     cudaError_t e = cudaSuccess;
-    if (!devImg) e = cudaMemcpyAsync(tmp, img, n, cudaMemcpyHostToDevice, nullptr);
+    if (!inImg) e = cudaMemcpyAsync(tmp, img, n, cudaMemcpyDefault, nullptr);
+    if (e == cudaSuccess && !inDesc && !hostDesc) e = cudaMemcpyAsync(dd, desc, n * 2, cudaMemcpyDefault, nullptr);
     const int edge = std::min(kBorder, H);  // full border rows at the top and at the bottom
-    const int side = std::min(kBorder * C, (int)row);
-    std::vector<uint16_t> keep;
-    if (!devDesc) {
-        keep.reserve(2 * edge * row + 2 * (size_t)side * H);
+    const size_t rowB = row * 2, sideB = std::min(2 * (size_t)kBorder * C, rowB);  // in bytes: the address may be odd
+    uint8_t* const out = (uint8_t*)desc;
+    std::vector<uint8_t> keep;
+    if (hostDesc) {
+        keep.reserve(2 * edge * rowB + 2 * sideB * H);
         for (int y = 0; y < H; ++y) {
-            const uint16_t* r = desc + (size_t)y * row;
+            const uint8_t* r = out + (size_t)y * rowB;
             if (y < edge || y >= H - edge) {
-                keep.insert(keep.end(), r, r + row);
+                keep.insert(keep.end(), r, r + rowB);
             } else {
-                keep.insert(keep.end(), r, r + side);
-                keep.insert(keep.end(), r + row - side, r + row);
+                keep.insert(keep.end(), r, r + sideB);
+                keep.insert(keep.end(), r + rowB - sideB, r + rowB);
             }
         }
     }
@@ -2134,20 +2146,20 @@ lvbgs_status lvbgs_lbsp_compute2(const uint8_t* img, int W, int H, int C, long a
         lvbgs_lbsp_dense<<<(unsigned)std::min<size_t>(blocks, 1u << 20), 256>>>(di, W, H, C, thr, rel, (unsigned)off, dd);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess && !devDesc) e = cudaMemcpyAsync(desc, dd, n * 2, cudaMemcpyDeviceToHost, nullptr);
+    if (e == cudaSuccess && !inDesc) e = cudaMemcpyAsync(desc, dd, n * 2, cudaMemcpyDefault, nullptr);
     if (tmp) cudaFreeAsync(tmp, nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    const uint16_t* k = keep.data();
-    if (!devDesc)
+    const uint8_t* k = keep.data();
+    if (hostDesc)
         for (int y = 0; y < H; ++y) {
-            uint16_t* r = desc + (size_t)y * row;
+            uint8_t* r = out + (size_t)y * rowB;
             if (y < edge || y >= H - edge) {
-                std::memcpy(r, k, row * 2);
-                k += row;
+                std::memcpy(r, k, rowB);
+                k += rowB;
             } else {
-                std::memcpy(r, k, (size_t)side * 2);
-                std::memcpy(r + row - side, k + side, (size_t)side * 2);
-                k += 2 * side;
+                std::memcpy(r, k, sideB);
+                std::memcpy(r + rowB - sideB, k + sideB, sideB);
+                k += 2 * sideB;
             }
         }
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "LBSP extraction");
