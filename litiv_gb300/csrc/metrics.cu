@@ -12,12 +12,11 @@
 
 #include <algorithm>
 #include <cmath>
-#include <condition_variable>
 #include <mutex>
-#include <vector>
 
 #include "../../include/lvbgs.h"
 #include "lvbgs_internal.h"
+#include "slots.h"
 #include "staging.h"
 
 namespace lvbgs {
@@ -117,36 +116,20 @@ bool on_device(const void* p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// The places of the calls in flight: an index into g_classif and a page-locked result of 64 bytes. A call takes
-// one and gives it back; more calls at once than places wait for one another.
+// The places of the calls in flight: an index into g_classif and a page-locked result of 64 bytes.
 struct ClassifSlots {
     std::mutex mu;
-    std::condition_variable cv;
-    std::vector<int> free_;
+    lvbgs::SlotPool pool{lvbgs::kClassifSlots};
     unsigned long long* host = nullptr;  // kClassifSlots * 8 words, page-locked, allocated once
-    cudaError_t take(int* slot) {
-        std::unique_lock<std::mutex> lk(mu);
-        if (!host) {
-            const cudaError_t e = cudaHostAlloc((void**)&host, lvbgs::kClassifSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped);
-            if (e != cudaSuccess) {
-                host = nullptr;
-                return e;
-            }
-            for (int i = lvbgs::kClassifSlots - 1; i >= 0; --i) free_.push_back(i);
-        }
-        cv.wait(lk, [&] { return !free_.empty(); });
-        *slot = free_.back();
-        free_.pop_back();
-        return cudaSuccess;
-    }
-    void give(int slot) {
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            free_.push_back(slot);
-        }
-        cv.notify_one();
+    cudaError_t ready() {
+        std::lock_guard<std::mutex> lk(mu);
+        if (host) return cudaSuccess;
+        const cudaError_t e = cudaHostAlloc((void**)&host, lvbgs::kClassifSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped);
+        if (e != cudaSuccess) host = nullptr;
+        return e;
     }
 };
+constexpr unsigned long long kNoCounts = ~0ull;  // in a result that the kernel has not written
 ClassifSlots& classif_slots() {
     static ClassifSlots s;
     return s;
@@ -171,6 +154,11 @@ extern "C" lvbgs_status lvbgs_classif_accumulate(const uint8_t* fgmask, const ui
         return report_error(LVBGS_DEVICE_ERROR, "cannot select the CUDA device");
     }
     cudaStream_t st = (cudaStream_t)cuda_stream;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return report_error(LVBGS_DEVICE_ERROR, "classification waits for its result and cannot be captured");
+    }
     // device inputs are read in place, host inputs copied to a stream-ordered staging buffer
     const uint8_t* src[3] = {fgmask, gt, roi};
     const uint8_t* dptr[3] = {nullptr, nullptr, nullptr};
@@ -193,22 +181,31 @@ extern "C" lvbgs_status lvbgs_classif_accumulate(const uint8_t* fgmask, const ui
         off += padded;
     }
     unsigned long long h[6] = {0, 0, 0, 0, 0, 0};
+    if (e == cudaSuccess) e = classif_slots().ready();
     if (e == cudaSuccess) {
-        int slot = -1, sms = 0;
-        e = classif_slots().take(&slot);
-        if (e == cudaSuccess) {
-            volatile unsigned long long* out = classif_slots().host + 8 * slot;
+        lvbgs::SlotLease place(classif_slots().pool);
+        if (place.slot() >= 0) {
+            volatile unsigned long long* out = classif_slots().host + 8 * place.slot();
+            out[0] = kNoCounts;
+            int sms = 0;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_id);
             const int vec = (((uintptr_t)dptr[0] | (uintptr_t)dptr[1] | (uintptr_t)dptr[2]) & 15) == 0;
             const int blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(sms, 1) * 8, (n + 4095) / 4096));
-            lvbgs::lvbgs_k_classif<<<blocks, 256, 0, st>>>(dptr[0], dptr[1], dptr[2], n, vec, slot, (unsigned long long*)out);
+            lvbgs::lvbgs_k_classif<<<blocks, 256, 0, st>>>(dptr[0], dptr[1], dptr[2], n, vec, place.slot(), (unsigned long long*)out);
             e = cudaGetLastError();
             if (tmp) cudaFreeAsync(tmp, st);
             tmp = nullptr;
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            // waited for also after an error, which may be an older one: the kernel may be running. The place is given
+            // back when the kernel has run to its end or was refused.
+            const cudaError_t waited = cudaStreamSynchronize(st);
+            const bool written = waited == cudaSuccess && out[0] != kNoCounts;
+            if (written || (waited == cudaSuccess && e != cudaSuccess)) place.done();
+            if (e == cudaSuccess) e = waited;
+            if (e == cudaSuccess && !written) e = cudaErrorUnknown;
             if (e == cudaSuccess)
                 for (int i = 0; i < 6; ++i) h[i] = out[i];
-            classif_slots().give(slot);
+        } else {
+            e = cudaErrorUnknown;
         }
     }
     if (tmp) cudaFreeAsync(tmp, st);
