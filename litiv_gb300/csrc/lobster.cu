@@ -800,7 +800,8 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
             // PBAS: every write into pixel p holds p's own colour and gradient
             const int q = ALG == ALG_PBAS ? p : p + (k / 3 - 1) * D.W + k % 3 - 1;
             const uint32_t c2 = ALG == ALG_LOBSTER ? __ldg(D.frame + (size_t)q * C + (C == 3 ? 2 : 0)) : 0u;
-            store_sample<C, ALG>(D, s, p, __ldg(D.wD + q), c2);
+            // (an ordinary load: the evaluation, which writes the words, may still run when this kernel's blocks arrive)
+            store_sample<C, ALG>(D, s, p, D.wD[q], c2);
         };
         const int nlist = nwr <= 5 ? nwr : 0;
         const int iters = (int)__reduce_max_sync(__activemask(), (unsigned)nlist);
@@ -1784,10 +1785,9 @@ void launch(const LobDev& D, int blocks, cudaStream_t st, A... args) {
 }
 template <int C, int ALG>
 struct Eval {
-    static void run(int b, cudaStream_t st, const LobDev& D) {
-        if (ALG == ALG_PBAS) lob_k_eval<C, ALG><<<b, kThreadsL, 0, st>>>(D);
-        else launch_chained(lob_k_eval<C, ALG>, dim3(b), dim3(kThreadsL), st, D);
-    }
+    // Not chained: what comes before may be a kernel of the caller's that writes the frame and lets dependents start
+    // early, and the read-only loads (ld.global.nc) of a kernel want memory that nothing writes while it is there.
+    static void run(int b, cudaStream_t st, const LobDev& D) { lob_k_eval<C, ALG><<<b, kThreadsL, 0, st>>>(D); }
 };
 template <int C, int ALG>
 struct First {
