@@ -2050,7 +2050,7 @@ size_t lvbgs_device_bytes(lvbgs_algo algo, int W, int H, int C, size_t N) {
     // four repair lists of one entry per pixel)
     const size_t npx = (size_t)W * H;
     return make_layout(W, H, C, N ? N : 50).total + sizeof(TickWork) + 8 * sizeof(StreamDev) +
-           9 * sizeof(unsigned long long) + 4 * sizeof(unsigned long long) * npx;
+           4 * sizeof(unsigned long long) * npx;
 }
 
 lvbgs_status lvbgs_spill(lvbgs_handle h, void* host, size_t bytes) {
