@@ -91,6 +91,8 @@ __device__ __forceinline__ unsigned long long mod64(uint32_t a, unsigned long lo
     return a % m32;
 }
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : v > hi ? hi : v; }
+// tiles of n pixels along a side. Tiles are numbered row by row in a grid of one dimension: the second one ends at 65,535
+LV_HD constexpr int tiles_across(int side, int n) { return (side + n - 1) / n; }
 
 // the 16 LBSP taps of channel c at pixel index p of a dense image, packed four to a word
 template <int C>
@@ -873,7 +875,8 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_median(LobDev D) {
     if (!ld_vol(&D.flags[LOB_F_CONV])) return;
     __shared__ MedSmem sm;
     const int r = D.medianK / 2, t = threadIdx.x, W = D.W;
-    const int x0 = blockIdx.x * 32 * kMedW, y0 = blockIdx.y * kMedH;
+    const int tilesX = tiles_across(W, 32 * kMedW);
+    const int x0 = (int)(blockIdx.x % tilesX) * 32 * kMedW, y0 = (int)(blockIdx.x / tilesX) * kMedH;
     for (int i = t; i < (kMedH + 2 * r) * (kMedW + 2); i += kThreadsL) {
         const int ry = i / (kMedW + 2), x = x0 + 32 * (i % (kMedW + 2) - 1);
         const int row = clampi(y0 - r + ry, 0, D.H - 1) * W;
@@ -914,8 +917,8 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_median(LobDev D) {
         if (KEEP) put(D.lastFG);  // PBAS keeps neither
     }
     if (KEEP) {
-        const size_t bytes = (size_t)D.npx * D.C, g = (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kThreadsL + t;
-        const size_t threads = (size_t)gridDim.x * gridDim.y * kThreadsL;
+        const size_t bytes = (size_t)D.npx * D.C, g = (size_t)blockIdx.x * kThreadsL + t;
+        const size_t threads = (size_t)gridDim.x * kThreadsL;
         // lastColor is aligned; a frame at any address is read as the aligned words that lie wholly inside it
         const uint32_t sh = 8u * (uint32_t)((uintptr_t)D.frame & 3);
         const uint32_t* src = (const uint32_t*)((uintptr_t)D.frame & ~(uintptr_t)3);
@@ -1022,7 +1025,8 @@ template <int C>
 __global__ void __launch_bounds__(kThreadsL) pbas_k_grad(LobDev D, const uint8_t* img) {
     using T = GradTile<C>;
     __shared__ T sm;
-    const int x0 = blockIdx.x * kGradW, y0 = blockIdx.y * kGradH, t = threadIdx.x;
+    const int tilesX = tiles_across(D.W, kGradW), t = threadIdx.x;
+    const int x0 = (int)(blockIdx.x % tilesX) * kGradW, y0 = (int)(blockIdx.x / tilesX) * kGradH;
     // frame bytes of rows y0 - 2 .. y0 + 17, pixels x0 - 2 .. x0 + 65, from byte kPad - 2 C of a row on
     constexpr int kBytes = (kGradW + 4) * C;
     // inside the frame's width a tile row is kRow aligned words from byte x0 C - kPad on (x0 C is a multiple of 64)
@@ -1807,7 +1811,7 @@ struct Commit {
 
 // PBAS's gradient image of a device frame into D.grad
 void pbas_gradient(const LobDev& D, const uint8_t* img, cudaStream_t st) {
-    const dim3 g((D.W + kGradW - 1) / kGradW, (D.H + kGradH - 1) / kGradH);
+    const dim3 g((unsigned)tiles_across(D.W, kGradW) * tiles_across(D.H, kGradH));
     if (D.C == 3) pbas_k_grad<3><<<g, kThreadsL, 0, st>>>(D, img);
     else pbas_k_grad<1><<<g, kThreadsL, 0, st>>>(D, img);
 }
@@ -1930,7 +1934,7 @@ lvbgs_status lob_apply(LobState& L, const uint8_t* dimg, uint8_t* dmask, uint8_t
         launch<Commit>(D, nb, st);
         // LOBSTER's median blur, last mask and last colour frame; PBAS's median blur (ViBe outputs its
         // raw mask)
-        const dim3 mg((D.W + 32 * kMedW - 1) / (32 * kMedW), (D.H + kMedH - 1) / kMedH);
+        const dim3 mg((unsigned)tiles_across(D.W, 32 * kMedW) * tiles_across(D.H, kMedH));
         if (D.alg == ALG_LOBSTER) launch_chained(lob_k_median<true>, mg, dim3(kThreadsL), st, D);
         else if (D.alg == ALG_PBAS) launch_chained(lob_k_median<false>, mg, dim3(kThreadsL), st, D);
         LOB_CUDA(cudaGetLastError(), "repair launch");
