@@ -798,20 +798,35 @@ __global__ void __launch_bounds__(kThreadsL) lob_k_commit(LobDev D) {
                 ++nwr;
             }
         }
-        auto write = [&](int k, int s) {
+        struct Write {
+            unsigned long long d;
+            uint32_t c2;
+            int s;
+        };
+        auto read = [&](int k, int s) -> Write {
             // PBAS: every write into pixel p holds p's own colour and gradient
             const int q = ALG == ALG_PBAS ? p : p + (k / 3 - 1) * D.W + k % 3 - 1;
             const uint32_t c2 = ALG == ALG_LOBSTER ? __ldg(D.frame + (size_t)q * C + (C == 3 ? 2 : 0)) : 0u;
             // (an ordinary load: the evaluation, which writes the words, may still run when this kernel's blocks arrive)
-            store_sample<C, ALG>(D, s, p, D.wD[q], c2);
+            return {D.wD[q], c2, s};
         };
+        auto entry = [&](int j) {
+            const uint32_t e = (uint32_t)(list >> (12 * j)) & 0xfffu;
+            return read((int)((e >> 6) & 15u), (int)(e & 63u));
+        };
+        // the next write's word is requested before this one is stored (an ordinary load does not pass a store)
         const int nlist = nwr <= 5 ? nwr : 0;
         const int iters = (int)__reduce_max_sync(__activemask(), (unsigned)nlist);
-        for (int j = 0; j < iters; ++j)
-            if (j < nlist) {
-                const uint32_t e = (uint32_t)(list >> (12 * j)) & 0xfffu;
-                write((int)((e >> 6) & 15u), (int)(e & 63u));
-            }
+        Write next = nlist > 0 ? entry(0) : Write{0ull, 0u, 0};
+        for (int j = 0; j < iters; ++j) {
+            const Write w = next;
+            if (j + 1 < nlist) next = entry(j + 1);
+            if (j < nlist) store_sample<C, ALG>(D, w.s, p, w.d, w.c2);
+        }
+        auto write = [&](int k, int s) {
+            const Write w = read(k, s);
+            store_sample<C, ALG>(D, w.s, p, w.d, w.c2);
+        };
         if (nwr > 5) {
 #pragma unroll 1
             for (int k = 0; k < 9; ++k) {
