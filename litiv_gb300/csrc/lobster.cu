@@ -671,8 +671,9 @@ __device__ __forceinline__ void round_end(const LobDev& D, int round) {
 // went through a list in memory. A block lasts as long as its slowest re-evaluation, so it takes 1,024 pixels:
 // with 256, LOBSTER 1277x719 BGR took 36 us and PBAS 1920x1080 BGR 67 us. A chain of latencies: more blocks at
 // once are worth some spilled registers (3 / 5 / 6 / 8 blocks per SM: LOBSTER 19.6 / 17.8 / 14.6 / 15.4 us, PBAS
-// 34 / 30 / 28 / 24 us). A frame of which four pixels a thread would make fewer than two blocks an SM takes one a
-// thread: 320x240 BGR ViBe 8.6 -> 7.7 us, 45 -> 40 us a frame.
+// 34 / 30 / 28 / 24 us). A frame of which four pixels a thread would make fewer than two blocks on each of this
+// chip's 152 SMs takes one a thread: 320x240 BGR ViBe 8.6 -> 7.7 us, 45 -> 40 us a frame (the one size measured in both forms;
+// on a chip with another count the line would lie elsewhere).
 constexpr int kFirstSmall = 304 * 1024;
 template <int C, int ALG, int PER>
 __global__ void __launch_bounds__(kThreadsL, ALG == ALG_PBAS ? 8 : 6) lob_k_first(LobDev D) {
@@ -1691,8 +1692,8 @@ lvbgs_status lob_setup(LobState& L, int alg, const lvbgs_params& prm, int W, int
     cudaFree(L.mem);
     L.mem = nullptr;
     const size_t npx = (size_t)W * H, N = prm.bg_samples;
-    // ViBe keeps only colour samples ([N][npx*C] bytes); PBAS colour and gradient samples and its maps;
-    // LOBSTER the packed descriptor plane and a colour byte
+    // ViBe keeps only colour samples, PBAS colour and gradient samples and its maps (words in two planes,
+    // load_sample), LOBSTER the packed descriptor plane and a colour byte
     const bool vibe = alg != ALG_LOBSTER, pbas = alg == ALG_PBAS;
     const size_t lob = vibe ? 0 : 1, pb = pbas ? 1 : 0;
     size_t off = 0;

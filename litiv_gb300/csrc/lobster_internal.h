@@ -5,10 +5,11 @@
 //
 // Device layout (one allocation per stream, each array 256-byte aligned):
 //   roi[npx], lastColor[npx*C], lastFG[npx], lastDesc[npx*C] (u16), kctr[npx] (u16, draws of the last
-//   frame), samples sD[N][npx] / sC[N][npx] (the SuBSENSE packing: for C=3 one u64 = desc0 | desc1<<16 |
+//   frame), samples sD[N][npx] / sC[N][npx] (for C=3 one u64 = desc0 | desc1<<16 |
 //   desc2<<32 | B<<48 | G<<56 and the R byte, for C=1 one u16 descriptor and the intensity),
-//   ViBe keeps only its samples, sC[N][npx*C] (the reference's layout: C colour bytes per sample);
-//   PBAS its colour and gradient samples sC / sG[N][npx*C], the R, T and D maps fm[2][3][npx] (by frame
+//   ViBe keeps only its samples, in words: for C=3 sC[N][npx] (u16, colours 0 and 1) and sG[N][npx] (u8, colour 2),
+//   for C=1 sC[N][npx] (u8); PBAS its colour and gradient samples, for C=3 sC[N][npx] (u32, the colours and gradient 0)
+//   and sG[N][npx] (u16, gradients 1 and 2), for C=1 sC[N][npx] (u16), the R, T and D maps fm[2][3][npx] (by frame
 //   parity), the frame's gradient image and the frame-level mean gradient distance;
 //   scratch of a frame step: intent[npx] (u32), wD[npx] (the sample word a pixel writes), rawBits (a bit a pixel),
 //   two repair lists and their dedupe stamps, flags and counters, the staged frame and mask.
@@ -58,7 +59,7 @@ struct LobDev {
     float R0, updateRate;   // m_nDefaultColorDistThreshold, m_fDefaultUpdateRate
     uint8_t *sG, *grad;
     float *fm, *meanGrad;
-    uint16_t* badVals;  // three channels: the bad samples' squared gradient distances, [N][npx]
+    uint16_t* badVals;  // three channels: the bad samples' squared gradient distances, [npx][N]
     uint32_t* badSum;
     uint8_t* badCnt;
     float* chunkAbout;  // three channels: about what each chunk of the mean's sum adds (in sumTr)

@@ -1574,7 +1574,8 @@ constexpr int kMaxBatchGroups = 4;
 constexpr int kSplitMinStreams = 8;
 // Batches from three million pixels on are split. One sequence / groups: 16 x 320x240 BGR (1.2 M) 365 / 403 us; 8 x
 // 640x480 (2.5 M) BGR 504 / 497, one channel 497 / 514; 12 mixed streams (3.5 M) 729 / 704, and from page-locked
-// memory, where one group's uploads overlap another's kernels, 813 / 736.
+// memory, where one group's uploads overlap another's kernels, 813 / 736. (Between 2.5 and 4 M that is the one batch that
+// was measured; at 2.5 M the forms are equal, so the line may as well lie anywhere between.)
 constexpr size_t kSplitMinPx = (size_t)3 << 20;
 
 // Large batches run as G groups of about equal pixels (the largest streams first, each to the lightest

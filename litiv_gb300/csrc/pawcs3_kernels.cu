@@ -161,7 +161,8 @@ __device__ void pw3_item_pixel(const PawcsDev& S, int p, const PwRec& R, uint32_
 // and 61 us by tiles and take 199, 342, 212, 86 and 59 us (a full warp of listed pixels whatever their number:
 // 214, 321, 236, 233, 108). Bound by DRAM's sectors: 860 MB in round 1, half of them for words beside the listed ones.
 // ------------------------------------------------------------------------------------------
-constexpr unsigned kPwLocalWarps = 152u * 3u * 8u;  // resident at once: three blocks on each of 152 SMs
+// resident at once on this chip: three blocks on each of 152 SMs (another count would spread the list otherwise, no more)
+constexpr unsigned kPwLocalWarps = 152u * 3u * 8u;
 template <bool FIRST>
 __device__ __forceinline__ void pw3_local(const PwParams& P) {
     PW_ROUND_GUARD(P);
@@ -833,7 +834,7 @@ extern "C" __global__ void __launch_bounds__(256) pw3_k_later_list(PwParams P) {
     }
     pw_list_append(S.dirty, &P.flags[PWF_NDIRTY], any, q);
 }
-constexpr unsigned kPwLaterWarps = 152u * 4u * 8u;
+constexpr unsigned kPwLaterWarps = 152u * 4u * 8u;  // likewise, four blocks
 extern "C" __global__ void __launch_bounds__(256, 4) pw3_k_later(PwParams P) {
     PW_TAIL_GATE(P);
     const PawcsDev& S = P.streams[0];

@@ -166,7 +166,10 @@ struct PawcsDev {
 // warm-up nearly always reach the true start: short segments keep all SMs busy (scan and walk of a 640x480
 // round: 66 + 46 us at 512 items, 29 + 18 at 128, 19 + 32 at 64 with 64 of warm-up). On one channel
 // replacements are rare, a segment seldom starts in the true state, and more segments are more of a walk
-// (33 + 5 us at 512, 19 + 10 at 256).
+// (33 + 5 us at 512, 19 + 10 at 256). How many segments the walk has to settle is the scene's matter, not the
+// model's age: of ten 640x480 scenes nine take 543 to 585 us a frame at 60 frames of age (563 to 604 with 512 items) and
+// the walk 5 us; in the tenth it settles nearly every segment, 208 us a launch, and the frame takes 1,000 us (870 with 512
+// items). 300 frames of moving blobs: median 692 us, 671 with 512 items.
 LV_HD constexpr int pw_gseg_items(int C) { return C == 3 ? 128 : 256; }
 LV_HD constexpr int pw_gseg_warm(int C) { return C == 3 ? 128 : 64; }
 constexpr int kPwGsegWords = 24;  // scratch words of a segment

@@ -1316,7 +1316,7 @@ extern "C" __global__ void __launch_bounds__(256) pw_k_epilogue(PwParams P, int 
     pc->reset_pending = 0;
     // automatic model reset (:1479-1513): the block is entered when the reset is enabled or the camera
     // moves; the camera-motion comparison of frames 500, 1000, ... (pw_k_motion_*) and the reset decision
-    // (pw_k_reset_decide) follow
+    // (pw_reset_decide) follow
     if (!ctl->auto_reset && ratio >= 45.0f * 2) ctl->auto_reset = 1;
     pc->reset_block = ctl->auto_reset || pc->moving_cam;
     if (decide) pw_reset_decide(S);

@@ -1508,8 +1508,8 @@ __device__ void stream_epilogue(const TickParams& P, const StreamDev& S);
 // a run that touches the ring (it holds x = 0 or x = W-1, or lies in the first or last row) stands for
 // node 0 without any memory access, so on a mostly empty mask few unions remain. The blocks past the rows
 // run the frame-level epilogue of one stream each (it touches nothing that these rows read).
-// Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before, 11 us now;
-// 320x240 4.9 us.
+// Latency-bound: 1920x1080 BGR frame, 46 us (one lane per pixel, after an 18 us label pass) before, 7 to 11 us now;
+// 320x240 4.7 us; a 640x480 BGR PAWCS frame 40 us.
 extern "C" __global__ void __launch_bounds__(256) lvbgs_k_unite(TickParams P) {
     pdl_entry();
     if (P.gate && ld_volatile(P.gate) == 0u) return;
@@ -1929,9 +1929,9 @@ extern "C" __global__ void __launch_bounds__(kThreads, 5) lvbgs_k_eval(TickParam
 
 // ------------------------------------------------------------------------------------------
 // long sample scans: the pixels whose ordered scan did not settle within the first kScanCap samples
-// (foreground pixels scan all N) continue here, one thread per pixel of the compacted list, from the
-// saved scan state; then the rest of their evaluation. Spatially sparse long scans would otherwise
-// keep whole warps of the evaluation waiting on a few lanes.
+// (foreground pixels scan all N) continue here from the saved scan state, over the compacted list: by
+// groups of eight lanes while the list is short, else a pixel a lane (coop_share); then the rest of their
+// evaluation. Spatially sparse long scans would otherwise keep whole warps of the evaluation waiting on a few lanes.
 // ------------------------------------------------------------------------------------------
 template <int C>
 __device__ void longscan_items(const TickParams& P, bool own, int m, unsigned long long key, unsigned long long sw) {
