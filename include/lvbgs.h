@@ -257,8 +257,9 @@ lvbgs_status lvbgs_get_scalars(lvbgs_handle h, lvbgs_scalars* out);
 lvbgs_status lvbgs_debug_set_timing(lvbgs_handle h, int batched, int n_ticks);
 int lvbgs_debug_tick_profile(lvbgs_handle h, int batched, double* out_ms, int max_n);
 /* Phase durations (microseconds) of the repair kernel of the last step launched by h (batched != 0:
- * its last batched step): the device timer at kernel entry and after every grid barrier, as
- * differences: re-match of round 0, re-resolution of round 0, re-match of round 1, ...; then the
+ * its last batched step): the device timer at kernel entry and after each phase of the rounds, as
+ * differences: re-match of round 0, re-resolution of round 0, re-match of round 1, ... (a round without
+ * ghost tests to resolve again has no barrier there and a re-resolution of next to nothing); then the
  * number of re-matched pixels of each round. Waits for the device. Returns the number of values
  * written. */
 int lvbgs_debug_repair_phases(lvbgs_handle h, int batched, double* out_us, int max_n);

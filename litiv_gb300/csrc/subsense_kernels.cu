@@ -2100,6 +2100,8 @@ extern "C" __global__ void __launch_bounds__(kThreads, 2) lvbgs_k_repair(TickPar
                 }
             }
             if (!grid_sync(w, ctas, P.barrierNs, due)) return;
+        } else if (blockIdx.x == 0 && threadIdx.x == 0 && w->nts < 40u) {
+            w->ts[w->nts++] = gtimer();  // the phase profile has two entries a round
         }
         ++iter;
     }
